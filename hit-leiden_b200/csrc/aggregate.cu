@@ -147,40 +147,18 @@ __device__ __forceinline__ void compress_out(u64 j, u64 a, double x, const u64* 
 }
 
 // In-order segmented sum over the records' weights gathered into sorted
-// order (sw); keep |w| > threshold.  Segments of RUN_FOLD_MIN or more terms
-// are listed for k_compress_runs.
-__global__ void k_compress(u32 U, const u32* start, u64 total, const u64* sk, const double* sw,
-                           double threshold, u32* ou, u32* ov, double* ow, u8* keepf, u32* longl,
-                           u32* longn) {
+// order (sw); keep |w| > threshold.
+__global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 total,
+                                                  const u64* sk, const double* sw,
+                                                  double threshold, u32* ou, u32* ov, double* ow,
+                                                  u8* keepf) {
+  __shared__ __align__(16) double chain[8][CHAIN_TILE];
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 j = warp; j < U; j += nwarps) {
-    u64 a = start[j], b = (j + 1 < U) ? start[j + 1] : total;
-    if (b - a >= RUN_FOLD_MIN) {
-      fold_defer(longl, longn, (u32)j);
-      continue;
-    }
-    double x = 0.0;
-    if (b - a == 1) {
-      x = sw[a];
-    } else {
-      x = warp_ordered_sum(a, b, 0.0, [&](u64 t) { return sw[t]; }, [](u64) { return true; });
-    }
-    compress_out(j, a, x, sk, threshold, ou, ov, ow, keepf);
-  }
-}
-
-// The long segments listed by k_compress, folded in runs (the same bits).
-__global__ void k_compress_runs(const u32* longl, const u32* longn, u32 U, const u32* start,
-                                u64 total, const u64* sk, const double* sw, double threshold,
-                                u32* ou, u32* ov, double* ow, u8* keepf) {
-  const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
-  const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  const u32 nl = *longn;
-  for (u64 i = warp; i < nl; i += nwarps) {
-    const u32 j = longl[i];
-    u64 a = start[j], b = (j + 1 < U) ? start[j + 1] : total;
-    double x = warp_fold_runs(a, b, 0.0, sw);
+    const u64 a = start[j], b = (j + 1 < U) ? start[j + 1] : total;
+    const double x =
+        b - a == 1 ? sw[a] : warp_chain_sum(a, b, 0.0, sw, chain[threadIdx.x >> 5]);
     compress_out(j, a, x, sk, threshold, ou, ov, ow, keepf);
   }
 }
@@ -231,13 +209,8 @@ static u64 compress_records(Engine& E, u64 R, double threshold, u32 id_bound) {
   S.op.ensure(E.mem, U);
   S.fvals.ensure(E.mem, R);
   ++E.nlaunch, k_gather_weights<<<grid_for(R), 256, 0, st>>>(vo, S.neww.p, R, S.fvals.p);
-  FoldList fl = fold_list(E, R, U);
   ++E.nlaunch, k_compress<<<grid_for((u64)U * 32), 256, 0, st>>>(
-      U, S.seg_start.p, R, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p, S.op.p, fl.seg,
-      fl.cnt);
-  ++E.nlaunch, k_compress_runs<<<FOLD_BLOCKS, 256, 0, st>>>(
-      fl.seg, fl.cnt, U, S.seg_start.p, R, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p,
-      S.op.p);
+      U, S.seg_start.p, R, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p, S.op.p);
   HL_LAUNCH_CHECK();
   S.eu2.ensure(E.mem, U);
   S.ev2.ensure(E.mem, U);

@@ -1,0 +1,49 @@
+// gang.cu — shapes and launches of the single-launch stage kernels (gang.cuh).
+#include "gang.cuh"
+
+namespace hl {
+
+static u32 sm_count(int device) {
+  static std::atomic<u32> cached[64];
+  if (device >= 0 && device < 64 && cached[device].load()) return cached[device].load();
+  int v = 0;
+  HL_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device));
+  if (device >= 0 && device < 64) cached[device].store((u32)v);
+  return (u32)v;
+}
+
+// One block up to a few thousand entries (its barrier is a block barrier), a
+// portable cluster of 8 up to a few hundred thousand, above that one block
+// per SM.
+GangShape gang_shape(Engine& E, u64 work) {
+  if (work <= 4096) return GangShape{1, false};
+  if (work <= 400000) return GangShape{8, false};
+  const u32 sms = sm_count(E.device);
+  return GangShape{sms < GANG_MAX_BLOCKS ? sms : GANG_MAX_BLOCKS, true};
+}
+
+void gang_launch(Engine& E, const void* kernel, const GangShape& s, size_t smem, void* args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(s.blocks);
+  cfg.blockDim = dim3(GANG_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = E.stream;
+  cudaLaunchAttribute at[1];
+  cfg.attrs = at;
+  if (s.grid) {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.numAttrs = 1;
+  } else if (s.blocks > 1) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = s.blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  }
+  void* params[1] = {args};
+  ++E.nlaunch;
+  HL_CUDA(cudaLaunchKernelExC(&cfg, kernel, params));
+}
+
+}  // namespace hl

@@ -1,0 +1,246 @@
+// gang.cuh — one launch for a whole stage of the update path.
+//
+// A batch on a small or mid-size level is bound by its launches and by the
+// host reads between them, not by memory: a stage is some twenty dependent
+// steps of a few microseconds each.  The gang kernels run all steps of a stage
+// in one launch, with a barrier over all of their blocks between steps and
+// every size kept on the device; the host reads one small result per stage.
+//
+// The blocks of a gang are one block, one thread-block cluster (its hardware
+// barrier costs a fraction of a microsecond, and clusters of different graphs
+// run side by side) or a cooperative grid of one block per SM for the large
+// levels.  All of them execute every barrier: branches around a barrier are
+// taken on values that every block reads alike.
+//
+// Arrays that a kernel writes and reads again after a barrier carry no
+// __restrict__ / const __restrict__ qualifiers (they must not go through the
+// non-coherent cache).
+#pragma once
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "hl_engine.cuh"
+
+namespace hl {
+
+constexpr u32 GANG_THREADS = 512;
+constexpr u32 GANG_WARPS = GANG_THREADS / 32;
+constexpr u32 GANG_MAX_BLOCKS = 148;
+constexpr u32 GSORT_CHUNK = 2048;  // records sorted by one block at a time
+constexpr u32 GSORT_ILP = 8;       // chunks a record's rank is looked up in at once
+
+struct Gang {
+  u32 rank, nct;
+  bool grid;
+  __device__ __forceinline__ u32 thread() const { return rank * GANG_THREADS + threadIdx.x; }
+  __device__ __forceinline__ u32 threads() const { return nct * GANG_THREADS; }
+  // consecutive warps sit on different blocks, so a short list spreads out
+  __device__ __forceinline__ u32 warp() const { return (threadIdx.x >> 5) * nct + rank; }
+  __device__ __forceinline__ u32 warps() const { return nct * GANG_WARPS; }
+  __device__ __forceinline__ void sync() const {
+    if (grid) {
+      cooperative_groups::this_grid().sync();
+    } else {
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    }
+  }
+};
+
+__device__ __forceinline__ Gang gang_make(bool grid) {
+  Gang G;
+  G.rank = blockIdx.x;
+  G.nct = gridDim.x;
+  G.grid = grid;
+  return G;
+}
+
+// Shared memory of the primitives below (one instance per kernel, static or
+// at the start of the dynamic block).
+struct GangSmem {
+  u64 key[GSORT_CHUNK];
+  u32 pos[GSORT_CHUNK];
+  u32 wsum[GANG_WARPS + 1];
+  u32 bcast[2];
+};
+
+// Sum of x over the block's threads, and the sum over the threads before this
+// one (exclusive).  Two block barriers.
+__device__ __forceinline__ u32 block_scan(GangSmem& S, u32 x, u32& total) {
+  const u32 lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  u32 inc = x;
+#pragma unroll
+  for (u32 o = 1; o < 32; o <<= 1) {
+    const u32 y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) S.wsum[wib] = inc;
+  __syncthreads();
+  u32 before = 0, tot = 0;
+#pragma unroll
+  for (u32 i = 0; i < GANG_WARPS; ++i) {
+    const u32 y = S.wsum[i];
+    if (i < wib) before += y;
+    tot += y;
+  }
+  __syncthreads();
+  total = tot;
+  return before + inc - x;
+}
+
+// Exclusive prefix sums of val(0..N-1), handed to out(i, prefix); returns the
+// total.  val is evaluated twice.  One gang barrier inside; the caller places
+// one before it reads what out wrote (which also frees `part`, nct words).
+template <typename V, typename O>
+__device__ __forceinline__ u32 gang_scan(const Gang& G, GangSmem& S, u32 N, V val, O out,
+                                         u32* part) {
+  const u32 per = ((N + G.nct - 1) / G.nct + GANG_THREADS - 1) / GANG_THREADS * GANG_THREADS;
+  const u32 lo = min(N, G.rank * per), hi = min(N, lo + per);
+  u32 base = 0, total = 0;
+  if (G.nct > 1) {
+    u32 sum = 0;
+    for (u32 i = lo + threadIdx.x; i < hi; i += GANG_THREADS) sum += val(i);
+    u32 tot;
+    block_scan(S, sum, tot);
+    if (threadIdx.x == 0) part[G.rank] = tot;
+    G.sync();
+    if (threadIdx.x < 32) {
+      u32 b = 0, t = 0;
+      for (u32 r = threadIdx.x; r < G.nct; r += 32) {
+        const u32 y = part[r];
+        if (r < G.rank) b += y;
+        t += y;
+      }
+      b = __reduce_add_sync(0xffffffffu, b);
+      t = __reduce_add_sync(0xffffffffu, t);
+      if (threadIdx.x == 0) {
+        S.bcast[0] = b;
+        S.bcast[1] = t;
+      }
+    }
+    __syncthreads();
+    base = S.bcast[0];
+    total = S.bcast[1];
+    __syncthreads();
+  }
+  u32 run = base;
+  for (u32 i0 = lo; i0 < hi; i0 += GANG_THREADS) {
+    const u32 i = i0 + threadIdx.x;
+    const u32 x = i < hi ? val(i) : 0u;
+    u32 tot;
+    const u32 ex = block_scan(S, x, tot);
+    if (i < hi) out(i, run + ex);
+    run += tot;
+  }
+  if (G.nct == 1) total = run;
+  return total;
+}
+
+// Stable ascending sort of N (key, value) records.  Blocks sort chunks of up
+// to GSORT_CHUNK records in shared memory (bitonic on (key, position)); after
+// a barrier every record finds its rank by a bisection in each other chunk and
+// is handed to emit(rank, key, value).  `tk`/`tv` take the sorted chunks.  Two
+// gang barriers inside (one when a single block does it all); the caller's
+// emitted output is visible after the last one.
+//
+// For a few thousand records this takes 5-10 us; a radix sort of the same
+// keys is six to nine dependent kernel launches.
+template <typename K, typename VL, typename EM>
+__device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K key_of, VL val_of,
+                                          u64* tk, u32* tv, EM emit) {
+  const u32 tid = threadIdx.x;
+  // few chunks: a record's rank costs one bisection per chunk
+  u32 ch = 64;
+  while (ch < GSORT_CHUNK && ch * min(G.nct, 8u) < N) ch <<= 1;
+  const u32 nch = (N + ch - 1) / ch;
+  for (u32 c = G.rank; c < nch; c += G.nct) {
+    const u32 base = c * ch;
+    const u32 cnt = min(ch, N - base);
+    u32 P = 64;  // the padded length of this chunk
+    while (P < cnt) P <<= 1;
+    for (u32 i = tid; i < P; i += GANG_THREADS) {
+      S.key[i] = i < cnt ? key_of(base + i) : ~0ull;
+      S.pos[i] = i;
+    }
+    __syncthreads();
+    for (u32 size = 2; size <= P; size <<= 1) {
+      for (u32 stride = size >> 1; stride > 0; stride >>= 1) {
+        for (u32 x = tid; x < P / 2; x += GANG_THREADS) {
+          const u32 i = 2 * x - (x & (stride - 1));
+          const u32 j = i + stride;
+          const bool up = (i & size) == 0;
+          const u64 ki = S.key[i], kj = S.key[j];
+          const u32 pi = S.pos[i], pj = S.pos[j];
+          const bool gt = ki > kj || (ki == kj && pi > pj);
+          if (gt == up) {
+            S.key[i] = kj;
+            S.key[j] = ki;
+            S.pos[i] = pj;
+            S.pos[j] = pi;
+          }
+        }
+        // strides up to 32 stay within the 64 elements of one warp
+        if (stride > 32) __syncthreads();
+        else __syncwarp();
+      }
+      if (size >= 64) __syncthreads();
+    }
+    for (u32 i = tid; i < cnt; i += GANG_THREADS) {
+      const u32 v = val_of(base + S.pos[i]);
+      if (nch == 1) {
+        emit(i, S.key[i], v);
+      } else {
+        tk[base + i] = S.key[i];
+        tv[base + i] = v;
+      }
+    }
+    __syncthreads();
+  }
+  G.sync();
+  if (nch == 1) return;
+  for (u32 e = G.thread(); e < N; e += G.threads()) {
+    const u64 k = tk[e];
+    const u32 mine = e / ch;
+    u32 rank = e - mine * ch;
+    // GSORT_ILP bisections side by side; equal keys: earlier chunks come first
+    for (u32 c0 = 0; c0 < nch; c0 += GSORT_ILP) {
+      u32 pos[GSORT_ILP];
+#pragma unroll
+      for (u32 j = 0; j < GSORT_ILP; ++j) pos[j] = 0;
+      for (u32 half = ch; half; half >>= 1) {
+        u64 probe[GSORT_ILP];
+        bool in[GSORT_ILP];
+#pragma unroll
+        for (u32 j = 0; j < GSORT_ILP; ++j) {
+          const u32 c = c0 + j;
+          const u32 at = c * ch + pos[j] + half;  // one past the probed record
+          in[j] = c < nch && c != mine && pos[j] + half <= ch && at <= N;
+          probe[j] = in[j] ? tk[at - 1] : 0ull;
+        }
+#pragma unroll
+        for (u32 j = 0; j < GSORT_ILP; ++j)
+          if (in[j] && (probe[j] < k || (probe[j] == k && c0 + j < mine))) pos[j] += half;
+      }
+#pragma unroll
+      for (u32 j = 0; j < GSORT_ILP; ++j) rank += pos[j];
+    }
+    emit(rank, k, tv[e]);
+  }
+  G.sync();
+}
+
+// ---------------------------------------------------------------------------
+// Host side: the shape of a gang.
+// ---------------------------------------------------------------------------
+struct GangShape {
+  u32 blocks;
+  bool grid;  // cooperative grid instead of a cluster
+};
+
+// Shape for a stage that touches about `work` entries.
+GangShape gang_shape(Engine& E, u64 work);
+// Launch of a gang kernel with one argument struct.
+void gang_launch(Engine& E, const void* kernel, const GangShape& s, size_t smem, void* args);
+
+}  // namespace hl

@@ -7,6 +7,7 @@
 // m edges, only the changed keys are resolved: weight updates are written in
 // place, and inserts/deletes become sorted row-operations that a warp-per-row
 // merge folds into a fresh CSR with rows still sorted by neighbour id.
+#include "csr_rebuild.cuh"
 #include "hl_engine.cuh"
 
 namespace hl {
@@ -203,8 +204,6 @@ __global__ void k_resolve(u32 U, const u32* seg_start, u64 k, const u64* sk, con
   }
 }
 
-constexpr u32 DEL_MARK = 0xFFFFFFFFu;
-
 __global__ void k_emit_rowops(u32 U, const u32* seg_start, const u64* sk, const u8* op,
                               const u32* pos_del, const u32* pos_ins, u64 ins_base, u64* rkeys,
                               u32* rvals) {
@@ -264,494 +263,115 @@ __global__ void k_del_flags(const u32* rvals, u64 R, u32* flag) {
     flag[t] = (t < R && rvals[t] == DEL_MARK) ? 1u : 0u;
 }
 
-__global__ void k_rowop_deg(const u64* rkeys, const u32* rvals, u64 R, int* ddeg, u8* touched) {
-  for (u64 t = blockIdx.x * (u64)blockDim.x + threadIdx.x; t < R; t += (u64)gridDim.x * blockDim.x) {
-    u32 r = (u32)(rkeys[t] >> 32);
-    atomicAdd(&ddeg[r], rvals[t] == DEL_MARK ? -1 : 1);
-    touched[r] = 1;
-  }
+__global__ void k_rowop_positions(const u64* rkeys, const u32* rvals, u64 R, const u64* off,
+                                  const u32* col, u64* opos) {
+  for (u64 t = blockIdx.x * (u64)blockDim.x + threadIdx.x; t < R; t += (u64)gridDim.x * blockDim.x)
+    opos[t] = rowop_position((u32)t, rkeys, rvals, off, col);
 }
 
-__global__ void k_new_degrees(u32 n, const u64* off, const int* ddeg, u64* nd) {
-  for (u64 v = blockIdx.x * (u64)blockDim.x + threadIdx.x; v <= n; v += (u64)gridDim.x * blockDim.x)
-    nd[v] = v < n ? (u64)((long long)(off[v + 1] - off[v]) + ddeg[v]) : 0ull;
-}
-
-// Untouched rows of the new CSR, copied by output position: each block takes
-// COPY_CH consecutive output entries and finds the rows they span with two
-// warp searches.  It stages those rows' new offsets, their shifts (old minus
-// new offset) and touched flags in shared memory, maps every entry to its row
-// there, and moves four entries per thread at a time.  Reads and writes
-// stream; entries of touched rows are left to k_merge_rows.
-constexpr u32 COPY_CH = 4096;
-constexpr u32 COPY_ROWS = 1024;
-constexpr u32 COPY_UNROLL = 4;
-
-// Largest i in [lo, hi) with a[i] <= x, given a[lo] <= x (a ascending).
-__device__ __forceinline__ u64 last_le_u64(const u64* a, u64 lo, u64 hi, u64 x) {
-  while (hi - lo > 1) {
-    const u64 mid = lo + (hi - lo) / 2;
-    if (a[mid] <= x) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// The same search by a whole warp: each step probes 32 evenly spaced
-// positions lo + span·k/32 at once and keeps the interval between the last
-// probe <= x and the next, so the span shrinks 32-fold per step.
-__device__ __forceinline__ u64 warp_last_le_u64(const u64* a, u64 lo, u64 hi, u64 x) {
-  const u32 lane = threadIdx.x & 31;
-  while (hi - lo > 32) {
-    const u64 span = hi - lo;
-    const u64 p = lo + span * lane / 32;
-    const u32 m = __ballot_sync(0xffffffffu, lane == 0 || a[p] <= x);
-    const u32 j = (u32)__popc(m) - 1;  // probes 0..j are <= x
-    const u64 nlo = lo + span * j / 32;
-    hi = j == 31 ? hi : lo + span * (j + 1) / 32;
-    lo = nlo;
-  }
-  const u64 p = lo + lane;
-  const u32 m = __ballot_sync(0xffffffffu, p < hi && (lane == 0 || a[p] <= x));
-  return lo + (u32)__popc(m) - 1;
-}
-
-__global__ void __launch_bounds__(256) k_copy_untouched(u32 n, const u64* off, const u32* col,
-                                                        const double* w, const u64* noff,
-                                                        u32* ncol, double* nw, const u8* touched,
-                                                        u64 nnz_new) {
-  __shared__ u64 s_noff[COPY_ROWS + 1];
-  __shared__ u64 s_shift[COPY_ROWS];
-  __shared__ u8 s_touched[COPY_ROWS];
-  __shared__ u32 s_rb, s_re;
-  const u32 wid = threadIdx.x >> 5;
-  for (u64 q0 = (u64)blockIdx.x * COPY_CH; q0 < nnz_new; q0 += (u64)gridDim.x * COPY_CH) {
-    const u64 q1 = q0 + COPY_CH < nnz_new ? q0 + COPY_CH : nnz_new;
-    // rows r with noff[r] <= q < noff[r + 1]; noff[0] = 0 <= q0, noff[n] = nnz_new > q
-    if (wid == 0) {
-      const u64 rb = warp_last_le_u64(noff, 0, (u64)n + 1, q0);
-      if ((threadIdx.x & 31) == 0) s_rb = (u32)rb;
-    } else if (wid == 1) {
-      const u64 re = warp_last_le_u64(noff, 0, (u64)n + 1, q1 - 1);
-      if ((threadIdx.x & 31) == 0) s_re = (u32)re;
-    }
-    __syncthreads();
-    const u32 rb = s_rb;
-    const u32 nrow = s_re - rb + 1;  // re <= n - 1, so rb + nrow <= n
-    const bool staged = nrow <= COPY_ROWS;
-    if (staged)
-      for (u32 x = threadIdx.x; x <= nrow; x += blockDim.x) {
-        const u64 no = noff[rb + x];
-        s_noff[x] = no;
-        if (x < nrow) {
-          s_shift[x] = off[rb + x] - no;  // modulo 2^64: src = q + shift
-          s_touched[x] = touched[rb + x];
-        }
-      }
-    __syncthreads();
-    for (u64 qb = q0 + threadIdx.x; qb < q1; qb += COPY_UNROLL * blockDim.x) {
-      u64 src[COPY_UNROLL];
-      bool mv[COPY_UNROLL];
-#pragma unroll
-      for (u32 u = 0; u < COPY_UNROLL; ++u) {
-        const u64 q = qb + (u64)u * blockDim.x;
-        mv[u] = false;
-        src[u] = 0;
-        if (q < q1) {
-          if (staged) {
-            u32 lo = 0, hi = nrow;
-            while (hi - lo > 1) {
-              const u32 mid = (lo + hi) >> 1;
-              if (s_noff[mid] <= q) lo = mid;
-              else hi = mid;
-            }
-            mv[u] = !s_touched[lo];
-            src[u] = q + s_shift[lo];
-          } else {
-            const u32 r = (u32)last_le_u64(noff, rb, (u64)rb + nrow, q);
-            mv[u] = !touched[r];
-            src[u] = off[r] + (q - noff[r]);
-          }
-        }
-      }
-      u32 c[COPY_UNROLL];
-      double v[COPY_UNROLL];
-#pragma unroll
-      for (u32 u = 0; u < COPY_UNROLL; ++u)
-        if (mv[u]) {
-          c[u] = col[src[u]];
-          v[u] = w[src[u]];
-        }
-#pragma unroll
-      for (u32 u = 0; u < COPY_UNROLL; ++u)
-        if (mv[u]) {
-          const u64 q = qb + (u64)u * blockDim.x;
-          ncol[q] = c[u];
-          nw[q] = v[u];
-        }
-    }
-    __syncthreads();
-  }
-}
-
-// Row-operation range [rstart[r], rend[r]) of every row that has operations
-// (row-operations sorted by (row, neighbour)).
-__global__ void k_row_ranges(const u64* rkeys, u64 R, u32* rstart, u32* rend) {
-  for (u64 t = blockIdx.x * (u64)blockDim.x + threadIdx.x; t < R; t += (u64)gridDim.x * blockDim.x) {
-    const u32 r = (u32)(rkeys[t] >> 32);
-    if (t == 0 || (u32)(rkeys[t - 1] >> 32) != r) rstart[r] = (u32)t;
-    if (t + 1 == R || (u32)(rkeys[t + 1] >> 32) != r) rend[r] = (u32)(t + 1);
-  }
-}
-
-// Merge of the row slice [s0, s1) (chunks of 32 from the row start o0) of a
-// touched row, by one warp (the row merge itself is described at
-// k_merge_rows).  The state on entry is that of the operations
-// consumed before the slice: p = first operation not consumed, drun / irun =
-// deletes / inserts consumed, del_key / del_same = neighbour of the last
-// consumed delete and the consumed deletes on it.  `row_end` marks the row's
-// last slice, whose last chunk takes every remaining operation.
-__device__ __forceinline__ void merge_slice(u64 o0, u64 s0, u64 s1, bool row_end, u64 no, u32 p,
-                                            u32 b, u32 drun, u32 irun, u32 del_key,
-                                            u32 del_same, const u32* col, const double* w,
-                                            u32* ncol, double* nw, const u64* rkeys,
-                                            const u32* rvals, const double* neww, u64 nnz_new,
-                                            u32* err) {
-  const u32 lane = threadIdx.x & 31;
-  // operation tile [tb, tb + 32) in registers: neighbour, value (DEL_MARK
-  // for a delete, else the index of the inserted weight)
-  u32 tb = p;
-  u32 tk = NONE32, tv = 0;
-  if (tb + lane < b) {
-    tk = (u32)rkeys[tb + lane];
-    tv = rvals[tb + lane];
-  }
-  // entry chunk prefetched one ahead
-  u32 c_n = s0 + lane < s1 ? col[s0 + lane] : NONE32;
-  double w_n = s0 + lane < s1 ? w[s0 + lane] : 0.0;
-  for (u64 base = s0;; base += 32) {
-    const bool chunk_last = base + 32 >= s1;
-    const bool last = chunk_last && row_end;  // the row's last chunk takes every remaining op
-    const u64 q = base + lane;
-    const bool valid = q < s1;
-    const u32 c = c_n;
-    const double wv = w_n;
-    if (!chunk_last) {
-      const u64 qn = q + 32;
-      c_n = qn < s1 ? col[qn] : NONE32;
-      w_n = qn < s1 ? w[qn] : 0.0;
-    }
-    const u32 vmask = __ballot_sync(0xffffffffu, valid);
-    const u32 c_last = vmask ? __shfl_sync(0xffffffffu, c, 31 - __clz(vmask)) : 0u;
-    const u32 d0 = drun, i0 = irun;
-    u32 dl = 0, il = 0;
-    // the two copies of a deleted self-loop may straddle two chunks: the
-    // earlier chunk consumed their deletes
-    bool deleted = valid && del_key != NONE32 && c == del_key;
-    while (p < b) {
-      const u32 o = p - tb;  // first unconsumed lane of the tile
-      const bool ok = tb + lane < b && lane >= o;
-      const u32 m = __ballot_sync(0xffffffffu, ok && (last || tk <= c_last));
-      const u32 cnt = __popc(m);  // lanes o .. o+cnt-1 (operations are sorted)
-      if (cnt) {
-        const u32 hiL = o + cnt;
-        const u32 delm = __ballot_sync(0xffffffffu, tv == DEL_MARK) & m;
-        // Entries: the consumed operations below c (lower bound of c among
-        // the tile's keys) and whether c itself is deleted.
-        u32 lo = o, hi = hiL;
-#pragma unroll
-        for (int it = 0; it < 6; ++it) {
-          const u32 mid = (lo + hi) >> 1;
-          const u32 km = __shfl_sync(0xffffffffu, tk, mid & 31);
-          if (lo < hi) {
-            if (km < c) lo = mid + 1;
-            else hi = mid;
-          }
-        }
-        const u32 ltm = m & (lo >= 32 ? 0xffffffffu : ((1u << lo) - 1u));
-        dl += __popc(ltm & delm);
-        il += __popc(ltm & ~delm);
-        const u32 kp = __shfl_sync(0xffffffffu, tk, lo & 31);
-        const u32 vp = __shfl_sync(0xffffffffu, tv, lo & 31);
-        if (valid && lo < hiL && kp == c && vp == DEL_MARK) deleted = true;
-        // Inserts: lower bound among the chunk's entries (padded with
-        // NONE32), earlier deletes below the key and earlier inserts.
-        u32 lo2 = 0, hi2 = 32;
-#pragma unroll
-        for (int it = 0; it < 6; ++it) {
-          const u32 mid = (lo2 + hi2) >> 1;
-          const u32 cm = __shfl_sync(0xffffffffu, c, mid & 31);
-          if (lo2 < hi2) {
-            if (cm < tk) lo2 = mid + 1;
-            else hi2 = mid;
-          }
-        }
-        const u32 grp = __match_any_sync(0xffffffffu, tk) & m;
-        const u32 before = (1u << lane) - 1u;
-        const bool ins = ((m >> lane) & 1u) && tv != DEL_MARK;
-        if (ins) {
-          const u32 dlt = drun + __popc(delm & before) - __popc(grp & delm & before) -
-                          (del_key == tk ? del_same : 0u);
-          const u64 out = no + (base + lo2 - o0) - dlt + irun + __popc(m & ~delm & before);
-          if (out >= nnz_new) {
-            atomicAdd(err, 1u);
-          } else {
-            ncol[out] = tk;
-            nw[out] = neww[tv];
-          }
-        }
-        if (delm) {
-          const u32 ld = 31 - __clz(delm);
-          const u32 kd = __shfl_sync(0xffffffffu, tk, ld);
-          const u32 same = __popc(__shfl_sync(0xffffffffu, grp, ld) & delm);
-          del_same = (del_key == kd) ? del_same + same : same;
-          del_key = kd;
-        }
-        drun += __popc(delm);
-        irun += cnt - __popc(delm);
-      }
-      p += cnt;
-      if (o + cnt < 32 || p >= b) break;
-      // the whole tile was consumed: load the next one
-      tb = p;
-      tk = NONE32;
-      tv = 0;
-      if (tb + lane < b) {
-        tk = (u32)rkeys[tb + lane];
-        tv = rvals[tb + lane];
-      }
-    }
-    if (valid && !deleted) {
-      const u64 out = no + (q - o0) - (d0 + dl) + (i0 + il);
-      if (out >= nnz_new) {
-        atomicAdd(err, 1u);
-      } else {
-        ncol[out] = c;
-        nw[out] = wv;
-      }
-    }
-    if (chunk_last) break;
-  }
-}
-
-// Touched rows, merged with their sorted row-operations, so the output row is
-// again sorted by neighbour id: deleted entries are skipped, every surviving
-// entry moves by (inserts before it) - (deletes before it), and an insert
-// lands at its lower bound in the old row, after the earlier inserts and
-// before the entries it precedes.  A warp walks the row in chunks of 32 and
-// consumes, per chunk, the operations whose neighbour is not above the
-// chunk's last one (all of them in the row's last chunk), 32 operations at a
-// time with bisections over lanes.  A self-loop is stored twice in its row and
-// its operations come in pairs; operations on one neighbour come deletes
-// first (a dropped self-loop replaced by an inserted one).
-//
-// Rows longer than MERGE_LONG go to `long_rows` for k_merge_long.
-constexpr u64 MERGE_LONG = 512;
-
-__global__ void k_merge_rows(u32 n, const u64* off, const u32* col, const double* w,
-                             const u64* noff, u32* ncol, double* nw, const u8* touched,
-                             const u64* rkeys, const u32* rvals, const u32* rstart,
-                             const u32* rend, const double* neww, u64 nnz_new, u32* err,
-                             u32* long_rows, u32* nlong) {
-  const u32 lane = threadIdx.x & 31;
-  const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
-  const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  for (u64 r = warp; r < n; r += nwarps) {
-    if (!touched[r]) continue;
-    const u64 o0 = off[r], o1 = off[r + 1];
-    if (o1 - o0 > MERGE_LONG) {
-      if (lane == 0) long_rows[atomicAdd(nlong, 1u)] = (u32)r;
-      continue;
-    }
-    merge_slice(o0, o0, o1, true, noff[r], rstart[r], rend[r], 0, 0, NONE32, 0, col, w, ncol, nw,
-                rkeys, rvals, neww, nnz_new, err);
-  }
-}
-
-// Long touched rows: a block per row, its warps on consecutive slices of
-// whole chunks.  A warp rebuilds the state at its slice start from the
-// operations whose neighbour is not above the entry before the slice (a
-// bisection, and the delete prefix of the sorted operations).
-__global__ void __launch_bounds__(256) k_merge_long(const u32* long_rows, const u32* nlong,
-                                                    const u64* off, const u32* col,
-                                                    const double* w, const u64* noff, u32* ncol,
-                                                    double* nw, const u64* rkeys,
-                                                    const u32* rvals, const u32* rstart,
-                                                    const u32* rend, const u32* delpre,
-                                                    const double* neww, u64 nnz_new, u32* err) {
-  const u32 lane = threadIdx.x & 31;
-  const u32 wib = threadIdx.x >> 5;
-  const u32 nw_ = blockDim.x >> 5;
-  const u32 cnt = *nlong;
-  for (u32 t = blockIdx.x; t < cnt; t += gridDim.x) {
-    const u32 r = long_rows[t];
-    const u64 o0 = off[r], o1 = off[r + 1];
-    const u64 chunks = (o1 - o0 + 31) / 32;  // > MERGE_LONG / 32 >= warps per block
-    const u64 c0 = chunks * wib / nw_, c1 = chunks * (wib + 1) / nw_;
-    const u64 s0 = o0 + 32 * c0;
-    const u64 s1 = (o0 + 32 * c1 < o1) ? o0 + 32 * c1 : o1;
-    const u32 a = rstart[r], b = rend[r];
-    u32 p = a, drun = 0, irun = 0, del_key = NONE32, del_same = 0;
-    if (s0 > o0) {
-      // operations consumed before the slice: neighbour <= cprev = col[s0 - 1]
-      const u32 cprev = col[s0 - 1];
-      u32 lo = a, hi = b;
-      while (lo < hi) {
-        const u32 mid = (lo + hi) >> 1;
-        if ((u32)rkeys[mid] <= cprev) lo = mid + 1;
-        else hi = mid;
-      }
-      p = lo;
-      drun = delpre[p] - delpre[a];
-      irun = (p - a) - drun;
-      // Only deletes on cprev itself matter from here on (a self-loop whose
-      // two copies the slice boundary separates): entries of this slice and
-      // the operations still to come are all >= cprev.
-      u32 x = p;
-      while (x > a && (u32)rkeys[x - 1] == cprev) --x;
-      for (; x < p; ++x)
-        if (rvals[x] == DEL_MARK) ++del_same;
-      if (del_same) del_key = cprev;
-    }
-    merge_slice(o0, s0, s1, c1 == chunks, noff[r], p, b, drun, irun, del_key, del_same, col, w,
-                ncol, nw, rkeys, rvals, neww, nnz_new, err);
-  }
+// The new CSR from the old one and its row-operations (csr_rebuild.cuh).
+__global__ void __launch_bounds__(256) k_rebuild(RowOps O, u32 n, u64 nnz, const u64* off,
+                                                 const u32* col, const double* w,
+                                                 const double* neww, u64* noff, u32* ncol,
+                                                 double* nw, u64 nnz_new, u32* err) {
+  const u64 thread = blockIdx.x * (u64)blockDim.x + threadIdx.x;
+  const u64 threads = (u64)gridDim.x * blockDim.x;
+  rebuild_inserts(O, neww, ncol, nw, nnz_new, err, thread, threads);
+  rebuild_offsets(O, n, off, noff, thread >> 5, threads >> 5);
+  rebuild_entries(O, nnz, col, w, ncol, nw, nnz_new, err, thread >> 5, threads >> 5);
 }
 
 // Row sums in CSR order (hit_leiden.rs:1063), left to right: the exact
-// rounding of the reference for any weights (warp per row, ordered fold).
-// `flags` (if set) restricts the rows to those flagged.  Rows of RUN_FOLD_MIN
-// or more entries are listed for k_row_sum_runs.
-__global__ void k_row_sum_serial(const u32* rows, u32 nr, const u64* off, const double* w,
-                                 double* k, const u8* flags, u32* longl, u32* longn) {
+// rounding of the reference for any weights.  A warp takes 32 rows at a time
+// and sums those whose flag is set (all without flags) one after another.
+__global__ void __launch_bounds__(256) k_row_sum_serial(u32 n, const u64* off, const double* w,
+                                                        double* k, const u8* flags) {
+  __shared__ __align__(16) double chain[8][CHAIN_TILE];
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  for (u64 i = warp; i < nr; i += nwarps) {
-    u32 v = rows ? rows[i] : (u32)i;
-    if (flags && !flags[v]) continue;
-    const u64 a = off[v], b = off[v + 1];
-    if (b - a >= RUN_FOLD_MIN) {
-      fold_defer(longl, longn, v);
-      continue;
+  for (u64 v0 = warp * 32; v0 < n; v0 += nwarps * 32) {
+    const u64 v = v0 + lane;
+    const bool on = v < n && (!flags || flags[v]);
+    const u64 a = on ? off[v] : 0, b = on ? off[v + 1] : 0;
+    double mine = 0.0;
+    for (u32 m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
+      const u32 j = __ffs(m) - 1;
+      const double s = warp_chain_sum(__shfl_sync(0xffffffffu, a, j),
+                                      __shfl_sync(0xffffffffu, b, j), 0.0, w,
+                                      chain[threadIdx.x >> 5]);
+      if (lane == j) mine = s;
     }
-    double s = warp_ordered_sum(a, b, 0.0, [&](u64 p) { return w[p]; },
-                                [](u64) { return true; });
-    if (lane == 0) k[v] = s;
-  }
-}
-
-// The long rows listed by k_row_sum_serial, folded in runs (the same bits).
-__global__ void k_row_sum_runs(const u32* longl, const u32* longn, const u64* off,
-                               const double* w, double* k) {
-  const u32 lane = threadIdx.x & 31;
-  const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
-  const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  const u32 nl = *longn;
-  for (u64 j = warp; j < nl; j += nwarps) {
-    const u32 v = longl[j];
-    double s = warp_fold_runs(off[v], off[v + 1], 0.0, w);
-    if (lane == 0) k[v] = s;
+    if (on) k[v] = mine;
   }
 }
 
 // Left-to-right sums of the segments [off[i], off[i+1]) of x from `init`:
-// PATH 0 is the library's pair (short segments here, long ones listed for
-// k_seq_sums_runs), 1 folds every segment in runs, 2 none.
-template <int PATH>
-__global__ void k_seq_sums(u32 nseg, const u64* off, const double* x, double init, double* out,
-                           u32* longl, u32* longn) {
+// the staged chain (paths 0 and 1) or the shuffled fold (path 2).
+template <bool STAGED>
+__global__ void __launch_bounds__(256) k_seq_sums(u32 nseg, const u64* off, const double* x,
+                                                  double init, double* out) {
+  __shared__ __align__(16) double chain[8][CHAIN_TILE];
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 i = warp; i < nseg; i += nwarps) {
     const u64 a = off[i], b = off[i + 1];
-    double s;
-    if constexpr (PATH == 1) {
-      s = warp_fold_runs(a, b, init, x);
-    } else {
-      if (PATH == 0 && b - a >= RUN_FOLD_MIN) {
-        fold_defer(longl, longn, (u32)i);
-        continue;
-      }
-      s = warp_ordered_sum(a, b, init, [&](u64 p) { return x[p]; }, [](u64) { return true; });
-    }
+    const double s = STAGED ? warp_chain_sum(a, b, init, x, chain[threadIdx.x >> 5])
+                            : warp_ordered_sum(a, b, init, [&](u64 p) { return x[p]; },
+                                               [](u64) { return true; });
     if (lane == 0) out[i] = s;
   }
-}
-
-__global__ void k_seq_sums_runs(const u32* longl, const u32* longn, const u64* off,
-                                const double* x, double init, double* out) {
-  const u32 lane = threadIdx.x & 31;
-  const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
-  const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  const u32 nl = *longn;
-  for (u64 j = warp; j < nl; j += nwarps) {
-    const u32 i = longl[j];
-    double s = warp_fold_runs(off[i], off[i + 1], init, x);
-    if (lane == 0) out[i] = s;
-  }
-}
-
-FoldList fold_list(Engine& E, u64 total, u32 nseg) {
-  Scratch& S = E.sc;
-  u64 cap = total / RUN_FOLD_MIN + 1;
-  if (cap > nseg) cap = nseg ? nseg : 1;
-  S.foldseg.ensure(E.mem, cap);
-  S.foldcnt.ensure(E.mem, 1);
-  HL_CUDA(cudaMemsetAsync(S.foldcnt.p, 0, sizeof(u32), E.stream));
-  return FoldList{S.foldseg.p, S.foldcnt.p};
 }
 
 void seq_sums(Engine& E, u32 nseg, const u64* off, const double* x, double init, int path,
               double* out) {
   if (!nseg) return;
   const u32 grid = grid_for((u64)nseg * 32);
-  if (path == 1) {
-    ++E.nlaunch, k_seq_sums<1><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out, nullptr,
-                                                            nullptr);
-  } else if (path == 2) {
-    ++E.nlaunch, k_seq_sums<2><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out, nullptr,
-                                                            nullptr);
-  } else {
-    // the total is only known on the device: room for every segment
-    FoldList fl = fold_list(E, (u64)nseg * RUN_FOLD_MIN, nseg);
-    ++E.nlaunch, k_seq_sums<0><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out, fl.seg,
-                                                            fl.cnt);
-    ++E.nlaunch, k_seq_sums_runs<<<FOLD_BLOCKS, 256, 0, E.stream>>>(fl.seg, fl.cnt, off, x, init,
-                                                                  out);
-  }
+  if (path == 2)
+    ++E.nlaunch, k_seq_sums<false><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
+  else
+    ++E.nlaunch, k_seq_sums<true><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
   HL_LAUNCH_CHECK();
 }
 
-// Ordered row sums of the flagged rows (all rows without flags): the short
-// rows in k_row_sum_serial, the long ones in k_row_sum_runs.
+// Ordered row sums of the flagged rows (all rows without flags).
 static void row_sums_ordered(Engine& E, Level& L, const u8* flags) {
-  const u32 n = L.g.n;
-  FoldList fl = fold_list(E, L.g.nnz, n);
-  ++E.nlaunch, k_row_sum_serial<<<grid_for((u64)n * 32), 256, 0, E.stream>>>(
-      nullptr, n, L.g.off.p, L.g.w.p, L.k.p, flags, fl.seg, fl.cnt);
-  ++E.nlaunch, k_row_sum_runs<<<FOLD_BLOCKS, 256, 0, E.stream>>>(fl.seg, fl.cnt, L.g.off.p,
-                                                                 L.g.w.p, L.k.p);
+  ++E.nlaunch, k_row_sum_serial<<<grid_for(L.g.n), 256, 0, E.stream>>>(
+      L.g.n, L.g.off.p, L.g.w.p, L.k.p, flags);
 }
 
 // Warp-parallel row sums; only used when every weight is integral, where any
 // summation order gives the same bits.
-__global__ void k_row_sum_warp(const u32* rows, u32 nr, const u64* off, const double* w,
-                               double* k, const u8* flags = nullptr) {
+__global__ void k_row_sum_warp(u32 n, const u64* off, const double* w, double* k,
+                               const u8* flags) {
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  for (u64 i = warp; i < nr; i += nwarps) {
-    u32 v = rows ? rows[i] : (u32)i;
-    if (flags && !flags[v]) continue;
-    double s = 0.0;
-    for (u64 p = off[v] + lane; p < off[v + 1]; p += 32) s += w[p];
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) k[v] = s;
+  for (u64 v0 = warp * 32; v0 < n; v0 += nwarps * 32) {
+    const u64 v = v0 + lane;
+    const bool on = v < n && (!flags || flags[v]);
+    const u64 a = on ? off[v] : 0, b = on ? off[v + 1] : 0;
+    double mine = 0.0;
+    for (u32 m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
+      const u32 j = __ffs(m) - 1;
+      const u64 hi = __shfl_sync(0xffffffffu, b, j);
+      u64 p = __shfl_sync(0xffffffffu, a, j) + lane;
+      double s = 0.0;
+      for (; p + 224 < hi; p += 256) {  // 8 loads in flight: hub rows
+        double y[8];
+#pragma unroll
+        for (u32 i = 0; i < 8; ++i) y[i] = w[p + 32 * i];
+#pragma unroll
+        for (u32 i = 0; i < 8; ++i) s += y[i];
+      }
+      for (; p < hi; p += 32) s += w[p];
+      for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == j) mine = s;
+    }
+    if (on) k[v] = mine;
   }
 }
-
 
 // Fixed-shape pairwise sum: tiles of 1024 (+0.0 padded) folded by stride
 // halving; repeated on the tile sums until one value remains.
@@ -797,8 +417,8 @@ static void recompute_flagged_rows(Engine& E, Level& L, const u8* flags) {
   if (!n) return;
   cudaEvent_t ev = E.kt_begin();
   if (E.integral)
-    ++E.nlaunch, k_row_sum_warp<<<grid_for((u64)n * 32), 256, 0, E.stream>>>(
-        nullptr, n, L.g.off.p, L.g.w.p, L.k.p, flags);
+    ++E.nlaunch, k_row_sum_warp<<<grid_for(n), 256, 0, E.stream>>>(n, L.g.off.p, L.g.w.p, L.k.p,
+                                                                    flags);
   else
     row_sums_ordered(E, L, flags);
   HL_LAUNCH_CHECK();
@@ -809,8 +429,8 @@ void recompute_all_degrees(Engine& E, Level& L) {
   u32 n = L.g.n;
   if (n) {
     if (E.integral)
-      ++E.nlaunch, k_row_sum_warp<<<grid_for((u64)n * 32), 256, 0, E.stream>>>(nullptr, n, L.g.off.p, L.g.w.p,
-                                                                   L.k.p);
+      ++E.nlaunch, k_row_sum_warp<<<grid_for(n), 256, 0, E.stream>>>(n, L.g.off.p, L.g.w.p, L.k.p,
+                                                                      nullptr);
     else
       row_sums_ordered(E, L, nullptr);
     HL_LAUNCH_CHECK();
@@ -830,6 +450,10 @@ void apply_delta(Engine& E, Level& L, const DevEdges& b, u32 new_n, bool keep_lo
   const u32 n = L.g.n;
   const bool drop_loops = !keep_loops && L.g.self_loop_entries > 0;
   if (b.k == 0 && !drop_loops) return;
+  if (gang_apply_fits(E, L, b, drop_loops)) {
+    gang_apply(E, L, b);
+    return;
+  }
   const u64 k = b.k;
 
   S.ktouched.ensure(E.mem, n ? n : 1);
@@ -947,11 +571,7 @@ void apply_delta(Engine& E, Level& L, const DevEdges& b, u32 new_n, bool keep_lo
     });
   }
   require(R < 0xFFFFFFFFull, "too many row operations in one batch");
-  // row-operation range of every row that has operations
-  S.delpre.ensure(E.mem, n ? n : 1);
-  S.inspre.ensure(E.mem, n ? n : 1);
-  ++E.nlaunch, k_row_ranges<<<grid_for(R), 256, 0, st>>>(S.rkeys2.p, R, S.delpre.p, S.inspre.p);
-  // deletes before every operation (for the long-row merge's slice starts)
+  // deletes before every operation, and its position in the old entries
   S.opdel.ensure(E.mem, R + 1);
   S.opdelpre.ensure(E.mem, R + 1);
   ++E.nlaunch, k_del_flags<<<grid_for(R + 1), 256, 0, st>>>(S.rvals2.p, R, S.opdel.p);
@@ -963,47 +583,26 @@ void apply_delta(Engine& E, Level& L, const DevEdges& b, u32 new_n, bool keep_lo
       return cub::DeviceScan::ExclusiveSum(t, bytes, a, o, (int64_t)R + 1, st);
     });
   }
-  S.ddeg.ensure(E.mem, n ? n : 1);
-  S.touched.ensure(E.mem, n ? n : 1);
-  HL_CUDA(cudaMemsetAsync(S.ddeg.p, 0, sizeof(int) * (n ? n : 1), st));
-  HL_CUDA(cudaMemsetAsync(S.touched.p, 0, n ? n : 1, st));
-  ++E.nlaunch, k_rowop_deg<<<grid_for(R), 256, 0, st>>>(S.rkeys2.p, S.rvals2.p, R, S.ddeg.p, S.touched.p);
-  S.newoff.ensure(E.mem, (size_t)n + 1);
-  ++E.nlaunch, k_new_degrees<<<grid_for((u64)n + 1), 256, 0, st>>>(n, L.g.off.p, S.ddeg.p, S.newoff.p);
+  S.opos.ensure(E.mem, R);
+  ++E.nlaunch, k_rowop_positions<<<grid_for(R), 256, 0, st>>>(S.rkeys2.p, S.rvals2.p, R,
+                                                               L.g.off.p, L.g.col.p, S.opos.p);
   HL_LAUNCH_CHECK();
-  {
-    u64* a = S.newoff.p;
-    cub_run(E, [&](void* t, size_t& bytes) {
-      return cub::DeviceScan::ExclusiveSum(t, bytes, a, a, (int64_t)n + 1, st);
-    });
-  }
-  u64 nnz_new = E.read_u64(S.newoff.p + n);
+  S.newoff.ensure(E.mem, (size_t)n + 1);
   DevGraph& G = L.g;
+  const u64 nnz_new = G.nnz + R - 2ull * E.read_u32(S.opdelpre.p + R);
   DBuf<u32>& ncol = G.col2;
   DBuf<double>& nw = G.w2;
   ncol.ensure(E.mem, nnz_new ? nnz_new : 1);
   nw.ensure(E.mem, nnz_new ? nnz_new : 1);
-  cudaEvent_t cev = E.kt_begin();
-  if (nnz_new)
-    ++E.nlaunch, k_copy_untouched<<<grid_for((nnz_new + COPY_CH - 1) / COPY_CH * 256), 256, 0, st>>>(
-        n, G.off.p, G.col.p, G.w.p, S.newoff.p, ncol.p, nw.p, S.touched.p, nnz_new);
-  E.kt_end(KT_COPY_ROWS, cev);
   cudaEvent_t kev = E.kt_begin();
-  if (n) {
-    S.ovf.ensure(E.mem, n);
-    S.ovf_cnt.ensure(E.mem, 4);
-    HL_CUDA(cudaMemsetAsync(S.ovf_cnt.p, 0, sizeof(u32), st));
-    ++E.nlaunch, k_merge_rows<<<grid_for((u64)n * 32), 256, 0, st>>>(
-        n, G.off.p, G.col.p, G.w.p, S.newoff.p, ncol.p, nw.p, S.touched.p, S.rkeys2.p, S.rvals2.p,
-        S.delpre.p, S.inspre.p, S.neww.p, nnz_new, S.cnt.p + 4, S.ovf.p, S.ovf_cnt.p);
-    ++E.nlaunch, k_merge_long<<<148 * 2, 256, 0, st>>>(
-        S.ovf.p, S.ovf_cnt.p, G.off.p, G.col.p, G.w.p, S.newoff.p, ncol.p, nw.p, S.rkeys2.p,
-        S.rvals2.p, S.delpre.p, S.inspre.p, S.opdelpre.p, S.neww.p, nnz_new, S.cnt.p + 4);
-  }
+  const RowOps O{(u32)R, S.rkeys2.p, S.rvals2.p, S.opdelpre.p, S.opos.p};
+  ++E.nlaunch, k_rebuild<<<grid_for(G.nnz / 8 + R + n), 256, 0, st>>>(
+      O, n, G.nnz, G.off.p, G.col.p, G.w.p, S.neww.p, S.newoff.p, ncol.p, nw.p, nnz_new,
+      S.cnt.p + 4);
   HL_LAUNCH_CHECK();
   E.kt_end(KT_MERGE_ROWS, kev);
-  // old and new offsets, touched flags, old and new (col, w) entries
-  E.kagg[KT_MERGE_ROWS].bytes += 16ull * ((u64)n + 1) + n + 12ull * (G.nnz + nnz_new);
+  // old and new offsets, old and new (col, w) entries
+  E.kagg[KT_MERGE_ROWS].bytes += 16ull * ((u64)n + 1) + 12ull * (G.nnz + nnz_new);
   u32 ce[3];  // merge errors, inserted and deleted self-loops
   E.read_u32s({S.cnt.p + 4, S.cnt.p + 0, S.cnt.p + 1}, ce);
   if (ce[0] != 0)

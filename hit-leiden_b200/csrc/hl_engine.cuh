@@ -49,12 +49,11 @@ struct Scratch {
   // delta application
   DBuf<u64> keys, keys2, rkeys, rkeys2;
   DBuf<u32> idx, idx2, segid, seg_start, rvals, rvals2;
-  DBuf<u8> op, touched, ktouched, isdel, isins;
+  DBuf<u8> op, ktouched, isdel, isins;
   DBuf<double> neww;
   DBuf<u32> nops_del, nops_ins, pos_del, pos_ins;
-  DBuf<u32> delpre, inspre;  // per-row operation ranges (start, end) of apply_delta
   DBuf<u32> opdel, opdelpre;  // apply_delta: delete flags of the sorted operations, their scan
-  DBuf<int> ddeg;
+  DBuf<u64> opos;             // apply_delta: their positions in the old entries
   DBuf<u64> newoff;
   DBuf<u32> rowlist;
   // node flags (level size)
@@ -89,7 +88,6 @@ struct Scratch {
   DBuf<u32> ovf, ovf_cnt;  // block kernel: rows deferred to the pass with global regions
   DBuf<u32> acc_cnt;       // inc-movement: accepted moves over all rounds
   DBuf<u32> hubk, hubk2, hubv;  // block bin ordered by degree (keys, sorted keys, list)
-  DBuf<u32> foldseg, foldcnt;   // ordered sums: long segments, folded in runs, and their count
   DBuf<double> fvals;           // ordered sums: the terms gathered into sum order
   DBuf<double> huge_val;
   // deterministic mode (det.cu)
@@ -119,6 +117,8 @@ struct Scratch {
   // per-level output: the level's s_cur before the batch, the changed nodes
   DBuf<u32> lvl_prev, lvl_nodes, lvl_ids;
   DBuf<u8> lvl_flag;
+  // single-launch stages (gang.cuh)
+  DBuf<u32> gang_part, gang_cnt, ga_touched;
 };
 
 // Per-kernel device timing (CUDA events on the engine's stream), enabled by
@@ -150,7 +150,7 @@ enum KernelId : int {
   KT_STAGE_REFINE,
   KT_STAGE_AGGREGATE,
   KT_HOST_SYNC,    // host waits on the stream (launches = count; no time)
-  KT_COPY_ROWS,    // untouched CSR rows copied into the new buffer
+  KT_GANG_APPLY,   // whole delta applications in one launch (gang_apply.cu)
   KT_MOVE_SMALL,   // movement rounds of a small frontier in one block (small.cu)
   KT_EVAL_PB,      // the partitioned pass of the block bin (inside KT_EVAL_HUGE)
   KT_COUNT
@@ -226,15 +226,13 @@ void recompute_all_degrees(Engine& E, Level& L);
 double tree_sum(Engine& E, const double* x, u64 n);
 void seq_sums(Engine& E, u32 nseg, const u64* off, const double* x, double init, int path,
               double* out);
-// List (and zeroed count) for the long segments of one ordered-sum kernel
-// pair: room for every segment of RUN_FOLD_MIN or more of `total` terms.
-struct FoldList {
-  u32* seg;
-  u32* cnt;
-};
-FoldList fold_list(Engine& E, u64 total, u32 nseg);
 bool edges_integral(Engine& E, const DevEdges& b);
 void check_endpoints(Engine& E, const DevEdges& b, u32 n);
+
+// gang_apply.cu: apply_delta in one launch, for batches it fits
+constexpr u64 GANG_BATCH_MAX = 32768;
+bool gang_apply_fits(Engine& E, const Level& L, const DevEdges& b, bool drop_loops);
+void gang_apply(Engine& E, Level& L, const DevEdges& b);
 
 // move.cu
 struct MoveOut {

@@ -1,0 +1,69 @@
+"""The single-launch stages on the GPU (one kernel per stage for batches and
+levels that fit it) against the oracle, at the sizes where their shape changes:
+one block, a cluster, a cooperative grid; sort chunks of 64 to 2048 records; the
+largest batch they take and the first one that goes to the multi-kernel path.
+
+Tolerance: bit-exact."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+gh = pytest.importorskip("tests.gpu_helpers")
+
+SHAPES = {"block": (300, 900), "cluster": (20000, 90000), "grid": (60000, 420000)}
+_graphs = {}
+
+
+def _base(shape, integral):
+    if (shape, integral) not in _graphs:
+        n, m = SHAPES[shape]
+        rng = np.random.default_rng(n + integral)
+        s, d, w = gh.random_graph(rng, n, m, integral)
+        # a hub whose row is summed apart and searched over many steps
+        hub = np.setdiff1d(rng.permutation(n)[: min(n // 2, 9000)], [7]).astype(np.uint32)
+        hw = np.full(len(hub), 2.0) if integral else rng.uniform(0.5, 2.0, len(hub))
+        s, d = np.concatenate([s, np.full(len(hub), 7, np.uint32)]), np.concatenate([d, hub])
+        g = O.Graph.from_edges(n, s, d, np.concatenate([w, hw]))
+        _graphs[shape, integral] = g.apply_delta([], [], [], keep_self_loops=True)
+    return _graphs[shape, integral]
+
+
+def _batch(g, k, integral, seed):
+    """k updates: inserts, exact deletes, weight changes, repeated keys, loops,
+    many of them in the hub's row."""
+    rng = np.random.default_rng(seed)
+    off, col, w = g.csr()
+    src = np.repeat(np.arange(g.n, dtype=np.uint32), np.diff(off).astype(np.int64))
+    ds = rng.integers(0, g.n, k).astype(np.uint32)
+    dd = rng.integers(0, g.n, k).astype(np.uint32)
+    dw = rng.integers(-2, 4, k).astype(float) if integral else rng.uniform(-1.0, 2.5, k)
+    old = rng.random(k) < 0.5
+    e = rng.integers(0, len(col), k)
+    ds[old], dd[old] = src[e[old]], col[e[old]]
+    gone = old & (rng.random(k) < 0.6)
+    dw[gone] = -w[e[gone]]
+    ds[rng.random(k) < 0.2] = 7
+    loop = rng.random(k) < 0.02
+    dd[loop] = ds[loop]
+    again = rng.random(k) < 0.1
+    at = rng.integers(0, k, k)
+    ds[again], dd[again] = ds[at[again]], dd[at[again]]
+    return ds, dd, dw
+
+
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("shape,k", [
+    ("block", 1), ("block", 64), ("block", 65), ("block", 513),
+    ("cluster", 1), ("cluster", 512), ("cluster", 1025), ("cluster", 16385),
+    ("grid", 2), ("grid", 2049), ("grid", 32768), ("grid", 32769)])
+def test_apply_delta_shapes(shape, k, integral):
+    g = _base(shape, integral)
+    for seed in range(2):
+        ds, dd, dw = _batch(g, k, integral, 10 * k + seed)
+        ref = g.apply_delta(ds, dd, dw, keep_self_loops=True)
+        got = gh.apply_delta(g, ds, dd, dw, keep_loops=True)
+        for a, b in zip(got, ref.csr()):
+            assert gh.same_bits(a, b)
