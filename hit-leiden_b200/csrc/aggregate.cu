@@ -409,32 +409,24 @@ void top_down(Engine& E) {
   HL_LAUNCH_CHECK();
 }
 
-__global__ void k_inherit(const u32* xs, const u32* os, u32 m, u32* s_pre, u32* s_cur, u32* gm) {
+// A new node takes the s_pre, s_cur and g of the node it was split from, and
+// joins K at its level (M6, M8).
+__global__ void k_inherit(u32 base, const u32* origin, u32 m, u32* s_pre, u32* s_cur, u32* gm,
+                          u8* kflag) {
   for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < m; i += (u64)gridDim.x * blockDim.x) {
-    u32 x = xs[i], o = os[i];
+    const u32 x = base + (u32)i, o = origin[i];
     s_pre[x] = s_pre[o];
     s_cur[x] = s_cur[o];
     gm[x] = gm[o];
+    kflag[x] = 1;
   }
 }
 
-void inherit_new_nodes(Engine& E, Level& hi, const std::vector<std::pair<u32, u32>>& ids) {
-  if (ids.empty()) return;
-  u32 m = (u32)ids.size();
-  std::vector<u32> xs(m), os(m);
-  for (u32 i = 0; i < m; ++i) {
-    xs[i] = ids[i].first;
-    os[i] = ids[i].second;
-  }
-  Scratch& S = E.sc;
-  S.upd_node.ensure(E.mem, m);
-  S.upd_to.ensure(E.mem, m);
-  HL_CUDA(cudaMemcpyAsync(S.upd_node.p, xs.data(), sizeof(u32) * m, cudaMemcpyHostToDevice, E.stream));
-  HL_CUDA(cudaMemcpyAsync(S.upd_to.p, os.data(), sizeof(u32) * m, cudaMemcpyHostToDevice, E.stream));
-  ++E.nlaunch, k_inherit<<<grid_for(m), 256, 0, E.stream>>>(S.upd_node.p, S.upd_to.p, m, hi.s_pre.p, hi.s_cur.p,
-                                               hi.gm.p);
+void inherit_new_nodes(Engine& E, Level& hi) {
+  if (!E.n_new) return;
+  ++E.nlaunch, k_inherit<<<grid_for(E.n_new), 256, 0, E.stream>>>(
+      E.new_base, E.sc.origin.p, E.n_new, hi.s_pre.p, hi.s_cur.p, hi.gm.p, E.sc.kflag.p);
   HL_LAUNCH_CHECK();
-  E.sync();  // host vectors go out of scope
 }
 
 }  // namespace hl

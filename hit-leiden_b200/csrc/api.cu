@@ -253,11 +253,6 @@ __global__ void k_gather_u32(const u32* idx, u32 m, const u32* src, u32* out) {
     out[i] = src[idx[i]];
 }
 
-__global__ void k_flag_ids(const u32* ids, u32 m, u32 n, u8* flags) {
-  for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < m; i += (u64)gridDim.x * blockDim.x)
-    if (ids[i] < n) flags[ids[i]] = 1;
-}
-
 static void level_snapshot(Engine& E, Level& L) {
   if (!E.level_fn || !L.g.n) return;
   E.sc.lvl_prev.ensure(E.mem, L.g.n);
@@ -365,50 +360,50 @@ static void hit_leiden_batch(EngineBox& B, const DevEdges& delta) {
     if (p == 0) st.refined = ro.refined;
     if (p + 1 >= P) break;
     Level& H = E.levels[p + 1];
-    // Grow level p+1 to hold every sub-community id handed out at level p.
-    u32 need = 0;
-    {
-      u32* o = E.sc.cnt.p + 12;
-      u32* sc = L.s_cur.p;
-      cub_run(E, [&](void* t, size_t& b) {
-        return cub::DeviceReduce::Max(t, b, sc, o, (int64_t)L.g.n, E.stream);
-      });
-      need = E.read_u32(o) + 1;
-      for (auto& xo : E.new_ids) need = need > xo.first + 1 ? need : xo.first + 1;
-    }
-    graph_grow_nodes(E, H, need);
-    inherit_new_nodes(E, H, E.new_ids);
-    // M8: the nodes level p+1 gains from this level's splits, and those whose
-    // community the projection changes, join K at level p+1
-    E.sc.kflag.ensure(E.mem, H.g.n ? H.g.n : 1);
-    HL_CUDA(cudaMemsetAsync(E.sc.kflag.p, 0, H.g.n ? H.g.n : 1, E.stream));
-    if (!E.new_ids.empty()) {
-      std::vector<u32> ids;
-      for (auto& xo : E.new_ids) ids.push_back(xo.first);
-      E.sc.kflag_ids.ensure(E.mem, ids.size());
-      HL_CUDA(cudaMemcpyAsync(E.sc.kflag_ids.p, ids.data(), sizeof(u32) * ids.size(),
-                              cudaMemcpyHostToDevice, E.stream));
-      ++E.nlaunch, k_flag_ids<<<(u32)std::min<size_t>((ids.size() + 255) / 256, 148 * 32), 256, 0,
-                                E.stream>>>(E.sc.kflag_ids.p, (u32)ids.size(), H.g.n,
-                                            E.sc.kflag.p);
-      HL_LAUNCH_CHECK();
-    }
-    project_up(E, L, H, E.sc.kflag.p);
-    E.k_flags_set = true;
-    if (cur.k == 0 && ro.refined == 0) {  // should_skip_aggregation (:1020-1022)
-      cur = DevEdges{};
-      cur_n = H.g.n;
-      continue;
+    // Grow level p+1 to hold every sub-community id handed out at level p
+    // (the ids of merged singletons included), project the communities onto
+    // it and aggregate; should_skip_aggregation (:1020-1022).
+    const bool aggregate = !(cur.k == 0 && ro.refined == 0);
+    const int slot = (p + 1) & 1;
+    u64 cnt = 0;
+    if (gang_aggregate_fits(E, L, cur)) {
+      e0 = E.kt_begin();
+      bool done;
+      {
+        NvtxScope r("aggregate");
+        done = gang_aggregate(E, L, H, cur, aggregate, B.bb.xu[slot], B.bb.xv[slot],
+                              B.bb.xw[slot], &cnt);
+      }
+      E.kt_end(KT_STAGE_AGGREGATE, e0);
+      E.k_flags_set = true;
+      if (done) {
+        cur = aggregate ? DevEdges{B.bb.xu[slot].p, B.bb.xv[slot].p, B.bb.xw[slot].p, cnt}
+                        : DevEdges{};
+        cur_n = H.g.n;
+        continue;
+      }
+    } else {
+      graph_grow_nodes(E, H, E.new_base + E.n_new);
+      // M8: the nodes level p+1 gains from this level's splits, and those whose
+      // community the projection changes, join K at level p+1
+      E.sc.kflag.ensure(E.mem, H.g.n ? H.g.n : 1);
+      HL_CUDA(cudaMemsetAsync(E.sc.kflag.p, 0, H.g.n ? H.g.n : 1, E.stream));
+      inherit_new_nodes(E, H);
+      project_up(E, L, H, E.sc.kflag.p);
+      E.k_flags_set = true;
+      if (!aggregate) {
+        cur = DevEdges{};
+        cur_n = H.g.n;
+        continue;
+      }
     }
     u32 nn = 0;
     e0 = E.kt_begin();
-    u64 cnt;
     {
       NvtxScope r("aggregate");
       cnt = inc_aggregation(E, L, cur, &nn, true, true);
     }
     E.kt_end(KT_STAGE_AGGREGATE, e0);
-    int slot = (p + 1) & 1;
     B.bb.xu[slot].ensure(E.mem, cnt ? cnt : 1);
     B.bb.xv[slot].ensure(E.mem, cnt ? cnt : 1);
     B.bb.xw[slot].ensure(E.mem, cnt ? cnt : 1);
@@ -674,7 +669,8 @@ static const char* kernel_names[KT_COUNT] = {
     "apply_and_mark",
     "refine_cc",   "t_filter",    "row_sums",         "delta_resolve",  "stage_apply",
     "stage_move",  "stage_refine", "stage_aggregate", "host_syncs",
-    "apply_one_launch", "move_small_rounds", "eval_huge_partitioned"};
+    "apply_one_launch", "move_small_rounds", "eval_huge_partitioned",
+    "refine_one_launch", "aggregate_one_launch"};
 
 hl_status hl_kernel_stats(const hl_graph* g, hl_kernel_stat* out, uint32_t cap, uint32_t* count) {
   HL_TRY(require(g && count, "NULL argument"); Engine& E = *const_cast<EngineBox*>(box(g))->E;
@@ -1082,6 +1078,7 @@ hl_status hl_dbg_inc_refinement(int32_t device, uint32_t n, const uint64_t* off,
     level_from_host(E, L, n, off, col, w);
     up(E, L.f, f, n);
     up(E, L.s_cur, s, n);
+    L.s_bound = 0;  // s is the caller's
     up(E, E.sc.affected, affected, n);
     inc_refinement(E, L, cc_same_community != 0);
     down(E, s, L.s_cur.p, n);

@@ -60,7 +60,7 @@ __device__ __forceinline__ Gang gang_make(bool grid) {
 // at the start of the dynamic block).
 struct GangSmem {
   u64 key[GSORT_CHUNK];
-  u32 pos[GSORT_CHUNK];
+  u32 val[GSORT_CHUNK];
   u32 wsum[GANG_WARPS + 1];
   u32 bcast[2];
 };
@@ -137,15 +137,16 @@ __device__ __forceinline__ u32 gang_scan(const Gang& G, GangSmem& S, u32 N, V va
   return total;
 }
 
-// Stable ascending sort of N (key, value) records.  Blocks sort chunks of up
-// to GSORT_CHUNK records in shared memory (bitonic on (key, position)); after
-// a barrier every record finds its rank by a bisection in each other chunk and
-// is handed to emit(rank, key, value).  `tk`/`tv` take the sorted chunks.  Two
-// gang barriers inside (one when a single block does it all); the caller's
-// emitted output is visible after the last one.
+// Ascending sort of N (key, value) records by (key, value); with the record's
+// index as its value, the stable sort by key.  Blocks sort chunks of up to
+// GSORT_CHUNK records in shared memory (bitonic); after a barrier every record
+// finds its rank by a bisection in each other chunk and is handed to
+// emit(rank, key, value).  `tk`/`tv` take the sorted chunks.  Two gang barriers
+// inside (one when a single chunk holds everything); the caller's emitted
+// output is visible after the last one.
 //
-// For a few thousand records this takes 5-10 us; a radix sort of the same
-// keys is six to nine dependent kernel launches.
+// For a few thousand records this takes 5-15 us; a radix sort of the same keys
+// is six to nine dependent kernel launches.
 template <typename K, typename VL, typename EM>
 __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K key_of, VL val_of,
                                           u64* tk, u32* tv, EM emit) {
@@ -161,7 +162,7 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
     while (P < cnt) P <<= 1;
     for (u32 i = tid; i < P; i += GANG_THREADS) {
       S.key[i] = i < cnt ? key_of(base + i) : ~0ull;
-      S.pos[i] = i;
+      S.val[i] = i < cnt ? val_of(base + i) : NONE32;
     }
     __syncthreads();
     for (u32 size = 2; size <= P; size <<= 1) {
@@ -171,13 +172,13 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
           const u32 j = i + stride;
           const bool up = (i & size) == 0;
           const u64 ki = S.key[i], kj = S.key[j];
-          const u32 pi = S.pos[i], pj = S.pos[j];
-          const bool gt = ki > kj || (ki == kj && pi > pj);
+          const u32 vi = S.val[i], vj = S.val[j];
+          const bool gt = ki > kj || (ki == kj && vi > vj);
           if (gt == up) {
             S.key[i] = kj;
             S.key[j] = ki;
-            S.pos[i] = pj;
-            S.pos[j] = pi;
+            S.val[i] = vj;
+            S.val[j] = vi;
           }
         }
         // strides up to 32 stay within the 64 elements of one warp
@@ -187,12 +188,11 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
       if (size >= 64) __syncthreads();
     }
     for (u32 i = tid; i < cnt; i += GANG_THREADS) {
-      const u32 v = val_of(base + S.pos[i]);
       if (nch == 1) {
-        emit(i, S.key[i], v);
+        emit(i, S.key[i], S.val[i]);
       } else {
         tk[base + i] = S.key[i];
-        tv[base + i] = v;
+        tv[base + i] = S.val[i];
       }
     }
     __syncthreads();
@@ -201,9 +201,10 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
   if (nch == 1) return;
   for (u32 e = G.thread(); e < N; e += G.threads()) {
     const u64 k = tk[e];
+    const u32 v = tv[e];
     const u32 mine = e / ch;
     u32 rank = e - mine * ch;
-    // GSORT_ILP bisections side by side; equal keys: earlier chunks come first
+    // GSORT_ILP bisections side by side; equal records: earlier chunks first
     for (u32 c0 = 0; c0 < nch; c0 += GSORT_ILP) {
       u32 pos[GSORT_ILP];
 #pragma unroll
@@ -219,15 +220,87 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
           probe[j] = in[j] ? tk[at - 1] : 0ull;
         }
 #pragma unroll
-        for (u32 j = 0; j < GSORT_ILP; ++j)
-          if (in[j] && (probe[j] < k || (probe[j] == k && c0 + j < mine))) pos[j] += half;
+        for (u32 j = 0; j < GSORT_ILP; ++j) {
+          if (!in[j] || probe[j] > k) continue;
+          if (probe[j] == k) {
+            const u32 y = tv[(c0 + j) * ch + pos[j] + half - 1];
+            if (y > v || (y == v && c0 + j > mine)) continue;
+          }
+          pos[j] += half;
+        }
       }
 #pragma unroll
       for (u32 j = 0; j < GSORT_ILP; ++j) rank += pos[j];
     }
-    emit(rank, k, tv[e]);
+    emit(rank, k, v);
   }
   G.sync();
+}
+
+// Stable counting sort of the vertices 0..n-1 by a label below 2^bits: sorted
+// labels in `lab`, vertices in `idx`, both ascending within.  8 bits a pass;
+// every warp of the gang owns a consecutive run of records, counts it per
+// digit (`hist`, 256 words a warp, digit-major), and after a scan places it in
+// order.  lab2 / idx2 are the other halves of the double buffers; the result is
+// in the buffers that *second names.  All barriers inside; the output is
+// visible on return.
+template <typename L0>
+__device__ __forceinline__ void gang_label_sort(const Gang& G, GangSmem& S, u32 n, u32 bits,
+                                                L0 label, u32* lab, u32* idx, u32* lab2,
+                                                u32* idx2, u32* hist, u32* part, bool* second) {
+  const u32 lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  // consecutive runs for consecutive (block, warp): run order is record order
+  const u32 run = G.rank * GANG_WARPS + wib, runs = G.warps();
+  const u32 per = ((n + runs - 1) / runs + 31) & ~31u;
+  const u32 lo = min(n, run * per), hi = min(n, lo + per);
+  u32* cnt = reinterpret_cast<u32*>(S.key) + wib * 256;  // 16 warps x 256 words
+  bool from_label = true;
+  u32 *ki = nullptr, *vi = nullptr, *ko = lab, *vo = idx;
+  for (u32 shift = 0; shift < bits; shift += 8) {
+    for (u32 d = lane; d < 256; d += 32) cnt[d] = 0;
+    __syncwarp();
+    for (u32 i0 = lo; i0 < hi; i0 += 32) {
+      const u32 i = i0 + lane;
+      const u32 k = i < hi ? (from_label ? label(i) : ki[i]) : 0u;
+      const u32 d = i < hi ? (k >> shift) & 255u : 256u;
+      const u32 grp = __match_any_sync(0xffffffffu, d);
+      if (i < hi && lane == (u32)(__ffs(grp) - 1)) cnt[d] += __popc(grp);
+      __syncwarp();
+    }
+    for (u32 d = lane; d < 256; d += 32) hist[d * runs + run] = cnt[d];
+    G.sync();
+    gang_scan(
+        G, S, 256 * runs, [&](u32 i) { return hist[i]; }, [&](u32 i, u32 ex) { hist[i] = ex; },
+        part);
+    G.sync();
+    for (u32 d = lane; d < 256; d += 32) cnt[d] = hist[d * runs + run];
+    __syncwarp();
+    for (u32 i0 = lo; i0 < hi; i0 += 32) {
+      const u32 i = i0 + lane;
+      const u32 k = i < hi ? (from_label ? label(i) : ki[i]) : 0u;
+      const u32 v = i < hi ? (from_label ? i : vi[i]) : 0u;
+      const u32 d = i < hi ? (k >> shift) & 255u : 256u;
+      const u32 grp = __match_any_sync(0xffffffffu, d);
+      if (i < hi) {
+        const u32 at = cnt[d] + __popc(grp & ((1u << lane) - 1u));
+        ko[at] = k;
+        vo[at] = v;
+      }
+      __syncwarp();
+      if (i < hi && lane == (u32)(__ffs(grp) - 1)) cnt[d] += __popc(grp);
+      __syncwarp();
+    }
+    __syncthreads();  // cnt aliases S.key, which gang_scan does not touch
+    G.sync();
+    from_label = false;
+    *second = ko == lab2;
+    u32* t = ko;
+    ko = t == lab ? lab2 : lab;
+    ki = t;
+    t = vo;
+    vo = t == idx ? idx2 : idx;
+    vi = t;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -67,6 +67,7 @@ void graph_init_empty(Engine& E, Level& L, u32 n) {
     HL_CUDA(cudaMemsetAsync(L.k.p, 0, sizeof(double) * n, E.stream));
   }
   L.tw = 0.0;
+  L.s_bound = n;
   HL_LAUNCH_CHECK();
 }
 
@@ -88,6 +89,7 @@ void graph_grow_nodes(Engine& E, Level& L, u32 n) {
   ++E.nlaunch, k_iota_range<<<grid_for(n - old), 256, 0, E.stream>>>(L.s_cur.p, old, n);
   ++E.nlaunch, k_fill_f64_range<<<grid_for(n - old), 256, 0, E.stream>>>(L.k.p, 0.0, old, n);
   L.g.n = n;
+  if (L.s_bound && L.s_bound < n) L.s_bound = n;
   HL_LAUNCH_CHECK();
 }
 

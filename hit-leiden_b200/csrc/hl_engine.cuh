@@ -30,6 +30,7 @@ struct Level {
   DBuf<u32> s_cur;  // current_subcommunity_mapping_per_level[p]
   DBuf<double> k;   // weighted degree of each level-p node
   double tw = 0.0;  // 2m of G^p
+  u32 s_bound = 0;  // every id in s_pre and s_cur is below this (0: not known)
 };
 
 // An edge list on the device (GraphInput): w == nullptr means weight 1.0.
@@ -110,7 +111,6 @@ struct Scratch {
   // [8] accepted moves, [9] refinement merges, [10] |B^1|
   DBuf<u64> bacc;
   DBuf<u8> kflag;     // K marks for the next level (M8), level-size bytes
-  DBuf<u32> kflag_ids;  // moved hubs whose rows k_mark_next_long marks
   // movement rounds of a small frontier (small.cu)
   DBuf<u32> sm_list_a, sm_list_b;
   DBuf<u64> sm_out;
@@ -118,7 +118,8 @@ struct Scratch {
   DBuf<u32> lvl_prev, lvl_nodes, lvl_ids;
   DBuf<u8> lvl_flag;
   // single-launch stages (gang.cuh)
-  DBuf<u32> gang_part, gang_cnt, ga_touched;
+  DBuf<u32> gang_part, gang_cnt, ga_touched, gr_bits;
+  DBuf<u64> gr_items;
 };
 
 // Per-kernel device timing (CUDA events on the engine's stream), enabled by
@@ -153,6 +154,8 @@ enum KernelId : int {
   KT_GANG_APPLY,   // whole delta applications in one launch (gang_apply.cu)
   KT_MOVE_SMALL,   // movement rounds of a small frontier in one block (small.cu)
   KT_EVAL_PB,      // the partitioned pass of the block bin (inside KT_EVAL_HUGE)
+  KT_GANG_REFINE,  // whole refinements in one launch (gang_refine.cu)
+  KT_GANG_AGG,     // whole aggregations in one launch (gang_aggregate.cu)
   KT_COUNT
 };
 
@@ -174,7 +177,9 @@ struct Engine {
   u64 launch_mark = 0;
   // per-call statistics
   hl_batch_stats st{};
-  std::vector<std::pair<u32, u32>> new_ids;  // (new sub-community id, origin) of the last refinement
+  // sub-community ids of the last refinement's splits: new_base ..
+  // new_base + n_new - 1, split from the ids in Scratch::origin
+  u32 n_new = 0, new_base = 0;
   // K marks handed to the next level's inc_movement (M8): the nodes it gained
   // from splits below and the nodes whose community the projection changed
   bool k_flags_set = false;
@@ -254,8 +259,15 @@ struct RefineOut {
   u64 splits = 0, merges = 0, refined = 0;
   u64 tfilter_exact = 0;  // candidates decided from the ordered sum
   u32 smax_before = 0;
+  u32 singles = 0;  // refined singletons (gang_refine)
 };
 RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community);
+
+// gang_refine.cu: the refinement in one launch; the status names the step the
+// multi-kernel path continues from
+enum : u32 { REF_DONE = 0, REF_HOST_ALL = 1, REF_HOST_MERGE = 2, REF_HOST_EVAL = 3 };
+bool gang_refine_fits(Engine& E, const Level& L);
+u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out);
 
 // api.cu: device-side batch statistics (Scratch::bacc)
 void stats_acc_u64(Engine& E, const unsigned long long* src, u32 count, u32 slot);
@@ -286,12 +298,17 @@ extern std::atomic<u32> g_dbg_hub_defer;
 extern std::atomic<u64> g_dbg_pb_round;
 
 // aggregate.cu
+// gang_aggregate.cu: the next level's growth and projection and the aggregation
+// in one launch
+bool gang_aggregate_fits(Engine& E, const Level& L, const DevEdges& delta);
+bool gang_aggregate(Engine& E, Level& L, Level& H, const DevEdges& delta, bool aggregate,
+                    DBuf<u32>& ou, DBuf<u32>& ov, DBuf<double>& ow, u64* count);
 u64 inc_aggregation(Engine& E, Level& L, const DevEdges& delta, u32* next_n,
                     bool changed_only, bool edge_weight_loops);  // output in sc.eu2/ev2/ew2
 u64 aggregate_full(Engine& E, Level& L, const u32* s, u32* out_u, u32* out_v, double* out_w);
 void project_up(Engine& E, Level& lo, Level& hi, u8* changed_flags = nullptr);
 void top_down(Engine& E);
-void inherit_new_nodes(Engine& E, Level& hi, const std::vector<std::pair<u32, u32>>& ids);
+void inherit_new_nodes(Engine& E, Level& hi);
 
 // modularity.cu
 double modularity(Engine& E, Level& L, const u32* part);

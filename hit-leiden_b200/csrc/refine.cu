@@ -120,13 +120,11 @@ __global__ void k_gather_keys(const u32* roots, u32 m, const u64* key, u64* out)
     out[i] = key[roots[i]];
 }
 
-__global__ void k_assign_newid(const u64* sorted, u32 m, u32 base, u32* newid, u32* origin_new,
-                               u32* origin_old) {
+__global__ void k_assign_newid(const u64* sorted, u32 m, u32 base, u32* newid, u32* origin) {
   for (u64 t = blockIdx.x * (u64)blockDim.x + threadIdx.x; t < m; t += (u64)gridDim.x * blockDim.x) {
     u32 r = (u32)sorted[t];
     newid[r] = base + (u32)t;
-    origin_new[t] = base + (u32)t;
-    origin_old[t] = (u32)(sorted[t] >> 32);
+    origin[t] = (u32)(sorted[t] >> 32);
   }
 }
 
@@ -418,16 +416,12 @@ static u32 select_flagged(Engine& E, const u8* flags, u32 n, u32* out, u32* cnt)
 
 std::atomic<int> g_exact_tfilter{0};
 
-RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
-  RefineOut out;
+// Connected-component split of the affected sub-communities, and R.
+static void refine_cc(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   Scratch& S = E.sc;
   cudaStream_t st = E.stream;
   const u32 n = L.g.n;
-  E.new_ids.clear();
-  S.refined.ensure(E.mem, n ? n : 1);
-  HL_CUDA(cudaMemsetAsync(S.refined.p, 0, n ? n : 1, st));
-  if (!n) return out;
-  S.cnt.ensure(E.mem, 16);
+  HL_CUDA(cudaMemsetAsync(S.refined.p, 0, n, st));
   u32* cnt = S.cnt.p;
   u32* s = L.s_cur.p;
 
@@ -465,8 +459,7 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
   if (m_new) {
     S.keys.ensure(E.mem, m_new);
     S.keys2.ensure(E.mem, m_new);
-    S.used.ensure(E.mem, m_new);
-    S.rank.ensure(E.mem, m_new);
+    S.origin.ensure(E.mem, m_new);
     ++E.nlaunch, k_gather_keys<<<grid_for(m_new), 256, 0, st>>>(S.act.p, m_new, S.gkey.p, S.keys.p);
     HL_LAUNCH_CHECK();
     u64* ki = S.keys.p;
@@ -474,17 +467,11 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
     cub_run(E, [&](void* t, size_t& b) {
       return cub::DeviceRadixSort::SortKeys(t, b, ki, ko, (int64_t)m_new, 0, 64, st);
     });
-    ++E.nlaunch, k_assign_newid<<<grid_for(m_new), 256, 0, st>>>(ko, m_new, smax + 1, S.newid.p, S.used.p,
-                                                     S.rank.p);
+    ++E.nlaunch, k_assign_newid<<<grid_for(m_new), 256, 0, st>>>(ko, m_new, smax + 1, S.newid.p,
+                                                     S.origin.p);
     ++E.nlaunch, k_apply_split<<<grid_for(n), 256, 0, st>>>(n, s, S.affsc.p, S.uroot.p, S.status.p, S.newid.p,
                                                S.refined.p);
     HL_LAUNCH_CHECK();
-    std::vector<u32> a(m_new), b(m_new);
-    HL_CUDA(cudaMemcpyAsync(a.data(), S.used.p, sizeof(u32) * m_new, cudaMemcpyDeviceToHost, st));
-    HL_CUDA(cudaMemcpyAsync(b.data(), S.rank.p, sizeof(u32) * m_new, cudaMemcpyDeviceToHost, st));
-    E.sync();
-    E.new_ids.resize(m_new);
-    for (u32 i = 0; i < m_new; ++i) E.new_ids[i] = {a[i], b[i]};
   }
   out.splits = m_new;
   E.kt_end(KT_REFINE_CC, ev_cc);
@@ -496,9 +483,38 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
   ++E.nlaunch, k_refine_all_if_identity<<<grid_for(n), 256, 0, st>>>(n, cnt + 5, S.refined.p);
   HL_LAUNCH_CHECK();
 
+  E.n_new = m_new;
+  E.new_base = smax + 1;
+  L.s_bound = n > smax + m_new + 1 ? n : smax + m_new + 1;
+}
+
+// The refined singletons' evaluation on the snapshot and the moves of all
+// that gain.
+static void merge_singletons(Engine& E, Level& L, const u32* single, u32 ns) {
+  Scratch& S = E.sc;
+  cudaStream_t st = E.stream;
+  u32* s = L.s_cur.p;
+  S.cand_to.ensure(E.mem, ns);
+  S.cand_gain.ensure(E.mem, ns);
+  run_eval(E, 1, single, ns, L, s, S.dS.p, S.blocked.p, false, S.cand_to.p, S.cand_gain.p,
+           nullptr);
+  u32* cnt = S.cnt.p;
+  HL_CUDA(cudaMemsetAsync(cnt + 9, 0, sizeof(u32), st));
+  ++E.nlaunch, k_apply_merges<<<grid_for(ns), 256, 0, st>>>(single, ns, S.cand_to.p,
+                                                            S.cand_gain.p, s, cnt + 9);
+  HL_LAUNCH_CHECK();
+  stats_acc_u32(E, cnt + 9, 9);  // merges, read when the call ends
+}
+
+// From the split on: singletons, T-filter, merges.
+static void refine_merge(Engine& E, Level& L, RefineOut& out) {
+  Scratch& S = E.sc;
+  cudaStream_t st = E.stream;
+  const u32 n = L.g.n;
+  u32* cnt = S.cnt.p;
+  u32* s = L.s_cur.p;
   // ---- 2. sub-community sizes ------------------------------------------------
-  u32 smax2 = m_new ? smax + m_new : smax;
-  const size_t s2cap = (size_t)smax2 + 1;
+  const size_t s2cap = (size_t)E.new_base + E.n_new;
   S.sizes.ensure(E.mem, s2cap);
   HL_CUDA(cudaMemsetAsync(S.sizes.p, 0, sizeof(u32) * s2cap, st));
   ++E.nlaunch, k_sizes<<<grid_for(n), 256, 0, st>>>(n, s, S.sizes.p);
@@ -507,7 +523,7 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
   // ---- 3. refined singletons ---------------------------------------------
   u32 nr = select_flagged(E, S.refined.p, n, S.act.p, cnt + 6);
   out.refined = nr;
-  if (!nr) return out;
+  if (!nr) return;
   if (E.cfg.mode == HL_MODE_DETERMINISTIC) {
     // sequential merges in (k, node) order with the live T-filter
     // (hit_leiden.rs:1392-1548)
@@ -517,7 +533,7 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
     S.dcomm.ensure(E.mem, fcap);
     recompute_comm_degrees(E, L, L.f.p, (u32)fcap, S.dcomm.p);
     out.merges = merge_singletons_det(E, L, S.act.p, nr, S.sizes.p, S.dS.p, S.dcomm.p, s2cap);
-    return out;
+    return;
   }
   S.nmask.ensure(E.mem, nr);
   ++E.nlaunch, k_singletons<<<grid_for(nr), 256, 0, st>>>(S.act.p, nr, s, S.sizes.p, S.nmask.p);
@@ -531,7 +547,7 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
     });
     ns = E.read_u32(cnt + 7);
   }
-  if (!ns) return out;
+  if (!ns) return;
   u32* single = S.cand_idx.p;
   // d_S and d_C serve only the T-filter and the singleton merges below
   S.dS.ensure(E.mem, s2cap);
@@ -619,15 +635,31 @@ RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
   E.kt_end(KT_TFILTER, ev_tf);
 
   // ---- 5. Jacobi singleton merge -------------------------------------------
-  S.cand_to.ensure(E.mem, ns);
-  S.cand_gain.ensure(E.mem, ns);
-  run_eval(E, 1, single, ns, L, s, S.dS.p, S.blocked.p, false, S.cand_to.p, S.cand_gain.p,
-           nullptr);
-  HL_CUDA(cudaMemsetAsync(cnt + 9, 0, sizeof(u32), st));
-  ++E.nlaunch, k_apply_merges<<<grid_for(ns), 256, 0, st>>>(single, ns, S.cand_to.p, S.cand_gain.p, s,
-                                               cnt + 9);
-  HL_LAUNCH_CHECK();
-  stats_acc_u32(E, cnt + 9, 9);  // merges, read when the call ends
+  merge_singletons(E, L, single, ns);
+}
+
+RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community) {
+  RefineOut out;
+  Scratch& S = E.sc;
+  const u32 n = L.g.n;
+  E.n_new = 0;
+  E.new_base = 0;
+  S.refined.ensure(E.mem, (((size_t)n + 3) & ~(size_t)3) + 4);
+  if (!n) return out;
+  S.cnt.ensure(E.mem, 16);
+  if (!L.s_bound) L.s_bound = reduce_max_u32(E, L.s_cur.p, n, S.cnt.p + 12) + 1;
+  if (gang_refine_fits(E, L)) {
+    switch (gang_refine(E, L, cc_same_community, out)) {
+      case REF_DONE: return out;
+      case REF_HOST_EVAL:
+        merge_singletons(E, L, S.cand_idx.p, out.singles);
+        return out;
+      case REF_HOST_MERGE: refine_merge(E, L, out); return out;
+      default: break;
+    }
+  }
+  refine_cc(E, L, cc_same_community, out);
+  refine_merge(E, L, out);
   return out;
 }
 

@@ -67,3 +67,51 @@ def test_apply_delta_shapes(shape, k, integral):
         got = gh.apply_delta(g, ds, dd, dw, keep_loops=True)
         for a, b in zip(got, ref.csr()):
             assert gh.same_bits(a, b)
+
+
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("share", [0.02, 1.0])
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_inc_refinement_shapes(shape, share, integral):
+    # sub-communities of 1 to a few hundred vertices inside 40 communities: rows
+    # cut into slices (the hub), splits, singletons with and without candidates,
+    # singletons above and below the warp table's 256 entries
+    g = _base(shape, integral)
+    rng = np.random.default_rng(len(shape))
+    f = gh.random_partition(rng, g.n, 40)
+    aff = rng.random(g.n) < share
+    for subs in (3, max(4, g.n // 400), g.n // 3):
+        s0 = (f.astype(np.int64) * subs + rng.integers(0, subs, g.n)) % (g.n + 5)
+        s0 = np.where(rng.random(g.n) < 0.7, f * np.uint32(subs), s0).astype(np.uint32) % g.n
+        for same_f in (False, True):
+            ref_s, ref_r = O.inc_refinement(g, f, s0.copy(), aff, 1.0, O.MODE_THROUGHPUT,
+                                            cc_same_community=same_f)
+            got_s, got_r = gh.inc_refinement(g, f, s0, aff, 1.0, same_f)
+            assert np.array_equal(ref_s, got_s) and np.array_equal(ref_r, got_r)
+
+
+# 40000 updates: the batch, and more than 65536 aggregation records, take the
+# multi-kernel path on the lower levels
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("shape,ks", [("block", (1, 40, 400)), ("cluster", (3, 700, 9000)),
+                                      ("grid", (50, 5000, 40000))])
+def test_levels_match_oracle(shape, ks, integral):
+    from tests.test_gpu_e2e import compare, oracle_state
+
+    import importlib
+    hl = importlib.import_module("hit-leiden_b200")
+    g = _base(shape, integral)
+    off, col, w = g.csr()
+    src = np.repeat(np.arange(g.n, dtype=np.uint32), np.diff(off).astype(np.int64))
+    once = src < col
+    edges = src[once], col[once], w[once]
+    gs = hl.PartitionState.load(hl.GraphInput.from_arrays(shape, g.n, *edges),
+                                hl.RunConfig(mode=hl.RunMode.Throughput))
+    ref = oracle_state(g.n, *edges, 10)
+    compare(gs, ref)
+    for i, k in enumerate(ks):
+        ds, dd, dw = _batch(g, k, integral, 77 + i)
+        gs.apply_batch(ds, dd, dw)
+        ref.hit_leiden(ds, dd, dw)
+        compare(gs, ref)
+    gs.close()
