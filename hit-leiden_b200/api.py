@@ -57,7 +57,7 @@ class RunConfig:
     batch_modularity: bool = False
     kernel_timing: bool = False
     autotune: bool = True        # degree-bin autotuner (HL_FLAG_NO_AUTOTUNE when off)
-    small_rounds: bool = True    # one-block rounds for small frontiers (HL_FLAG_NO_SMALL_ROUNDS)
+    small_rounds: bool = True    # one-launch rounds for small frontiers (HL_FLAG_NO_SMALL_ROUNDS)
 
     def validate(self) -> None:
         if self.max_iterations == 0:

@@ -669,7 +669,7 @@ static const char* kernel_names[KT_COUNT] = {
     "apply_and_mark",
     "refine_cc",   "t_filter",    "row_sums",         "delta_resolve",  "stage_apply",
     "stage_move",  "stage_refine", "stage_aggregate", "host_syncs",
-    "apply_one_launch", "move_small_rounds", "eval_huge_partitioned",
+    "apply_one_launch", "move_one_launch", "eval_huge_partitioned",
     "refine_one_launch", "aggregate_one_launch"};
 
 hl_status hl_kernel_stats(const hl_graph* g, hl_kernel_stat* out, uint32_t cap, uint32_t* count) {

@@ -111,14 +111,15 @@ struct Scratch {
   // [8] accepted moves, [9] refinement merges, [10] |B^1|
   DBuf<u64> bacc;
   DBuf<u8> kflag;     // K marks for the next level (M8), level-size bytes
-  // movement rounds of a small frontier (small.cu)
+  // movement in one launch (gang_move.cu): frontier lists
   DBuf<u32> sm_list_a, sm_list_b;
-  DBuf<u64> sm_out;
   // per-level output: the level's s_cur before the batch, the changed nodes
   DBuf<u32> lvl_prev, lvl_nodes, lvl_ids;
   DBuf<u8> lvl_flag;
   // single-launch stages (gang.cuh)
-  DBuf<u32> gang_part, gang_cnt, ga_touched, gr_bits;
+  DBuf<u32> gang_part, gang_cnt, ga_touched, gr_bits, gm_bits, gm_hist;
+  DBuf<unsigned short> gm_slot;
+  DBuf<double> gm_w;
   DBuf<u64> gr_items;
 };
 
@@ -152,7 +153,7 @@ enum KernelId : int {
   KT_STAGE_AGGREGATE,
   KT_HOST_SYNC,    // host waits on the stream (launches = count; no time)
   KT_GANG_APPLY,   // whole delta applications in one launch (gang_apply.cu)
-  KT_MOVE_SMALL,   // movement rounds of a small frontier in one block (small.cu)
+  KT_GANG_MOVE,    // movement rounds of small frontiers in one launch (gang_move.cu)
   KT_EVAL_PB,      // the partitioned pass of the block bin (inside KT_EVAL_HUGE)
   KT_GANG_REFINE,  // whole refinements in one launch (gang_refine.cu)
   KT_GANG_AGG,     // whole aggregations in one launch (gang_aggregate.cu)
@@ -274,11 +275,16 @@ void stats_acc_u64(Engine& E, const unsigned long long* src, u32 count, u32 slot
 void stats_acc_u32(Engine& E, const u32* src, u32 slot);
 void stats_count_flags(Engine& E, const u8* flags, u32 n, u32 slot);
 
-// small.cu: movement rounds of a small frontier in one block.  Returns true
-// when the movement stage is finished, false when the host rounds continue
-// from S.active (*big_degree: an active vertex exceeds the block's tables).
-bool move_rounds_small(Engine& E, Level& L, bool mark_moved, u32& it, u64& moves, u64& cands,
-                       u64& trav, u64& sum_nv, bool* big_degree);
+// gang_move.cu: the movement in one launch; the status says why the host's
+// rounds go on from S.active
+enum : u32 { MOVE_DONE = 0, MOVE_BIG_FRONTIER = 1, MOVE_BIG_HUB = 2, MOVE_LABELS = 3 };
+struct GangMoveStats {
+  u64 moves = 0, cands = 0, trav = 0;
+};
+constexpr u32 GM_FRONTIER = 32768;  // frontier (and candidate) limit
+bool gang_move_fits(Engine& E, const Level& L);
+u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_active,
+              bool mark_moved, u32 frontier, u32& it, GangMoveStats& ms);
 
 // eval.cu: degree-bin autotuner (once per handle)
 void autotune_bins(Engine& E, const u32* verts, u32 nv, const Level& L, const u32* s,

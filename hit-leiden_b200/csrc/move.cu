@@ -12,6 +12,7 @@
 //      every endpoint community whose role is still open;
 //   4. accepted moves are applied, d(C) updated in selected order, and the
 //      next frontier / K set marked.
+#include <algorithm>
 #include <cstring>
 
 #include "hl_engine.cuh"
@@ -526,30 +527,53 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   Scratch& S = E.sc;
   cudaStream_t st = E.stream;
   const u32 n = L.g.n;
-  // flag arrays padded to whole 32-bit words (small.cu marks them by word)
+  // flag arrays padded to whole 32-bit words (gang_move.cu clears them by word)
   const size_t nflag = (((size_t)n + 3) & ~(size_t)3) ? (((size_t)n + 3) & ~(size_t)3) : 4;
   S.active.ensure(E.mem, nflag);
   S.next.ensure(E.mem, nflag);
-  S.changed.ensure(E.mem, n ? n : 1);
-  S.affected.ensure(E.mem, n ? n : 1);
-  HL_CUDA(cudaMemsetAsync(S.active.p, all_active ? 1 : 0, n ? n : 1, st));
-  HL_CUDA(cudaMemsetAsync(S.changed.p, 0, n ? n : 1, st));
-  HL_CUDA(cudaMemsetAsync(S.affected.p, 0, n ? n : 1, st));
-  if (!n) return out;
-  if (delta.k)
-    ++E.nlaunch, k_seed<<<grid_for(delta.k), 256, 0, st>>>(delta.u, delta.v, delta.w, delta.k, L.f.p,
-                                               L.s_cur.p, S.active.p, S.affected.p);
-  HL_LAUNCH_CHECK();
-  if (E.k_flags_set) {  // M8: K marks handed up from the level below
-    ++E.nlaunch, k_or_flags<<<grid_for(n), 256, 0, st>>>(S.kflag.p, n, S.affected.p);
-    HL_LAUNCH_CHECK();
-    E.k_flags_set = false;
-  }
-  // Community ids must stay below n so that n + v is a fresh empty community.
-  compact_labels_if_needed(E, L.f.p, n, n);
+  S.changed.ensure(E.mem, nflag);
+  S.affected.ensure(E.mem, nflag);
   const size_t ncap = 2 * (size_t)n + 2;
-  ensure_comm_arrays(E, ncap);
-  recompute_comm_degrees(E, L, L.f.p, (u32)ncap, S.d.p);
+  u32 it = 0;
+  GangMoveStats gm;
+  bool gang_on = gang_move_fits(E, L);
+  if (gang_on) {
+    S.cnt.ensure(E.mem, 16);
+    const u32 fr = all_active ? n : (u32)std::min<u64>(n, 2 * delta.k);
+    u32 why = gang_move(E, L, delta, true, all_active, mark_moved, fr, it, gm);
+    if (why == MOVE_LABELS) {
+      // Community ids must stay below n so that n + v is a fresh empty community.
+      compact_labels_if_needed(E, L.f.p, n, n);
+      why = gang_move(E, L, delta, true, all_active, mark_moved, fr, it, gm);
+    }
+    if (why == MOVE_DONE) {
+      out.iterations = it;
+      out.moves = gm.moves;
+      out.candidates = gm.cands;
+      out.traversed = gm.trav;
+      return out;
+    }
+    if (why == MOVE_BIG_HUB) gang_on = false;
+  } else {
+    HL_CUDA(cudaMemsetAsync(S.active.p, all_active ? 1 : 0, n ? n : 1, st));
+    HL_CUDA(cudaMemsetAsync(S.changed.p, 0, n ? n : 1, st));
+    HL_CUDA(cudaMemsetAsync(S.affected.p, 0, n ? n : 1, st));
+    if (!n) return out;
+    if (delta.k)
+      ++E.nlaunch, k_seed<<<grid_for(delta.k), 256, 0, st>>>(delta.u, delta.v, delta.w, delta.k,
+                                                             L.f.p, L.s_cur.p, S.active.p,
+                                                             S.affected.p);
+    HL_LAUNCH_CHECK();
+    if (E.k_flags_set) {  // M8: K marks handed up from the level below
+      ++E.nlaunch, k_or_flags<<<grid_for(n), 256, 0, st>>>(S.kflag.p, n, S.affected.p);
+      HL_LAUNCH_CHECK();
+      E.k_flags_set = false;
+    }
+    // Community ids must stay below n so that n + v is a fresh empty community.
+    compact_labels_if_needed(E, L.f.p, n, n);
+    ensure_comm_arrays(E, ncap);
+    recompute_comm_degrees(E, L, L.f.p, (u32)ncap, S.d.p);
+  }
   if (E.cfg.mode == HL_MODE_DETERMINISTIC) {
     // sequential Gauss–Seidel (hit_leiden.rs:1103-1191): one iteration
     inc_movement_det(E, L, S.d.p, ncap, mark_moved, &out.moves, &out.traversed);
@@ -578,20 +602,16 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   u32* cnt = S.cnt.p;
 
   const u32 max_rounds = E.cfg.max_rounds ? E.cfg.max_rounds : 20;
-  u32 it = 0;
   S.acc_cnt.ensure(E.mem, 1);
   HL_CUDA(cudaMemsetAsync(S.acc_cnt.p, 0, sizeof(u32), st));  // accepted moves, all rounds
-  // Small frontiers run whole rounds in one block (small.cu); the host
-  // rounds below take over while the frontier is large or a hub is active.
-  u64 sm_moves = 0, sm_cands = 0, sm_trav = 0, sm_nv = 0;
-  bool small_on = !(E.cfg.flags & HL_FLAG_NO_SMALL_ROUNDS);
-  u32 last_na = 0;
+  // Small frontiers run whole rounds in one launch (gang_move.cu); the host
+  // rounds take over while the frontier is large or a hub outgrows its tables.
+  u32 last_na = NONE32;
   while (it < max_rounds) {
-    if (small_on && last_na <= 16384) {
-      bool big = false;
-      if (move_rounds_small(E, L, mark_moved, it, sm_moves, sm_cands, sm_trav, sm_nv, &big))
-        break;
-      if (big) small_on = false;
+    if (gang_on && last_na <= GM_FRONTIER) {
+      const u32 why = gang_move(E, L, DevEdges{}, false, false, mark_moved, last_na, it, gm);
+      if (why == MOVE_DONE) break;
+      if (why == MOVE_BIG_HUB) gang_on = false;
       if (it >= max_rounds) break;
     }
     // Active list, ascending (iter_ones order).
@@ -699,9 +719,9 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   stats_acc_u64(E, reinterpret_cast<const unsigned long long*>(S.red64.p), 8, 0);
   stats_acc_u32(E, S.acc_cnt.p, 8);
   E.sum_nv_batch += sum_nv;
-  out.moves += sm_moves;
-  out.candidates += sm_cands;
-  out.traversed += sm_trav;
+  out.moves += gm.moves;
+  out.candidates += gm.cands;
+  out.traversed += gm.trav;
   return out;
 }
 

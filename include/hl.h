@@ -92,9 +92,10 @@ typedef struct {
  * pair for the handle (hl_autotune_info). */
 #define HL_FLAG_NO_AUTOTUNE (1u << 3)
 /* Keep every throughput movement round on the multi-kernel path.  By default
- * rounds whose frontier has at most 4096 vertices of at most 256 entries each
- * (levels of up to 2^18 nodes) run whole inside one block, without host round
- * trips between them; the results are identical either way. */
+ * rounds whose frontier has at most 32768 vertices run whole inside one
+ * launch, without host round trips between them, while hub rows have at most
+ * 16384 entries and 2048 distinct neighbour communities; the results are
+ * identical either way. */
 #define HL_FLAG_NO_SMALL_ROUNDS (1u << 4)
 
 typedef struct {

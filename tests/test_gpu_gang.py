@@ -115,3 +115,27 @@ def test_levels_match_oracle(shape, ks, integral):
         ref.hit_leiden(ds, dd, dw)
         compare(gs, ref)
     gs.close()
+
+
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("labels", ["few", "many", "high"])
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_inc_movement_shapes(shape, labels, integral):
+    # few: the hub's row holds 40 keys, long chains; many: more than 2048 keys,
+    # so the round goes to the multi-kernel path; high: ids of n and above are
+    # compacted first.  From a batch, and from all vertices (60,000 of them
+    # outgrow the frontier lists).
+    g = _base(shape, integral)
+    rng = np.random.default_rng(len(labels))
+    f = gh.random_partition(rng, g.n, 40 if labels == "few" else g.n // 2)
+    if labels == "high":
+        f = (f + np.uint32(g.n // 2 + 3)).astype(np.uint32)
+    s = gh.random_partition(rng, g.n, g.n // 3)
+    for k in (0, min(2000, g.n // 4)):
+        ds, dd, dw = _batch(g, k, integral, 5) if k else ([], [], [])
+        for rounds in ((1, 20) if shape == "block" else (2,)):
+            ref = O.inc_movement(g, ds, dd, dw, f.copy(), s, 1.0, O.MODE_THROUGHPUT,
+                                 max_rounds=rounds)
+            got = gh.inc_movement(g, ds, dd, dw, f, s, 1.0, max_rounds=rounds)
+            assert np.array_equal(ref[0], got[0])
+            assert np.array_equal(ref[1], got[1]) and np.array_equal(ref[2], got[2])
