@@ -533,7 +533,9 @@ static void finish_stats(EngineBox& B, hl_batch_stats* stats) {
   // offsets, f, k, d(f) and outputs; per adjacency entry the neighbour,
   // weight and neighbour community; per evaluated candidate its d(C).
   E.kagg[KT_MOVE_EVAL].bytes += 52ull * E.sum_nv_batch + 16ull * trav + 8ull * ncand;
-  E.st.traversed += trav;
+  // the rows of vertices a bound ruled out count as traversed (they are, in the
+  // reference) but move no bytes
+  E.st.traversed += trav + acc[11];
   E.st.moves += acc[8];
   E.st.merges += acc[9];
   E.st.changed = acc[10];

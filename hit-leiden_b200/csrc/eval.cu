@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "hl_engine.cuh"
+#include "prune.cuh"
 
 namespace hl {
 
@@ -66,6 +67,7 @@ struct EvalArgs {
   u32* work;            // block kernel: next idx position to take (zeroed per launch)
   u64 defer_deg;        // block kernel pass 1: rows longer than this go to the
                         // partitioned pass unread (0: none)
+  Prune prune;          // movement bounds (kernels of longer rows)
 };
 
 constexpr u32 MID_MAX = 128;
@@ -147,7 +149,11 @@ __device__ __forceinline__ void finish(const EvalArgs& A, u32 i, u32 v, u32 cur,
     to = best_key;
   }
   if (KIND == EVAL_MOVE && A.allow_empty && A.tw != 0.0) {
-    double eg = empty_gain(wcur, A.tw, A.gamma, kv, A.d[cur]);
+    const double dcur = A.d[cur];
+    double eg = empty_gain(wcur, A.tw, A.gamma, kv, dcur);
+    if (A.prune.b)
+      prune_store(A.prune, *A.prune.shift, v, has_best && best_g > eg ? best_g : eg, kv, dcur,
+                  A.tw, A.gamma);
     if (eg > g) {
       g = eg;
       to = A.n + v;
@@ -1467,12 +1473,17 @@ __global__ void k_pb_final(EvalArgs A, PbArgs P, u32* fail_list, u32* fail_count
 // Host side: bin the list by degree and launch the three kernels.
 // ---------------------------------------------------------------------------
 // Bins: 0-2 sub-warp (deg <= 8, 16, 32), 3 warp table (<= mid_max), 4 wide
-// (<= WIDE_SPLIT), 6 wide (<= wide_max) with full-size tables, 5 block.
-constexpr int NBINS = 7;
+// (<= WIDE_SPLIT), 6 wide (<= wide_max) with full-size tables, 5 block, 7 ruled
+// out by their bounds (prune.cuh).
+constexpr int NBINS = 8;
 
 __global__ void k_bin(const u32* verts, u32 nv, const u64* off, u32* bin, u32* idx,
-                      u32* counts, unsigned long long* maxdeg, u32 mid_max, u32 wide_max) {
+                      u32* counts, unsigned long long* maxdeg, u32 mid_max, u32 wide_max,
+                      Prune prune, const u32* f, const double* d, const double* kdeg, double tw,
+                      double gamma, u32* out_to, double* out_gain,
+                      unsigned long long* pruned_entries) {
   __shared__ u32 sc[NBINS];
+  unsigned long long pruned = 0;
   if (threadIdx.x < NBINS) sc[threadIdx.x] = 0;
   __syncthreads();
   for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < nv; i += (u64)gridDim.x * blockDim.x) {
@@ -1480,6 +1491,15 @@ __global__ void k_bin(const u32* verts, u32 nv, const u64* off, u32* bin, u32* i
     u64 deg = off[v + 1] - off[v];
     u32 b = deg <= 8 ? 0 : deg <= 16 ? 1 : deg <= 32 ? 2 : deg <= mid_max ? 3
           : deg <= wide_max ? (deg <= WIDE_SPLIT ? 4 : 6) : 5;
+    if (deg > PRUNE_MIN_DEG && prune_valid(prune, v)) {
+      const u32 c = f[v];
+      if (prune_rules_out(prune, *prune.shift, v, kdeg[v], d[c], tw, gamma)) {
+        b = 7;
+        out_to[i] = c;
+        out_gain[i] = 0.0;
+        pruned += deg;
+      }
+    }
     bin[i] = b;
     idx[i] = (u32)i;
     atomicAdd(&sc[b], 1u);
@@ -1487,6 +1507,8 @@ __global__ void k_bin(const u32* verts, u32 nv, const u64* off, u32* bin, u32* i
   }
   __syncthreads();
   if (threadIdx.x < NBINS && sc[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sc[threadIdx.x]);
+  for (int o = 16; o; o >>= 1) pruned += __shfl_xor_sync(0xffffffffu, pruned, o);
+  if ((threadIdx.x & 31) == 0 && pruned && pruned_entries) atomicAdd(pruned_entries, pruned);
 }
 
 // Sort keys that order vertices by degree, largest first.
@@ -1711,8 +1733,11 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   // compile-time table sizes: mid <= MID_MAX, wide <= WIDE_MAX)
   const u32 mid_max = E.tune.mid_max ? E.tune.mid_max : MID_MAX;
   const u32 wide_max = E.tune.wide_max ? E.tune.wide_max : WIDE_MAX;
+  const Prune prune = kind == EVAL_MOVE ? E.prune : Prune{};
   ++E.nlaunch, k_bin<<<grid_for(nv), 256, 0, st>>>(verts, nv, L.g.off.p, S.used.p, S.order.p, cnt,
-                                                    maxdeg, mid_max, wide_max);
+                                                    maxdeg, mid_max, wide_max, prune, L.f.p, d,
+                                                    L.k.p, L.tw, E.cfg.resolution, out_to,
+                                                    out_gain, counters ? counters + 8 : nullptr);
   HL_LAUNCH_CHECK();
   u32* ki = S.used.p;
   u32* ko = S.rank.p;
@@ -1728,6 +1753,10 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   E.sync();
   std::memcpy(c, E.hs.p, sizeof(c));
   const u64 big_maxdeg = E.hs.p[4];
+  // bounds that rule out few of the rows they could are not worth keeping up
+  // (R-MAT: every round moves neighbours of every hub)
+  if (prune.b && ++E.prune_rounds > 3 && (u64)c[7] * 8 < (u64)c[4] + c[5] + c[6])
+    E.prune = Prune{};
   u32 start[NBINS + 1] = {0};
   for (int b = 0; b < NBINS; ++b) start[b + 1] = start[b] + c[b];
 
@@ -1832,6 +1861,7 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   if (c[4]) {
     EvalArgs a = A;
     a.counters = counters ? counters + 4 : nullptr;
+    a.prune = prune;
     a.idx = vo + start[4];
     a.nidx = c[4];
     u32 blocks = grid_for((u64)c[4] * 32, WIDE_WARPS * 32);
@@ -1846,6 +1876,7 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   if (c[6]) {
     EvalArgs a = A;
     a.counters = counters ? counters + 4 : nullptr;
+    a.prune = prune;
     a.idx = vo + start[6];
     a.nidx = c[6];
     u32 blocks = grid_for((u64)c[6] * 32, WIDE_WARPS * 32);
@@ -1864,6 +1895,7 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
     // are deferred to an overflow list.
     EvalArgs a = A;
     a.counters = counters ? counters + 6 : nullptr;
+    a.prune = prune;
     // the bin's list by degree, largest first
     S.hubk.ensure(E.mem, c[5]);
     S.hubk2.ensure(E.mem, c[5]);
@@ -1966,6 +1998,8 @@ void autotune_bins(Engine& E, const u32* verts, u32 nv, const Level& L, const u3
   HL_CUDA(cudaEventCreate(&a));
   HL_CUDA(cudaEventCreate(&b));
   const bool kt = E.ktiming;
+  const Prune prune = E.prune;
+  E.prune = Prune{};  // every trial evaluates the whole frontier
   E.ktiming = false;  // the trial runs stay out of the kernel statistics
   float best = 0.f;
   u32 bm = MID_MAX, bw = WIDE_MAX;
@@ -2009,6 +2043,7 @@ void autotune_bins(Engine& E, const u32* verts, u32 nv, const Level& L, const u3
     best = bdt;
   }
   E.ktiming = kt;
+  E.prune = prune;
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   E.tune.hub_defer = bd;

@@ -335,8 +335,8 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
     gang_launch(E, fn, shape, 0, &A);
     result();
     if (o.nops) {
-      Gr.col2.ensure(E.mem, o.nnz_new ? o.nnz_new : 1);
-      Gr.w2.ensure(E.mem, o.nnz_new ? o.nnz_new : 1);
+      Gr.col2.ensure_slack(E.mem, o.nnz_new ? o.nnz_new : 1);
+      Gr.w2.ensure_slack(E.mem, o.nnz_new ? o.nnz_new : 1);
     }
     A.structure_only = false;
     A.finish_only = true;

@@ -12,6 +12,7 @@
 #include "csr_rebuild.cuh"
 #include "gang.cuh"
 #include "hub_sums.cuh"
+#include "prune.cuh"
 
 namespace hl {
 
@@ -24,19 +25,19 @@ enum : u32 { GM_EMIT = 1, GM_ACC = 2 };
 enum : u32 { GM_UNDECIDED = 0, GM_ACCEPTED = 1, GM_REJECTED = 2 };
 
 struct MoveRound {  // of one parity; the other one's is cleared meanwhile
-  u32 nv, nh, ncand, nops, nitems, work, hwork, big;
+  u32 nv, nh, ncand, nops, nitems, work, hwork, big, wv, wh;
 };
 
 struct MoveCnt {  // zeroed by the host
   MoveRound r[2];
   u32 maxlab, und[2], pad_;
-  unsigned long long moves, cands, trav, nfront;
+  unsigned long long moves, cands, trav, nfront, pruned;
 };
 
 struct MoveOutDev {
   u32 status, it, round, pad_;
   u64 epoch;
-  unsigned long long moves, cands, trav, nfront;
+  unsigned long long moves, cands, trav, nfront, pruned;
 };
 
 struct WarpTabs {
@@ -74,6 +75,8 @@ struct GangMoveArgs {
   u32* verts[2];     // frontier: rows of up to GM_MAXDEG entries
   u32* hubs[2];      // ... and longer ones
   u32 list_cap;
+  u32 *wverts, *whubs;  // those of them that need an evaluation
+  Prune prune;
   u32* to;           // per vertex: its candidate's target
   u64* ckey;
   u32* cnode;
@@ -121,7 +124,7 @@ __device__ __forceinline__ void gm_activate(const GangMoveArgs& A, u32 b, u32 v)
 // listed.
 __device__ __forceinline__ void gm_finish(const GangMoveArgs& A, MoveRound& R, u32 v, u32 cur,
                                           double kv, double wcur, double dcur, double g, u32 p,
-                                          u32 kk) {
+                                          u32 kk, bool bound, double shift) {
   u32 to = cur;
   double gain = 0.0;
   if (p != NONE32 && g > 0.0) {
@@ -130,6 +133,8 @@ __device__ __forceinline__ void gm_finish(const GangMoveArgs& A, MoveRound& R, u
   }
   if (A.tw != 0.0) {
     const double eg = empty_gain(wcur, A.tw, A.gamma, kv, dcur);
+    if (bound && A.prune.b)
+      prune_store(A.prune, shift, v, p != NONE32 && g > eg ? g : eg, kv, dcur, A.tw, A.gamma);
     if (eg > gain) {
       gain = eg;
       to = A.n + v;
@@ -146,7 +151,7 @@ __device__ __forceinline__ void gm_finish(const GangMoveArgs& A, MoveRound& R, u
 // Best move of v by one warp: up to 256 entries loaded together, their labels
 // gathered together, then folded in CSR order into the warp's table.
 __device__ __forceinline__ void gm_eval(const GangMoveArgs& A, WarpTabs& W, MoveRound& R, u32 v,
-                                        unsigned long long& trav) {
+                                        double shift, unsigned long long& trav) {
   const u32 lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   u32* tk = W.tk[wib];
   u32* tp = W.tp[wib];
@@ -246,7 +251,8 @@ __device__ __forceinline__ void gm_eval(const GangMoveArgs& A, WarpTabs& W, Move
       kk = ok;
     }
   }
-  if (lane == 0) gm_finish(A, R, v, cur, kv, wcur, dcur, g, p, kk);
+  if (lane == 0)
+    gm_finish(A, R, v, cur, kv, wcur, dcur, g, p, kk, deg > PRUNE_MIN_DEG, shift);
   __syncwarp();
 }
 
@@ -266,7 +272,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
   const u32 gt = G.thread(), gts = G.threads();
   MoveCnt& C = *A.cnt;
   const u32 words = (A.n + 31) / 32;
-  unsigned long long trav = 0, trav_round = 0;
+  unsigned long long trav = 0, trav_round = 0, pruned = 0;
   u32 b = 0;  // parity of the current frontier
   // ---- clear; the largest label ----
   for (u32 i = gt; i < words; i += gts) A.bits[0][i] = A.bits[1][i] = 0;
@@ -280,6 +286,14 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0 && mx) atomicMax(&C.maxlab, mx);
     for (u64 c = gt; c < A.dcap; c += gts) A.d[c] = 0.0;
+    if (A.prune.b) {
+      for (u32 i = gt; i < words; i += gts) A.prune.valid[i] = 0;
+      for (u64 c = gt; c < A.dcap; c += gts) A.prune.drop[c] = 0.0;
+      if (gt == 0) {
+        *A.prune.shift = 0.0;
+        *A.prune.worst = 0;
+      }
+    }
   }
   G.sync();
   if (A.setup) {
@@ -353,9 +367,17 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
   u32 it = A.it0, round = A.round0;
   u64 epoch = A.epoch0;
   u32 status = MOVE_DONE;
+  u32 m_last = 0;  // candidates of the round before
   while (true) {
     MoveRound& R = C.r[b];
     const u32 nv = R.nv, nh = R.nh;
+    double shift = 0.0;
+    if (A.prune.b) {
+      shift = *A.prune.shift + prune_worst_now(A.prune);
+      for (u32 r = gt; r < m_last; r += gts)
+        if (A.status[r] == GM_ACCEPTED) A.prune.drop[A.sel_from[r]] = 0.0;
+      m_last = 0;
+    }
     if (it >= A.max_rounds || nv + nh == 0) break;
     if (nv > A.list_cap || nh > A.list_cap || nv + nh > A.list_cap) {
       status = MOVE_BIG_FRONTIER;
@@ -364,16 +386,39 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     // ---- best moves on the snapshot: hubs by block, the rest by warp ----
     if (gt == 0) {
       MoveRound& N = C.r[b ^ 1];
-      N.nv = N.nh = N.ncand = N.nops = N.nitems = N.work = N.hwork = N.big = 0;
+      N.nv = N.nh = N.ncand = N.nops = N.nitems = N.work = N.hwork = N.big = N.wv = N.wh = 0;
     }
-    if (nh) {
+    const u32 *verts = A.verts[b], *hubs = A.hubs[b];
+    u32 ev = nv, eh = nh;  // vertices to evaluate
+    unsigned long long pruned_round = 0;
+    if (A.prune.b && it > 0) {
+      // rows of earlier rounds hold bounds: most need no evaluation
+      for (u32 i = gt; i < nv + nh; i += gts) {
+        const bool hub = i >= nv;
+        const u32 v = hub ? hubs[i - nv] : verts[i];
+        if (prune_valid(A.prune, v) &&
+            prune_rules_out(A.prune, shift, v, A.k[v], A.d[A.f[v]], A.tw, A.gamma)) {
+          pruned_round += A.off[v + 1] - A.off[v];
+        } else if (hub) {
+          A.whubs[atomicAdd(&R.wh, 1u)] = v;
+        } else {
+          A.wverts[atomicAdd(&R.wv, 1u)] = v;
+        }
+      }
+      G.sync();
+      ev = R.wv;
+      eh = R.wh;
+      verts = A.wverts;
+      hubs = A.whubs;
+    }
+    if (eh) {
       for (;;) {
         __syncthreads();
         if (tid == 0) s_next = atomicAdd(&R.hwork, 1u);
         __syncthreads();
         const u32 i = s_next;
-        if (i >= nh) break;
-        const u32 v = A.hubs[b][i];
+        if (i >= eh) break;
+        const u32 v = hubs[i];
         const u64 o0 = A.off[v], o1 = A.off[v + 1];
         const u32 cur = A.f[v];
         if (o1 - o0 > HUB_MAXDEG ||
@@ -392,13 +437,13 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
                              p, kk);
         if (tid == 0) {
           trav_round += o1 - o0;
-          gm_finish(A, R, v, cur, kv, M.h.wcur, dcur, g, p, kk);
+          gm_finish(A, R, v, cur, kv, M.h.wcur, dcur, g, p, kk, true, shift);
         }
       }
       __syncthreads();
     }
-    for (u32 i = G.warp(); i < nv;) {
-      gm_eval(A, M.w, R, A.verts[b][i], trav_round);
+    for (u32 i = G.warp(); i < ev;) {
+      gm_eval(A, M.w, R, verts[i], shift, trav_round);
       if (lane == 0) i = G.warps() + atomicAdd(&R.work, 1u);
       i = __shfl_sync(0xffffffffu, i, 0);
     }
@@ -408,12 +453,13 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       break;
     }
     trav += trav_round;
+    pruned += pruned_round;
     trav_round = 0;
     const u32 m = R.ncand;
     ++it;
     if (gt == 0) {
       C.cands += m;
-      C.nfront += nv + nh;
+      C.nfront += ev + eh;
     }
     if (m == 0) {
       b ^= 1;  // nothing selected: the next frontier is empty
@@ -495,9 +541,15 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       }
     }
     // ---- the accepted moves (throughput.rs:182-187) ----
+    if (gt == 0 && A.prune.b) {
+      *A.prune.shift = shift;
+      *A.prune.worst = 0;
+    }
+    m_last = m;
     for (u32 r = gt; r < m; r += gts) {
       if (A.status[r] != GM_ACCEPTED) continue;
       const u32 v = A.sel_node[r], from = A.sel_from[r], to = A.sel_to[r];
+      prune_moved(A.prune, v, from, A.k[v]);
       A.f[v] = to;
       A.changed[v] = 1;
       if (A.mark_moved) A.affected[v] = 1;
@@ -545,6 +597,8 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     for (u32 i = G.warp(); i < nitems; i += G.warps()) {
       const u64 item = A.items[i];
       const u32 v = A.sel_node[(u32)(item >> 32)], to = A.sel_to[(u32)(item >> 32)];
+      const u32 from = A.sel_from[(u32)(item >> 32)];
+      if (lane == 0 && (u32)item == 0) prune_worst(A.prune, from);
       const u64 lo = A.off[v] + (u64)(u32)item * GM_SLICE;
       const u64 hi = min(A.off[v + 1], lo + GM_SLICE);
       const u32 sv = A.s[v];
@@ -562,7 +616,11 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (nb[j] == NONE32) continue;
-          if (fn[j] != to) gm_activate(A, b ^ 1, nb[j]);
+          if (fn[j] != to) {
+            gm_activate(A, b ^ 1, nb[j]);
+            if (prune_valid(A.prune, nb[j]))
+              prune_raise(A.prune, nb[j], fn[j], from, A.w[p0 + 32 * j]);
+          }
           if (sn[j] == sv) {
             A.affected[nb[j]] = 1;
             any = true;
@@ -575,11 +633,17 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     G.sync();
   }
   for (int o = 16; o; o >>= 1) trav += __shfl_xor_sync(0xffffffffu, trav, o);
+  for (int o = 16; o; o >>= 1) pruned += __shfl_xor_sync(0xffffffffu, pruned, o);
   if (lane == 0 && trav) atomicAdd(&C.trav, trav);
+  if (lane == 0 && pruned) atomicAdd(&C.pruned, pruned);
   if (status != MOVE_DONE)  // the frontier for the host's rounds
     for (u32 v = gt; v < A.n; v += gts) A.active[v] = (A.bits[b][v >> 5] >> (v & 31)) & 1u;
   G.sync();
   if (gt == 0) {
+    if (A.prune.b) {  // for the host's rounds
+      *A.prune.shift += prune_worst_now(A.prune);
+      *A.prune.worst = 0;
+    }
     A.out->status = status;
     A.out->it = it;
     A.out->round = round;
@@ -588,6 +652,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     A.out->cands = C.cands;
     A.out->trav = C.trav;
     A.out->nfront = C.nfront;
+    A.out->pruned = C.pruned;
   }
 }
 
@@ -623,7 +688,7 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   S.affected.ensure(E.mem, nflag);
   ensure_comm_arrays(E, ncap);
   S.gm_bits.ensure(E.mem, 2 * (((size_t)n + 31) / 32));
-  S.sm_list_a.ensure(E.mem, 2 * (size_t)fr);
+  S.sm_list_a.ensure(E.mem, 4 * (size_t)fr);
   S.sm_list_b.ensure(E.mem, 2 * (size_t)fr);
   S.cand_to.ensure(E.mem, n);
   S.gkey.ensure(E.mem, fr);
@@ -672,7 +737,7 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   }
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
   S.gang_cnt.ensure(E.mem, 64);
-  static_assert(sizeof(MoveCnt) <= 32 * sizeof(u32) && sizeof(MoveOutDev) <= 32 * sizeof(u32),
+  static_assert(sizeof(MoveCnt) <= 44 * sizeof(u32) && sizeof(MoveOutDev) <= 20 * sizeof(u32),
                 "both fit the counter block");
   HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 64 * sizeof(u32), st));
   u32 round0 = E.sel_round;
@@ -707,7 +772,10 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   A.verts[1] = S.sm_list_b.p;
   A.hubs[0] = S.sm_list_a.p + fr;
   A.hubs[1] = S.sm_list_b.p + fr;
+  A.wverts = S.sm_list_a.p + 2 * (size_t)fr;
+  A.whubs = S.sm_list_a.p + 3 * (size_t)fr;
   A.list_cap = fr;
+  A.prune = E.prune;
   A.to = S.cand_to.p;
   A.ckey = S.gkey.p;
   A.cnode = S.cand_node.p;
@@ -729,7 +797,7 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   A.epoch0 = E.epoch;
   A.label_bits = (u32)bits_for(n - 1);
   A.cnt = reinterpret_cast<MoveCnt*>(S.gang_cnt.p);
-  A.out = reinterpret_cast<MoveOutDev*>(S.gang_cnt.p + 32);
+  A.out = reinterpret_cast<MoveOutDev*>(S.gang_cnt.p + 44);
   cudaEvent_t ev = E.kt_begin();
   gang_launch(E, reinterpret_cast<const void*>(&k_gang_move), shape, sizeof(MoveSmem), &A);
   E.kt_end(KT_GANG_MOVE, ev);
@@ -742,7 +810,7 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   it = o.it;
   ms.moves += o.moves;
   ms.cands += o.cands;
-  ms.trav += o.trav;
+  ms.trav += o.trav + o.pruned;  // rows ruled out count as traversed
   E.sel_round = o.round;
   E.epoch = o.epoch;
   E.kagg[KT_GANG_MOVE].bytes += 52ull * o.nfront + 16ull * o.trav + 8ull * o.cands;

@@ -594,8 +594,8 @@ void apply_delta(Engine& E, Level& L, const DevEdges& b, u32 new_n, bool keep_lo
   const u64 nnz_new = G.nnz + R - 2ull * E.read_u32(S.opdelpre.p + R);
   DBuf<u32>& ncol = G.col2;
   DBuf<double>& nw = G.w2;
-  ncol.ensure(E.mem, nnz_new ? nnz_new : 1);
-  nw.ensure(E.mem, nnz_new ? nnz_new : 1);
+  ncol.ensure_slack(E.mem, nnz_new ? nnz_new : 1);
+  nw.ensure_slack(E.mem, nnz_new ? nnz_new : 1);
   cudaEvent_t kev = E.kt_begin();
   const RowOps O{(u32)R, S.rkeys2.p, S.rvals2.p, S.opdelpre.p, S.opos.p};
   ++E.nlaunch, k_rebuild<<<grid_for(G.nnz / 8 + R + n), 256, 0, st>>>(

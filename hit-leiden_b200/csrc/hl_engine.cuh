@@ -108,9 +108,13 @@ struct Scratch {
   DBuf<u32> mark_long_cnt;
   // batch statistics accumulated on the device and read once at the end of
   // the call: [0..7] traversed / candidates of the four evaluation bins,
-  // [8] accepted moves, [9] refinement merges, [10] |B^1|
+  // [8] accepted moves, [9] refinement merges, [10] |B^1|, [11] entries of
+  // vertices whose bound ruled a move out
   DBuf<u64> bacc;
   DBuf<u8> kflag;     // K marks for the next level (M8), level-size bytes
+  // movement bounds (prune.cuh)
+  DBuf<double> pr_b, pr_shift, pr_drop;
+  DBuf<u32> pr_valid;
   // movement in one launch (gang_move.cu): frontier lists
   DBuf<u32> sm_list_a, sm_list_b;
   // per-level output: the level's s_cur before the batch, the changed nodes
@@ -160,6 +164,16 @@ enum KernelId : int {
   KT_COUNT
 };
 
+// Bounds that rule a move out without reading the row (prune.cuh): from one
+// movement's start to its end.
+struct Prune {
+  double* b = nullptr;    // per vertex, where `valid` is set
+  u32* valid = nullptr;   // bit per vertex
+  double* shift = nullptr;// S: how far any community's degree may have fallen
+  double* drop = nullptr; // per community: degree leaving it in this round
+  unsigned long long* worst = nullptr;  // bits of the largest of them, not yet in S
+};
+
 struct Engine {
   hl_config cfg{};
   int device = 0;
@@ -184,6 +198,8 @@ struct Engine {
   // K marks handed to the next level's inc_movement (M8): the nodes it gained
   // from splits below and the nodes whose community the projection changed
   bool k_flags_set = false;
+  u32 prune_rounds = 0;  // multi-kernel evaluations of the running movement
+  Prune prune;           // the running movement's bounds (b == nullptr: off)
   u64 sum_nv_batch = 0;  // frontier sizes of the multi-kernel evaluations, this call
   // degree-bin thresholds picked by the autotuner (0 = compile-time default)
   struct Tune {
@@ -251,6 +267,7 @@ void recompute_comm_degrees(Engine& E, Level& L, const u32* part, u32 ncomm_cap,
 void compact_labels_if_needed(Engine& E, u32* labels, u32 n, u32 limit);
 void select_decoupled_dev(Engine& E, u32 M);
 void ensure_comm_arrays(Engine& E, size_t ncap);
+void prune_begin(Engine& E, const Level& L);
 void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, const u32* s,
               const double* d, const u8* blocked, bool allow_empty, u32* out_to, double* out_gain,
               unsigned long long* traversed);

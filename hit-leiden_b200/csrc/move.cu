@@ -16,6 +16,7 @@
 #include <cstring>
 
 #include "hl_engine.cuh"
+#include "prune.cuh"
 
 namespace hl {
 
@@ -338,7 +339,7 @@ __global__ void k_gather_sel(const u32* order, u32 M, const u32* act, const u32*
 __global__ void k_apply_moves(u32 M, const u8* status, const u32* sel_node, const u32* sel_from,
                               const u32* sel_to, u32* f, const double* kdeg, double* d,
                               bool atomic_d, u8* changed, u8* affected, bool mark_moved,
-                              u32* accepted) {
+                              u32* accepted, Prune prune) {
   u32 local = 0;
   for (u64 r = blockIdx.x * (u64)blockDim.x + threadIdx.x; r < M; r += (u64)gridDim.x * blockDim.x) {
     if (status[r] != ST_ACCEPTED) continue;
@@ -346,6 +347,7 @@ __global__ void k_apply_moves(u32 M, const u8* status, const u32* sel_node, cons
     f[v] = sel_to[r];
     changed[v] = 1;
     if (mark_moved) affected[v] = 1;
+    prune_moved(prune, v, sel_from[r], kdeg[v]);
     if (atomic_d) {
       double kv = kdeg[v];
       atomicAdd(&d[sel_from[r]], -kv);
@@ -401,9 +403,10 @@ constexpr u64 MARK_LONG = 4096;
 // One row's marks over entries [p_lo, p_hi): four entries per lane in
 // flight, their neighbours, then their labels.  Returns whether a neighbour
 // shares v's sub-community.
-__device__ __forceinline__ bool mark_entries(u64 p_lo, u64 p_hi, u32 lane, u32 to, u32 sv,
-                                             const u32* col, const u32* f, const u32* s, u8* next,
-                                             u8* affected) {
+__device__ __forceinline__ bool mark_entries(u64 p_lo, u64 p_hi, u32 lane, u32 from, u32 to,
+                                             u32 sv, const u32* col, const double* w,
+                                             const u32* f, const u32* s, u8* next, u8* affected,
+                                             const Prune& prune) {
   bool any_same = false;
   for (u64 p0 = p_lo + lane; p0 < p_hi; p0 += 128) {
     u32 nb[4], fn[4], sn[4];
@@ -418,7 +421,10 @@ __device__ __forceinline__ bool mark_entries(u64 p_lo, u64 p_hi, u32 lane, u32 t
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (nb[j] != NONE32) {
-        if (fn[j] != to) next[nb[j]] = 1;
+        if (fn[j] != to) {
+          next[nb[j]] = 1;
+          if (prune_valid(prune, nb[j])) prune_raise(prune, nb[j], fn[j], from, w[p0 + 32 * j]);
+        }
         if (sn[j] == sv) {
           affected[nb[j]] = 1;
           any_same = true;
@@ -428,15 +434,18 @@ __device__ __forceinline__ bool mark_entries(u64 p_lo, u64 p_hi, u32 lane, u32 t
   return any_same;
 }
 
-__global__ void k_mark_next(u32 M, const u8* status, const u32* sel_node, const u32* sel_to,
-                            const u64* off, const u32* col, const u32* f, const u32* s, u8* next,
-                            u8* affected, unsigned long long* long_list, u32* long_count) {
+__global__ void k_mark_next(u32 M, const u8* status, const u32* sel_node, const u32* sel_from,
+                            const u32* sel_to, const u64* off, const u32* col, const double* w,
+                            const u32* f, const u32* s, u8* next, u8* affected,
+                            unsigned long long* long_list, u32* long_count, Prune prune) {
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 r = warp; r < M; r += nwarps) {
     if (status[r] != ST_ACCEPTED) continue;
     u32 v = sel_node[r], to = sel_to[r];
+    const u32 from = sel_from[r];
+    if (lane == 0) prune_worst(prune, from);
     const u64 deg = off[v + 1] - off[v];
     if (deg > MARK_LONG) {
       const u32 nseg = (u32)((deg + MARK_LONG - 1) / MARK_LONG);
@@ -447,18 +456,29 @@ __global__ void k_mark_next(u32 M, const u8* status, const u32* sel_node, const 
         long_list[at + x] = ((unsigned long long)r << 32) | x;
       continue;
     }
-    const bool any_same = mark_entries(off[v], off[v + 1], lane, to, s[v], col, f, s, next,
-                                       affected);
+    const bool any_same = mark_entries(off[v], off[v + 1], lane, from, to, s[v], col, w, f, s,
+                                       next, affected, prune);
     if (__any_sync(0xffffffffu, any_same) && lane == 0) affected[v] = 1;
   }
 }
 
 // The segments of long rows k_mark_next listed: a warp per segment, the same
 // marks (every segment that meets v's sub-community marks v itself).
+// The round's drops are done with: S takes the largest, the counters clear.
 __global__ void k_mark_next_long(const unsigned long long* long_list, const u32* long_count,
-                                 const u32* sel_node, const u32* sel_to, const u64* off,
-                                 const u32* col, const u32* f, const u32* s, u8* next,
-                                 u8* affected) {
+                                 u32 M, const u8* status, const u32* sel_node,
+                                 const u32* sel_from, const u32* sel_to, const u64* off,
+                                 const u32* col, const double* w, const u32* f, const u32* s,
+                                 u8* next, u8* affected, Prune prune) {
+  if (prune.b) {
+    const u64 gt = blockIdx.x * (u64)blockDim.x + threadIdx.x;
+    if (gt == 0) {
+      *prune.shift += prune_worst_now(prune);
+      *prune.worst = 0;
+    }
+    for (u64 r = gt; r < M; r += (u64)gridDim.x * blockDim.x)
+      if (status[r] == ST_ACCEPTED) prune.drop[sel_from[r]] = 0.0;
+  }
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
@@ -470,7 +490,8 @@ __global__ void k_mark_next_long(const unsigned long long* long_list, const u32*
     const u64 o0 = off[v], o1 = off[v + 1];
     const u64 lo = o0 + (u64)seg * MARK_LONG;
     const u64 hi = lo + MARK_LONG < o1 ? lo + MARK_LONG : o1;
-    const bool any_same = mark_entries(lo, hi, lane, to, s[v], col, f, s, next, affected);
+    const bool any_same =
+        mark_entries(lo, hi, lane, sel_from[r], to, s[v], col, w, f, s, next, affected, prune);
     if (__any_sync(0xffffffffu, any_same) && lane == 0) affected[v] = 1;
   }
 }
@@ -521,6 +542,27 @@ void select_decoupled_dev(Engine& E, u32 M) {
   E.kagg[KT_SELECT].bytes += (u64)M * 9 * iters;  // from/to/status/nmask per iteration
 }
 
+// The bounds of one movement; off where they do not hold (γ < 0) or no row is
+// long enough for them.
+void prune_begin(Engine& E, const Level& L) {
+  E.prune = Prune{};
+  E.prune_rounds = 0;
+  const u32 n = L.g.n;
+  if (!n || E.cfg.mode == HL_MODE_DETERMINISTIC || !(E.cfg.resolution >= 0.0) ||
+      !(L.tw > 0.0) || L.g.nnz <= PRUNE_MIN_DEG)
+    return;
+  Scratch& S = E.sc;
+  S.pr_b.ensure(E.mem, n);
+  S.pr_valid.ensure(E.mem, ((size_t)n + 31) / 32);
+  S.pr_drop.ensure(E.mem, 2 * (size_t)n + 2);
+  S.pr_shift.ensure(E.mem, 2);
+  E.prune.b = S.pr_b.p;
+  E.prune.valid = S.pr_valid.p;
+  E.prune.drop = S.pr_drop.p;
+  E.prune.shift = S.pr_shift.p;
+  E.prune.worst = reinterpret_cast<unsigned long long*>(S.pr_shift.p + 1);
+}
+
 MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active,
                      bool mark_moved) {
   MoveOut out;
@@ -537,6 +579,7 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   u32 it = 0;
   GangMoveStats gm;
   bool gang_on = gang_move_fits(E, L);
+  prune_begin(E, L);
   if (gang_on) {
     S.cnt.ensure(E.mem, 16);
     const u32 fr = all_active ? n : (u32)std::min<u64>(n, 2 * delta.k);
@@ -573,6 +616,11 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
     compact_labels_if_needed(E, L.f.p, n, n);
     ensure_comm_arrays(E, ncap);
     recompute_comm_degrees(E, L, L.f.p, (u32)ncap, S.d.p);
+    if (E.prune.b) {
+      HL_CUDA(cudaMemsetAsync(E.prune.valid, 0, sizeof(u32) * (((size_t)n + 31) / 32), st));
+      HL_CUDA(cudaMemsetAsync(E.prune.drop, 0, sizeof(double) * ncap, st));
+      HL_CUDA(cudaMemsetAsync(E.prune.shift, 0, 2 * sizeof(double), st));
+    }
   }
   if (E.cfg.mode == HL_MODE_DETERMINISTIC) {
     // sequential Gauss–Seidel (hit_leiden.rs:1103-1191): one iteration
@@ -596,8 +644,8 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   S.gkey.ensure(E.mem, n);
   S.gkey2.ensure(E.mem, n);
   S.cnt.ensure(E.mem, 16);
-  S.red64.ensure(E.mem, 8);
-  HL_CUDA(cudaMemsetAsync(S.red64.p, 0, 8 * sizeof(u64), st));
+  S.red64.ensure(E.mem, 9);
+  HL_CUDA(cudaMemsetAsync(S.red64.p, 0, 9 * sizeof(u64), st));
   u64 sum_nv = 0;
   u32* cnt = S.cnt.p;
 
@@ -657,7 +705,8 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
     cudaEvent_t ev_mark = E.kt_begin();
     ++E.nlaunch, k_apply_moves<<<grid_for(M), 256, 0, st>>>(M, S.status.p, S.sel_node.p, S.sel_from.p,
                                                S.sel_to.p, L.f.p, L.k.p, S.d.p, E.integral,
-                                               S.changed.p, S.affected.p, mark_moved, S.acc_cnt.p);
+                                               S.changed.p, S.affected.p, mark_moved, S.acc_cnt.p,
+                                               E.prune);
     HL_LAUNCH_CHECK();
     if (!E.integral) {
       // Replay d(C) -= k / += k in selected order, per community.
@@ -700,15 +749,12 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
     S.mark_long.ensure(E.mem, (size_t)M + L.g.nnz / MARK_LONG + 1);
     S.mark_long_cnt.ensure(E.mem, 1);
     HL_CUDA(cudaMemsetAsync(S.mark_long_cnt.p, 0, sizeof(u32), st));
-    ++E.nlaunch, k_mark_next<<<grid_for((u64)M * 32), 256, 0, st>>>(M, S.status.p, S.sel_node.p, S.sel_to.p,
-                                                        L.g.off.p, L.g.col.p, L.f.p, L.s_cur.p,
-                                                        S.next.p, S.affected.p, S.mark_long.p,
-                                                        S.mark_long_cnt.p);
-    ++E.nlaunch, k_mark_next_long<<<148 * 8, 256, 0, st>>>(S.mark_long.p, S.mark_long_cnt.p,
-                                                           S.sel_node.p,
-                                                           S.sel_to.p, L.g.off.p, L.g.col.p,
-                                                           L.f.p, L.s_cur.p, S.next.p,
-                                                           S.affected.p);
+    ++E.nlaunch, k_mark_next<<<grid_for((u64)M * 32), 256, 0, st>>>(
+        M, S.status.p, S.sel_node.p, S.sel_from.p, S.sel_to.p, L.g.off.p, L.g.col.p, L.g.w.p,
+        L.f.p, L.s_cur.p, S.next.p, S.affected.p, S.mark_long.p, S.mark_long_cnt.p, E.prune);
+    ++E.nlaunch, k_mark_next_long<<<148 * 8, 256, 0, st>>>(
+        S.mark_long.p, S.mark_long_cnt.p, M, S.status.p, S.sel_node.p, S.sel_from.p, S.sel_to.p,
+        L.g.off.p, L.g.col.p, L.g.w.p, L.f.p, L.s_cur.p, S.next.p, S.affected.p, E.prune);
     HL_LAUNCH_CHECK();
     E.kt_end(KT_MARK_NEXT, ev_mark);
     S.active.swap(S.next);
@@ -717,6 +763,7 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   // The evaluation counters and the accepted moves stay on the device until
   // the call ends (Scratch::bacc; the algorithmic bytes are counted there).
   stats_acc_u64(E, reinterpret_cast<const unsigned long long*>(S.red64.p), 8, 0);
+  stats_acc_u64(E, reinterpret_cast<const unsigned long long*>(S.red64.p) + 8, 1, 11);
   stats_acc_u32(E, S.acc_cnt.p, 8);
   E.sum_nv_batch += sum_nv;
   out.moves += gm.moves;

@@ -103,7 +103,9 @@ typedef struct {
   uint32_t levels;       /* levels in the state                                    */
   uint64_t moves;        /* accepted movement moves, all levels                    */
   uint64_t candidates;   /* positive-gain candidates, all levels                   */
-  uint64_t traversed;    /* adjacency entries scanned by movement, all levels      */
+  uint64_t traversed;    /* adjacency entries of the vertices movement decided on, */
+                         /* all levels (a vertex whose bound rules a move out      */
+                         /* counts without its row being read)                     */
   uint64_t splits;       /* sub-community components split off                     */
   uint64_t merges;       /* singleton refinement merges                            */
   uint64_t changed;      /* |B^1| level-0 vertices whose community changed         */

@@ -68,7 +68,7 @@ fn main() {
     for h in ["hl.h", "hl_debug.h"] {
         println!("cargo:rerun-if-changed={}", include.join(h).display());
     }
-    for h in ["hl_engine.cuh", "hl_internal.cuh", "csr_rebuild.cuh", "gang.cuh", "hub_sums.cuh"] {
+    for h in ["hl_engine.cuh", "hl_internal.cuh", "csr_rebuild.cuh", "gang.cuh", "hub_sums.cuh", "prune.cuh"] {
         println!("cargo:rerun-if-changed={}", csrc.join(h).display());
     }
 

@@ -139,3 +139,33 @@ def test_inc_movement_shapes(shape, labels, integral):
             got = gh.inc_movement(g, ds, dd, dw, f, s, 1.0, max_rounds=rounds)
             assert np.array_equal(ref[0], got[0])
             assert np.array_equal(ref[1], got[1]) and np.array_equal(ref[2], got[2])
+
+
+# Rows above 64 entries carry bounds from round to round (prune.cuh): dense
+# graphs with few communities keep whole neighbourhoods active for 20 rounds,
+# in the one-launch and in the multi-kernel rounds.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("gamma", [0.0, 0.7, 3.0])
+@pytest.mark.parametrize("multi", [False, True])
+def test_bounds_change_nothing(integral, gamma, multi):
+    import importlib
+    hl = importlib.import_module("hit-leiden_b200")
+    rng = np.random.default_rng(int(10 * gamma) + integral)
+    n = 1500
+    s, d, w = gh.random_graph(rng, n, 90000, integral)
+    cfg = hl.RunConfig(mode=hl.RunMode.Throughput, resolution=gamma, small_rounds=not multi)
+    gs = hl.PartitionState.load(hl.GraphInput.from_arrays("dense", n, s, d, w), cfg)
+    ref = O.State(n, gamma=gamma, mode=O.MODE_THROUGHPUT)
+    ref.bootstrap(s, d, w, max_levels=10)
+    for i in range(3):
+        ds = rng.integers(0, n, 400).astype(np.uint32)
+        dd = rng.integers(0, n, 400).astype(np.uint32)
+        dw = rng.integers(1, 9, 400).astype(float) if integral else rng.uniform(0.1, 9.0, 400)
+        gs.apply_batch(ds, dd, dw)
+        ref.hit_leiden(ds, dd, dw)
+        assert gs.levels == ref.levels
+        for p in range(ref.levels):
+            assert np.array_equal(gs.community_mapping_per_level[p], ref.get_map(p, O.MAP_F))
+            assert np.array_equal(gs.current_subcommunity_mapping_per_level[p],
+                                  ref.get_map(p, O.MAP_S_CUR))
+    gs.close()
