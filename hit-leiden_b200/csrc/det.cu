@@ -119,7 +119,7 @@ struct DetMoveArgs {
   const double* k;
   double* d;
   u64 dcap;            // entries of d (and of bw / bp): community ids stay below it
-  u32* act;            // active bitset, (n + 31) / 32 words
+  const u32* act;      // active bitset, (n + 31) / 32 words
   u8* changed;
   u8* affected;
   bool mark_moved;
@@ -129,68 +129,381 @@ struct DetMoveArgs {
   double tw, gamma;
   u32 next_empty;      // id of the next empty community (hit_leiden.rs:1104)
   bool ordered;
+  bool f_local;        // the labels are kept in shared memory too
+  bool d_local;        // ... and d of the ids below n
+  u32* gbits;          // the bit sets, when they exceed shared memory
   u64 max_pops;
   unsigned long long* out;  // [0] pops, [1] moves, [2] traversed, [3] status, [4] next_empty
 };
 
-// hit_leiden.rs:1103-1191.
+// The walk pops the lowest active vertex, evaluates it, perhaps moves it, and
+// most pops move nothing (25 pops a move on the 9.9k-vertex graph).  A pop that
+// moves nothing changes nothing that later evaluations read, so the next
+// vertices in order are evaluated together on the current state, a warp each;
+// up to and including the first one that moves they are the reference's pops,
+// the rest stay active and are evaluated again after the move.  The number taken
+// grows while nothing moves.  The active set is a three-level bit set in shared
+// memory, and so are the labels and the community degrees of small levels.
+// Rows above DET_WARP_ROW entries take the whole block, one at a time.
+constexpr u32 DET_AHEAD = 128;       // vertices evaluated together at most
+constexpr u32 DET_WARP_ROW = 128;
+constexpr u32 DET_TAB = 2 * DET_WARP_ROW;
+constexpr u32 DET_F_LOCAL = 32768;   // nodes whose labels fit shared memory
+constexpr u32 DET_D_LOCAL = 10240;   // ... whose community degrees do, too
+constexpr size_t DET_SMEM_MAX = 216 * 1024;
+constexpr u32 DET_BITS_LOCAL = 1u << 20;  // nodes whose bit sets fit shared memory
+constexpr u32 DET_BIG = 0xFFFFFFFDu;      // result of a row left to the block
+
+struct DetWarp {
+  double tv[DET_TAB];
+  double sw[DET_WARP_ROW];
+  u32 tk[DET_TAB], tp[DET_TAB];
+};
+struct DetSmem {
+  DetWarp warp[DET_WARPS];
+};
+
+// The active set: words of 32 vertices, and one bit per non-zero word, twice.
+struct DetBits {
+  u32 *l0, *l1, *l2;
+  __device__ __forceinline__ void set(u32 v) {
+    atomicOr(&l0[v >> 5], 1u << (v & 31));
+    atomicOr(&l1[v >> 10], 1u << ((v >> 5) & 31));
+    atomicOr(&l2[v >> 15], 1u << ((v >> 10) & 31));
+  }
+  // Several threads may clear at once, but none may set meanwhile.
+  __device__ __forceinline__ void clear(u32 v) {
+    const u32 m0 = ~(1u << (v & 31)), m1 = ~(1u << ((v >> 5) & 31));
+    if (atomicAnd(&l0[v >> 5], m0) & m0) return;
+    if (atomicAnd(&l1[v >> 10], m1) & m1) return;
+    atomicAnd(&l2[v >> 15], ~(1u << ((v >> 10) & 31)));
+  }
+};
+
+__device__ __forceinline__ u32 det_word(const u32* p) { return *(const volatile u32*)p; }
+
+// The lowest active vertex (NONE32: none), by one warp; n2 words at the top.
+__device__ __forceinline__ u32 det_lowest(const DetBits& B, u32 n2) {
+  const u32 lane = threadIdx.x & 31;
+  for (u32 i0 = 0; i0 < n2; i0 += 32) {
+    const u32 x = i0 + lane < n2 ? det_word(&B.l2[i0 + lane]) : 0u;
+    const u32 m = __ballot_sync(0xffffffffu, x != 0);
+    if (!m) continue;
+    const u32 j = __ffs(m) - 1;
+    const u32 i2 = ((i0 + j) << 5) + (u32)__ffs(__shfl_sync(0xffffffffu, x, j)) - 1;
+    const u32 i1 = (i2 << 5) + (u32)__ffs(det_word(&B.l1[i2])) - 1;
+    return (i1 << 5) + (u32)__ffs(det_word(&B.l0[i1])) - 1;
+  }
+  return NONE32;
+}
+
+// Largest gain over the lanes (g of lanes without a candidate: 0), ties to the
+// smallest position; the winning lane, or 32 when no gain is positive.
+__device__ __forceinline__ u32 det_warp_best(double g, u32 p) {
+  const u64 key = g > 0.0 ? (u64)__double_as_longlong(g) : 0ull;  // positive: bits ascend
+  const u32 hi = (u32)(key >> 32), lo = (u32)key;
+  const u32 mh = __reduce_max_sync(0xffffffffu, hi);
+  if (!mh) return 32;
+  const u32 ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const bool best = hi == mh && lo == ml;
+  const u32 mp = __reduce_min_sync(0xffffffffu, best ? p : NONE32);
+  return __ffs(__ballot_sync(0xffffffffu, best && p == mp)) - 1;
+}
+
+// False when the computed gain of moving to (w_to, d_to) is certainly <= 0: the
+// division-free proxy Q = 2m·c·gain lies below zero by more than the rounding
+// of both (GainScreen in hl_internal.cuh).  Two divisions cost as much as the
+// rest of a step, and few candidates gain.
+__device__ __forceinline__ bool det_may_gain(double w_to, double d_to, double w_cur, double tw,
+                                             double gamma, double kv, double d_cur) {
+  const double p1 = __dmul_rn(__dsub_rn(w_to, w_cur), __dmul_rn(tw, tw));
+  const double p2 =
+      __dmul_rn(__dmul_rn(__dmul_rn(gamma, kv), __dsub_rn(__dsub_rn(d_cur, kv), d_to)), tw);
+  const double t = __dadd_rn(fabs(p1), fabs(p2));
+  return !(__dadd_rn(p1, p2) < -__dadd_rn(__dmul_rn(1.7763568394002505e-15, t), 1e-300));
+}
+
+// hit_leiden.rs:1103-1191.  What bounds it: the chain of a step (barriers and
+// dependent loads, about 6 us) times the moves.  9.9k vertices, 1,672 pops with
+// 67 moves: 128 steps, 0.83 ms, against 2.9 ms one pop at a time by the block
+// (two divisions, eight barriers and global atomics a pop).
 __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
-  __shared__ u32 s_lo, s_found, s_nk, s_best, s_stop;
+  extern __shared__ __align__(16) unsigned char det_raw[];
+  DetSmem& M = *reinterpret_cast<DetSmem*>(det_raw);
+  __shared__ u32 s_list[DET_AHEAD], s_to[DET_AHEAD], s_deg[DET_AHEAD];
+  __shared__ u32 s_nlist, s_first, s_nk, s_best, s_stop;
   __shared__ double s_bestg;
   __shared__ double r_g[DET_WARPS];
   __shared__ u32 r_p[DET_WARPS], r_k[DET_WARPS];
   __shared__ double tile[32];
-  const u32 tid = threadIdx.x;
-  const u32 nwords = (A.n + 31) >> 5;
-  unsigned long long pops = 0, moves = 0, trav = 0;
-  u32 next_empty = A.next_empty;
+  __shared__ unsigned long long s_pops, s_moves, s_trav;
+  __shared__ u32 s_empty;
+  const u32 tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+  const u32 n0 = (A.n + 31) >> 5, n1 = (n0 + 31) >> 5, n2 = (n1 + 31) >> 5;
+  u32* local = reinterpret_cast<u32*>(det_raw + sizeof(DetSmem));
+  DetBits B;
+  B.l0 = A.gbits ? A.gbits : local;
+  B.l1 = B.l0 + n0;
+  B.l2 = B.l1 + n1;
+  u32* fl = A.f_local ? local + (A.gbits ? 0 : n0 + n1 + n2) : nullptr;
+  u32* f = fl ? fl : A.f;
+  // d of ids below n; written through to A.d
+  double* dl = A.d_local ? reinterpret_cast<double*>(
+                               det_raw + ((sizeof(DetSmem) + 4 * (size_t)(n0 + n1 + n2 + A.n) + 7) &
+                                          ~(size_t)7))
+                         : nullptr;
+  auto d_of = [&](u32 c) { return dl && c < A.n ? dl[c] : A.d[c]; };
+  auto d_put = [&](u32 c, double x) {
+    if (dl && c < A.n) dl[c] = x;
+    A.d[c] = x;
+  };
+  for (u32 i = tid; i < n0; i += DET_THREADS) B.l0[i] = A.act[i];
+  for (u32 i = tid; i < n1 + n2; i += DET_THREADS) B.l1[i] = 0;
+  if (fl)
+    for (u32 i = tid; i < A.n; i += DET_THREADS) fl[i] = A.f[i];
+  if (dl)
+    for (u32 i = tid; i < A.n; i += DET_THREADS) dl[i] = A.d[i];
   if (tid == 0) {
-    s_lo = 0;
     s_stop = DET_OK;
+    s_pops = s_moves = s_trav = 0;
+    s_empty = A.next_empty;
   }
   __syncthreads();
+  for (u32 i = tid; i < n0; i += DET_THREADS)
+    if (det_word(&B.l0[i])) {
+      atomicOr(&B.l1[i >> 5], 1u << (i & 31));
+      atomicOr(&B.l2[i >> 10], 1u << ((i >> 5) & 31));
+    }
+  __syncthreads();
+  u32 ahead = DET_WARPS;  // vertices taken together
   while (true) {
-    // 1. the lowest active vertex (iter_ones().next(), :1109)
-    if (tid == 0) s_found = NONE32;
-    __syncthreads();
-    for (u32 base = s_lo; base < nwords; base += DET_THREADS) {
-      const u32 wi = base + tid;
-      const bool hit = wi < nwords && A.act[wi] != 0u;
-      if (hit) atomicMin(&s_found, wi);
-      if (__syncthreads_or(hit)) break;
+    // ---- the next active vertices in order ----
+    if (wib == 0) {
+      const u32 first = det_lowest(B, n2);
+      u32 cnt = 0;
+      if (first != NONE32) {
+        u32 w0 = first >> 5;
+        for (u32 win = 0; win < 16 && w0 < n0 && cnt < ahead; ++win, w0 += 32) {
+          u32 x = w0 + lane < n0 ? det_word(&B.l0[w0 + lane]) : 0u;
+          if (!__any_sync(0xffffffffu, x != 0)) continue;
+          u32 inc = __popc(x);
+#pragma unroll
+          for (u32 o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+          }
+          for (u32 at = cnt + inc - __popc(x); x && at < ahead; x &= x - 1, ++at)
+            s_list[at] = ((w0 + lane) << 5) + (u32)__ffs(x) - 1;
+          cnt = min(ahead, cnt + __shfl_sync(0xffffffffu, inc, 31));
+        }
+      }
+      if (lane == 0) {
+        s_nlist = cnt;
+        s_first = NONE32;
+        s_nk = 0;
+      }
     }
-    const u32 word = s_found;
-    if (word == NONE32) break;
-    const u32 bits = A.act[word];
-    const u32 v = (word << 5) + (u32)(__ffs(bits) - 1);
     __syncthreads();
+    const u32 nlist = s_nlist;
+    if (nlist == 0) break;
+    // ---- their best moves on the current state ----
+    for (u32 i = wib; i < nlist; i += DET_WARPS) {
+      const u32 v = s_list[i];
+      const u64 o0 = A.off[v];
+      const u32 deg = (u32)(A.off[v + 1] - o0);
+      if (deg > DET_WARP_ROW) {
+        if (lane == 0) {
+          s_deg[i] = 0;  // counted by the block
+          s_to[i] = DET_BIG;
+          atomicMin(&s_first, i);
+        }
+        continue;
+      }
+      const u32 cur = f[v];
+      const double kv = A.k[v];
+      const double dcur = d_of(cur);
+      // Σw per neighbour community, self-loops included (:1119-1125): this
+      // lane's candidate (key, first position, gain)
+      double wcur = 0.0, g = 0.0;
+      u32 key = NONE32, pos = NONE32;
+      DetWarp& T = M.warp[wib];
+      if (deg <= 32) {
+        u32 c = NONE32;
+        if (lane < deg) {
+          c = f[A.col[o0 + lane]];
+          T.sw[lane] = A.w[o0 + lane];
+        }
+        __syncwarp();
+        const u32 grp = __match_any_sync(0xffffffffu, c);
+        const bool lead = c != NONE32 && !(grp & ((1u << lane) - 1u));
+        double sum = 0.0, dkey = 0.0;
+        if (lead) {
+          dkey = d_of(c);
+          for (u32 m = grp; m; m &= m - 1) sum = __dadd_rn(sum, T.sw[__ffs(m) - 1]);
+        }
+        const u32 cm = __ballot_sync(0xffffffffu, lead && c == cur);
+        const double wc = __shfl_sync(0xffffffffu, sum, cm ? __ffs(cm) - 1 : 0);
+        wcur = cm ? wc : 0.0;
+        if (lead && c != cur && det_may_gain(sum, dkey, wcur, A.tw, A.gamma, kv, dcur)) {
+          g = move_gain(sum, wcur, A.tw, A.gamma, kv, dcur, dkey);
+          key = c;
+          pos = lane;
+        }
+      } else {
+        u32 cap = 64;
+        while (cap < 2 * deg) cap <<= 1;
+        const u32 mask = cap - 1;
+        for (u32 x = lane; x < cap; x += 32) T.tk[x] = NONE32;
+        u32 cq[DET_WARP_ROW / 32];
+#pragma unroll
+        for (u32 j = 0; j < DET_WARP_ROW / 32; ++j) {
+          const u32 q = 32 * j + lane;
+          cq[j] = q < deg ? A.col[o0 + q] : NONE32;
+          if (q < deg) T.sw[q] = A.w[o0 + q];
+        }
+#pragma unroll
+        for (u32 j = 0; j < DET_WARP_ROW / 32; ++j)
+          if (cq[j] != NONE32) cq[j] = f[cq[j]];
+        __syncwarp();
+#pragma unroll
+        for (u32 j = 0; j < DET_WARP_ROW / 32; ++j) {
+          if (32 * j >= deg) break;
+          const u32 c = cq[j];
+          const u32 grp = __match_any_sync(0xffffffffu, c);
+          if (c != NONE32 && !(grp & ((1u << lane) - 1u))) {
+            u32 slot = ((c * 2654435761u) >> 7) & mask;
+            while (true) {  // the table holds at most deg < cap keys
+              const u32 prev = atomicCAS(&T.tk[slot], NONE32, c);
+              if (prev == NONE32 || prev == c) {
+                double sum = prev == NONE32 ? 0.0 : T.tv[slot];
+                for (u32 m = grp; m; m &= m - 1)
+                  sum = __dadd_rn(sum, T.sw[32 * j + __ffs(m) - 1]);
+                T.tv[slot] = sum;
+                if (prev == NONE32) T.tp[slot] = 32 * j + lane;
+                break;
+              }
+              slot = (slot + 1) & mask;
+            }
+          }
+          __syncwarp();
+        }
+        bool found = false;
+        for (u32 x = lane; x < cap; x += 32)
+          if (T.tk[x] == cur) {
+            wcur = T.tv[x];
+            found = true;
+          }
+        const u32 fm = __ballot_sync(0xffffffffu, found);
+        wcur = __shfl_sync(0xffffffffu, wcur, fm ? __ffs(fm) - 1 : 0);
+        if (!fm) wcur = 0.0;
+        for (u32 x = lane; x < cap; x += 32) {
+          const u32 c = T.tk[x];
+          if (c == NONE32 || c == cur) continue;
+          const double dc = d_of(c);
+          if (!det_may_gain(T.tv[x], dc, wcur, A.tw, A.gamma, kv, dcur)) continue;
+          const double gn = move_gain(T.tv[x], wcur, A.tw, A.gamma, kv, dcur, dc);
+          const u32 pc = T.tp[x];
+          if (gn > 0.0 && (pos == NONE32 || gn > g || (gn == g && pc < pos))) {
+            g = gn;
+            pos = pc;
+            key = c;
+          }
+        }
+      }
+      // best candidate (:1127-1146), then the empty community (:1150-1162)
+      const bool may_empty = det_may_gain(0.0, 0.0, wcur, A.tw, A.gamma, kv, dcur);
+      const u32 bl = det_warp_best(g, pos);
+      u32 to = NONE32;
+      double bestg = 0.0;
+      if (bl < 32) {
+        bestg = __shfl_sync(0xffffffffu, g, bl);
+        to = __shfl_sync(0xffffffffu, key, bl);
+      }
+      if (may_empty && empty_gain(wcur, A.tw, A.gamma, kv, dcur) > bestg) to = DET_EMPTY;
+      if (lane == 0) {
+        s_deg[i] = deg;
+        s_to[i] = to;
+        if (to != NONE32) atomicMin(&s_first, i);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    // ---- the pops: all up to the first that moves ----
+    const u32 first = s_first;
+    const u32 popped = first == NONE32 ? nlist : first + 1;
+    if (tid < popped) {
+      B.clear(s_list[tid]);
+      atomicAdd(&s_trav, (unsigned long long)s_deg[tid]);
+    }
     if (tid == 0) {
-      A.act[word] = bits & (bits - 1u);
-      s_lo = word;
-      s_nk = 0;
-      if (++pops > A.max_pops) s_stop = DET_POP_LIMIT;
+      s_pops += popped;
+      if (s_pops > A.max_pops) s_stop = DET_POP_LIMIT;
     }
     __syncthreads();
+    ahead = first == NONE32 ? min(2 * ahead, DET_AHEAD) : DET_WARPS;
     if (s_stop != DET_OK) break;
+    if (first == NONE32) continue;
+    const u32 v = s_list[first];
+    const u32 cur = f[v];
     const u64 o0 = A.off[v], o1 = A.off[v + 1];
-    const u32 cur = A.f[v];
+    u32 best = s_to[first];
+    if (best != DET_BIG) {
+      // ---- the move (:1168-1187), by one warp ----
+      if (wib == 0) {
+        const double kv = A.k[v];
+        if (best == DET_EMPTY) {
+          best = s_empty;
+          if ((u64)best >= A.dcap) {
+            best = NONE32;
+            if (lane == 0) s_stop = DET_ID_SPACE;
+          }
+        }
+        if (best != NONE32) {
+          const double dcur = d_of(cur), dbest = d_of(best);
+          __syncwarp();
+          if (lane == 0) {
+            if (s_to[first] == DET_EMPTY) s_empty = best + 1;
+            A.f[v] = best;
+            if (fl) fl[v] = best;
+            A.changed[v] = 1;
+            if (A.mark_moved) A.affected[v] = 1;
+            d_put(cur, __dsub_rn(dcur, kv));
+            d_put(best, __dadd_rn(dbest, kv));
+            ++s_moves;
+          }
+          __syncwarp();
+          const u32 sv = A.s[v];
+          bool any = false;
+          for (u64 q = o0 + lane; q < o1; q += 32) {
+            const u32 nb = A.col[q];
+            if (f[nb] != best) B.set(nb);
+            if (A.s[nb] == sv) {
+              any = true;
+              A.affected[nb] = 1;
+            }
+          }
+          if (__any_sync(0xffffffffu, any) && lane == 0) A.affected[v] = 1;
+        }
+      }
+      __syncthreads();
+      if (s_stop != DET_OK) break;
+      continue;
+    }
+    // ---- a long row, by the whole block ----
     const double kv = A.k[v];
-    // 2. Σw per neighbour community, self-loops included (:1119-1125)
-    const u32* f = A.f;
     const u32* col = A.col;
     det_row_sums(o0, o1, A.w, A.ordered, [&](u64 q) { return f[col[q]]; }, A.bw, A.bp, A.klist,
                  &s_nk, tile);
     __syncthreads();
-    // 3. best candidate (:1127-1146), then the empty community (:1150-1162)
     const double wcur = A.bw[cur];
-    const double dcur = A.d[cur];
+    const double dcur = d_of(cur);
     const u32 nk = s_nk;
     double g = 0.0;
     u32 p = NONE32, kk = NONE32;
     for (u32 i = tid; i < nk; i += DET_THREADS) {
       const u32 c = A.klist[i];
       if (c == cur) continue;
-      const double gn = move_gain(A.bw[c], wcur, A.tw, A.gamma, kv, dcur, A.d[c]);
+      const double gn = move_gain(A.bw[c], wcur, A.tw, A.gamma, kv, dcur, d_of(c));
       const u32 pc = A.bp[c];
       if (gn > 0.0 && (p == NONE32 || gn > g || (gn == g && pc < p))) {
         g = gn;
@@ -200,7 +513,7 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
     }
     det_argmax(g, p, kk, r_g, r_p, r_k);
     if (tid == 0) {
-      u32 best = cur;
+      best = cur;
       double bestg = 0.0;
       if (p != NONE32) {
         best = kk;
@@ -211,9 +524,24 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
         bestg = eg;
         best = DET_EMPTY;
       }
+      s_trav += o1 - o0;
+      if (bestg > 0.0) {
+        if (best == DET_EMPTY) {
+          if ((u64)s_empty >= A.dcap) s_stop = DET_ID_SPACE;
+          else best = s_empty++;
+        }
+        if (s_stop == DET_OK) {
+          A.f[v] = best;
+          if (fl) fl[v] = best;
+          A.changed[v] = 1;
+          if (A.mark_moved) A.affected[v] = 1;
+          d_put(cur, __dsub_rn(dcur, kv));
+          d_put(best, __dadd_rn(d_of(best), kv));
+          ++s_moves;
+        }
+      }
       s_best = best;
       s_bestg = bestg;
-      trav += o1 - o0;
     }
     __syncthreads();
     for (u32 i = tid; i < nk; i += DET_THREADS) {
@@ -221,66 +549,27 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
       A.bw[c] = 0.0;
       A.bp[c] = NONE32;
     }
-    if (!(s_bestg > 0.0)) {  // :1164-1166
-      __syncthreads();
-      continue;
-    }
-    // 4. the move (:1168-1181)
-    if (tid == 0) {
-      u32 best = s_best;
-      if (best == DET_EMPTY) {
-        if ((u64)next_empty >= A.dcap) {
-          s_stop = DET_ID_SPACE;
-        } else {
-          best = next_empty++;
-        }
-      }
-      if (s_stop == DET_OK) {
-        A.f[v] = best;
-        A.changed[v] = 1;
-        if (A.mark_moved) A.affected[v] = 1;
-        A.d[cur] = __dsub_rn(A.d[cur], kv);
-        A.d[best] = __dadd_rn(A.d[best], kv);
-        s_best = best;
-        ++moves;
-      }
-    }
-    __syncthreads();
     if (s_stop != DET_OK) break;
-    // 5. re-activate neighbours outside the new community, mark K (:1182-1187)
-    const u32 best = s_best;
-    const u32 sv = A.s[v];
-    for (u64 q = o0 + tid; q < o1; q += DET_THREADS) {
-      const u32 nb = A.col[q];
-      if (A.f[nb] != best) {
-        atomicOr(&A.act[nb >> 5], 1u << (nb & 31));
-        atomicMin(&s_lo, nb >> 5);
-      }
-      if (A.s[nb] == sv) {
-        A.affected[v] = 1;
-        A.affected[nb] = 1;
+    if (s_bestg > 0.0) {
+      best = s_best;
+      const u32 sv = A.s[v];
+      for (u64 q = o0 + tid; q < o1; q += DET_THREADS) {
+        const u32 nb = A.col[q];
+        if (f[nb] != best) B.set(nb);
+        if (A.s[nb] == sv) {
+          A.affected[v] = 1;
+          A.affected[nb] = 1;
+        }
       }
     }
     __syncthreads();
   }
   if (tid == 0) {
-    A.out[0] = pops;
-    A.out[1] = moves;
-    A.out[2] = trav;
+    A.out[0] = s_pops;
+    A.out[1] = s_moves;
+    A.out[2] = s_trav;
     A.out[3] = s_stop;
-    A.out[4] = next_empty;
-  }
-}
-
-__global__ void k_bits_from_flags(const u8* flags, u32 n, u32* bits) {
-  const u32 nwords = (n + 31) >> 5;
-  for (u64 wi = blockIdx.x * (u64)blockDim.x + threadIdx.x; wi < nwords;
-       wi += (u64)gridDim.x * blockDim.x) {
-    u32 x = 0;
-    const u64 b = wi << 5;
-    for (u32 j = 0; j < 32 && b + j < n; ++j)
-      if (flags[b + j]) x |= 1u << j;
-    bits[wi] = x;
+    A.out[4] = s_empty;
   }
 }
 
@@ -298,20 +587,38 @@ static void det_status(Engine& E, const u64* out, const char* stage) {
   (void)E;
 }
 
-// The deterministic branch of inc_movement, after seeding and d(C) (`active`
-// holds A as 0/1 bytes).  Returns moves and traversed entries.
-void inc_movement_det(Engine& E, Level& L, double* d, size_t dcap, bool mark_moved,
-                      u64* moves, u64* traversed) {
+static std::atomic<bool> g_det_attr[64];
+
+// The deterministic branch of inc_movement, after seeding and d(C) (`act`: the
+// active bit set).  Returns moves and traversed entries.
+void inc_movement_det(Engine& E, Level& L, const u32* act, double* d, size_t dcap,
+                      bool mark_moved, u64* moves, u64* traversed) {
   Scratch& S = E.sc;
   cudaStream_t st = E.stream;
   const u32 n = L.g.n;
-  const u32 nwords = (n + 31) / 32;
-  S.det_bits.ensure(E.mem, nwords ? nwords : 1);
+  const u64 n0 = ((u64)n + 31) / 32, n1 = (n0 + 31) / 32, n2 = (n1 + 31) / 32;
+  const bool bits_local = n <= DET_BITS_LOCAL, f_local = n <= DET_F_LOCAL;
+  if (!bits_local) S.det_bits.ensure(E.mem, n0 + n1 + n2);
+  const bool d_local = n <= DET_D_LOCAL;
+  size_t smem = sizeof(DetSmem) + (bits_local ? 4 * (n0 + n1 + n2) : 0) +
+                (f_local ? 4 * (size_t)n : 0);
+  if (d_local) smem = ((smem + 7) & ~(size_t)7) + 8 * (size_t)n;
+  // bit sets: n / 8 bytes and a little more than a 32nd of that above them
+  constexpr auto bits = [](size_t x) { return x / 8 + x / 128; };
+  static_assert(sizeof(DetSmem) + 12 * DET_D_LOCAL + bits(DET_D_LOCAL) <= DET_SMEM_MAX &&
+                    sizeof(DetSmem) + 4 * DET_F_LOCAL + bits(DET_F_LOCAL) <= DET_SMEM_MAX &&
+                    sizeof(DetSmem) + bits(DET_BITS_LOCAL) <= DET_SMEM_MAX,
+                "the largest levels kept in shared memory fit it");
+  const int dev = E.device;
+  if (dev >= 0 && dev < 64 && !g_det_attr[dev]) {
+    HL_CUDA(cudaFuncSetAttribute(k_det_move, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)DET_SMEM_MAX));
+    g_det_attr[dev] = true;
+  }
   S.det_bw.ensure(E.mem, dcap);
   S.det_bp.ensure(E.mem, dcap);
   S.det_keys.ensure(E.mem, dcap);
   S.det_out.ensure(E.mem, 8);
-  ++E.nlaunch, k_bits_from_flags<<<grid_for(nwords), 256, 0, st>>>(S.active.p, n, S.det_bits.p);
   HL_CUDA(cudaMemsetAsync(S.det_bw.p, 0, sizeof(double) * dcap, st));
   ++E.nlaunch, k_fill_u32_det<<<grid_for(dcap), 256, 0, st>>>(S.det_bp.p, NONE32, dcap);
   HL_CUDA(cudaMemsetAsync(S.det_out.p, 0, 8 * sizeof(u64), st));
@@ -326,7 +633,10 @@ void inc_movement_det(Engine& E, Level& L, double* d, size_t dcap, bool mark_mov
   A.k = L.k.p;
   A.d = d;
   A.dcap = dcap;
-  A.act = S.det_bits.p;
+  A.act = act;
+  A.f_local = f_local;
+  A.d_local = d_local;
+  A.gbits = bits_local ? nullptr : S.det_bits.p;
   A.changed = S.changed.p;
   A.affected = S.affected.p;
   A.mark_moved = mark_moved;
@@ -339,7 +649,7 @@ void inc_movement_det(Engine& E, Level& L, double* d, size_t dcap, bool mark_mov
   A.ordered = !E.integral;
   A.max_pops = 4096ull * (u64)n + (1ull << 20);
   A.out = reinterpret_cast<unsigned long long*>(S.det_out.p);
-  ++E.nlaunch, k_det_move<<<1, DET_THREADS, 0, st>>>(A);
+  ++E.nlaunch, k_det_move<<<1, DET_THREADS, smem, st>>>(A);
   HL_LAUNCH_CHECK();
   u64 out[8];
   HL_CUDA(cudaMemcpyAsync(E.hs.p, S.det_out.p, 8 * sizeof(u64), cudaMemcpyDeviceToHost, st));
@@ -433,6 +743,195 @@ __device__ double det_wsp(const DetRefArgs& A, u32 S, u32 parent, double* r_g) {
   return acc;  // thread 0 (all of warp 0)
 }
 
+// w(S, C_parent) by one warp (det_wsp's sums and order).  With integral weights
+// (any order) a lane takes a member, rows above 32 entries the whole warp.
+__device__ __forceinline__ double det_wsp_warp(const DetRefArgs& A, u32 S, u32 parent) {
+  const u32 lane = threadIdx.x & 31;
+  const u32 ms = A.mstart[S];
+  const u32 mc = ms == NONE32 ? 0u : A.mcount[S];
+  const u32* f = A.f;
+  const u32* col = A.col;
+  const double* w = A.w;
+  double acc = 0.0;
+  u32 x = A.xhead[S];
+  if (A.ordered) {
+    u32 i = 0;
+    while (i < mc || x != NONE32) {
+      u32 m;
+      if (x == NONE32 || (i < mc && A.members[ms + i] < x)) {
+        m = A.members[ms + i];
+        ++i;
+      } else {
+        m = x;
+        x = A.xnext[x];
+      }
+      acc = warp_ordered_sum(A.off[m], A.off[m + 1], acc, [&](u64 t) { return w[t]; },
+                             [&](u64 t) { return f[col[t]] == parent; });
+    }
+    return acc;
+  }
+  for (u32 i0 = 0; i0 < mc; i0 += 32) {
+    const u32 m = i0 + lane < mc ? A.members[ms + i0 + lane] : NONE32;
+    const u64 a = m != NONE32 ? A.off[m] : 0, b = m != NONE32 ? A.off[m + 1] : 0;
+    if (b - a <= 32)
+      for (u64 q = a; q < b; ++q)
+        if (f[col[q]] == parent) acc += w[q];
+    for (u32 big = __ballot_sync(0xffffffffu, b - a > 32); big; big &= big - 1) {
+      const u32 j = __ffs(big) - 1;
+      const u64 bb = __shfl_sync(0xffffffffu, b, j);
+      for (u64 q = __shfl_sync(0xffffffffu, a, j) + lane; q < bb; q += 32)
+        if (f[col[q]] == parent) acc += w[q];
+    }
+  }
+  for (; x != NONE32; x = A.xnext[x])
+    for (u64 q = A.off[x] + lane; q < A.off[x + 1]; q += 32)
+      if (f[col[q]] == parent) acc += w[q];
+  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
+// The merge of v into `best` (lane 0 / thread 0).  w(best, C) grows by v's own
+// w(v, C) (`wv`), exactly so with integral weights; otherwise (wv < 0: not
+// known) it is summed again when next needed.
+__device__ __forceinline__ void det_merge(const DetRefArgs& A, u32 v, u32 cs, u32 best, double kv,
+                                          double wv) {
+  A.s[v] = best;
+  A.sizes[cs] -= 1u;
+  A.sizes[best] += 1u;
+  A.dS[cs] = __dsub_rn(A.dS[cs], kv);
+  A.dS[best] = __dadd_rn(A.dS[best], kv);
+  // v joins best's members, in node order
+  u32* link = &A.xhead[best];
+  while (*link != NONE32 && *link < v) link = &A.xnext[*link];
+  A.xnext[v] = *link;
+  *link = v;
+  if (wv < 0.0) A.wvalid[best] = 0;
+  else if (A.wvalid[best]) A.wsp[best] += wv;
+}
+
+// One singleton by one warp (rows of up to DET_WARP_ROW entries): per-key sums
+// in the warp's table, the candidates in gain order until the T-filter lets one
+// pass.  No block barriers: they were most of a step.
+__device__ __forceinline__ bool det_refine_warp(const DetRefArgs& A, DetWarp& T, u32 v, u32 cs) {
+  const u32 lane = threadIdx.x & 31;
+  const u64 o0 = A.off[v];
+  const u32 deg = (u32)(A.off[v + 1] - o0);
+  const u32 cc = A.f[v];
+  const double kv = A.k[v];
+  const double dcs = A.dS[cs], dpar = A.dcomm[cc];
+  u32 cap = 64;
+  while (cap < 2 * deg) cap <<= 1;
+  const u32 mask = cap - 1;
+  for (u32 x = lane; x < cap; x += 32) T.tk[x] = NONE32;
+  u32 cq[DET_WARP_ROW / 32];
+#pragma unroll
+  for (u32 j = 0; j < DET_WARP_ROW / 32; ++j) {
+    const u32 q = 32 * j + lane;
+    cq[j] = q < deg ? A.col[o0 + q] : NONE32;
+    if (q < deg) T.sw[q] = A.w[o0 + q];
+  }
+#pragma unroll
+  for (u32 j = 0; j < DET_WARP_ROW / 32; ++j)
+    if (cq[j] != NONE32) cq[j] = A.f[cq[j]] == cc ? A.s[cq[j]] : NONE32;
+  double wv = -1.0;  // w(v, C), kept with integral weights
+  if (!A.ordered) {
+    wv = 0.0;
+#pragma unroll
+    for (u32 j = 0; j < DET_WARP_ROW / 32; ++j)
+      if (cq[j] != NONE32) wv += T.sw[32 * j + lane];
+    for (int o = 16; o; o >>= 1) wv += __shfl_xor_sync(0xffffffffu, wv, o);
+  }
+  __syncwarp();
+#pragma unroll
+  for (u32 j = 0; j < DET_WARP_ROW / 32; ++j) {
+    if (32 * j >= deg) break;
+    const u32 c = cq[j];
+    const u32 grp = __match_any_sync(0xffffffffu, c);
+    if (c != NONE32 && !(grp & ((1u << lane) - 1u))) {
+      u32 slot = ((c * 2654435761u) >> 7) & mask;
+      while (true) {  // the table holds at most deg < cap keys
+        const u32 prev = atomicCAS(&T.tk[slot], NONE32, c);
+        if (prev == NONE32 || prev == c) {
+          double sum = prev == NONE32 ? 0.0 : T.tv[slot];
+          for (u32 m = grp; m; m &= m - 1) sum = __dadd_rn(sum, T.sw[32 * j + __ffs(m) - 1]);
+          T.tv[slot] = sum;
+          if (prev == NONE32) T.tp[slot] = 32 * j + lane;
+          break;
+        }
+        slot = (slot + 1) & mask;
+      }
+    }
+    __syncwarp();
+  }
+  double wcur = 0.0;
+  bool found = false;
+  for (u32 x = lane; x < cap; x += 32)
+    if (T.tk[x] == cs) {
+      wcur = T.tv[x];
+      found = true;
+    }
+  const u32 fm = __ballot_sync(0xffffffffu, found);
+  wcur = __shfl_sync(0xffffffffu, wcur, fm ? __ffs(fm) - 1 : 0);
+  if (!fm) wcur = 0.0;
+  // gains in place of the sums; candidates without a positive one leave the table
+  for (u32 x = lane; x < cap; x += 32) {
+    const u32 c = T.tk[x];
+    if (c == NONE32) continue;
+    double gn = 0.0;
+    if (c != cs) {
+      const double dc = A.dS[c];
+      if (det_may_gain(T.tv[x], dc, wcur, A.tw, A.gamma, kv, dcs))
+        gn = move_gain(T.tv[x], wcur, A.tw, A.gamma, kv, dcs, dc);
+    }
+    if (gn > 0.0) T.tv[x] = gn;
+    else T.tk[x] = NONE32;
+  }
+  __syncwarp();
+  // The best candidate the T-filter lets through wins (the same choice as the
+  // reference's strict '>' over the filtered list).
+  while (true) {
+    double g = 0.0;
+    u32 p = NONE32, at = 0;
+    for (u32 x = lane; x < cap; x += 32) {
+      if (T.tk[x] == NONE32) continue;
+      const double gn = T.tv[x];
+      const u32 pc = T.tp[x];
+      if (p == NONE32 || gn > g || (gn == g && pc < p)) {
+        g = gn;
+        p = pc;
+        at = x;
+      }
+    }
+    const u32 bl = det_warp_best(g, p);
+    if (bl == 32) return false;
+    const u32 slot = __shfl_sync(0xffffffffu, at, bl);
+    const u32 cand = T.tk[slot];
+    const double ds = A.dS[cand];  // (:1514-1548)
+    bool skip = false;
+    if (ds > 0.0) {
+      double x;
+      if (A.wvalid[cand]) {
+        x = A.wsp[cand];
+      } else {
+        x = det_wsp_warp(A, cand, cc);
+        if (lane == 0) {
+          A.wsp[cand] = x;
+          A.wvalid[cand] = 1;
+        }
+      }
+      skip = remove_gain(x, A.tw, A.gamma, ds, dpar) > 1e-9;
+    }
+    __syncwarp();
+    if (!skip) {
+      if (lane == 0) det_merge(A, v, cs, cand, kv, wv);
+      __syncwarp();
+      return true;
+    }
+    if (lane == 0) T.tk[slot] = NONE32;
+    __syncwarp();
+  }
+}
+
 // hit_leiden.rs:1392-1413 → try_merge_singleton_refinement (:1419-1511) with
 // should_skip_candidate_t_filter (:1514-1548).
 __global__ void __launch_bounds__(DET_THREADS) k_det_refine(DetRefArgs A) {
@@ -443,10 +942,26 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_refine(DetRefArgs A) {
   __shared__ double tile[32];
   const u32 tid = threadIdx.x;
   unsigned long long merges = 0;
-  for (u32 i = 0; i < A.nr; ++i) {
+  __shared__ DetWarp s_warp;
+  __shared__ u32 s_i;
+  for (u32 i = 0;; ++i) {
+    // the first warp walks until a row needs the block
+    if (tid < 32) {
+      for (; i < A.nr; ++i) {
+        const u32 v = A.rlist[i];
+        const u32 cs = A.s[v];
+        if (A.sizes[cs] != 1u) continue;  // singleton check (:1398-1400)
+        if (A.off[v + 1] - A.off[v] > DET_WARP_ROW) break;
+        if (det_refine_warp(A, s_warp, v, cs)) ++merges;
+      }
+      if (tid == 0) s_i = i;
+    }
+    __syncthreads();
+    i = s_i;
+    if (i >= A.nr) break;
+    // ---- a long row, by the whole block ----
     const u32 v = A.rlist[i];
     const u32 cs = A.s[v];
-    if (A.sizes[cs] != 1u) continue;  // singleton check (:1398-1400), uniform
     const u32 cc = A.f[v];
     const double kv = A.k[v];
     if (tid == 0) s_nk = 0;
@@ -539,21 +1054,12 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_refine(DetRefArgs A) {
     __syncthreads();
     if (best != cs && bestg > 0.0) {
       if (tid == 0) {
-        A.s[v] = best;
-        A.sizes[cs] -= 1u;
-        A.sizes[best] += 1u;
-        A.dS[cs] = __dsub_rn(A.dS[cs], kv);
-        A.dS[best] = __dadd_rn(A.dS[best], kv);
+        det_merge(A, v, cs, best, kv, -1.0);
         ++merges;
-        // v joins best's members, in node order
-        u32* link = &A.xhead[best];
-        while (*link != NONE32 && *link < v) link = &A.xnext[*link];
-        A.xnext[v] = *link;
-        *link = v;
-        A.wvalid[best] = 0;  // w(best, C) is summed again when next needed
       }
       __syncthreads();
     }
+    __syncthreads();
   }
   if (tid == 0) A.out[0] = merges;
 }

@@ -659,11 +659,12 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
 static std::atomic<bool> g_move_attr[64];
 
 bool gang_move_fits(Engine& E, const Level& L) {
-  return L.g.n > 0 && L.g.n < (1u << 30) && E.cfg.mode != HL_MODE_DETERMINISTIC &&
-         !(E.cfg.flags & HL_FLAG_NO_SMALL_ROUNDS);
+  return L.g.n > 0 &&
+         (E.cfg.mode == HL_MODE_DETERMINISTIC || !(E.cfg.flags & HL_FLAG_NO_SMALL_ROUNDS));
 }
 
-// Movement rounds from the seeds (`setup`) or from the frontier in S.active.
+// Movement rounds from the seeds (`setup`) or from the frontier in S.active.  In
+// deterministic mode the setup alone: the active set is left in S.gm_bits.
 // Returns MOVE_DONE, or why the host's rounds continue from S.active
 // (MOVE_LABELS: the labels need compaction first; nothing else has happened).
 u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_active,
@@ -792,7 +793,7 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   A.items_cap = (u32)std::min<u64>(items_cap, 0xFFFFFFFFull);
   A.part = S.gang_part.p;
   A.it0 = it;
-  A.max_rounds = E.cfg.max_rounds ? E.cfg.max_rounds : 20;
+  A.max_rounds = E.cfg.mode == HL_MODE_DETERMINISTIC ? 0 : E.cfg.max_rounds ? E.cfg.max_rounds : 20;
   A.round0 = round0;
   A.epoch0 = E.epoch;
   A.label_bits = (u32)bits_for(n - 1);

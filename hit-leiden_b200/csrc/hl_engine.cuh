@@ -308,8 +308,8 @@ void autotune_bins(Engine& E, const u32* verts, u32 nv, const Level& L, const u3
                    const double* d, u32* out_to, double* out_gain);
 
 // det.cu: the sequential (RunMode::Deterministic) steps
-void inc_movement_det(Engine& E, Level& L, double* d, size_t dcap, bool mark_moved, u64* moves,
-                      u64* traversed);
+void inc_movement_det(Engine& E, Level& L, const u32* act, double* d, size_t dcap,
+                      bool mark_moved, u64* moves, u64* traversed);
 u64 merge_singletons_det(Engine& E, Level& L, const u32* rv, u32 nr, u32* sizes, double* dS,
                          const double* dcomm, size_t scap);
 

@@ -582,12 +582,20 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   prune_begin(E, L);
   if (gang_on) {
     S.cnt.ensure(E.mem, 16);
-    const u32 fr = all_active ? n : (u32)std::min<u64>(n, 2 * delta.k);
+    const bool det = E.cfg.mode == HL_MODE_DETERMINISTIC;
+    const u32 fr = det ? 0 : all_active ? n : (u32)std::min<u64>(n, 2 * delta.k);
     u32 why = gang_move(E, L, delta, true, all_active, mark_moved, fr, it, gm);
     if (why == MOVE_LABELS) {
       // Community ids must stay below n so that n + v is a fresh empty community.
       compact_labels_if_needed(E, L.f.p, n, n);
       why = gang_move(E, L, delta, true, all_active, mark_moved, fr, it, gm);
+    }
+    if (det) {
+      // sequential Gauss–Seidel (hit_leiden.rs:1103-1191): one iteration
+      inc_movement_det(E, L, S.gm_bits.p, S.d.p, ncap, mark_moved, &out.moves, &out.traversed);
+      out.iterations = 1;
+      E.kagg[KT_MOVE_EVAL].bytes += 16ull * out.traversed;
+      return out;
     }
     if (why == MOVE_DONE) {
       out.iterations = it;
@@ -622,14 +630,6 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
       HL_CUDA(cudaMemsetAsync(E.prune.shift, 0, 2 * sizeof(double), st));
     }
   }
-  if (E.cfg.mode == HL_MODE_DETERMINISTIC) {
-    // sequential Gauss–Seidel (hit_leiden.rs:1103-1191): one iteration
-    inc_movement_det(E, L, S.d.p, ncap, mark_moved, &out.moves, &out.traversed);
-    out.iterations = 1;
-    E.kagg[KT_MOVE_EVAL].bytes += 16ull * out.traversed;
-    return out;
-  }
-
   S.act.ensure(E.mem, n);
   S.cand_to.ensure(E.mem, n);
   S.cand_gain.ensure(E.mem, n);

@@ -169,3 +169,34 @@ def test_bounds_change_nothing(integral, gamma, multi):
             assert np.array_equal(gs.current_subcommunity_mapping_per_level[p],
                                   ref.get_map(p, O.MAP_S_CUR))
     gs.close()
+
+
+# Deterministic mode takes up to 128 pops together and keeps its state in shared
+# memory by size: bit sets, labels (32768 nodes) and community degrees (10240).
+# Rows above 128 entries take the whole block.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("n,m", [(60, 200), (10240, 21000), (10241, 21000), (33000, 60000)])
+def test_deterministic_sizes(n, m, integral):
+    import importlib
+    hl = importlib.import_module("hit-leiden_b200")
+    rng = np.random.default_rng(n)
+    s, d, w = gh.random_graph(rng, n, m, integral)
+    hub = rng.permutation(n)[: min(n // 2, 700)].astype(np.uint32)
+    hub = hub[hub != 3]
+    s, d = np.concatenate([s, np.full(len(hub), 3, np.uint32)]), np.concatenate([d, hub])
+    w = np.concatenate([w, np.ones(len(hub)) if integral else rng.uniform(0.5, 2.0, len(hub))])
+    gs = hl.PartitionState.load(hl.GraphInput.from_arrays("det", n, s, d, w),
+                                hl.RunConfig(mode=hl.RunMode.Deterministic, max_iterations=1))
+    ref = O.State(n, levels=1, mode=O.MODE_DETERMINISTIC)
+    ref.push_empty_graph()
+    ref.hit_leiden(s, d, w)
+    for i in range(2):
+        ds = rng.integers(0, n, 200).astype(np.uint32)
+        dd = rng.integers(0, n, 200).astype(np.uint32)
+        dw = rng.integers(1, 4, 200).astype(float) if integral else rng.uniform(0.5, 2.0, 200)
+        gs.apply_batch(ds, dd, dw)
+        ref.hit_leiden(ds, dd, dw)
+        assert np.array_equal(gs.community_mapping_per_level[0], ref.get_map(0, O.MAP_F))
+        assert np.array_equal(gs.current_subcommunity_mapping_per_level[0],
+                              ref.get_map(0, O.MAP_S_CUR))
+    gs.close()
