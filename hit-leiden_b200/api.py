@@ -465,7 +465,7 @@ def run(graph: GraphInput, config: Optional[RunConfig] = None, keep_state: bool 
         if p < len(subs):
             chain = subs[p][chain]
     res = PartitionResult(run_id=f"run:{graph.dataset_id}", node_to_community=part,
-                          hierarchy_levels=levels, community_count=int(len(np.unique(part))),
+                          hierarchy_levels=levels, community_count=int(part.max()) + 1 if len(part) else 0,
                           quality_score=q, iteration_count=0)
     out = RunOutcome(partition=res, state=st if keep_state else None)
     if not keep_state:

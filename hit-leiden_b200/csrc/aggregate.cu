@@ -28,14 +28,17 @@ __device__ __forceinline__ bool agg_emit(u32 v, u32 nb, const u8* refined, const
   return changed_only && !refined[nb];
 }
 
-__device__ __forceinline__ u64 pair_key(u32 a, u32 b) {
-  return a <= b ? (((u64)a << 32) | b) : (((u64)b << 32) | a);
+// Key of an unordered pair of ids below 2^bits, larger id in the low bits: a
+// radix sort passes over 2·bits of it (38 for 300k ids: 5 passes, where ids in
+// the two halves of 64 bits take 7).
+__device__ __forceinline__ u64 pair_key(u32 a, u32 b, u32 bits) {
+  return a <= b ? (((u64)a << bits) | b) : (((u64)b << bits) | a);
 }
 
 __global__ void k_agg_lift(const u32* u, const u32* v, const double* w, u64 k, const u32* s_pre,
-                           u64* keys, double* vals, u32* seq) {
+                           u32 bits, u64* keys, double* vals, u32* seq) {
   for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < k; i += (u64)gridDim.x * blockDim.x) {
-    keys[i] = pair_key(s_pre[u[i]], s_pre[v[i]]);
+    keys[i] = pair_key(s_pre[u[i]], s_pre[v[i]], bits);
     vals[i] = w ? w[i] : 1.0;
     seq[i] = (u32)i;
   }
@@ -47,8 +50,8 @@ __global__ void k_agg_lift(const u32* u, const u32* v, const double* w, u64 k, c
 // With `pos == nullptr` only the per-vertex record count is produced.
 __global__ void k_agg_rows(u32 n, const u64* off, const u32* col, const double* w,
                            const u8* refined, const u32* s_pre, const u32* s_cur,
-                           bool changed_only, bool edge_weight_loops, u64* cnt, const u64* pos,
-                           u64 base, u64* keys, double* vals, u32* seq) {
+                           bool changed_only, bool edge_weight_loops, u32 bits, u64* cnt,
+                           const u64* pos, u64 base, u64* keys, double* vals, u32* seq) {
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
@@ -89,10 +92,10 @@ __global__ void k_agg_rows(u32 n, const u64* off, const u32* col, const double* 
         const u32 m = __ballot_sync(0xffffffffu, emit);
         if (pos && emit) {
           const u64 at = o + 2ull * __popc(m & ((1u << lane) - 1u));
-          keys[at] = pair_key(sp, np_[j]);
+          keys[at] = pair_key(sp, np_[j], bits);
           vals[at] = -x[j];
           seq[at] = (u32)at;
-          keys[at + 1] = pair_key(sc, nc[j]);
+          keys[at + 1] = pair_key(sc, nc[j], bits);
           vals[at + 1] = x[j];
           seq[at + 1] = (u32)(at + 1);
         }
@@ -112,10 +115,10 @@ __global__ void k_agg_rows(u32 n, const u64* off, const u32* col, const double* 
       if (!pos) {
         cnt[v] = c + (loop ? 2 : 0);
       } else if (loop) {
-        keys[o] = pair_key(sp, sp);
+        keys[o] = pair_key(sp, sp, bits);
         vals[o] = -slw;
         seq[o] = (u32)o;
-        keys[o + 1] = pair_key(sc, sc);
+        keys[o + 1] = pair_key(sc, sc, bits);
         vals[o + 1] = slw;
         seq[o + 1] = (u32)(o + 1);
       }
@@ -133,33 +136,43 @@ __global__ void k_seg_start64(const u32* head, const u32* segid, u64 n, u32* sta
     if (head[i]) start[segid[i]] = (u32)i;
 }
 
-// One compressed record: the key of segment j (starting at a), its sum x.
-__device__ __forceinline__ void compress_out(u64 j, u64 a, double x, const u64* sk,
-                                             double threshold, u32* ou, u32* ov, double* ow,
-                                             u8* keepf) {
-  if ((threadIdx.x & 31) == 0) {
-    u64 key = sk[a];
-    ou[j] = (u32)(key >> 32);
-    ov[j] = (u32)key;
-    ow[j] = x;
-    keepf[j] = fabs(x) > threshold ? 1 : 0;
-  }
-}
-
 // In-order segmented sum over the records' weights gathered into sorted
-// order (sw); keep |w| > threshold.
-__global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 total,
+// order (sw); keep |w| > threshold.  Most keys have a few records: a lane each
+// (a warp each took 340 us for 300k segments, 32 lanes for one addition);
+// longer segments take the warp, one after another.
+constexpr u32 COMPRESS_LANE = 16;
+
+__global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 total, u32 bits,
                                                   const u64* sk, const double* sw,
                                                   double threshold, u32* ou, u32* ov, double* ow,
                                                   u8* keepf) {
   __shared__ __align__(16) double chain[8][CHAIN_TILE];
+  const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  for (u64 j = warp; j < U; j += nwarps) {
-    const u64 a = start[j], b = (j + 1 < U) ? start[j + 1] : total;
-    const double x =
-        b - a == 1 ? sw[a] : warp_chain_sum(a, b, 0.0, sw, chain[threadIdx.x >> 5]);
-    compress_out(j, a, x, sk, threshold, ou, ov, ow, keepf);
+  for (u64 j0 = warp * 32; j0 < U; j0 += nwarps * 32) {
+    const u64 j = j0 + lane;
+    const u64 a = j < U ? start[j] : 0, b = j < U ? (j + 1 < U ? start[j + 1] : total) : 0;
+    double x = 0.0;
+    if (b - a == 1) {
+      x = sw[a];
+    } else if (b - a <= COMPRESS_LANE) {
+      for (u64 t = a; t < b; ++t) x = __dadd_rn(x, sw[t]);
+    }
+    for (u32 m = __ballot_sync(0xffffffffu, b - a > COMPRESS_LANE); m; m &= m - 1) {
+      const u32 l = __ffs(m) - 1;
+      const double y = warp_chain_sum(__shfl_sync(0xffffffffu, a, l),
+                                      __shfl_sync(0xffffffffu, b, l), 0.0, sw,
+                                      chain[threadIdx.x >> 5]);
+      if (lane == l) x = y;
+    }
+    if (j < U) {
+      const u64 key = sk[a];
+      ou[j] = (u32)(key >> bits);
+      ov[j] = (u32)(key & ((1ull << bits) - 1));
+      ow[j] = x;
+      keepf[j] = fabs(x) > threshold ? 1 : 0;
+    }
   }
 }
 
@@ -176,8 +189,8 @@ __global__ void k_set_spre(u32 n, const u8* refined, const u32* s_cur, u32* s_pr
 
 // Sort (key, seq) records, sum each key in push order, drop |w| <= threshold.
 // Output edges land in sc.eu2 / ev2 / ew2 in ascending key order.
-// Keys are pair_key(a, b) of ids below id_bound.
-static u64 compress_records(Engine& E, u64 R, double threshold, u32 id_bound) {
+// Keys are pair_key(a, b, bits).
+static u64 compress_records(Engine& E, u64 R, double threshold, u32 bits) {
   Scratch& S = E.sc;
   cudaStream_t st = E.stream;
   if (!R) return 0;
@@ -186,8 +199,7 @@ static u64 compress_records(Engine& E, u64 R, double threshold, u32 id_bound) {
   u32* vi = S.idx.p;
   u32* vo = S.idx2.p;
   cub_run(E, [&](void* t, size_t& b) {
-    return cub::DeviceRadixSort::SortPairs(t, b, ki, ko, vi, vo, (int64_t)R, 0,
-                                           32 + bits_for(id_bound ? id_bound - 1 : 0), st);
+    return cub::DeviceRadixSort::SortPairs(t, b, ki, ko, vi, vo, (int64_t)R, 0, (int)(2 * bits), st);
   });
   S.rowlist.ensure(E.mem, R);
   S.segid.ensure(E.mem, R);
@@ -209,8 +221,8 @@ static u64 compress_records(Engine& E, u64 R, double threshold, u32 id_bound) {
   S.op.ensure(E.mem, U);
   S.fvals.ensure(E.mem, R);
   ++E.nlaunch, k_gather_weights<<<grid_for(R), 256, 0, st>>>(vo, S.neww.p, R, S.fvals.p);
-  ++E.nlaunch, k_compress<<<grid_for((u64)U * 32), 256, 0, st>>>(
-      U, S.seg_start.p, R, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p, S.op.p);
+  ++E.nlaunch, k_compress<<<grid_for(U), 256, 0, st>>>(
+      U, S.seg_start.p, R, bits, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p, S.op.p);
   HL_LAUNCH_CHECK();
   S.eu2.ensure(E.mem, U);
   S.ev2.ensure(E.mem, U);
@@ -261,11 +273,12 @@ u64 inc_aggregation(Engine& E, Level& L, const DevEdges& delta, u32* next_n, boo
     }
     *next_n = (m1 > m2 ? m1 : m2) + 1;
   }
+  const u32 bits = (u32)bits_for(*next_n - 1);
   S.newoff.ensure(E.mem, (size_t)n + 1);
   S.gkey2.ensure(E.mem, (size_t)n + 1);
   ++E.nlaunch, k_agg_rows<<<grid_for((u64)n * 32), 256, 0, st>>>(
       n, L.g.off.p, L.g.col.p, L.g.w.p, S.refined.p, L.s_pre.p, L.s_cur.p, changed_only,
-      edge_weight_loops, S.newoff.p, nullptr, 0, nullptr, nullptr, nullptr);
+      edge_weight_loops, bits, S.newoff.p, nullptr, 0, nullptr, nullptr, nullptr);
   HL_CUDA(cudaMemsetAsync(S.newoff.p + n, 0, sizeof(u64), st));
   HL_LAUNCH_CHECK();
   u64* a = S.newoff.p;
@@ -283,13 +296,13 @@ u64 inc_aggregation(Engine& E, Level& L, const DevEdges& delta, u32* next_n, boo
     S.neww.ensure(E.mem, R);
     if (delta.k)
       ++E.nlaunch, k_agg_lift<<<grid_for(delta.k), 256, 0, st>>>(delta.u, delta.v, delta.w, delta.k, L.s_pre.p,
-                                                    S.keys.p, S.neww.p, S.idx.p);
+                                                    bits, S.keys.p, S.neww.p, S.idx.p);
     ++E.nlaunch, k_agg_rows<<<grid_for((u64)n * 32), 256, 0, st>>>(
         n, L.g.off.p, L.g.col.p, L.g.w.p, S.refined.p, L.s_pre.p, L.s_cur.p, changed_only,
-        edge_weight_loops, nullptr, pos, delta.k, S.keys.p, S.neww.p, S.idx.p);
+        edge_weight_loops, bits, nullptr, pos, delta.k, S.keys.p, S.neww.p, S.idx.p);
     HL_LAUNCH_CHECK();
   }
-  u64 out = compress_records(E, R, 1e-9, *next_n);
+  u64 out = compress_records(E, R, 1e-9, bits);
   ++E.nlaunch, k_set_spre<<<grid_for(n), 256, 0, st>>>(n, S.refined.p, L.s_cur.p, L.s_pre.p);
   HL_LAUNCH_CHECK();
   E.kt_end(KT_AGGREGATE, kev);
@@ -302,31 +315,34 @@ u64 inc_aggregation(Engine& E, Level& L, const DevEdges& delta, u32* next_n, boo
 
 // Bootstrap aggregation of G^p by s: every undirected edge once (a self-loop
 // counted once), summed per (s(u), s(v)) in (u ascending, CSR) order.
-__global__ void k_full_count(u32 n, const u64* off, const u32* col, u64* cnt) {
-  for (u64 v = blockIdx.x * (u64)blockDim.x + threadIdx.x; v < n; v += (u64)gridDim.x * blockDim.x) {
-    u64 c = 0;
-    for (u64 p = off[v]; p < off[v + 1]; ++p) {
-      u32 nb = col[p];
-      if (nb < v) continue;
-      if (nb == v && p + 1 < off[v + 1] && col[p + 1] == (u32)v) continue;
-      ++c;
-    }
-    cnt[v] = c;
-  }
+// The counted entries of row v are its last ones: neighbours above v, and the
+// second copy of its self-loop.
+__device__ __forceinline__ u64 full_first(u32 v, u64 o0, u64 o1, const u32* col) {
+  const u64 p = lower_bound_u32(col, o0, o1, v);
+  return p + 1 < o1 && col[p + 1] == v ? p + 1 : p;
 }
 
+__global__ void k_full_count(u32 n, const u64* off, const u32* col, u64* cnt) {
+  for (u64 v = blockIdx.x * (u64)blockDim.x + threadIdx.x; v < n; v += (u64)gridDim.x * blockDim.x)
+    cnt[v] = off[v + 1] - full_first((u32)v, off[v], off[v + 1], col);
+}
+
+// Eight lanes a row (a thread a row walked hub rows alone, uncoalesced: 0.8 ms
+// for 300k rows of 20, where this streams).
 __global__ void k_full_emit(u32 n, const u64* off, const u32* col, const double* w, const u32* s,
-                            const u64* pos, u64* keys, double* vals, u32* seq) {
-  for (u64 v = blockIdx.x * (u64)blockDim.x + threadIdx.x; v < n; v += (u64)gridDim.x * blockDim.x) {
-    u64 o = pos[v];
-    for (u64 p = off[v]; p < off[v + 1]; ++p) {
-      u32 nb = col[p];
-      if (nb < v) continue;
-      if (nb == v && p + 1 < off[v + 1] && col[p + 1] == (u32)v) continue;
-      keys[o] = pair_key(s[v], s[nb]);
+                            const u64* pos, u32 bits, u64* keys, double* vals, u32* seq) {
+  const u32 sub = threadIdx.x & 7;
+  const u64 group = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 3;
+  const u64 ngroups = ((u64)gridDim.x * blockDim.x) >> 3;
+  for (u64 v = group; v < n; v += ngroups) {
+    const u64 o0 = pos[v], o1 = pos[v + 1];
+    const u64 p0 = off[v + 1] - (o1 - o0);
+    const u32 sv = s[v];
+    for (u64 o = o0 + sub; o < o1; o += 8) {
+      const u64 p = p0 + (o - o0);
+      keys[o] = pair_key(sv, s[col[p]], bits);
       vals[o] = w[p];
       seq[o] = (u32)o;
-      ++o;
     }
   }
 }
@@ -352,10 +368,11 @@ u64 aggregate_full(Engine& E, Level& L, const u32* s, u32*, u32*, double*) {
   S.idx.ensure(E.mem, R);
   S.idx2.ensure(E.mem, R);
   S.neww.ensure(E.mem, R);
-  ++E.nlaunch, k_full_emit<<<grid_for(n), 256, 0, st>>>(n, L.g.off.p, L.g.col.p, L.g.w.p, s, pos, S.keys.p,
-                                           S.neww.p, S.idx.p);
+  const u32 bits = (u32)bits_for(n - 1);
+  ++E.nlaunch, k_full_emit<<<grid_for((u64)n * 8), 256, 0, st>>>(
+      n, L.g.off.p, L.g.col.p, L.g.w.p, s, pos, bits, S.keys.p, S.neww.p, S.idx.p);
   HL_LAUNCH_CHECK();
-  return compress_records(E, R, -1.0, n);
+  return compress_records(E, R, -1.0, bits);
 }
 
 // f^{p+1}(s^p(v)) := f^p(v); with several members the largest v writes last,

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 
 #include "../../include/hl_debug.h"
 #include "hl_engine.cuh"
@@ -19,6 +20,48 @@ void hl_set_error_message(const std::string& m) { g_err = m; }
 
 
 namespace hl {
+
+// Blocks of 64 words, portable across devices; at most PINNED_KEEP wait for
+// their next use, the rest are given back at once.
+constexpr size_t PINNED_KEEP = 64;
+struct PinnedPool {
+  std::mutex mu;
+  std::vector<u64*> free;
+  ~PinnedPool() {
+    for (u64* p : free) cudaFreeHost(p);
+  }
+};
+static PinnedPool& pinned_pool() {
+  static PinnedPool pool;
+  return pool;
+}
+u64* pinned_take() {
+  PinnedPool& P = pinned_pool();
+  {
+    std::lock_guard<std::mutex> lk(P.mu);
+    if (!P.free.empty()) {
+      u64* p = P.free.back();
+      P.free.pop_back();
+      return p;
+    }
+  }
+  u64* p = nullptr;
+  HL_CUDA(cudaHostAlloc((void**)&p, 64 * sizeof(u64), cudaHostAllocPortable));
+  return p;
+}
+// The owner's stream has been waited for: no copy into the block is in flight.
+void pinned_give(u64* p) {
+  if (!p) return;
+  PinnedPool& P = pinned_pool();
+  {
+    std::lock_guard<std::mutex> lk(P.mu);
+    if (P.free.size() < PINNED_KEEP) {
+      P.free.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
 
 u64 Engine::read_u64(const u64* d) {
   if (ktiming) ++kagg[KT_HOST_SYNC].launches;

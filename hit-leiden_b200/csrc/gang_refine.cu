@@ -592,10 +592,11 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) 
 
 static std::atomic<bool> g_ref_attr[64];
 
-// The bootstrap refines every vertex of every level from the identity, which
-// the kernel hands back.
+// The bootstrap refines every vertex of every level from the identity: worth
+// one launch while one block per SM has few singletons a warp.
 bool gang_refine_fits(Engine& E, const Level& L) {
-  return L.g.n > 0 && L.g.n < (1u << 30) && !E.in_bootstrap;
+  return L.g.n > 0 && L.g.n < (1u << 30) &&
+         (!E.in_bootstrap || L.g.n <= 16 * GANG_WARPS * GANG_MAX_BLOCKS);
 }
 
 // One launch of the refinement.  The caller continues on the multi-kernel path
@@ -612,7 +613,8 @@ u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   }
   const u64 nslice = L.g.nnz / REF_SLICE + 1;
   const u64 scap = (u64)L.s_bound + n;
-  const GangShape shape = gang_shape(E, 2ull * n + L.g.nnz / 8);
+  const GangShape shape =
+      gang_shape(E, 2ull * n + L.g.nnz / 8 + (E.in_bootstrap ? 128ull * n : 0));
   S.refined.ensure(E.mem, ((size_t)n + 3) & ~(size_t)3);
   S.gr_bits.ensure(E.mem, (L.s_bound + 31) / 32 + (scap + 31) / 32 + (2ull * n + 33) / 32);
   S.par.ensure(E.mem, n);

@@ -175,6 +175,10 @@ struct Prune {
 };
 
 struct Engine {
+  // the staging block and the buffers go back with nothing in flight
+  ~Engine() {
+    if (stream) cudaStreamSynchronize(stream);
+  }
   hl_config cfg{};
   int device = 0;
   cudaStream_t stream = nullptr;

@@ -147,13 +147,17 @@ struct DBuf {
   T* get() const { return p; }
 };
 
-// Pinned host staging for small scalar read-backs.
+// Pinned host staging for small scalar read-backs.  Blocks come from a bounded
+// process-wide pool (api.cu): pinning 512 bytes and unpinning them costs more
+// than a small call's kernels (hl_canonicalize of 1,000 labels: 250 us).
+u64* pinned_take();
+void pinned_give(u64* p);
 struct HostScalars {
-  u64* p = nullptr;
-  explicit HostScalars() { HL_CUDA(cudaMallocHost((void**)&p, 64 * sizeof(u64))); }
-  ~HostScalars() {
-    if (p) cudaFreeHost(p);
-  }
+  u64* p = pinned_take();
+  HostScalars() = default;
+  HostScalars(const HostScalars&) = delete;
+  HostScalars& operator=(const HostScalars&) = delete;
+  ~HostScalars() { pinned_give(p); }
 };
 
 inline u32 div_up(u64 a, u64 b) { return (u32)((a + b - 1) / b); }
