@@ -650,7 +650,14 @@ namespace hl {
 // Entry points for the multi-graph executors (multi.cu): one batch on one
 // handle, with the error captured for the calling thread; device bytes held.
 hl_status apply_on_handle(hl_graph* g, const uint32_t* src, const uint32_t* dst, const double* w,
-                          uint64_t k, hl_batch_stats* stats, std::string* err) {
+                          uint64_t k, bool shared, hl_batch_stats* stats, std::string* err) {
+  struct Shared {  // for this batch only
+    Engine* E;
+    ~Shared() {
+      if (E) E->shared = false;
+    }
+  } guard{g ? box(g)->E.get() : nullptr};
+  if (guard.E) guard.E->shared = shared;
   try {
     apply_impl(g, src, dst, w, k, false, stats);
     return HL_OK;
@@ -811,10 +818,13 @@ static void get_partition_impl(const hl_graph* g, uint32_t* out) {
   Level& L = E.levels[0];
   u32 n = L.g.n;
   if (!n) return;
-  DBuf<u32> tmp;
-  tmp.ensure(E.mem, n);
-  canonicalize_device(E, L.f.p, n, tmp.p);
-  HL_CUDA(cudaMemcpyAsync(out, tmp.p, sizeof(u32) * n, cudaMemcpyDeviceToHost, E.stream));
+  // a level's community ids come from the levels above it: below twice the
+  // size of the largest, plus two
+  u32 top = 0;
+  for (const Level& l : E.levels) top = std::max(top, l.g.n);
+  E.sc.canon.ensure(E.mem, n);
+  canonicalize_bounded(E, L.f.p, n, 2 * top + 2, E.sc.canon.p);
+  HL_CUDA(cudaMemcpyAsync(out, E.sc.canon.p, sizeof(u32) * n, cudaMemcpyDeviceToHost, E.stream));
   E.sync();
 }
 

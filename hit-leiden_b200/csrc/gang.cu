@@ -14,10 +14,17 @@ static u32 sm_count(int device) {
 
 // One block up to a few thousand entries (its barrier is a block barrier), a
 // portable cluster of 8 up to a few hundred thousand, above that one block
-// per SM.
+// per SM.  While other graphs are being updated too, a grid that needs every SM
+// at once waits for all of their kernels: there clusters go on to a few million
+// entries (48 graphs of 1k-30k vertices on 16 host threads: 18.5 ms a batch
+// each with grids, 12 ms with clusters; one graph at a time: 97 and 104 ms).
+constexpr u64 GANG_BLOCK_WORK = 4096;
+constexpr u64 GANG_CLUSTER_WORK = 400000;
+constexpr u64 GANG_SHARED_WORK = 4000000;
+
 GangShape gang_shape(Engine& E, u64 work) {
-  if (work <= 4096) return GangShape{1, false};
-  if (work <= 400000) return GangShape{8, false};
+  if (work <= GANG_BLOCK_WORK) return GangShape{1, false};
+  if (work <= (E.shared ? GANG_SHARED_WORK : GANG_CLUSTER_WORK)) return GangShape{8, false};
   const u32 sms = sm_count(E.device);
   return GangShape{sms < GANG_MAX_BLOCKS ? sms : GANG_MAX_BLOCKS, true};
 }

@@ -121,6 +121,7 @@ struct Scratch {
   DBuf<u32> lvl_prev, lvl_nodes, lvl_ids;
   DBuf<u8> lvl_flag;
   // single-launch stages (gang.cuh)
+  DBuf<u32> canon;  // the canonical partition before it is copied out
   DBuf<u32> gang_part, gang_cnt, ga_touched, gr_bits, gm_bits, gm_hist;
   DBuf<unsigned short> gm_slot;
   DBuf<double> gm_w;
@@ -204,6 +205,7 @@ struct Engine {
   bool k_flags_set = false;
   u32 prune_rounds = 0;  // multi-kernel evaluations of the running movement
   Prune prune;           // the running movement's bounds (b == nullptr: off)
+  bool shared = false;   // other graphs are being updated on the GPU meanwhile
   u64 sum_nv_batch = 0;  // frontier sizes of the multi-kernel evaluations, this call
   // degree-bin thresholds picked by the autotuner (0 = compile-time default)
   struct Tune {
@@ -337,8 +339,10 @@ void project_up(Engine& E, Level& lo, Level& hi, u8* changed_flags = nullptr);
 void top_down(Engine& E);
 void inherit_new_nodes(Engine& E, Level& hi);
 
-// modularity.cu
+// gang_modularity.cu
 double modularity(Engine& E, Level& L, const u32* part);
+void canonicalize_bounded(Engine& E, const u32* labels, u32 n, u32 bound, u32* out);
+// modularity.cu
 void canonicalize_device(Engine& E, u32* labels, u64 n, u32* out);
 u32 rank_compact(Engine& E, u32* labels, u32 n, u32 id_bound);
 

@@ -34,7 +34,7 @@
 
 namespace hl {
 hl_status apply_on_handle(hl_graph* g, const uint32_t* src, const uint32_t* dst, const double* w,
-                          uint64_t k, hl_batch_stats* stats, std::string* err);
+                          uint64_t k, bool shared, hl_batch_stats* stats, std::string* err);
 uint64_t handle_device_bytes(const hl_graph* g);
 }  // namespace hl
 
@@ -202,11 +202,17 @@ struct hl_server {
       lc->have_l0 = false;
       if (level_fn.load()) hl_set_level_callback(g, level_trampoline, lc);
       else hl_set_level_callback(g, nullptr, nullptr);
+      bool shared;  // more than two graphs may be updated side by side
+      {
+        std::lock_guard<std::mutex> lk(mu);
+        shared = std::min(workers.size(), graphs.size()) > 2;
+      }
       const Clock::time_point t0 = Clock::now();
       hl_batch_stats st{};
       std::string err;
       const hl_status rc = hl::apply_on_handle(g, src.data(), dst.data(),
-                                               any_w ? w.data() : nullptr, src.size(), &st, &err);
+                                               any_w ? w.data() : nullptr, src.size(), shared,
+                                               &st, &err);
       const Clock::time_point t1 = Clock::now();
       const uint64_t held = hl::handle_device_bytes(g);  // this worker owns g here
       {
@@ -314,7 +320,7 @@ HL_API hl_status hl_apply_batches(hl_graph* const* graphs, const uint32_t* const
       if (t >= count) return;
       const uint32_t i = order[t];
       rc[i] = hl::apply_on_handle(graphs[i], src[i], dst[i], w ? w[i] : nullptr, k[i],
-                                  stats ? &stats[i] : nullptr, &msg[i]);
+                                  workers > 2, stats ? &stats[i] : nullptr, &msg[i]);
     }
   };
   std::vector<std::thread> pool;

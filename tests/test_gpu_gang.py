@@ -200,3 +200,28 @@ def test_deterministic_sizes(n, m, integral):
         assert np.array_equal(gs.current_subcommunity_mapping_per_level[0],
                               ref.get_map(0, O.MAP_S_CUR))
     gs.close()
+
+
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_modularity_and_partition_shapes(shape, integral):
+    # labels: one community, a few large ones, one vertex each, values far above
+    # n; the hub's row and long communities take a whole warp
+    import importlib
+    hl = importlib.import_module("hit-leiden_b200")
+    g = _base(shape, integral)
+    off, col, w = g.csr()
+    src = np.repeat(np.arange(g.n, dtype=np.uint32), np.diff(off).astype(np.int64))
+    once = src < col
+    st = hl.PartitionState.load(
+        hl.GraphInput.from_arrays(shape, g.n, src[once], col[once], w[once]),
+        hl.RunConfig(mode=hl.RunMode.Throughput, max_iterations=1))
+    ref = O.Graph.from_edges(g.n, src[once], col[once], w[once])
+    rng = np.random.default_rng(3)
+    for part in (np.zeros(g.n, np.uint32), rng.integers(0, 5, g.n).astype(np.uint32),
+                 np.arange(g.n, dtype=np.uint32),
+                 (rng.integers(0, 300, g.n) * 70001).astype(np.uint32)):
+        q = O.modularity_csr(ref, part)
+        assert abs(st.modularity(part) - q) <= 1e-12 * max(1.0, abs(q))
+    assert np.array_equal(st.partition(), O.canonicalize(st.community_mapping_per_level[0]))
+    st.close()
