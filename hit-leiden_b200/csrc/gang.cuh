@@ -137,9 +137,90 @@ __device__ __forceinline__ u32 gang_scan(const Gang& G, GangSmem& S, u32 N, V va
   return total;
 }
 
+// Ascending sort of P (key, value) records (a power of two from 64 to
+// GSORT_CHUNK) by (key, value) into S.key / S.val, by the block: every warp
+// sorts 32 records through its lanes, then runs merge pairwise, each record
+// finding its place by a bisection in the sibling run.  2048 records: 24 us as
+// a bitonic network in shared memory (66 stages of 48 KB traffic), a third of
+// that this way.
+template <typename K, typename VL>
+__device__ __forceinline__ void block_sort(GangSmem& S, u32 P, K key_of, VL val_of) {
+  constexpr u32 PER = GSORT_CHUNK / GANG_THREADS;
+  const u32 tid = threadIdx.x, lane = tid & 31;
+  u64 k[PER];
+  u32 v[PER];
+#pragma unroll
+  for (u32 j = 0; j < PER; ++j) {
+    const u32 e = tid + j * GANG_THREADS;
+    if (e >= P) break;  // warp-uniform
+    k[j] = key_of(e);
+    v[j] = val_of(e);
+  }
+#pragma unroll
+  for (u32 j = 0; j < PER; ++j) {
+    const u32 e = tid + j * GANG_THREADS;
+    if (e >= P) break;
+#pragma unroll
+    for (u32 size = 2; size <= 32; size <<= 1)
+#pragma unroll
+      for (u32 stride = size >> 1; stride; stride >>= 1) {
+        const u64 ok = __shfl_xor_sync(0xffffffffu, k[j], stride);
+        const u32 ov = __shfl_xor_sync(0xffffffffu, v[j], stride);
+        const bool less = ok < k[j] || (ok == k[j] && ov < v[j]);
+        const bool want_less = ((lane & size) == 0 || size == 32) == ((lane & stride) == 0);
+        const bool differ = ok != k[j] || ov != v[j];
+        if (differ && less == want_less) {
+          k[j] = ok;
+          v[j] = ov;
+        }
+      }
+    S.key[e] = k[j];
+    S.val[e] = v[j];
+  }
+  __syncthreads();
+  for (u32 run = 32; run < P; run <<= 1) {
+    u32 pos[PER];
+#pragma unroll
+    for (u32 j = 0; j < PER; ++j) {
+      const u32 e = tid + j * GANG_THREADS;
+      pos[j] = 0;
+      if (e >= P) break;
+      k[j] = S.key[e];
+      v[j] = S.val[e];
+    }
+    for (u32 half = run; half; half >>= 1) {
+#pragma unroll
+      for (u32 j = 0; j < PER; ++j) {
+        const u32 e = tid + j * GANG_THREADS;
+        if (e >= P) break;
+        const u32 sib = (e & ~(run - 1)) ^ run;
+        if (pos[j] + half > run) continue;
+        const u32 at = sib + pos[j] + half - 1;
+        const u64 x = S.key[at];
+        bool before = x < k[j];
+        if (x == k[j]) {  // equal records: the left run's come first
+          const u32 y = S.val[at];
+          before = y < v[j] || (y == v[j] && sib < e);
+        }
+        if (before) pos[j] += half;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (u32 j = 0; j < PER; ++j) {
+      const u32 e = tid + j * GANG_THREADS;
+      if (e >= P) break;
+      const u32 to = (e & ~(2 * run - 1)) + (e & (run - 1)) + pos[j];
+      S.key[to] = k[j];
+      S.val[to] = v[j];
+    }
+    __syncthreads();
+  }
+}
+
 // Ascending sort of N (key, value) records by (key, value); with the record's
 // index as its value, the stable sort by key.  Blocks sort chunks of up to
-// GSORT_CHUNK records in shared memory (bitonic); after a barrier every record
+// GSORT_CHUNK records in shared memory; after a barrier every record
 // finds its rank by a bisection in each other chunk and is handed to
 // emit(rank, key, value).  `tk`/`tv` take the sorted chunks.  Two gang barriers
 // inside (one when a single chunk holds everything); the caller's emitted
@@ -160,33 +241,9 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
     const u32 cnt = min(ch, N - base);
     u32 P = 64;  // the padded length of this chunk
     while (P < cnt) P <<= 1;
-    for (u32 i = tid; i < P; i += GANG_THREADS) {
-      S.key[i] = i < cnt ? key_of(base + i) : ~0ull;
-      S.val[i] = i < cnt ? val_of(base + i) : NONE32;
-    }
-    __syncthreads();
-    for (u32 size = 2; size <= P; size <<= 1) {
-      for (u32 stride = size >> 1; stride > 0; stride >>= 1) {
-        for (u32 x = tid; x < P / 2; x += GANG_THREADS) {
-          const u32 i = 2 * x - (x & (stride - 1));
-          const u32 j = i + stride;
-          const bool up = (i & size) == 0;
-          const u64 ki = S.key[i], kj = S.key[j];
-          const u32 vi = S.val[i], vj = S.val[j];
-          const bool gt = ki > kj || (ki == kj && vi > vj);
-          if (gt == up) {
-            S.key[i] = kj;
-            S.key[j] = ki;
-            S.val[i] = vj;
-            S.val[j] = vi;
-          }
-        }
-        // strides up to 32 stay within the 64 elements of one warp
-        if (stride > 32) __syncthreads();
-        else __syncwarp();
-      }
-      if (size >= 64) __syncthreads();
-    }
+    block_sort(
+        S, P, [&](u32 i) { return i < cnt ? key_of(base + i) : ~0ull; },
+        [&](u32 i) { return i < cnt ? val_of(base + i) : NONE32; });
     for (u32 i = tid; i < cnt; i += GANG_THREADS) {
       if (nch == 1) {
         emit(i, S.key[i], S.val[i]);
@@ -300,6 +357,68 @@ __device__ __forceinline__ void gang_label_sort(const Gang& G, GangSmem& S, u32 
     t = vo;
     vo = t == idx ? idx2 : idx;
     vi = t;
+  }
+}
+
+// Ordered sums of x over the segments of equal values in the ascending labels
+// lab[0..n): done(label, sum) is called by one lane per segment.  A warp takes
+// 32 positions and the segments that start there; one that ends within the next
+// position is the last of its 32, found by a 32-way search.  Segments of up to
+// 16 terms take a lane, longer ones the warp (`buf`: CHAIN_TILE doubles of it).
+template <typename T, typename DN>
+__device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T* lab,
+                                                  const double* x, double* buf, DN done) {
+  const u32 lane = threadIdx.x & 31;
+  for (u32 t0 = G.warp() * 32; t0 < n; t0 += G.warps() * 32) {
+    const u32 t = t0 + lane;
+    const T c = t < n ? lab[t] : T(0);
+    const T before = t < n && t > 0 ? lab[t - 1] : T(0);
+    const u32 hm = __ballot_sync(0xffffffffu, t < n && (t == 0 || before != c));
+    if (!hm) continue;
+    // the last segment's end
+    const u32 last = 31 - __clz(hm);
+    const T cl = __shfl_sync(0xffffffffu, c, last);
+    u32 lo = t0 + last, hi = n;  // lab[lo] == cl
+    u32 step = 1;                // most segments are short: gallop first
+    while (true) {
+      const u64 p = (u64)lo + (u64)step * (lane + 1);
+      const u32 m = __ballot_sync(0xffffffffu, p < hi && lab[p] == cl);
+      const u32 j = (u32)__popc(m);
+      if (j == 32) {
+        lo += 32 * step;
+        step *= 32;
+        continue;
+      }
+      const u64 nhi = (u64)lo + (u64)step * (j + 1);
+      lo += step * j;
+      hi = nhi < hi ? (u32)nhi : hi;
+      if (step == 1) break;
+      step /= 32;
+    }
+    const u32 end_last = lo + 1;
+    const bool head = (hm >> lane) & 1u;
+    const u32 above = hm & ~((2u << lane) - 1u);
+    const u32 end = above ? t0 + __ffs(above) - 1 : end_last;
+    const u32 len = head ? end - t : 0;
+    if (len && len <= 16) {
+      double s = 0.0;
+      u32 q = t;
+      for (; q + 4 <= end; q += 4) {
+        const double y0 = x[q], y1 = x[q + 1], y2 = x[q + 2], y3 = x[q + 3];
+        s = __dadd_rn(s, y0);
+        s = __dadd_rn(s, y1);
+        s = __dadd_rn(s, y2);
+        s = __dadd_rn(s, y3);
+      }
+      for (; q < end; ++q) s = __dadd_rn(s, x[q]);
+      done(c, s);
+    }
+    for (u32 bm = __ballot_sync(0xffffffffu, len > 16); bm; bm &= bm - 1) {
+      const u32 l = __ffs(bm) - 1;
+      const u32 e = __shfl_sync(0xffffffffu, end, l);
+      const double s = warp_chain_sum(t0 + l, e, 0.0, x, buf);
+      if (lane == l) done(c, s);
+    }
   }
 }
 

@@ -102,31 +102,9 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_modularity(GangModArgs
   G.sync();
   // ---- Σ_C d(C)²/2m ----
   DD expected{0.0, 0.0}, intra{0.0, 0.0};
-  for (u32 t0 = G.warp() * 32; t0 < A.n; t0 += G.warps() * 32) {
-    const u32 t = t0 + lane;
-    const u32 c = t < A.n ? lab[t] : NONE32;
-    const bool head = t < A.n && (t == 0 || lab[t - 1] != c);
-    bool more = false;
-    if (head) {  // small communities: a lane each
-      double x = 0.0;
-      u32 j = t;
-      for (; j < A.n && j < t + 16 && lab[j] == c; ++j) x = __dadd_rn(x, A.kval[j]);
-      more = j < A.n && lab[j] == c;
-      if (!more) expected = dd_add(expected, __ddiv_rn(__dmul_rn(x, x), A.tw));
-    }
-    for (u32 hm = __ballot_sync(0xffffffffu, more); hm; hm &= hm - 1) {
-      const u32 a = t0 + __ffs(hm) - 1;
-      const u32 ca = lab[a];
-      u32 lo = a + 16, hi = A.n;  // first index past the community
-      while (lo < hi) {
-        const u32 mid = lo + (hi - lo) / 2;
-        if (lab[mid] <= ca) lo = mid + 1;
-        else hi = mid;
-      }
-      const double x = warp_chain_sum(a, lo, 0.0, A.kval, chain[threadIdx.x >> 5]);
-      if (lane == 0) expected = dd_add(expected, __ddiv_rn(__dmul_rn(x, x), A.tw));
-    }
-  }
+  gang_segment_sums(G, A.n, lab, A.kval, chain[threadIdx.x >> 5], [&](u32, double x) {
+    expected = dd_add(expected, __ddiv_rn(__dmul_rn(x, x), A.tw));
+  });
   // ---- intra weight: eight lanes a row, taken by the warps as they come ----
   const u32 sub = lane & 7;
   const u32 chunks = (A.n + MOD_ROWS - 1) / MOD_ROWS;

@@ -331,32 +331,8 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       const u32* idx = second ? A.idx2 : A.idx;
       for (u32 t = gt; t < A.n; t += gts) A.kval[t] = A.k[idx[t]];
       G.sync();
-      double* buf = M.w.sw[tid >> 5];
-      for (u32 t0 = G.warp() * 32; t0 < A.n; t0 += G.warps() * 32) {
-        const u32 t = t0 + lane;
-        const u32 c = t < A.n ? lab[t] : NONE32;
-        const bool head = t < A.n && (t == 0 || lab[t - 1] != c);
-        bool more = false;
-        if (head) {  // small communities: a lane each
-          double x = 0.0;
-          u32 j = t;
-          for (; j < A.n && j < t + 16 && lab[j] == c; ++j) x = __dadd_rn(x, A.kval[j]);
-          more = j < A.n && lab[j] == c;
-          if (!more) A.d[c] = x;
-        }
-        for (u32 hm = __ballot_sync(0xffffffffu, more); hm; hm &= hm - 1) {
-          const u32 a = t0 + __ffs(hm) - 1;
-          const u32 ca = lab[a];
-          u32 lo = a + 16, hi = A.n;  // first index past the community
-          while (lo < hi) {
-            const u32 mid = lo + (hi - lo) / 2;
-            if (lab[mid] <= ca) lo = mid + 1;
-            else hi = mid;
-          }
-          const double x = warp_chain_sum(a, lo, 0.0, A.kval, buf);
-          if (lane == 0) A.d[ca] = x;
-        }
-      }
+      gang_segment_sums(G, A.n, lab, A.kval, M.w.sw[tid >> 5],
+                        [&](u32 c, double x) { A.d[c] = x; });
     }
     G.sync();
   } else {

@@ -21,7 +21,6 @@ constexpr u32 REF_SLICE = 256;
 constexpr u32 REF_MAXDEG = 256;    // singleton rows evaluated here
 constexpr u32 REF_TAB = 2 * REF_MAXDEG;
 constexpr u32 REF_MAX_REC = 65536;  // records sorted here
-constexpr u32 SEG_LANE = 16;       // ordered segments up to this length: a lane each
 
 struct RefCnt {  // zeroed by the host
   u32 smax, nitems, nsplit, nrefined, nsingle, nsitems, nbig, ncand;
@@ -61,7 +60,7 @@ struct GangRefArgs {
   u32 *sidx, *sidx2;
   u32* origin;           // per new id: the sub-community it was split from
   u32 *rlist, *single, *clist, *plist;
-  u64 *rec, *rec2, *rtmp;  // (id << 33 | is community << 32 | vertex)
+  u64 *rec, *rid, *rtmp;  // (id << 33 | is community << 32 | vertex)
   u32 *ridx, *rtidx;
   double* rval;
   double *dS, *dcomm, *wsp;
@@ -507,32 +506,12 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) 
       gang_sort(
           G, S, nrec, [&](u32 i) { return A.rec[i]; }, [](u32 i) { return i; }, A.rtmp, A.rtidx,
           [&](u32 r, u64 key, u32) {
-            A.rec2[r] = key;
+            A.rid[r] = key >> 32;
             A.rval[r] = A.k[(u32)key];
           });
-      double* buf = W.tv[threadIdx.x >> 5];
-      for (u32 t0 = G.warp() * 32; t0 < nrec; t0 += G.warps() * 32) {
-        const u32 t = t0 + lane;
-        const bool head = t < nrec && (t == 0 || (A.rec2[t] >> 32) != (A.rec2[t - 1] >> 32));
-        const u64 id = t < nrec ? A.rec2[t] >> 32 : 0;
-        double* d = id & 1 ? A.dcomm : A.dS;
-        bool more = false;
-        if (head) {  // short segments: a lane each
-          double x = 0.0;
-          u32 j = t;
-          for (; j < nrec && j < t + SEG_LANE && (A.rec2[j] >> 32) == id; ++j)
-            x = __dadd_rn(x, A.rval[j]);
-          more = j < nrec && (A.rec2[j] >> 32) == id;
-          if (!more) d[id >> 1] = x;
-        }
-        for (u32 hm = __ballot_sync(0xffffffffu, more); hm; hm &= hm - 1) {
-          const u32 a = t0 + __ffs(hm) - 1;
-          const u64 aid = A.rec2[a] >> 32;
-          const u32 b = warp_bound_u64<false>(A.rec2, a, nrec, (aid + 1) << 32);
-          const double x = warp_chain_sum(a, b, 0.0, A.rval, buf);
-          if (lane == 0) (aid & 1 ? A.dcomm : A.dS)[aid >> 1] = x;
-        }
-      }
+      gang_segment_sums(G, nrec, A.rid, A.rval, W.tv[threadIdx.x >> 5], [&](u64 id, double x) {
+        (id & 1 ? A.dcomm : A.dS)[id >> 1] = x;
+      });
       G.sync();
     }
     // ---- T-filter decisions (the rounding window of k_blocked_bounds) ----
@@ -686,7 +665,7 @@ u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   A.clist = S.cand_node.p;
   A.plist = S.sel_node.p;
   A.rec = S.rkeys.p;
-  A.rec2 = S.rkeys2.p;
+  A.rid = S.rkeys2.p;
   A.rtmp = S.keys.p;
   A.rtidx = S.idx.p;
   A.rval = S.fvals.p;
