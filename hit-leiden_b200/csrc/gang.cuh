@@ -137,64 +137,70 @@ __device__ __forceinline__ u32 gang_scan(const Gang& G, GangSmem& S, u32 N, V va
   return total;
 }
 
-// Ascending sort of P (key, value) records (a power of two from 64 to
-// GSORT_CHUNK) by (key, value) into S.key / S.val, by the block: every warp
-// sorts 32 records through its lanes, then runs merge pairwise, each record
-// finding its place by a bisection in the sibling run.  2048 records: 24 us as
-// a bitonic network in shared memory (66 stages of 48 KB traffic), a third of
-// that this way.
-template <typename K, typename VL>
-__device__ __forceinline__ void block_sort(GangSmem& S, u32 P, K key_of, VL val_of) {
+// Ascending sort of the P (key, value) records (a power of two from 64 to
+// GSORT_CHUNK) in S.key / S.val by (key, value), by the block: every warp sorts
+// 32 records through its lanes, then runs merge pairwise, each record finding
+// its place by a bisection in the sibling run.
+//
+// What bounds it: a stage runs once per launch, so straight-line code costs its
+// instruction fetches.  2048 records take 24 us as a bitonic network in shared
+// memory (66 stages), 55 us with the 15 lane stages unrolled four times over
+// (29 us of it fetching them), and %SORT% us as written, rolled and shared by all
+// sorts of a kernel.
+static __device__ __noinline__ void block_sort(GangSmem* Sp, u32 P) {
+  __builtin_assume(__isShared(Sp));
+  GangSmem& S = *Sp;
   constexpr u32 PER = GSORT_CHUNK / GANG_THREADS;
   const u32 tid = threadIdx.x, lane = tid & 31;
+  const u32 per = (P + GANG_THREADS - 1) / GANG_THREADS;  // uniform
   u64 k[PER];
-  u32 v[PER];
+  u32 v[PER], pos[PER];
 #pragma unroll
   for (u32 j = 0; j < PER; ++j) {
     const u32 e = tid + j * GANG_THREADS;
-    if (e >= P) break;  // warp-uniform
-    k[j] = key_of(e);
-    v[j] = val_of(e);
+    k[j] = e < P ? S.key[e] : ~0ull;
+    v[j] = e < P ? S.val[e] : NONE32;
   }
+#pragma unroll 1
+  for (u32 size = 2; size <= 32; size <<= 1) {
+#pragma unroll 1
+    for (u32 stride = size >> 1; stride; stride >>= 1) {
+      const bool want_less = ((lane & size) == 0) == ((lane & stride) == 0);
 #pragma unroll
-  for (u32 j = 0; j < PER; ++j) {
-    const u32 e = tid + j * GANG_THREADS;
-    if (e >= P) break;
-#pragma unroll
-    for (u32 size = 2; size <= 32; size <<= 1)
-#pragma unroll
-      for (u32 stride = size >> 1; stride; stride >>= 1) {
+      for (u32 j = 0; j < PER; ++j) {
+        if (j >= per) break;
         const u64 ok = __shfl_xor_sync(0xffffffffu, k[j], stride);
         const u32 ov = __shfl_xor_sync(0xffffffffu, v[j], stride);
         const bool less = ok < k[j] || (ok == k[j] && ov < v[j]);
-        const bool want_less = ((lane & size) == 0 || size == 32) == ((lane & stride) == 0);
         const bool differ = ok != k[j] || ov != v[j];
         if (differ && less == want_less) {
           k[j] = ok;
           v[j] = ov;
         }
       }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (u32 j = 0; j < PER; ++j) {
+    const u32 e = tid + j * GANG_THREADS;
+    if (e >= P) continue;
     S.key[e] = k[j];
     S.val[e] = v[j];
   }
   __syncthreads();
+#pragma unroll 1
   for (u32 run = 32; run < P; run <<= 1) {
-    u32 pos[PER];
 #pragma unroll
-    for (u32 j = 0; j < PER; ++j) {
-      const u32 e = tid + j * GANG_THREADS;
-      pos[j] = 0;
-      if (e >= P) break;
-      k[j] = S.key[e];
-      v[j] = S.val[e];
-    }
+    for (u32 j = 0; j < PER; ++j) pos[j] = 0;
+#pragma unroll 1
     for (u32 half = run; half; half >>= 1) {
 #pragma unroll
       for (u32 j = 0; j < PER; ++j) {
+        if (j >= per) break;
         const u32 e = tid + j * GANG_THREADS;
-        if (e >= P) break;
+        if (e >= P || pos[j] + half > run) continue;
         const u32 sib = (e & ~(run - 1)) ^ run;
-        if (pos[j] + half > run) continue;
         const u32 at = sib + pos[j] + half - 1;
         const u64 x = S.key[at];
         bool before = x < k[j];
@@ -209,13 +215,58 @@ __device__ __forceinline__ void block_sort(GangSmem& S, u32 P, K key_of, VL val_
 #pragma unroll
     for (u32 j = 0; j < PER; ++j) {
       const u32 e = tid + j * GANG_THREADS;
-      if (e >= P) break;
+      if (e >= P) continue;
       const u32 to = (e & ~(2 * run - 1)) + (e & (run - 1)) + pos[j];
       S.key[to] = k[j];
       S.val[to] = v[j];
     }
     __syncthreads();
+#pragma unroll
+    for (u32 j = 0; j < PER; ++j) {
+      const u32 e = tid + j * GANG_THREADS;
+      if (e >= P) continue;
+      k[j] = S.key[e];
+      v[j] = S.val[e];
+    }
   }
+}
+
+// How many records of the sorted chunks first, first + GSORT_ILP, ... come
+// before record (k, v) of chunk `mine` (tk / tv: N records in chunks of ch);
+// GSORT_ILP bisections side by side; equal records: earlier chunks first.
+static __device__ __noinline__ u32 gang_rank(const u64* tk, const u32* tv, u32 N, u32 ch, u32 nch,
+                                             u32 first, u32 step, u32 mine, u64 k, u32 v) {
+  u32 rank = 0;
+#pragma unroll 1
+  for (u32 c0 = first; c0 < nch; c0 += step) {
+    u32 pos[GSORT_ILP];
+#pragma unroll
+    for (u32 j = 0; j < GSORT_ILP; ++j) pos[j] = 0;
+#pragma unroll 1
+    for (u32 half = ch; half; half >>= 1) {
+      u64 probe[GSORT_ILP];
+      bool in[GSORT_ILP];
+#pragma unroll
+      for (u32 j = 0; j < GSORT_ILP; ++j) {
+        const u32 c = c0 + j;
+        const u32 at = c * ch + pos[j] + half;  // one past the probed record
+        in[j] = c < nch && c != mine && pos[j] + half <= ch && at <= N;
+        probe[j] = in[j] ? tk[at - 1] : 0ull;
+      }
+#pragma unroll
+      for (u32 j = 0; j < GSORT_ILP; ++j) {
+        if (!in[j] || probe[j] > k) continue;
+        if (probe[j] == k) {
+          const u32 y = tv[(c0 + j) * ch + pos[j] + half - 1];
+          if (y > v || (y == v && c0 + j > mine)) continue;
+        }
+        pos[j] += half;
+      }
+    }
+#pragma unroll
+    for (u32 j = 0; j < GSORT_ILP; ++j) rank += pos[j];
+  }
+  return rank;
 }
 
 // Ascending sort of N (key, value) records by (key, value); with the record's
@@ -232,18 +283,23 @@ template <typename K, typename VL, typename EM>
 __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K key_of, VL val_of,
                                           u64* tk, u32* tv, EM emit) {
   const u32 tid = threadIdx.x;
-  // few chunks: a record's rank costs one bisection per chunk
+  // Few chunks, because a record's rank costs one bisection per chunk, and at
+  // most one a block: on a grid 32 (512 records sort in 8 us, 2048 in 33 us,
+  // a rank among 32 chunks takes four lanes what one among 8 takes one).
   u32 ch = 64;
-  while (ch < GSORT_CHUNK && ch * min(G.nct, 8u) < N) ch <<= 1;
+  while (ch < GSORT_CHUNK && ch * min(G.nct, 32u) < N) ch <<= 1;
   const u32 nch = (N + ch - 1) / ch;
   for (u32 c = G.rank; c < nch; c += G.nct) {
     const u32 base = c * ch;
     const u32 cnt = min(ch, N - base);
     u32 P = 64;  // the padded length of this chunk
     while (P < cnt) P <<= 1;
-    block_sort(
-        S, P, [&](u32 i) { return i < cnt ? key_of(base + i) : ~0ull; },
-        [&](u32 i) { return i < cnt ? val_of(base + i) : NONE32; });
+    for (u32 i = tid; i < P; i += GANG_THREADS) {
+      S.key[i] = i < cnt ? key_of(base + i) : ~0ull;
+      S.val[i] = i < cnt ? val_of(base + i) : NONE32;
+    }
+    __syncthreads();
+    block_sort(&S, P);
     for (u32 i = tid; i < cnt; i += GANG_THREADS) {
       if (nch == 1) {
         emit(i, S.key[i], S.val[i]);
@@ -256,40 +312,21 @@ __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K k
   }
   G.sync();
   if (nch == 1) return;
-  for (u32 e = G.thread(); e < N; e += G.threads()) {
-    const u64 k = tk[e];
-    const u32 v = tv[e];
+  // a warp takes 32 / L records, L lanes a record share its chunks; consecutive
+  // warps sit on different blocks, which spreads the probes over the chip
+  u32 L = 1;
+  while (L < 32 && L * GSORT_ILP < nch) L <<= 1;
+  const u32 per = 32 / L, g = (tid & 31) / per;
+  for (u32 e0 = G.warp() * per; e0 < N; e0 += G.warps() * per) {
+    const u32 e = e0 + ((tid & 31) & (per - 1));
+    const bool on = e < N;
+    const u64 k = on ? tk[e] : 0ull;
+    const u32 v = on ? tv[e] : 0u;
     const u32 mine = e / ch;
-    u32 rank = e - mine * ch;
-    // GSORT_ILP bisections side by side; equal records: earlier chunks first
-    for (u32 c0 = 0; c0 < nch; c0 += GSORT_ILP) {
-      u32 pos[GSORT_ILP];
-#pragma unroll
-      for (u32 j = 0; j < GSORT_ILP; ++j) pos[j] = 0;
-      for (u32 half = ch; half; half >>= 1) {
-        u64 probe[GSORT_ILP];
-        bool in[GSORT_ILP];
-#pragma unroll
-        for (u32 j = 0; j < GSORT_ILP; ++j) {
-          const u32 c = c0 + j;
-          const u32 at = c * ch + pos[j] + half;  // one past the probed record
-          in[j] = c < nch && c != mine && pos[j] + half <= ch && at <= N;
-          probe[j] = in[j] ? tk[at - 1] : 0ull;
-        }
-#pragma unroll
-        for (u32 j = 0; j < GSORT_ILP; ++j) {
-          if (!in[j] || probe[j] > k) continue;
-          if (probe[j] == k) {
-            const u32 y = tv[(c0 + j) * ch + pos[j] + half - 1];
-            if (y > v || (y == v && c0 + j > mine)) continue;
-          }
-          pos[j] += half;
-        }
-      }
-#pragma unroll
-      for (u32 j = 0; j < GSORT_ILP; ++j) rank += pos[j];
-    }
-    emit(rank, k, v);
+    u32 rank = 0;
+    if (on) rank = gang_rank(tk, tv, N, ch, nch, g * GSORT_ILP, L * GSORT_ILP, mine, k, v);
+    for (u32 o = per; o < 32; o <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    if (on && g == 0) emit(rank + e - mine * ch, k, v);
   }
   G.sync();
 }
