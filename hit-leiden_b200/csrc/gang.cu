@@ -29,6 +29,18 @@ GangShape gang_shape(Engine& E, u64 work) {
   return GangShape{sms < GANG_MAX_BLOCKS ? sms : GANG_MAX_BLOCKS, true};
 }
 
+u32* gang_counters(Engine& E, u32** next) {
+  Scratch& S = E.sc;
+  if (!S.gang_cnt.p) {
+    S.gang_cnt.ensure(E.mem, 2 * GANG_CNT);
+    HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 2 * GANG_CNT * sizeof(u32), E.stream));
+    E.gang_set = 0;
+  }
+  *next = S.gang_cnt.p + (E.gang_set ^ 1u) * GANG_CNT;
+  return S.gang_cnt.p + E.gang_set * GANG_CNT;
+}
+void gang_turn(Engine& E) { E.gang_set ^= 1u; }
+
 void gang_launch(Engine& E, const void* kernel, const GangShape& s, size_t smem, void* args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s.blocks);

@@ -59,6 +59,7 @@ struct GangAggArgs {
   u32 *ou, *ov;
   double* ow;
   AggCnt* cnt;
+  u32* cnt_next;
   AggOut* out;
 };
 
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_aggregate(GangAggArgs 
   const u32 lane = threadIdx.x & 31;
   const u32 gt = G.thread(), gts = G.threads();
   AggCnt& C = *A.cnt;
+  gang_clear_next(G, A.cnt_next);
   // ---- new nodes of the level above start isolated with identity maps ----
   for (u32 x = gt; x < A.hn; x += gts) {
     A.last[x] = 0;
@@ -311,8 +313,6 @@ bool gang_aggregate(Engine& E, Level& L, Level& H, const DevEdges& delta, bool a
   S.kflag.ensure(E.mem, hn ? hn : 1);
   S.minmem.ensure(E.mem, (size_t)hn + 1);
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
-  S.gang_cnt.ensure(E.mem, 64);
-  HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 64 * sizeof(u32), st));
   GangAggArgs A{};
   if (aggregate) {
     const u64 nit = (u64)n + L.g.nnz / AGG_SLICE + 1;
@@ -380,10 +380,11 @@ bool gang_aggregate(Engine& E, Level& L, Level& H, const DevEdges& delta, bool a
   A.aggregate = aggregate;
   A.grid = shape.grid;
   A.part = S.gang_part.p;
-  A.cnt = reinterpret_cast<AggCnt*>(S.gang_cnt.p);
-  A.out = reinterpret_cast<AggOut*>(S.gang_cnt.p + 32);
+  A.cnt = reinterpret_cast<AggCnt*>(gang_counters(E, &A.cnt_next));
+  A.out = reinterpret_cast<AggOut*>(E.hs.p);
   cudaEvent_t ev = E.kt_begin();
   gang_launch(E, reinterpret_cast<const void*>(&k_gang_aggregate), shape, 0, &A);
+  gang_turn(E);
   E.kt_end(KT_GANG_AGG, ev);
   H.g.n = hn;
   if (H.s_bound && H.s_bound < hn) H.s_bound = hn;
@@ -392,7 +393,6 @@ bool gang_aggregate(Engine& E, Level& L, Level& H, const DevEdges& delta, bool a
     return true;
   }
   AggOut o;
-  HL_CUDA(cudaMemcpyAsync(E.hs.p, A.out, sizeof(AggOut), cudaMemcpyDeviceToHost, st));
   E.sync();
   std::memcpy(&o, E.hs.p, sizeof(o));
   *count = o.count;

@@ -48,6 +48,7 @@ struct GangApplyArgs {
   double *red, *red2;
   u32* part;
   ApplyCnt* cnt;
+  u32* cnt_next;
   ApplyOut* out;
 };
 
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_apply(GangApplyArgs A)
   const Gang G = gang_make(A.grid);
   const u32 tid = threadIdx.x, lane = tid & 31;
   ApplyCnt& C = *A.cnt;
+  gang_clear_next(G, A.cnt_next);
   if (!A.finish_only) {
     // ---- the batch by key, stable (batch order within a key) ----
     for (u32 i = G.thread(); i < (A.n + 31) / 32; i += G.threads()) A.touched[i] = 0;
@@ -285,8 +287,6 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   S.red.ensure(E.mem, tiles + 1);
   S.red2.ensure(E.mem, (tiles + 1023) / 1024 + 1);
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
-  S.gang_cnt.ensure(E.mem, 64);
-  HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 64 * sizeof(u32), st));
   GangApplyArgs A{};
   A.n = n;
   A.nnz = Gr.nnz;
@@ -318,14 +318,13 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   A.red = S.red.p;
   A.red2 = S.red2.p;
   A.part = S.gang_part.p;
-  A.cnt = reinterpret_cast<ApplyCnt*>(S.gang_cnt.p);
-  A.out = reinterpret_cast<ApplyOut*>(S.gang_cnt.p + 32);
+  A.cnt = reinterpret_cast<ApplyCnt*>(gang_counters(E, &A.cnt_next));
+  A.out = reinterpret_cast<ApplyOut*>(E.hs.p);
   const u64 bound = Gr.nnz + rmax;
   cudaEvent_t ev = E.kt_begin();
   ApplyOut o;
   const void* fn = reinterpret_cast<const void*>(&k_gang_apply);
   auto result = [&]() {
-    HL_CUDA(cudaMemcpyAsync(E.hs.p, A.out, sizeof(ApplyOut), cudaMemcpyDeviceToHost, st));
     E.sync();
     std::memcpy(&o, E.hs.p, sizeof(o));
   };
@@ -333,6 +332,7 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
     // the second buffer may have to grow: only by what the batch needs
     A.structure_only = true;
     gang_launch(E, fn, shape, 0, &A);
+    gang_turn(E);  // the second launch goes on with these counters
     result();
     if (o.nops) {
       Gr.col2.ensure_slack(E.mem, o.nnz_new ? o.nnz_new : 1);
@@ -344,6 +344,7 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   A.ncol = Gr.col2.p;
   A.nw = Gr.w2.p;
   gang_launch(E, fn, shape, 0, &A);
+  if (!A.finish_only) gang_turn(E);
   result();
   E.kt_end(KT_GANG_APPLY, ev);
   if (o.err)

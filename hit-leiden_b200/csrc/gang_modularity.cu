@@ -48,6 +48,7 @@ struct GangModArgs {
   double* kval;
   double* partial;  // per block: intra hi, lo, expected hi, lo
   ModCnt* cnt;
+  u32* cnt_next;
   double* out;      // intra, expected
 };
 
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_modularity(GangModArgs
   const u32 lane = threadIdx.x & 31;
   const u32 gt = G.thread(), gts = G.threads();
   ModCnt& C = *A.cnt;
+  gang_clear_next(G, A.cnt_next);
   // ---- the largest label ----
   {
     u32 mx = 0;
@@ -175,9 +177,7 @@ double modularity(Engine& E, Level& L, const u32* part) {
   S.fvals.ensure(E.mem, n);
   S.gm_hist.ensure(E.mem, (size_t)256 * GANG_WARPS * shape.blocks);
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
-  S.gang_cnt.ensure(E.mem, 64);
-  S.red.ensure(E.mem, 4 * GANG_MAX_BLOCKS + 2);
-  HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 64 * sizeof(u32), st));
+  S.red.ensure(E.mem, 4 * GANG_MAX_BLOCKS);
   GangModArgs A{};
   A.n = n;
   A.off = L.g.off.p;
@@ -195,10 +195,10 @@ double modularity(Engine& E, Level& L, const u32* part) {
   A.gpart = S.gang_part.p;
   A.kval = S.fvals.p;
   A.partial = S.red.p;
-  A.cnt = reinterpret_cast<ModCnt*>(S.gang_cnt.p);
-  A.out = S.red.p + 4 * GANG_MAX_BLOCKS;
+  A.cnt = reinterpret_cast<ModCnt*>(gang_counters(E, &A.cnt_next));
+  A.out = reinterpret_cast<double*>(E.hs.p);
   gang_launch(E, reinterpret_cast<const void*>(&k_gang_modularity), shape, 0, &A);
-  HL_CUDA(cudaMemcpyAsync(E.hs.p, A.out, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  gang_turn(E);
   E.sync();
   double q[2];
   std::memcpy(q, E.hs.p, sizeof(q));

@@ -99,6 +99,7 @@ struct GangMoveArgs {
   u64 epoch0;
   u32 label_bits;
   MoveCnt* cnt;
+  u32* cnt_next;
   MoveOutDev* out;
 };
 
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
   const u32 tid = threadIdx.x, lane = tid & 31;
   const u32 gt = G.thread(), gts = G.threads();
   MoveCnt& C = *A.cnt;
+  gang_clear_next(G, A.cnt_next);
   const u32 words = (A.n + 31) / 32;
   unsigned long long trav = 0, trav_round = 0, pruned = 0;
   u32 b = 0;  // parity of the current frontier
@@ -713,10 +715,8 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
     }
   }
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
-  S.gang_cnt.ensure(E.mem, 64);
-  static_assert(sizeof(MoveCnt) <= 44 * sizeof(u32) && sizeof(MoveOutDev) <= 20 * sizeof(u32),
-                "both fit the counter block");
-  HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 64 * sizeof(u32), st));
+  static_assert(sizeof(MoveCnt) <= GANG_CNT * sizeof(u32), "fits the counter block");
+  static_assert(sizeof(MoveOutDev) <= 64 * sizeof(u64), "fits the pinned block");
   u32 round0 = E.sel_round;
   if (round0 + E.cfg.max_rounds + 2 >= (1u << 29)) round0 = E.sel_round = 1;
   A.n = n;
@@ -773,13 +773,13 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   A.round0 = round0;
   A.epoch0 = E.epoch;
   A.label_bits = (u32)bits_for(n - 1);
-  A.cnt = reinterpret_cast<MoveCnt*>(S.gang_cnt.p);
-  A.out = reinterpret_cast<MoveOutDev*>(S.gang_cnt.p + 44);
+  A.cnt = reinterpret_cast<MoveCnt*>(gang_counters(E, &A.cnt_next));
+  A.out = reinterpret_cast<MoveOutDev*>(E.hs.p);
   cudaEvent_t ev = E.kt_begin();
   gang_launch(E, reinterpret_cast<const void*>(&k_gang_move), shape, sizeof(MoveSmem), &A);
+  gang_turn(E);
   E.kt_end(KT_GANG_MOVE, ev);
   MoveOutDev o;
-  HL_CUDA(cudaMemcpyAsync(E.hs.p, A.out, sizeof(o), cudaMemcpyDeviceToHost, st));
   E.sync();
   std::memcpy(&o, E.hs.p, sizeof(o));
   if (o.status == MOVE_LABELS) return o.status;

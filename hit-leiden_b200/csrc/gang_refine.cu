@@ -72,6 +72,7 @@ struct GangRefArgs {
   double tw, gamma;
   u32* part;
   RefCnt* cnt;
+  u32* cnt_next;
   RefOut* out;
 };
 
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) 
   const u32 lane = threadIdx.x & 31;
   const u32 gt = G.thread(), gts = G.threads();
   RefCnt& C = *A.cnt;
+  gang_clear_next(G, A.cnt_next);
   // ---- clear; the largest sub-community id ----
   for (u32 i = gt; i < A.s_words; i += gts) A.affsc[i] = 0;
   for (u32 i = gt; i < (A.n + 3) / 4; i += gts) reinterpret_cast<u32*>(A.refined)[i] = 0;
@@ -625,8 +627,6 @@ u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   S.cand_to.ensure(E.mem, n);
   S.cand_gain.ensure(E.mem, n);
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
-  S.gang_cnt.ensure(E.mem, 64);
-  HL_CUDA(cudaMemsetAsync(S.gang_cnt.p, 0, 64 * sizeof(u32), st));
   GangRefArgs A{};
   A.n = n;
   A.off = L.g.off.p;
@@ -680,13 +680,13 @@ u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   A.tw = L.tw;
   A.gamma = E.cfg.resolution;
   A.part = S.gang_part.p;
-  A.cnt = reinterpret_cast<RefCnt*>(S.gang_cnt.p);
-  A.out = reinterpret_cast<RefOut*>(S.gang_cnt.p + 32);
+  A.cnt = reinterpret_cast<RefCnt*>(gang_counters(E, &A.cnt_next));
+  A.out = reinterpret_cast<RefOut*>(E.hs.p);
   cudaEvent_t ev = E.kt_begin();
   gang_launch(E, reinterpret_cast<const void*>(&k_gang_refine), shape, sizeof(RefSmem), &A);
+  gang_turn(E);
   E.kt_end(KT_GANG_REFINE, ev);
   RefOut o;
-  HL_CUDA(cudaMemcpyAsync(E.hs.p, A.out, sizeof(RefOut), cudaMemcpyDeviceToHost, st));
   E.sync();
   std::memcpy(&o, E.hs.p, sizeof(o));
   if (o.status == REF_HOST_ALL) return o.status;

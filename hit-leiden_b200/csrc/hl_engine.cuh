@@ -192,6 +192,7 @@ struct Engine {
   HostScalars hs;
   u64 epoch = 1;         // selection epochs (reservation keys)
   u32 sel_round = 0;     // role tag of the current selection
+  u32 gang_set = 0;      // counter block of the next gang launch
   u64 stats_sel_iters = 0;
   u64 nlaunch = 0;       // launches of this library's kernels
   u64 launch_mark = 0;
