@@ -265,9 +265,10 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   const u32 n = Gr.n;
   const u32 k = (u32)b.k;
   const u32 rmax = 2 * k;
-  // a sorted record costs about 64 streamed entries (17.5k updates: two sorts
-  // 310 us on 8 blocks, 140 us on 148)
-  const GangShape shape = gang_shape(E, Gr.nnz + n + 64ull * k);
+  // A sorted record costs about 64 streamed entries (17.5k updates: two sorts
+  // 310 us on 8 blocks, 140 us on 148), and less while a single block sorts all
+  // of them in one go (70 updates of 1.3k entries: 25 us on one block, 40 on 8).
+  const GangShape shape = gang_shape(E, Gr.nnz + n + (k <= 128 ? 16ull : 64ull) * k);
   S.keys.ensure(E.mem, rmax);
   S.idx.ensure(E.mem, rmax);
   S.keys2.ensure(E.mem, k);
