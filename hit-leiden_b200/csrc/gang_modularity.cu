@@ -52,7 +52,8 @@ struct GangModArgs {
   double* out;      // intra, expected
 };
 
-constexpr u32 MOD_ROWS = 128;     // rows a warp takes at a time
+constexpr u32 MOD_ROWS = 32;      // rows a warp takes at a time
+constexpr u32 MOD_AHEAD = 4;      // groups of four rows whose loads are in flight together
 constexpr u32 MOD_LONG = 256;     // rows above this take the whole warp
 
 // Sum of the 32 lanes' double-doubles of this warp's share, block by block, to
@@ -75,7 +76,8 @@ __device__ __forceinline__ void mod_block_sum(DD x, DD* sh, double* out) {
 // bytes an entry); a large community's ordered degree sum is one chain (10
 // cycles a member) that runs beside it.  500k vertices, 12M entries, 4,000
 // communities: row sums 133 us, ordered degrees 56 us and some twenty launches
-// with five host reads, 490 us a call, become one launch.
+// with five host reads, 520 us a call, become one launch and 375 us (with one
+// group of rows in flight a warp and 128 rows taken at a time: 458).
 __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_modularity(GangModArgs A) {
   __shared__ GangSmem S;
   __shared__ __align__(16) double chain[GANG_WARPS][CHAIN_TILE];
@@ -115,37 +117,68 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_modularity(GangModArgs
     if (lane == 0) ch = atomicAdd(&C.work, 1u);
     ch = __shfl_sync(0xffffffffu, ch, 0);
     if (ch >= chunks) break;
-    for (u32 r = 0; r < MOD_ROWS; r += 4) {
-      const u64 v = (u64)ch * MOD_ROWS + r + (lane >> 3);
-      const bool live = v < A.n;
-      const u64 a = live ? A.off[v] : 0, b = live ? A.off[v + 1] : 0;
-      const u32 c = live ? A.part[v] : 0;
-      const bool big = b - a > MOD_LONG;
-      DD s{0.0, 0.0};
-      if (!big)
-        for (u64 p = a + sub; p < b; p += 32) {
-          u32 nb[4];
-          double x[4];
+    // MOD_AHEAD groups of four rows at once: a group is a chain of three
+    // dependent loads (offsets, neighbours, labels) that one warp would wait
+    // for in turn
+    for (u32 r = 0; r < MOD_ROWS; r += 4 * MOD_AHEAD) {
+      u64 a[MOD_AHEAD], b[MOD_AHEAD];
+      u32 c[MOD_AHEAD], nb[MOD_AHEAD][4];
+      double x[MOD_AHEAD][4];
 #pragma unroll
-          for (u32 j = 0; j < 4; ++j) nb[j] = p + 8 * j < b ? A.col[p + 8 * j] : NONE32;
+      for (u32 k = 0; k < MOD_AHEAD; ++k) {
+        const u64 v = (u64)ch * MOD_ROWS + r + 4 * k + (lane >> 3);
+        const bool live = v < A.n;
+        a[k] = live ? A.off[v] : 0;
+        b[k] = live ? A.off[v + 1] : 0;
+        c[k] = live ? A.part[v] : 0;
+      }
 #pragma unroll
-          for (u32 j = 0; j < 4; ++j) x[j] = nb[j] != NONE32 ? A.w[p + 8 * j] : 0.0;
+      for (u32 k = 0; k < MOD_AHEAD; ++k) {
+        const u64 stop = b[k] - a[k] > MOD_LONG ? a[k] : b[k];
 #pragma unroll
-          for (u32 j = 0; j < 4; ++j)
-            if (nb[j] != NONE32 && A.part[nb[j]] == c) s = dd_add(s, x[j]);
+        for (u32 j = 0; j < 4; ++j) {
+          const u64 p = a[k] + sub + 8 * j;
+          nb[k][j] = p < stop ? A.col[p] : NONE32;
+          x[k][j] = p < stop ? A.w[p] : 0.0;
         }
-      for (u32 o = 4; o; o >>= 1) s = dd_add(s, dd_shfl_xor(s, o));
-      // a row's sum is rounded before the total, as the reference adds rows
-      if (live && !big && sub == 0) intra = dd_add(intra, s.hi + s.lo);
-      for (u32 bm = __ballot_sync(0xffffffffu, big && sub == 0); bm; bm &= bm - 1) {
-        const u32 l = __ffs(bm) - 1;
-        const u64 ba = __shfl_sync(0xffffffffu, a, l), bb = __shfl_sync(0xffffffffu, b, l);
-        const u32 bc = __shfl_sync(0xffffffffu, c, l);
-        DD t{0.0, 0.0};
-        for (u64 p = ba + lane; p < bb; p += 32)
-          if (A.part[A.col[p]] == bc) t = dd_add(t, A.w[p]);
-        for (u32 o = 16; o; o >>= 1) t = dd_add(t, dd_shfl_xor(t, o));
-        if (lane == 0) intra = dd_add(intra, t.hi + t.lo);
+      }
+#pragma unroll
+      for (u32 k = 0; k < MOD_AHEAD; ++k)
+#pragma unroll
+        for (u32 j = 0; j < 4; ++j)
+          if (nb[k][j] == NONE32 || A.part[nb[k][j]] != c[k]) x[k][j] = 0.0;
+#pragma unroll
+      for (u32 k = 0; k < MOD_AHEAD; ++k) {
+        const bool big = b[k] - a[k] > MOD_LONG;
+        DD s{0.0, 0.0};
+#pragma unroll
+        for (u32 j = 0; j < 4; ++j)
+          if (x[k][j] != 0.0) s = dd_add(s, x[k][j]);
+        if (!big)
+          for (u64 p0 = a[k] + sub + 32; p0 < b[k]; p0 += 32) {
+            u32 m[4];
+            double y[4];
+#pragma unroll
+            for (u32 j = 0; j < 4; ++j) m[j] = p0 + 8 * j < b[k] ? A.col[p0 + 8 * j] : NONE32;
+#pragma unroll
+            for (u32 j = 0; j < 4; ++j) y[j] = m[j] != NONE32 ? A.w[p0 + 8 * j] : 0.0;
+#pragma unroll
+            for (u32 j = 0; j < 4; ++j)
+              if (m[j] != NONE32 && A.part[m[j]] == c[k]) s = dd_add(s, y[j]);
+          }
+        for (u32 o = 4; o; o >>= 1) s = dd_add(s, dd_shfl_xor(s, o));
+        // a row's sum is rounded before the total, as the reference adds rows
+        if (!big && sub == 0) intra = dd_add(intra, s.hi + s.lo);
+        for (u32 bm = __ballot_sync(0xffffffffu, big && sub == 0); bm; bm &= bm - 1) {
+          const u32 l = __ffs(bm) - 1;
+          const u64 ba = __shfl_sync(0xffffffffu, a[k], l), bb = __shfl_sync(0xffffffffu, b[k], l);
+          const u32 bc = __shfl_sync(0xffffffffu, c[k], l);
+          DD t{0.0, 0.0};
+          for (u64 p = ba + lane; p < bb; p += 32)
+            if (A.part[A.col[p]] == bc) t = dd_add(t, A.w[p]);
+          for (u32 o = 16; o; o >>= 1) t = dd_add(t, dd_shfl_xor(t, o));
+          if (lane == 0) intra = dd_add(intra, t.hi + t.lo);
+        }
       }
     }
   }
