@@ -28,7 +28,8 @@ namespace hl {
 constexpr u32 GANG_THREADS = 512;
 constexpr u32 GANG_WARPS = GANG_THREADS / 32;
 constexpr u32 GANG_MAX_BLOCKS = 148;
-constexpr u32 GSORT_CHUNK = 2048;  // records sorted by one block at a time
+constexpr u32 GSORT_CHUNK = 1024;  // records sorted by one block at a time
+constexpr u32 GANG_WORDS = 2048;   // 64-bit words of a block's shared memory (GangSmem)
 constexpr u32 GSORT_ILP = 8;       // chunks a record's rank is looked up in at once
 
 struct Gang {
@@ -68,7 +69,7 @@ __device__ __forceinline__ void gang_clear_next(const Gang& G, u32* next) {
 // Shared memory of the primitives below (one instance per kernel, static or
 // at the start of the dynamic block).
 struct GangSmem {
-  u64 key[GSORT_CHUNK];
+  u64 key[GANG_WORDS];
   u32 val[GSORT_CHUNK];
   u32 wsum[GANG_WARPS + 1];
   u32 bcast[2];
@@ -151,11 +152,11 @@ __device__ __forceinline__ u32 gang_scan(const Gang& G, GangSmem& S, u32 N, V va
 // 32 records through its lanes, then runs merge pairwise, each record finding
 // its place by a bisection in the sibling run.
 //
-// What bounds it: a stage runs once per launch, so straight-line code costs its
-// instruction fetches.  2048 records take 24 us as a bitonic network in shared
-// memory (66 stages), 55 us with the 15 lane stages unrolled four times over
-// (29 us of it fetching them), and %SORT% us as written, rolled and shared by all
-// sorts of a kernel.
+// What bounds it: a sort runs once or twice per launch, so straight-line code
+// costs its instruction fetches: with the 15 lane stages unrolled four times,
+// 2048 records took 55 us, 29 us of it in those stages; rolled and shared by all
+// sorts of a kernel, 33 us.  512 records take 8 us, 1024 take 15; chunks above
+// that lose more than a rank among fewer chunks gains.
 static __device__ __noinline__ void block_sort(GangSmem* Sp, u32 P) {
   __builtin_assume(__isShared(Sp));
   GangSmem& S = *Sp;
@@ -286,15 +287,15 @@ static __device__ __noinline__ u32 gang_rank(const u64* tk, const u32* tv, u32 N
 // inside (one when a single chunk holds everything); the caller's emitted
 // output is visible after the last one.
 //
-// For a few thousand records this takes 5-15 us; a radix sort of the same keys
+// For a few thousand records this takes 10-20 us; a radix sort of the same keys
 // is six to nine dependent kernel launches.
 template <typename K, typename VL, typename EM>
 __device__ __forceinline__ void gang_sort(const Gang& G, GangSmem& S, u32 N, K key_of, VL val_of,
                                           u64* tk, u32* tv, EM emit) {
   const u32 tid = threadIdx.x;
   // Few chunks, because a record's rank costs one bisection per chunk, and at
-  // most one a block: on a grid 32 (512 records sort in 8 us, 2048 in 33 us,
-  // a rank among 32 chunks takes four lanes what one among 8 takes one).
+  // most one a block: on a grid 32 (a rank among 32 chunks takes four lanes what
+  // one among 8 takes one).
   u32 ch = 64;
   while (ch < GSORT_CHUNK && ch * min(G.nct, 32u) < N) ch <<= 1;
   const u32 nch = (N + ch - 1) / ch;

@@ -127,17 +127,18 @@ struct DBuf {
     c.used += bytes;
     if (c.used > c.peak) c.peak = c.used;
   }
-  // Capacity for n elements with room for later batches, where the budget
-  // allows it: a graph's CSR grows by a few entries a batch, and a buffer that
-  // only just fits would be regrown (by half, hundreds of megabytes a level)
-  // by the first batch that inserts more than it deletes.
+  // Capacity for n elements with room for later batches: a graph's CSR grows by
+  // a few entries a batch, and a buffer that only just fits would be regrown (by
+  // half, hundreds of megabytes a level) by the first batch that inserts more
+  // than it deletes.  A handle with a budget takes no more than ensure() does:
+  // what the room took could be missing later.
   void ensure_slack(MemCtx& c, size_t n) {
     if (n <= cap) return;
-    const size_t want = n + n / 16;
-    const u64 bytes = (u64)(want + 256) * sizeof(T);
-    const bool fits = !c.budget || c.used - (u64)cap * sizeof(T) + bytes <= c.budget;
-    release();  // contents are not kept
-    ensure(c, fits ? want : n);
+    if (!c.budget) {
+      release();  // contents are not kept
+      n += n / 16;
+    }
+    ensure(c, n);
   }
   void swap(DBuf& o) {
     std::swap(p, o.p);
