@@ -94,6 +94,19 @@ double Engine::read_f64(const double* d) {
   std::memcpy(&x, hs.p, sizeof(double));
   return x;
 }
+void Engine::side_begin() {
+  if (!side_done) {
+    if (!side) HL_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    if (!side_go) HL_CUDA(cudaEventCreateWithFlags(&side_go, cudaEventDisableTiming));
+    HL_CUDA(cudaEventCreateWithFlags(&side_done, cudaEventDisableTiming));
+  }
+  HL_CUDA(cudaEventRecord(side_go, stream));
+  HL_CUDA(cudaStreamWaitEvent(side, side_go, 0));
+}
+void Engine::side_end() {
+  cudaEventRecord(side_done, side);
+  cudaStreamWaitEvent(stream, side_done, 0);
+}
 void Engine::sync() {
   if (ktiming) ++kagg[KT_HOST_SYNC].launches;
   HL_CUDA(cudaStreamSynchronize(stream));
@@ -110,17 +123,17 @@ static cudaEvent_t pool_get(std::vector<cudaEvent_t>& pool) {
   return e;
 }
 
-cudaEvent_t Engine::kt_begin() {
+cudaEvent_t Engine::kt_begin(cudaStream_t s) {
   if (!ktiming) return nullptr;
   cudaEvent_t e = pool_get(ev_pool);
-  HL_CUDA(cudaEventRecord(e, stream));
+  HL_CUDA(cudaEventRecord(e, s ? s : stream));
   return e;
 }
 
-void Engine::kt_end(int id, cudaEvent_t a) {
+void Engine::kt_end(int id, cudaEvent_t a, cudaStream_t s) {
   if (!ktiming || !a) return;
   cudaEvent_t b = pool_get(ev_pool);
-  HL_CUDA(cudaEventRecord(b, stream));
+  HL_CUDA(cudaEventRecord(b, s ? s : stream));
   ev_pending.push_back({id, {a, b}});
 }
 

@@ -607,6 +607,8 @@ __global__ void __launch_bounds__(WIDE_WARPS * 32) k_eval_wide(EvalArgs A) {
 // regions, moving a row's table there when it passes the same bound.
 // ---------------------------------------------------------------------------
 constexpr u32 BIG_TAB = 4096;
+constexpr u32 FORK_HUBS = 148;     // hub rows and
+constexpr u32 FORK_ROWS = 65536;   // other rows from which the two run side by side
 constexpr u32 BIG_SCAN_UNROLL = 4;  // table slots a thread scans at a time
 // Used-slot list of the shared table: a row is checked against BIG_TAB / 2
 // distinct keys after every tile, so it holds at most that plus one tile's
@@ -1818,77 +1820,97 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   }
 
   cudaEvent_t ev = E.kt_begin();
-  cudaEvent_t e_s = E.kt_begin();
-  for (int b = 0; b < 3; ++b) {
-    if (!c[b]) continue;
-    EvalArgs a = A;
-    a.counters = counters;
-    a.idx = vo + start[b];
-    a.nidx = c[b];
-    u32 G = b == 0 ? 8 : b == 1 ? 16 : 32;
-    u32 blocks = grid_for((u64)c[b] * G, 256);
-    if (kind == EVAL_MOVE) {
-      if (G == 8) ++E.nlaunch, k_eval_small<EVAL_MOVE, 8><<<blocks, 256, 0, st>>>(a);
-      else if (G == 16) ++E.nlaunch, k_eval_small<EVAL_MOVE, 16><<<blocks, 256, 0, st>>>(a);
-      else ++E.nlaunch, k_eval_small<EVAL_MOVE, 32><<<blocks, 256, 0, st>>>(a);
-    } else {
-      if (G == 8) ++E.nlaunch, k_eval_small<EVAL_REFINE, 8><<<blocks, 256, 0, st>>>(a);
-      else if (G == 16) ++E.nlaunch, k_eval_small<EVAL_REFINE, 16><<<blocks, 256, 0, st>>>(a);
-      else ++E.nlaunch, k_eval_small<EVAL_REFINE, 32><<<blocks, 256, 0, st>>>(a);
+  // The rows below the hub bin.  With many of them beside many hub rows they run
+  // on a stream of their own: the hub passes leave part of the chip idle (three
+  // blocks an SM in the first, host reads before the partitioned one).  R-MAT
+  // 2^21, batches of 80 and 60 rounds: 292 -> 280 and 221 -> 211 ms; 2^25, where
+  // the hub passes fill the chip: equal (2.17, 2.18 s).  Below the lines the rounds
+  // take as long either way (R-MAT 2^17, 1M-vertex communities).
+  const u32 below = c[0] + c[1] + c[2] + c[3] + c[4] + c[6];
+  const bool fork = c[5] >= FORK_HUBS && below >= FORK_ROWS;
+  auto rest = [&](cudaStream_t on) {
+    cudaEvent_t e_s = E.kt_begin(on);
+    for (int b = 0; b < 3; ++b) {
+      if (!c[b]) continue;
+      EvalArgs a = A;
+      a.counters = counters;
+      a.idx = vo + start[b];
+      a.nidx = c[b];
+      u32 G = b == 0 ? 8 : b == 1 ? 16 : 32;
+      u32 blocks = grid_for((u64)c[b] * G, 256);
+      if (kind == EVAL_MOVE) {
+        if (G == 8) ++E.nlaunch, k_eval_small<EVAL_MOVE, 8><<<blocks, 256, 0, on>>>(a);
+        else if (G == 16) ++E.nlaunch, k_eval_small<EVAL_MOVE, 16><<<blocks, 256, 0, on>>>(a);
+        else ++E.nlaunch, k_eval_small<EVAL_MOVE, 32><<<blocks, 256, 0, on>>>(a);
+      } else {
+        if (G == 8) ++E.nlaunch, k_eval_small<EVAL_REFINE, 8><<<blocks, 256, 0, on>>>(a);
+        else if (G == 16) ++E.nlaunch, k_eval_small<EVAL_REFINE, 16><<<blocks, 256, 0, on>>>(a);
+        else ++E.nlaunch, k_eval_small<EVAL_REFINE, 32><<<blocks, 256, 0, on>>>(a);
+      }
     }
-  }
-  HL_LAUNCH_CHECK();
-  E.kt_end(KT_EVAL_SMALL, e_s);
-  E.kagg[KT_EVAL_SMALL].items += (u64)c[0] + c[1] + c[2];
-  E.kagg[KT_EVAL_MID].items += c[3];
-  E.kagg[KT_EVAL_BIG].items += (u64)c[4] + c[6];
-  E.kagg[KT_EVAL_HUGE].items += c[5];
-  cudaEvent_t e_m = E.kt_begin();
-  if (c[3]) {
-    EvalArgs a = A;
-    a.counters = counters ? counters + 2 : nullptr;
-    a.idx = vo + start[3];
-    a.nidx = c[3];
-    u32 blocks = grid_for((u64)c[3] * 32, MID_WARPS * 32);
-    if (kind == EVAL_MOVE)
-      ++E.nlaunch, k_eval_mid<EVAL_MOVE><<<blocks, MID_WARPS * 32, 0, st>>>(a);
-    else
-      ++E.nlaunch, k_eval_mid<EVAL_REFINE><<<blocks, MID_WARPS * 32, 0, st>>>(a);
-  }
-  HL_LAUNCH_CHECK();
-  E.kt_end(KT_EVAL_MID, e_m);
-  cudaEvent_t e_b = E.kt_begin();
-  if (c[4]) {
-    EvalArgs a = A;
-    a.counters = counters ? counters + 4 : nullptr;
-    a.prune = prune;
-    a.idx = vo + start[4];
-    a.nidx = c[4];
-    u32 blocks = grid_for((u64)c[4] * 32, WIDE_WARPS * 32);
-    if (blocks > WIDE_SPLIT_MAX_BLOCKS) blocks = WIDE_SPLIT_MAX_BLOCKS;
-    constexpr u32 T = 2 * WIDE_SPLIT;
-    if (kind == EVAL_MOVE)
-      ++E.nlaunch, k_eval_wide<EVAL_MOVE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), st>>>(a);
-    else
-      ++E.nlaunch, k_eval_wide<EVAL_REFINE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), st>>>(a);
     HL_LAUNCH_CHECK();
-  }
-  if (c[6]) {
-    EvalArgs a = A;
-    a.counters = counters ? counters + 4 : nullptr;
-    a.prune = prune;
-    a.idx = vo + start[6];
-    a.nidx = c[6];
-    u32 blocks = grid_for((u64)c[6] * 32, WIDE_WARPS * 32);
-    if (blocks > WIDE_MAX_BLOCKS) blocks = WIDE_MAX_BLOCKS;
-    constexpr u32 T = 2 * WIDE_MAX;
-    if (kind == EVAL_MOVE)
-      ++E.nlaunch, k_eval_wide<EVAL_MOVE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), st>>>(a);
-    else
-      ++E.nlaunch, k_eval_wide<EVAL_REFINE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), st>>>(a);
+    E.kt_end(KT_EVAL_SMALL, e_s, on);
+    E.kagg[KT_EVAL_SMALL].items += (u64)c[0] + c[1] + c[2];
+    E.kagg[KT_EVAL_MID].items += c[3];
+    E.kagg[KT_EVAL_BIG].items += (u64)c[4] + c[6];
+    E.kagg[KT_EVAL_HUGE].items += c[5];
+    cudaEvent_t e_m = E.kt_begin(on);
+    if (c[3]) {
+      EvalArgs a = A;
+      a.counters = counters ? counters + 2 : nullptr;
+      a.idx = vo + start[3];
+      a.nidx = c[3];
+      u32 blocks = grid_for((u64)c[3] * 32, MID_WARPS * 32);
+      if (kind == EVAL_MOVE)
+        ++E.nlaunch, k_eval_mid<EVAL_MOVE><<<blocks, MID_WARPS * 32, 0, on>>>(a);
+      else
+        ++E.nlaunch, k_eval_mid<EVAL_REFINE><<<blocks, MID_WARPS * 32, 0, on>>>(a);
+    }
     HL_LAUNCH_CHECK();
-  }
-  E.kt_end(KT_EVAL_BIG, e_b);
+    E.kt_end(KT_EVAL_MID, e_m, on);
+    cudaEvent_t e_b = E.kt_begin(on);
+    if (c[4]) {
+      EvalArgs a = A;
+      a.counters = counters ? counters + 4 : nullptr;
+      a.prune = prune;
+      a.idx = vo + start[4];
+      a.nidx = c[4];
+      u32 blocks = grid_for((u64)c[4] * 32, WIDE_WARPS * 32);
+      if (blocks > WIDE_SPLIT_MAX_BLOCKS) blocks = WIDE_SPLIT_MAX_BLOCKS;
+      constexpr u32 T = 2 * WIDE_SPLIT;
+      if (kind == EVAL_MOVE)
+        ++E.nlaunch, k_eval_wide<EVAL_MOVE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), on>>>(a);
+      else
+        ++E.nlaunch, k_eval_wide<EVAL_REFINE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), on>>>(a);
+      HL_LAUNCH_CHECK();
+    }
+    if (c[6]) {
+      EvalArgs a = A;
+      a.counters = counters ? counters + 4 : nullptr;
+      a.prune = prune;
+      a.idx = vo + start[6];
+      a.nidx = c[6];
+      u32 blocks = grid_for((u64)c[6] * 32, WIDE_WARPS * 32);
+      if (blocks > WIDE_MAX_BLOCKS) blocks = WIDE_MAX_BLOCKS;
+      constexpr u32 T = 2 * WIDE_MAX;
+      if (kind == EVAL_MOVE)
+        ++E.nlaunch, k_eval_wide<EVAL_MOVE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), on>>>(a);
+      else
+        ++E.nlaunch, k_eval_wide<EVAL_REFINE, T><<<blocks, WIDE_WARPS * 32, sizeof(WideSmem<T>), on>>>(a);
+      HL_LAUNCH_CHECK();
+    }
+    E.kt_end(KT_EVAL_BIG, e_b, on);
+  };
+  struct Join {  // the engine's stream goes on after the other one, also on an exception
+    Engine& E;
+    bool forked = false;
+    void now() {
+      if (forked) E.side_end();
+      forked = false;
+    }
+    ~Join() { now(); }
+  } join{E};
+  if (!fork) rest(st);
   cudaEvent_t e_h = E.kt_begin();
   if (c[5]) {
     // Pass 1: shared tables only; rows with more than BIG_TAB / 2 distinct keys
@@ -1918,12 +1940,17 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
     S.ovf.ensure(E.mem, c[5]);
     a.ovf_list = S.ovf.p;
     a.ovf_count = S.ovf_cnt.p;  // zeroed with the bin counters
+    if (fork) {
+      E.side_begin();
+      join.forked = true;
+    }
     u32 blocks = c[5] < BIG_MAX_BLOCKS ? c[5] : BIG_MAX_BLOCKS;
     if (kind == EVAL_MOVE)
       ++E.nlaunch, k_eval_big<EVAL_MOVE><<<blocks, BIG_THREADS, big_smem(), st>>>(a);
     else
       ++E.nlaunch, k_eval_big<EVAL_REFINE><<<blocks, BIG_THREADS, big_smem(), st>>>(a);
     HL_LAUNCH_CHECK();
+    if (fork) rest(E.side);
     const u32* pass2_list = S.ovf.p;
     const u32* pass2_count = S.ovf_cnt.p;
     bool pass2 = big_maxdeg > BIG_TAB / 2;
@@ -1977,6 +2004,7 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
     }
   }
   E.kt_end(KT_EVAL_HUGE, e_h);
+  join.now();
   E.kt_end(kind == EVAL_MOVE ? KT_MOVE_EVAL : KT_REFINE_EVAL, ev);
 }
 

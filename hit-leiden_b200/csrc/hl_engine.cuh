@@ -178,11 +178,24 @@ struct Prune {
 struct Engine {
   // the staging block and the buffers go back with nothing in flight
   ~Engine() {
+    if (side) cudaStreamSynchronize(side);
     if (stream) cudaStreamSynchronize(stream);
+    if (side_go) cudaEventDestroy(side_go);
+    if (side_done) cudaEventDestroy(side_done);
+    if (side) cudaStreamDestroy(side);
   }
   hl_config cfg{};
   int device = 0;
   cudaStream_t stream = nullptr;
+  // A second stream for launches that need nothing from the engine's current
+  // ones (created by the first large frontier that has both kinds of rows):
+  // side_begin lets it start where the engine's stream is now, side_end makes
+  // the engine's stream wait for all of it, before anything reads or frees what
+  // it uses.
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_go = nullptr, side_done = nullptr;
+  void side_begin();
+  void side_end();
   MemCtx mem;
   Scratch sc;
   std::vector<Level> levels;
@@ -225,8 +238,9 @@ struct Engine {
   KernelAgg kagg[KT_COUNT];
   std::vector<cudaEvent_t> ev_pool;
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> ev_pending;
-  cudaEvent_t kt_begin();
-  void kt_end(int id, cudaEvent_t a);
+  // on `s`, or on the engine's stream
+  cudaEvent_t kt_begin(cudaStream_t s = nullptr);
+  void kt_end(int id, cudaEvent_t a, cudaStream_t s = nullptr);
   void kt_collect();
 
   u64 read_u64(const u64* dptr);

@@ -1,6 +1,6 @@
 """The single-launch stages on the GPU (one kernel per stage for batches and
 levels that fit it) against the oracle, at the sizes where their shape changes:
-one block, a cluster, a cooperative grid; sort chunks of 64 to 2048 records; the
+one block, a cluster, a cooperative grid; sort chunks of 64 to 1024 records; the
 largest batch they take and the first one that goes to the multi-kernel path.
 
 Tolerance: bit-exact."""
@@ -225,3 +225,23 @@ def test_modularity_and_partition_shapes(shape, integral):
         assert abs(st.modularity(part) - q) <= 1e-12 * max(1.0, abs(q))
     assert np.array_equal(st.partition(), O.canonicalize(st.community_mapping_per_level[0]))
     st.close()
+
+
+# From 148 rows above 512 entries and 65,536 others on, the two kinds are
+# evaluated on two streams; one hub or one vertex fewer keeps a single one.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("hubs,others", [(148, 65536), (147, 65536), (148, 65535)])
+def test_hub_rows_beside_the_others(hubs, others, integral):
+    n = hubs + others
+    rng = np.random.default_rng(n + integral)
+    s = np.concatenate([np.repeat(np.arange(hubs), 700), rng.integers(hubs, n, 2 * n),
+                        np.arange(hubs, n)])
+    d = np.concatenate([rng.integers(hubs, n, 700 * hubs), rng.integers(hubs, n, 2 * n),
+                        np.roll(np.arange(hubs, n), 1)])
+    w = np.ones(len(s)) if integral else rng.uniform(0.5, 2.0, len(s))
+    g = O.Graph.from_edges(n, s.astype(np.uint32), d.astype(np.uint32), w)
+    f = gh.random_partition(rng, n, n // 20)
+    sub = np.arange(n, dtype=np.uint32)
+    ref = O.inc_movement(g, [], [], [], f.copy(), sub, 1.0, O.MODE_THROUGHPUT, max_rounds=3)
+    got = gh.inc_movement(g, [], [], [], f, sub, 1.0, max_rounds=3)
+    assert all(np.array_equal(ref[i], got[i]) for i in range(3))
