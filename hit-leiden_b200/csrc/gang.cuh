@@ -412,7 +412,8 @@ __device__ __forceinline__ void gang_label_sort(const Gang& G, GangSmem& S, u32 
 // 32 positions and the segments that start there; one that ends within the next
 // position is the last of its 32, found by a 32-way search.  Segments of up to
 // 16 terms take a lane, longer ones the warp (`buf`: CHAIN_TILE doubles of it).
-template <typename T, typename DN>
+// ANY_ORDER: sums that are exact in every order, the long ones lane by lane.
+template <bool ANY_ORDER = false, typename T, typename DN>
 __device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T* lab,
                                                   const double* x, double* buf, DN done) {
   const u32 lane = threadIdx.x & 31;
@@ -463,7 +464,14 @@ __device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T*
     for (u32 bm = __ballot_sync(0xffffffffu, len > 16); bm; bm &= bm - 1) {
       const u32 l = __ffs(bm) - 1;
       const u32 e = __shfl_sync(0xffffffffu, end, l);
-      const double s = warp_chain_sum(t0 + l, e, 0.0, x, buf);
+      double s = 0.0;
+      if (ANY_ORDER) {
+#pragma unroll 8
+        for (u32 q = t0 + l + lane; q < e; q += 32) s += x[q];
+        for (u32 o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      } else {
+        s = warp_chain_sum(t0 + l, e, 0.0, x, buf);
+      }
       if (lane == l) done(c, s);
     }
   }

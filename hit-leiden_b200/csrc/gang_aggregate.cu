@@ -135,8 +135,8 @@ __device__ __forceinline__ u32 gg_slice(const GangAggArgs& A, u64 it, u32 at) {
 // What bounds it: the chain of its two sorts, scans and barriers.  Against the
 // multi-kernel form (some thirty launches and five host reads a level), the
 // stage with the next level's growth and projection: 5 levels of 250-400 nodes
-// 290 -> 45 us, 10 levels of 10-50k nodes 370 -> 90 us, 10 levels of 0.13-1M
-// nodes 420 -> 95 us.
+// 290 -> 22 us, 10 levels of 10-50k nodes 370 -> 79 us, 10 levels of 0.13-1M
+// nodes 420 -> 61 us (events around the launch).
 __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_aggregate(GangAggArgs A) {
   __shared__ GangSmem S;
   __shared__ __align__(16) double chain[GANG_WARPS][CHAIN_TILE];

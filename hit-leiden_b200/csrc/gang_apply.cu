@@ -95,8 +95,10 @@ __device__ __forceinline__ void ga_tree_tiles(const Gang& G, GangSmem& S, const 
 // 29.0M entries in 173 us, 4.0 TB/s), on small ones the chain of sorts,
 // searches and barriers.  Against the multi-kernel form it replaces (some
 // forty launches and five host reads a level), the whole stage of one level:
-// 5 levels of 250-400 nodes 240 -> 50 us, 20k nodes / 400k entries 460 -> 180
-// us, 10 levels of 0.13-1M nodes with f64 weights 830 -> 390 us.
+// 5 levels of 250-400 nodes 240 -> 36 us, 10 levels of 10-50k nodes 460 -> 113
+// us, 10 levels of 0.13-1M nodes with f64 weights 830 -> 350 us (of which the
+// rewrite 90-220, the chains of hub rows 40-110, two sorts 65; events around
+// the launch).
 __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_apply(GangApplyArgs A) {
   __shared__ GangSmem S;
   __shared__ __align__(16) double chain[GANG_WARPS][CHAIN_TILE];

@@ -43,7 +43,7 @@ struct GangModArgs {
   const double* k;
   const u32* part;
   double tw;
-  bool grid;
+  bool grid, integral;
   u32 *lab, *idx, *lab2, *idx2, *hist, *gpart;
   double* kval;
   double* partial;  // per block: intra hi, lo, expected hi, lo
@@ -95,20 +95,62 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_modularity(GangModArgs
     if (lane == 0 && mx) atomicMax(&C.maxlab, mx);
   }
   G.sync();
-  // ---- members by community, their degrees in that order ----
-  const u32 bits = C.maxlab ? 32 - __clz(C.maxlab) : 1;
-  bool second;
-  gang_label_sort(G, S, A.n, bits, [&](u32 i) { return A.part[i]; }, A.lab, A.idx, A.lab2,
-                  A.idx2, A.hist, A.gpart, &second);
-  const u32* lab = second ? A.lab2 : A.lab;
-  const u32* idx = second ? A.idx2 : A.idx;
-  for (u32 t = gt; t < A.n; t += gts) A.kval[t] = A.k[idx[t]];
-  G.sync();
-  // ---- Σ_C d(C)²/2m ----
   DD expected{0.0, 0.0}, intra{0.0, 0.0};
-  gang_segment_sums(G, A.n, lab, A.kval, chain[threadIdx.x >> 5], [&](u32, double x) {
+  auto square = [&](u32, double x) {
     expected = dd_add(expected, __ddiv_rn(__dmul_rn(x, x), A.tw));
-  });
+  };
+  if (A.integral && C.maxlab < A.n) {
+    // ---- Σ_C d(C)²/2m: integral degrees add up in any order, in shared memory
+    // while the labels fit it.  A sort and one ordered chain a community instead
+    // take 890 us on a partition of a few large communities, this form 320.
+    const u32 nc = C.maxlab + 1;
+    const bool local = nc <= GANG_WORDS;
+    for (u32 c = gt; c < nc; c += gts) A.kval[c] = 0.0;
+    if (local)
+      for (u32 c = threadIdx.x; c < nc; c += GANG_THREADS) S.key[c] = 0;
+    __syncthreads();
+    G.sync();
+    for (u32 t0 = G.warp() * 32; t0 < A.n; t0 += G.warps() * 32) {
+      const u32 v = t0 + lane;
+      const bool ok = v < A.n;
+      const u32 c = ok ? A.part[v] : 0;
+      unsigned long long x = ok ? (unsigned long long)A.k[v] : 0ull;
+      const u32 grp = __match_any_sync(0xffffffffu, ok ? c : NONE32);
+      const bool lead = ok && lane == (u32)(__ffs(grp) - 1);
+      // lanes of one community add up first
+      for (u32 m = __ballot_sync(0xffffffffu, lead && (grp & (grp - 1))); m; m &= m - 1) {
+        const u32 l = __ffs(m) - 1;
+        const u32 gm = __shfl_sync(0xffffffffu, grp, l);
+        unsigned long long y = (gm >> lane) & 1u ? x : 0ull;
+        for (u32 o = 16; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        if (lane == l) x = y;
+      }
+      if (!lead) continue;
+      if (local) atomicAdd(reinterpret_cast<unsigned long long*>(&S.key[c]), x);
+      else atomicAdd(&A.kval[c], (double)x);
+    }
+    __syncthreads();
+    if (local)
+      for (u32 c = threadIdx.x; c < nc; c += GANG_THREADS)
+        if (S.key[c]) atomicAdd(&A.kval[c], (double)S.key[c]);
+    G.sync();
+    for (u32 c = gt; c < nc; c += gts) square(c, A.kval[c]);
+  } else {
+    // ---- members by community, their degrees in that order ----
+    const u32 bits = C.maxlab ? 32 - __clz(C.maxlab) : 1;
+    bool second;
+    gang_label_sort(G, S, A.n, bits, [&](u32 i) { return A.part[i]; }, A.lab, A.idx, A.lab2,
+                    A.idx2, A.hist, A.gpart, &second);
+    const u32* lab = second ? A.lab2 : A.lab;
+    const u32* idx = second ? A.idx2 : A.idx;
+    for (u32 t = gt; t < A.n; t += gts) A.kval[t] = A.k[idx[t]];
+    G.sync();
+    // ---- Σ_C d(C)²/2m ----
+    if (A.integral)
+      gang_segment_sums<true>(G, A.n, lab, A.kval, chain[threadIdx.x >> 5], square);
+    else
+      gang_segment_sums(G, A.n, lab, A.kval, chain[threadIdx.x >> 5], square);
+  }
   // ---- intra weight: eight lanes a row, taken by the warps as they come ----
   const u32 sub = lane & 7;
   const u32 chunks = (A.n + MOD_ROWS - 1) / MOD_ROWS;
@@ -219,6 +261,7 @@ double modularity(Engine& E, Level& L, const u32* part) {
   A.k = L.k.p;
   A.part = part;
   A.tw = L.tw;
+  A.integral = E.integral;
   A.grid = shape.grid;
   A.lab = S.used.p;
   A.lab2 = S.rank.p;

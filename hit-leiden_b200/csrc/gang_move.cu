@@ -260,9 +260,10 @@ __device__ __forceinline__ void gm_eval(const GangMoveArgs& A, WarpTabs& W, Move
 // What bounds it: the chain of its steps (barriers and dependent L2 accesses);
 // with many active rows, the gathers of their neighbours' labels.  Against the
 // multi-kernel rounds and the one-block rounds it replaces, the stage of one
-// level: 5 levels of 250-400 nodes 88 -> 45 us, 3 levels of 7-10k nodes
-// 415 -> 100 us, 10 levels of 10-50k nodes 410 -> 100 us, one level of 100k
-// nodes 570 -> 230 us, 10 levels of 0.13-1M nodes with f64 weights 750 -> 510 us.
+// level: 5 levels of 250-400 nodes 88 -> 23 us, 3 levels of 7-10k nodes
+// 415 -> 79 us, 10 levels of 10-50k nodes 410 -> 54 us, one level of 100k nodes
+// 570 -> 210 us, 10 levels of 0.13-1M nodes with f64 weights 750 -> 440 us (events
+// around the launch).
 __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
   extern __shared__ __align__(16) unsigned char gm_raw[];
   MoveSmem& M = *reinterpret_cast<MoveSmem*>(gm_raw);

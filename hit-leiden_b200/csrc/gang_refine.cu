@@ -225,9 +225,9 @@ __device__ __forceinline__ void gr_result(const Gang& G, const GangRefArgs& A, u
 // What bounds it: a chain of some fifteen dependent steps of 1-10 us each
 // (barriers, L2 round trips); on hub levels the unions.  Against the
 // multi-kernel form (some fifty launches and six host reads a level), the
-// stage of one level: 5 levels of 250-400 nodes 330 -> 45 us, 3 levels of
-// 7-10k nodes 370 -> 70 us, 10 levels of 10-50k nodes 445 -> 130 us, 10 levels
-// of 0.13-1M nodes with f64 weights 235 -> 85 us.
+// stage of one level: 5 levels of 250-400 nodes 330 -> 27 us, 3 levels of
+// 7-10k nodes 370 -> 51 us, 10 levels of 10-50k nodes 445 -> 88 us, 10 levels
+// of 0.13-1M nodes with f64 weights 235 -> 66 us (events around the launch).
 __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) {
   extern __shared__ __align__(16) unsigned char gr_raw[];
   RefSmem& W = *reinterpret_cast<RefSmem*>(gr_raw);

@@ -136,7 +136,11 @@ struct DBuf {
     if (n <= cap) return;
     if (!c.budget) {
       release();  // contents are not kept
-      n += n / 16;
+      try {
+        ensure(c, n + n / 16);
+        return;
+      } catch (const Error&) {  // the device is that full: without the room
+      }
     }
     ensure(c, n);
   }
