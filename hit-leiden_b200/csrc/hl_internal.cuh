@@ -323,15 +323,28 @@ __device__ __forceinline__ double warp_chain_sum(u64 a, u64 b, double acc, const
     }
     const u32 cnt = b - base < CHAIN_TILE ? (u32)(b - base) : CHAIN_TILE;
     const double2* b2 = reinterpret_cast<const double2*>(buf);
+    // 16 terms at a time, the next 16 on their way while these are added (they
+    // may lie beyond the tile's end, not beyond the buffer's)
     u32 i = 0;
+    double2 y[8], z[8];
+#pragma unroll
+    for (u32 j = 0; j < 8; ++j) y[j] = b2[j];
+#pragma unroll 1
     for (; i + 32 <= cnt; i += 32) {
-      double2 y[16];
 #pragma unroll
-      for (u32 j = 0; j < 16; ++j) y[j] = b2[i / 2 + j];
+      for (u32 j = 0; j < 8; ++j) z[j] = b2[i / 2 + 8 + j];
 #pragma unroll
-      for (u32 j = 0; j < 16; ++j) {
+      for (u32 j = 0; j < 8; ++j) {
         acc = __dadd_rn(acc, y[j].x);
         acc = __dadd_rn(acc, y[j].y);
+      }
+      const u32 nx = i + 32 < CHAIN_TILE ? i / 2 + 16 : 0;
+#pragma unroll
+      for (u32 j = 0; j < 8; ++j) y[j] = b2[nx + j];
+#pragma unroll
+      for (u32 j = 0; j < 8; ++j) {
+        acc = __dadd_rn(acc, z[j].x);
+        acc = __dadd_rn(acc, z[j].y);
       }
     }
     for (; i + 4 <= cnt; i += 4) {
