@@ -1171,6 +1171,11 @@ hl_status hl_dbg_set_bins(uint32_t mid_max, uint32_t wide_max) {
   return HL_OK;
 }
 
+hl_status hl_dbg_set_selection(hl_graph* g, uint32_t round, uint64_t epoch) {
+  HL_TRY(require(g && epoch, "NULL handle or epoch 0"); Engine& E = *box(g)->E;
+         E.sel_round = round; E.epoch = epoch);
+}
+
 hl_status hl_dbg_set_bucket_slots(uint32_t slots) {
   g_pb_slots.store(slots);  // 0 (or out of range): the fold kernel's full table
   return HL_OK;

@@ -96,6 +96,7 @@ struct GangMoveArgs {
   double* gw;
   u32* part;
   u32 it0, max_rounds, round0;
+  bool more;  // max_rounds is this launch's own limit, not the movement's
   u64 epoch0;
   u32 label_bits;
   MoveCnt* cnt;
@@ -357,7 +358,10 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
         if (A.status[r] == GM_ACCEPTED) A.prune.drop[A.sel_from[r]] = 0.0;
       m_last = 0;
     }
-    if (it >= A.max_rounds || nv + nh == 0) break;
+    if (it >= A.max_rounds || nv + nh == 0) {
+      if (A.more && nv + nh) status = MOVE_BIG_FRONTIER;
+      break;
+    }
     if (nv > A.list_cap || nh > A.list_cap || nv + nh > A.list_cap) {
       status = MOVE_BIG_FRONTIER;
       break;
@@ -718,8 +722,9 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
   static_assert(sizeof(MoveCnt) <= GANG_CNT * sizeof(u32), "fits the counter block");
   static_assert(sizeof(MoveOutDev) <= 64 * sizeof(u64), "fits the pinned block");
-  u32 round0 = E.sel_round;
-  if (round0 + E.cfg.max_rounds + 2 >= (1u << 29)) round0 = E.sel_round = 1;
+  selection_room(E);
+  const u32 max_rounds =
+      E.cfg.mode == HL_MODE_DETERMINISTIC ? 0 : E.cfg.max_rounds ? E.cfg.max_rounds : 20;
   A.n = n;
   A.off = L.g.off.p;
   A.col = L.g.col.p;
@@ -770,8 +775,9 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   A.items_cap = (u32)std::min<u64>(items_cap, 0xFFFFFFFFull);
   A.part = S.gang_part.p;
   A.it0 = it;
-  A.max_rounds = E.cfg.mode == HL_MODE_DETERMINISTIC ? 0 : E.cfg.max_rounds ? E.cfg.max_rounds : 20;
-  A.round0 = round0;
+  A.more = max_rounds > it && max_rounds - it > SEL_ROUNDS;
+  A.max_rounds = A.more ? it + SEL_ROUNDS : max_rounds;
+  A.round0 = E.sel_round;
   A.epoch0 = E.epoch;
   A.label_bits = (u32)bits_for(n - 1);
   A.cnt = reinterpret_cast<MoveCnt*>(gang_counters(E, &A.cnt_next));

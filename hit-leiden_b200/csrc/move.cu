@@ -506,6 +506,19 @@ void ensure_comm_arrays(Engine& E, size_t ncap) {
   if (S.role.cap != old_role) HL_CUDA(cudaMemsetAsync(S.role.p, 0, S.role.cap * sizeof(u32), E.stream));
 }
 
+// Role tags hold a round below 2^29 and reservation keys an epoch below 2^32.
+// Before SEL_ROUNDS more rounds could pass either bound, both counters start
+// again, and the tags and keys of the old count go with them: a tag that
+// another movement left under the same number would read as this round's.
+void selection_room(Engine& E) {
+  if ((u64)E.sel_round + SEL_ROUNDS < (1u << 29) && E.epoch < (1ull << 31)) return;
+  Scratch& S = E.sc;
+  if (S.role.p) HL_CUDA(cudaMemsetAsync(S.role.p, 0, S.role.cap * sizeof(u32), E.stream));
+  if (S.res.p) HL_CUDA(cudaMemsetAsync(S.res.p, 0, S.res.cap * sizeof(u64), E.stream));
+  E.sel_round = 0;
+  E.epoch = 1;
+}
+
 // Decides every sorted candidate in S.sel_from / S.sel_to (rank order):
 // S.status[r] = accepted / rejected exactly as the sequential greedy would.
 void select_decoupled_dev(Engine& E, u32 M) {
@@ -514,8 +527,8 @@ void select_decoupled_dev(Engine& E, u32 M) {
   u32* cnt = S.cnt.p;
   cudaEvent_t ev = E.kt_begin();
   HL_CUDA(cudaMemsetAsync(S.status.p, ST_UNDECIDED, M, st));
-  u32 round = ++E.sel_round;
-  if (round >= (1u << 29)) E.sel_round = round = 1;
+  selection_room(E);
+  const u32 round = ++E.sel_round;
   u32 iters = 0;
   while (true) {
     for (int rep = 0; rep < 4; ++rep) {

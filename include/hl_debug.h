@@ -116,6 +116,11 @@ HL_API hl_status hl_dbg_set_pb_round(uint64_t entries);
  * from.  Results do not depend on them. */
 HL_API hl_status hl_dbg_set_bins(uint32_t mid_max, uint32_t wide_max);
 
+/* The handle's selection counters: the round its role tags and the epoch its
+ * reservation keys stand at.  Both start again near 2^29 and 2^31; tests set
+ * them there (between calls on the handle).  Results do not depend on them. */
+HL_API hl_status hl_dbg_set_selection(hl_graph* g, uint32_t round, uint64_t epoch);
+
 /* Modularity of `part` on the CSR (hit_leiden.rs:121-161). */
 HL_API hl_status hl_dbg_modularity(int32_t device, uint32_t n, const uint64_t* off, const uint32_t* col,
                             const double* w, const uint32_t* part, double* q);
