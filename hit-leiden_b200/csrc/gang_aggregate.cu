@@ -17,7 +17,9 @@ constexpr u32 AGG_LANE = 16;         // sums up to this length: a lane each
 constexpr u32 AGG_MAX_REC = 65536;
 
 struct AggCnt {  // zeroed by the host
-  u32 nitems, nlong, pad_[30];
+  u32 nitems, nlong;
+  unsigned long long total;  // records of the changed rows
+  u32 pad_[28];
 };
 
 struct AggOut {
@@ -195,28 +197,40 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_aggregate(GangAggArgs 
   }
   u32 R = A.dk;
   const u32 nitems = C.nitems;
+  // Everything is counted before anything is sorted: the sort's ranks cost
+  // nitems^2 / 1024 searches (a split star of 1M leaves: 27 ms), and the total
+  // of up to AGG_MAX_REC slices fits 32 bits.
+  bool fits = nitems <= AGG_MAX_REC;
+  if (fits && nitems) {
+    unsigned long long mine = 0;
+    for (u32 i = G.warp(); i < nitems; i += G.warps()) {
+      const u32 c = gg_slice<false>(A, A.items[i], 0);
+      if (lane == 0) A.ipos[i] = c;
+      mine += c;
+    }
+    if (lane == 0 && mine) atomicAdd(&C.total, mine);
+    G.sync();
+    fits = C.total + A.dk <= AGG_MAX_REC;
+  }
+  if (!fits) {
+    if (gt == 0) {
+      A.out->status = 1;
+      A.out->count = 0;
+      A.out->records = 0;
+    }
+    return;
+  }
   if (nitems) {
     // ---- records of every changed row, in vertex and CSR order ----
     gang_sort(
         G, S, nitems, [&](u32 i) { return A.items[i]; }, [](u32 i) { return i; }, A.itmp, A.itv,
-        [&](u32 r, u64 key, u32) { A.items2[r] = key; });
-    for (u32 i = G.warp(); i < nitems; i += G.warps()) {
-      const u32 c = gg_slice<false>(A, A.items2[i], 0);
-      if (lane == 0) A.icnt[i] = c;
-    }
-    G.sync();
-    const u32 total = gang_scan(
+        [&](u32 r, u64 key, u32 i) {
+          A.items2[r] = key;
+          A.icnt[r] = A.ipos[i];
+        });
+    R += gang_scan(
         G, S, nitems, [&](u32 i) { return A.icnt[i]; }, [&](u32 i, u32 ex) { A.ipos[i] = ex; },
         A.part);
-    if ((u64)total + A.dk > AGG_MAX_REC) {
-      if (gt == 0) {
-        A.out->status = 1;
-        A.out->count = 0;
-        A.out->records = 0;
-      }
-      return;
-    }
-    R += total;
     G.sync();
     for (u32 i = G.warp(); i < nitems; i += G.warps())
       gg_slice<true>(A, A.items2[i], A.dk + A.ipos[i]);

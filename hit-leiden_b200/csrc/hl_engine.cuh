@@ -288,9 +288,10 @@ void recompute_comm_degrees(Engine& E, Level& L, const u32* part, u32 ncomm_cap,
 void compact_labels_if_needed(Engine& E, u32* labels, u32 n, u32 limit);
 void select_decoupled_dev(Engine& E, u32 M);
 void ensure_comm_arrays(Engine& E, size_t ncap);
-// Rounds one launch of gang_move runs at most before it hands back; a round
-// takes at most 65 epochs.
-constexpr u32 SEL_ROUNDS = 1u << 24;
+// Rounds one launch of gang_move runs at most before it hands back, so that a
+// movement without a cap that never settles is a chain of launches of some 10 ms
+// (10 us a round) and not one without an end; a round takes at most 65 epochs.
+constexpr u32 SEL_ROUNDS = 1024;
 void selection_room(Engine& E);
 void prune_begin(Engine& E, const Level& L);
 void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, const u32* s,
