@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 t
     }
     for (u32 m = __ballot_sync(0xffffffffu, b - a > COMPRESS_LANE); m; m &= m - 1) {
       const u32 l = __ffs(m) - 1;
-      const double y = warp_chain_sum(__shfl_sync(0xffffffffu, a, l),
+      const double y = warp_long_sum(__shfl_sync(0xffffffffu, a, l),
                                       __shfl_sync(0xffffffffu, b, l), 0.0, sw,
                                       chain[threadIdx.x >> 5]);
       if (lane == l) x = y;

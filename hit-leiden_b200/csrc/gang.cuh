@@ -470,7 +470,7 @@ __device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T*
         for (u32 q = t0 + l + lane; q < e; q += 32) s += x[q];
         for (u32 o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       } else {
-        s = warp_chain_sum(t0 + l, e, 0.0, x, buf);
+        s = warp_long_sum(t0 + l, e, 0.0, x, buf);
       }
       if (lane == l) done(c, s);
     }

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_aggregate(GangAggArgs 
       for (u32 i = G.warp(); i < nlong; i += G.warps()) {
         const u32 t = A.longs[i];
         const u32 b = warp_bound_u64<true>(A.keys2, t, R, A.keys2[t]);
-        const double x = warp_chain_sum(t, b, 0.0, A.sw, chain[threadIdx.x >> 5]);
+        const double x = warp_long_sum(t, b, 0.0, A.sw, chain[threadIdx.x >> 5]);
         if (lane == 0) A.xs[t] = fabs(x) > 1e-9 ? x : 0.0;
       }
       G.sync();

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_apply(GangApplyArgs A)
     double* buf = chain[tid >> 5];
     for (u32 i = G.warp(); i < nlong + nrows;) {
       const u32 v = i < nlong ? A.longrows[i] : A.rows[i - nlong];
-      const double s = warp_chain_sum(off[v], off[v + 1], 0.0, w, buf);
+      const double s = warp_long_sum(off[v], off[v + 1], 0.0, w, buf);
       if (lane == 0) {
         A.k[v] = s;
         i = G.warps() + atomicAdd(&C.work, 1u);  // the next row not yet taken

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256) k_row_sum_serial(u32 n, const u64* off, c
     double mine = 0.0;
     for (u32 m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
       const u32 j = __ffs(m) - 1;
-      const double s = warp_chain_sum(__shfl_sync(0xffffffffu, a, j),
+      const double s = warp_long_sum(__shfl_sync(0xffffffffu, a, j),
                                       __shfl_sync(0xffffffffu, b, j), 0.0, w,
                                       chain[threadIdx.x >> 5]);
       if (lane == j) mine = s;
@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(256) k_row_sum_serial(u32 n, const u64* off, c
 }
 
 // Left-to-right sums of the segments [off[i], off[i+1]) of x from `init`:
-// the staged chain (paths 0 and 1) or the shuffled fold (path 2).
-template <bool STAGED>
+// the library's own choice (path 0), the run fold (1) or the shuffled fold (2).
+template <int PATH>
 __global__ void __launch_bounds__(256) k_seq_sums(u32 nseg, const u64* off, const double* x,
                                                   double init, double* out) {
   __shared__ __align__(16) double chain[8][CHAIN_TILE];
@@ -319,9 +319,10 @@ __global__ void __launch_bounds__(256) k_seq_sums(u32 nseg, const u64* off, cons
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 i = warp; i < nseg; i += nwarps) {
     const u64 a = off[i], b = off[i + 1];
-    const double s = STAGED ? warp_chain_sum(a, b, init, x, chain[threadIdx.x >> 5])
-                            : warp_ordered_sum(a, b, init, [&](u64 p) { return x[p]; },
-                                               [](u64) { return true; });
+    const double s = PATH == 0   ? warp_long_sum(a, b, init, x, chain[threadIdx.x >> 5])
+                     : PATH == 1 ? warp_fold_runs(a, b, init, x)
+                                 : warp_ordered_sum(a, b, init, [&](u64 p) { return x[p]; },
+                                                    [](u64) { return true; });
     if (lane == 0) out[i] = s;
   }
 }
@@ -331,9 +332,11 @@ void seq_sums(Engine& E, u32 nseg, const u64* off, const double* x, double init,
   if (!nseg) return;
   const u32 grid = grid_for((u64)nseg * 32);
   if (path == 2)
-    ++E.nlaunch, k_seq_sums<false><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
+    ++E.nlaunch, k_seq_sums<2><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
+  else if (path == 1)
+    ++E.nlaunch, k_seq_sums<1><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
   else
-    ++E.nlaunch, k_seq_sums<true><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
+    ++E.nlaunch, k_seq_sums<0><<<grid, 256, 0, E.stream>>>(nseg, off, x, init, out);
   HL_LAUNCH_CHECK();
 }
 

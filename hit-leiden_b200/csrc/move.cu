@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) k_comm_deg_ordered(const u32* seg_last,
   const u32 nu = *seg_last + *head_last;
   for (u64 j = warp; j < nu; j += nwarps) {
     const u32 a = ustart[j], b = (j + 1 < nu) ? ustart[j + 1] : n;
-    const double s = warp_chain_sum(a, b, 0.0, vals, chain[threadIdx.x >> 5]);
+    const double s = warp_long_sum(a, b, 0.0, vals, chain[threadIdx.x >> 5]);
     if (lane == 0) d[ukeys[j]] = s;
   }
 }

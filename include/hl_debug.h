@@ -71,9 +71,10 @@ HL_API hl_status hl_dbg_tree_sum(int32_t device, const double* x, uint64_t n, do
 /* Left-to-right f64 sums, out[i] = init + x[off[i]] + ... + x[off[i+1]-1]
  * with every addition rounded in that order: the fold behind the row sums
  * (hit_leiden.rs:1063), the community degrees and the aggregation's
- * per-super-edge sums.  paths 0 and 1 are the library's chain (terms staged in
- * shared memory, one addition after another), 2 the fold that shuffles the
- * terms through a warp's lanes; all three give the same bits.  No
+ * per-super-edge sums.  path 0 is the library's own choice (one addition after
+ * another on terms staged in shared memory, runs of same-binade terms for long
+ * segments of one sign), 1 always folds in runs, 2 shuffles the terms through a
+ * warp's lanes; all three give the same bits.  No
  * reference counterpart: the entry point exposes the fold to tests. */
 HL_API hl_status hl_dbg_seq_sums(int32_t device, uint32_t nseg, const uint64_t* off,
                                  const double* x, double init, int32_t path, double* out);

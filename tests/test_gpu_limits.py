@@ -85,6 +85,39 @@ def test_changed_rows_are_not_sorted_in_vain():
     assert ms < 5.0, ms
 
 
+# Long ordered sums choose a fold every 65,536 terms by the signs they meet, and
+# one addition after another below 16,384: at and around both lengths, sums that
+# change sign inside a piece and at its edge, zeros and values that are not
+# finite.  All three paths, bit for bit.
+@pytest.mark.parametrize("kind", ["positive", "negative", "late", "edge", "mixed", "zeros", "inf"])
+def test_long_sums_choose_their_fold(kind):
+    rng = np.random.default_rng(len(kind))
+    segs = []
+    for n in (16383, 16384, 16385, 65536, 65537, 81919, 81920, 150001):
+        x = rng.uniform(0.5, 60.0, n)
+        if kind == "negative":
+            x = -x
+        elif kind == "late":  # after the first terms that are looked at
+            x[100::7] *= -3.0
+        elif kind == "edge":
+            x[65536:] *= -1.0
+        elif kind == "mixed":
+            x[::2] *= -1.0
+        elif kind == "zeros":
+            x[rng.random(n) < 0.9] = 0.0
+        elif kind == "inf":
+            x[n // 2] = np.inf
+        segs.append(x)
+    L = gh.L
+    off = np.concatenate([[0], np.cumsum([len(s) for s in segs])]).astype(np.uint64)
+    x = np.concatenate(segs)
+    want = np.array([np.cumsum(np.concatenate([[0.0], s]))[-1] for s in segs])
+    for path in (0, 1, 2):
+        got = np.zeros(len(segs))
+        L.check(L.lib.hl_dbg_seq_sums(0, len(segs), L.ptr(off), L.ptr(x), 0.0, path, L.ptr(got)))
+        assert gh.same_bits(got, want), (kind, path)
+
+
 # Tags and reservation keys of earlier selections stay in memory.  When their
 # counters start again, a batch must not read them as its own: round numbers
 # repeat those of the batches before.  One-launch rounds and multi-kernel ones.
