@@ -139,13 +139,14 @@ __global__ void k_seg_start64(const u32* head, const u32* segid, u64 n, u32* sta
 // In-order segmented sum over the records' weights gathered into sorted
 // order (sw); keep |w| > threshold.  Most keys have a few records: a lane each
 // (a warp each took 340 us for 300k segments, 32 lanes for one addition);
-// longer segments take the warp, one after another.
+// longer segments take the warp, one after another, and those of LONG_SEG terms
+// or more (a super-edge between two giant nodes) a second launch.
 constexpr u32 COMPRESS_LANE = 16;
 
 __global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 total, u32 bits,
                                                   const u64* sk, const double* sw,
                                                   double threshold, u32* ou, u32* ov, double* ow,
-                                                  u8* keepf) {
+                                                  u8* keepf, LongList ll) {
   __shared__ __align__(16) double chain[8][CHAIN_TILE];
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
@@ -159,7 +160,9 @@ __global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 t
     } else if (b - a <= COMPRESS_LANE) {
       for (u64 t = a; t < b; ++t) x = __dadd_rn(x, sw[t]);
     }
-    for (u32 m = __ballot_sync(0xffffffffu, b - a > COMPRESS_LANE); m; m &= m - 1) {
+    if (b - a >= LONG_SEG) ll.seg[atomicAdd(ll.cnt, 1u)] = (u32)j;
+    for (u32 m = __ballot_sync(0xffffffffu, b - a > COMPRESS_LANE && b - a < LONG_SEG); m;
+         m &= m - 1) {
       const u32 l = __ffs(m) - 1;
       const double y = warp_long_sum(__shfl_sync(0xffffffffu, a, l),
                                       __shfl_sync(0xffffffffu, b, l), 0.0, sw,
@@ -170,6 +173,27 @@ __global__ void __launch_bounds__(256) k_compress(u32 U, const u32* start, u64 t
       const u64 key = sk[a];
       ou[j] = (u32)(key >> bits);
       ov[j] = (u32)(key & ((1ull << bits) - 1));
+      ow[j] = x;  // a listed segment's sum and flag are written once more
+      keepf[j] = fabs(x) > threshold ? 1 : 0;
+    }
+  }
+}
+
+// The listed segments: integral weights (exact in any order) a block each,
+// others a warp each, in order.
+template <bool ANY_ORDER>
+__global__ void __launch_bounds__(256) k_compress_long(LongList ll, u32 U, const u32* start,
+                                                       u64 total, const double* sw,
+                                                       double threshold, double* ow, u8* keepf) {
+  __shared__ __align__(16) double chain[ANY_ORDER ? 1 : 8][CHAIN_TILE];
+  const u32 cnt = *ll.cnt;
+  const u32 per = ANY_ORDER ? 1 : 8, wib = threadIdx.x >> 5;
+  for (u32 i = blockIdx.x * per + (ANY_ORDER ? 0 : wib); i < cnt; i += gridDim.x * per) {
+    const u32 j = ll.seg[i];
+    const u64 a = start[j], b = j + 1 < U ? start[j + 1] : total;
+    const double x = ANY_ORDER ? block_sum_any(sw, a, b, chain[0])
+                               : warp_long_sum(a, b, 0.0, sw, chain[ANY_ORDER ? 0 : wib]);
+    if (ANY_ORDER ? threadIdx.x == 0 : (threadIdx.x & 31) == 0) {
       ow[j] = x;
       keepf[j] = fabs(x) > threshold ? 1 : 0;
     }
@@ -221,8 +245,15 @@ static u64 compress_records(Engine& E, u64 R, double threshold, u32 bits) {
   S.op.ensure(E.mem, U);
   S.fvals.ensure(E.mem, R);
   ++E.nlaunch, k_gather_weights<<<grid_for(R), 256, 0, st>>>(vo, S.neww.p, R, S.fvals.p);
+  const LongList ll = long_list(E, R, U);
   ++E.nlaunch, k_compress<<<grid_for(U), 256, 0, st>>>(
-      U, S.seg_start.p, R, bits, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p, S.op.p);
+      U, S.seg_start.p, R, bits, ko, S.fvals.p, threshold, S.eu.p, S.ev.p, S.ew.p, S.op.p, ll);
+  if (E.integral)
+    ++E.nlaunch, k_compress_long<true><<<LONG_BLOCKS, 256, 0, st>>>(
+        ll, U, S.seg_start.p, R, S.fvals.p, threshold, S.ew.p, S.op.p);
+  else
+    ++E.nlaunch, k_compress_long<false><<<LONG_BLOCKS, 256, 0, st>>>(
+        ll, U, S.seg_start.p, R, S.fvals.p, threshold, S.ew.p, S.op.p);
   HL_LAUNCH_CHECK();
   S.eu2.ensure(E.mem, U);
   S.ev2.ensure(E.mem, U);

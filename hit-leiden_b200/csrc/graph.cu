@@ -283,19 +283,33 @@ __global__ void __launch_bounds__(256) k_rebuild(RowOps O, u32 n, u64 nnz, const
   rebuild_entries(O, nnz, col, w, ncol, nw, nnz_new, err, thread >> 5, threads >> 5);
 }
 
+LongList long_list(Engine& E, u64 total, u32 nseg) {
+  Scratch& S = E.sc;
+  const u64 cap = std::min<u64>(total / LONG_SEG + 1, nseg ? nseg : 1);
+  S.longseg.ensure(E.mem, cap);
+  S.longcnt.ensure(E.mem, 1);
+  HL_CUDA(cudaMemsetAsync(S.longcnt.p, 0, sizeof(u32), E.stream));
+  return LongList{S.longseg.p, S.longcnt.p};
+}
+
 // Row sums in CSR order (hit_leiden.rs:1063), left to right: the exact
 // rounding of the reference for any weights.  A warp takes 32 rows at a time
-// and sums those whose flag is set (all without flags) one after another.
+// and sums those whose flag is set (all without flags) one after another; the
+// long ones are listed for k_row_sum_serial_long.
 __global__ void __launch_bounds__(256) k_row_sum_serial(u32 n, const u64* off, const double* w,
-                                                        double* k, const u8* flags) {
+                                                        double* k, const u8* flags, LongList ll) {
   __shared__ __align__(16) double chain[8][CHAIN_TILE];
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 v0 = warp * 32; v0 < n; v0 += nwarps * 32) {
     const u64 v = v0 + lane;
-    const bool on = v < n && (!flags || flags[v]);
+    bool on = v < n && (!flags || flags[v]);
     const u64 a = on ? off[v] : 0, b = on ? off[v + 1] : 0;
+    if (b - a >= LONG_SEG) {
+      ll.seg[atomicAdd(ll.cnt, 1u)] = (u32)v;
+      on = false;
+    }
     double mine = 0.0;
     for (u32 m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
       const u32 j = __ffs(m) - 1;
@@ -305,6 +319,18 @@ __global__ void __launch_bounds__(256) k_row_sum_serial(u32 n, const u64* off, c
       if (lane == j) mine = s;
     }
     if (on) k[v] = mine;
+  }
+}
+
+// The listed rows, a warp each.
+__global__ void __launch_bounds__(256) k_row_sum_serial_long(LongList ll, const u64* off,
+                                                             const double* w, double* k) {
+  __shared__ __align__(16) double chain[8][CHAIN_TILE];
+  const u32 cnt = *ll.cnt;
+  for (u32 i = blockIdx.x * 8 + (threadIdx.x >> 5); i < cnt; i += gridDim.x * 8) {
+    const u32 v = ll.seg[i];
+    const double s = warp_long_sum(off[v], off[v + 1], 0.0, w, chain[threadIdx.x >> 5]);
+    if ((threadIdx.x & 31) == 0) k[v] = s;
   }
 }
 
@@ -342,28 +368,35 @@ void seq_sums(Engine& E, u32 nseg, const u64* off, const double* x, double init,
 
 // Ordered row sums of the flagged rows (all rows without flags).
 static void row_sums_ordered(Engine& E, Level& L, const u8* flags) {
+  const LongList ll = long_list(E, L.g.nnz, L.g.n);
   ++E.nlaunch, k_row_sum_serial<<<grid_for(L.g.n), 256, 0, E.stream>>>(
-      L.g.n, L.g.off.p, L.g.w.p, L.k.p, flags);
+      L.g.n, L.g.off.p, L.g.w.p, L.k.p, flags, ll);
+  ++E.nlaunch, k_row_sum_serial_long<<<LONG_BLOCKS, 256, 0, E.stream>>>(ll, L.g.off.p, L.g.w.p,
+                                                                        L.k.p);
 }
 
 // Warp-parallel row sums; only used when every weight is integral, where any
 // summation order gives the same bits.
 __global__ void k_row_sum_warp(u32 n, const u64* off, const double* w, double* k,
-                               const u8* flags) {
+                               const u8* flags, LongList ll) {
   const u32 lane = threadIdx.x & 31;
   const u64 warp = (blockIdx.x * (u64)blockDim.x + threadIdx.x) >> 5;
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 v0 = warp * 32; v0 < n; v0 += nwarps * 32) {
     const u64 v = v0 + lane;
-    const bool on = v < n && (!flags || flags[v]);
+    bool on = v < n && (!flags || flags[v]);
     const u64 a = on ? off[v] : 0, b = on ? off[v + 1] : 0;
+    if (b - a >= LONG_SEG) {
+      ll.seg[atomicAdd(ll.cnt, 1u)] = (u32)v;
+      on = false;
+    }
     double mine = 0.0;
     for (u32 m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
       const u32 j = __ffs(m) - 1;
       const u64 hi = __shfl_sync(0xffffffffu, b, j);
       u64 p = __shfl_sync(0xffffffffu, a, j) + lane;
       double s = 0.0;
-      for (; p + 224 < hi; p += 256) {  // 8 loads in flight: hub rows
+      for (; p + 224 < hi; p += 256) {  // 8 loads in flight
         double y[8];
 #pragma unroll
         for (u32 i = 0; i < 8; ++i) y[i] = w[p + 32 * i];
@@ -376,6 +409,27 @@ __global__ void k_row_sum_warp(u32 n, const u64* off, const double* w, double* k
     }
     if (on) k[v] = mine;
   }
+}
+
+// The listed rows, a block each.
+__global__ void __launch_bounds__(256) k_row_sum_warp_long(LongList ll, const u64* off,
+                                                           const double* w, double* k) {
+  __shared__ double sh[8];
+  const u32 cnt = *ll.cnt;
+  for (u32 i = blockIdx.x; i < cnt; i += gridDim.x) {
+    const u32 v = ll.seg[i];
+    const double s = block_sum_any(w, off[v], off[v + 1], sh);
+    if (threadIdx.x == 0) k[v] = s;
+  }
+}
+
+// Row sums in any order of the flagged rows (all rows without flags).
+static void row_sums_integral(Engine& E, Level& L, const u8* flags) {
+  const LongList ll = long_list(E, L.g.nnz, L.g.n);
+  ++E.nlaunch, k_row_sum_warp<<<grid_for(L.g.n), 256, 0, E.stream>>>(
+      L.g.n, L.g.off.p, L.g.w.p, L.k.p, flags, ll);
+  ++E.nlaunch, k_row_sum_warp_long<<<LONG_BLOCKS, 256, 0, E.stream>>>(ll, L.g.off.p, L.g.w.p,
+                                                                      L.k.p);
 }
 
 // Fixed-shape pairwise sum: tiles of 1024 (+0.0 padded) folded by stride
@@ -421,11 +475,8 @@ static void recompute_flagged_rows(Engine& E, Level& L, const u8* flags) {
   const u32 n = L.g.n;
   if (!n) return;
   cudaEvent_t ev = E.kt_begin();
-  if (E.integral)
-    ++E.nlaunch, k_row_sum_warp<<<grid_for(n), 256, 0, E.stream>>>(n, L.g.off.p, L.g.w.p, L.k.p,
-                                                                    flags);
-  else
-    row_sums_ordered(E, L, flags);
+  if (E.integral) row_sums_integral(E, L, flags);
+  else row_sums_ordered(E, L, flags);
   HL_LAUNCH_CHECK();
   E.kt_end(KT_ROW_SUMS, ev);
 }
@@ -433,11 +484,8 @@ static void recompute_flagged_rows(Engine& E, Level& L, const u8* flags) {
 void recompute_all_degrees(Engine& E, Level& L) {
   u32 n = L.g.n;
   if (n) {
-    if (E.integral)
-      ++E.nlaunch, k_row_sum_warp<<<grid_for(n), 256, 0, E.stream>>>(n, L.g.off.p, L.g.w.p, L.k.p,
-                                                                      nullptr);
-    else
-      row_sums_ordered(E, L, nullptr);
+    if (E.integral) row_sums_integral(E, L, nullptr);
+    else row_sums_ordered(E, L, nullptr);
     HL_LAUNCH_CHECK();
   }
   L.tw = tree_sum(E, L.k.p, n);

@@ -89,6 +89,7 @@ struct Scratch {
   DBuf<u32> ovf, ovf_cnt;  // block kernel: rows deferred to the pass with global regions
   DBuf<u32> acc_cnt;       // inc-movement: accepted moves over all rounds
   DBuf<u32> hubk, hubk2, hubv;  // block bin ordered by degree (keys, sorted keys, list)
+  DBuf<u32> longseg, longcnt;   // long rows or segments, summed apart, and their count
   DBuf<double> fvals;           // ordered sums: the terms gathered into sum order
   DBuf<double> huge_val;
   // deterministic mode (det.cu)
@@ -269,6 +270,17 @@ void recompute_all_degrees(Engine& E, Level& L);
 double tree_sum(Engine& E, const double* x, u64 n);
 void seq_sums(Engine& E, u32 nseg, const u64* off, const double* x, double init, int path,
               double* out);
+// Kernels that take 32 rows or segments a warp leave those of LONG_SEG terms or
+// more to a second launch: hub rows stand side by side (R-MAT's first vertices),
+// and one warp would sum all of its 32 one after another.  List (and zeroed
+// count) with room for every such segment of `total` terms.
+constexpr u64 LONG_SEG = 512;
+constexpr u32 LONG_BLOCKS = 148 * 4;
+struct LongList {
+  u32* seg;
+  u32* cnt;
+};
+LongList long_list(Engine& E, u64 total, u32 nseg);
 bool edges_integral(Engine& E, const DevEdges& b);
 void check_endpoints(Engine& E, const DevEdges& b, u32 n);
 

@@ -515,6 +515,24 @@ __device__ __forceinline__ double warp_long_sum(u64 a, u64 b, double acc, const 
   }
 }
 
+// Sum of xs[a..b) in any order, exact for integral terms, by a block of 256
+// threads (sh: 8 words); thread 0 holds it.
+__device__ __forceinline__ double block_sum_any(const double* xs, u64 a, u64 b, double* sh) {
+  double s = 0.0;
+  u64 p = a + threadIdx.x;
+  for (; p + 3 * 256 < b; p += 4 * 256) {
+    const double y0 = xs[p], y1 = xs[p + 256], y2 = xs[p + 512], y3 = xs[p + 768];
+    s += (y0 + y1) + (y2 + y3);
+  }
+  for (; p < b; p += 256) s += xs[p];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  for (u32 x = 1; x < 8 && threadIdx.x == 0; ++x) s += sh[x];
+  return s;
+}
+
 // First position in [lo, hi) of the ascending array a whose value is >= x.
 __device__ __forceinline__ u64 lower_bound_u32(const u32* a, u64 lo, u64 hi, u32 x) {
   while (lo < hi) {

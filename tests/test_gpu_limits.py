@@ -85,6 +85,57 @@ def test_changed_rows_are_not_sorted_in_vain():
     assert ms < 5.0, ms
 
 
+# Hub rows side by side, in a batch above the one-launch limit: their sums run
+# beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
+# weights).  Same bits as the oracle's CSR and degrees.
+@pytest.mark.parametrize("integral", [True, False])
+def test_adjacent_hub_rows(integral):
+    rng = np.random.default_rng(5)
+    n, hubs, deg = 30000, 64, 20000
+    s = np.repeat(np.arange(hubs, dtype=np.uint32), deg)
+    d = np.concatenate([rng.choice(np.arange(hubs, n), deg, replace=False)
+                        for _ in range(hubs)]).astype(np.uint32)
+    w = np.ones(len(s)) if integral else rng.uniform(0.5, 2.0, len(s))
+    gs = _load(n, (s, d, w), max_iterations=1, kernel_timing=True)
+    ref = O.State(n, levels=1, mode=O.MODE_THROUGHPUT)
+    ref.push_empty_graph()
+    ref.hit_leiden(s, d, w)
+    e = rng.choice(len(s), 40000, replace=False)
+    b = s[e], d[e], np.ones(len(e)) if integral else rng.uniform(0.5, 2.0, len(e))
+    gs.apply_batch(*b)
+    before = gs.kernel_stats()["row_sums"]
+    gs.apply_batch(*b)
+    after = gs.kernel_stats()["row_sums"]
+    ref.hit_leiden(*b)
+    ref.hit_leiden(*b)
+    _same(gs, ref)
+    off, col, wt = gs.supergraph(0)
+    ro, rc, rw = ref.graph(0).csr()
+    assert np.array_equal(off, ro) and np.array_equal(col, rc) and gh.same_bits(wt, rw)
+    assert gs.modularity() == pytest.approx(ref.modularity(0), abs=1e-12)
+    assert after["launches"] - before["launches"] == 1
+    assert after["ms"] - before["ms"] < 1.0, after["ms"] - before["ms"]
+    gs.close()
+
+
+# Two hubs whose half a million leaves each are split and merged again: the
+# upper level's edges are sums of half a million records each, which must not
+# wait for one another.
+@pytest.mark.parametrize("integral", [True, False])
+def test_long_segments_of_the_aggregation(integral):
+    n, edges = _double_star(500000, integral)
+    gs, ref = _load(n, edges), _oracle(n, edges)
+    b = np.array([2], np.uint32), np.array([3], np.uint32), np.ones(1)
+    gs.apply_batch(*b)
+    ref.hit_leiden(*b)
+    _same(gs, ref)
+    for p in range(ref.levels):
+        off, col, wt = gs.supergraph(p)
+        ro, rc, rw = ref.graph(p).csr()
+        assert np.array_equal(off, ro) and np.array_equal(col, rc) and gh.same_bits(wt, rw)
+    gs.close()
+
+
 # Long ordered sums choose a fold every 65,536 terms by the signs they meet, and
 # one addition after another below 16,384: at and around both lengths, sums that
 # change sign inside a piece and at its edge, zeros and values that are not
