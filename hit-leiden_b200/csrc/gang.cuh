@@ -99,6 +99,23 @@ __device__ __forceinline__ u32 block_scan(GangSmem& S, u32 x, u32& total) {
   return before + inc - x;
 }
 
+// d[c] += x for the lanes with `on` (the whole warp calls it), where sums are
+// exact in any order: the lanes of one id add up first.  One community may hold
+// most of a level, and 2M atomics on its word take 3 ms, a sixteenth of that so.
+__device__ __forceinline__ void warp_add_by_id(double* d, u32 c, double x, bool on) {
+  const u32 lane = threadIdx.x & 31;
+  const u32 grp = __match_any_sync(0xffffffffu, on ? c : NONE32);
+  const bool lead = on && !(grp & ((1u << lane) - 1u));
+  for (u32 m = __ballot_sync(0xffffffffu, lead && (grp & (grp - 1))); m; m &= m - 1) {
+    const u32 l = __ffs(m) - 1;
+    const u32 of = __shfl_sync(0xffffffffu, grp, l);
+    double y = (of >> lane) & 1u ? x : 0.0;
+    for (u32 o = 16; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (lane == l) x = y;
+  }
+  if (lead) atomicAdd(&d[c], x);
+}
+
 // Exclusive prefix sums of val(0..N-1), handed to out(i, prefix); returns the
 // total.  val is evaluated twice.  One gang barrier inside; the caller places
 // one before it reads what out wrote (which also frees `part`, nct words).

@@ -326,7 +326,11 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       for (u32 v = gt; v < A.n; v += gts) gm_activate(A, 0, v);
     // ---- community degrees (hit_leiden.rs:1060-1066) ----
     if (A.integral) {
-      for (u32 v = gt; v < A.n; v += gts) atomicAdd(&A.d[A.f[v]], A.k[v]);
+      for (u32 v0 = gt - lane; v0 < A.n; v0 += gts) {
+        const u32 v = v0 + lane;
+        const bool on = v < A.n;
+        warp_add_by_id(A.d, on ? A.f[v] : 0, on ? A.k[v] : 0.0, on);
+      }
     } else {
       bool second;
       gang_label_sort(G, S, A.n, A.label_bits, [&](u32 i) { return A.f[i]; }, A.lab, A.idx,

@@ -435,14 +435,15 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) 
   // ---- their members ----
   const u32 ncand = C.ncand;
   if (ncand) {
-    for (u32 v = gt; v < A.n; v += gts) {
-      const u32 x = A.s[v];
-      if (!bit_test(A.cand, x)) continue;
+    for (u32 v0 = gt - lane; v0 < A.n; v0 += gts) {
+      const u32 v = v0 + lane;
+      const u32 x = v < A.n ? A.s[v] : 0;
+      const bool on = v < A.n && bit_test(A.cand, x);
+      if (A.integral) warp_add_by_id(A.dS, x, on ? A.k[v] : 0.0, on);
+      if (!on) continue;
       atomicMin(&A.minmem[x], v);
       push_row(A.mitems, &C.nmitems, v, A.off[v + 1] - A.off[v]);
-      if (A.integral) {
-        atomicAdd(&A.dS[x], A.k[v]);
-      } else {
+      if (!A.integral) {
         const u32 at = atomicAdd(&C.nrec, 1u);
         if (at < REF_MAX_REC) A.rec[at] = ((u64)x << 33) | v;
       }
@@ -487,12 +488,13 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) 
         atomicAdd(&A.wcnt[x], (unsigned long long)c);
       }
     }
-    for (u32 v = gt; v < A.n; v += gts) {
-      const u32 c = A.f[v];
-      if (!bit_test(A.parent, c)) continue;
+    for (u32 v0 = gt - lane; v0 < A.n; v0 += gts) {
+      const u32 v = v0 + lane;
+      const u32 c = v < A.n ? A.f[v] : 0;
+      const bool on = v < A.n && bit_test(A.parent, c);
       if (A.integral) {
-        atomicAdd(&A.dcomm[c], A.k[v]);
-      } else {
+        warp_add_by_id(A.dcomm, c, on ? A.k[v] : 0.0, on);
+      } else if (on) {
         const u32 at = atomicAdd(&C.nrec, 1u);
         if (at < REF_MAX_REC) A.rec[at] = ((u64)c << 33) | (1ull << 32) | v;
       }

@@ -85,6 +85,23 @@ def test_changed_rows_are_not_sorted_in_vain():
     assert ms < 5.0, ms
 
 
+# Two million vertices in two communities: their integral degrees add up in the
+# warp before they meet on one word (3.1 ms for this batch's two levels without).
+def test_degrees_of_giant_communities():
+    n, edges = _double_star(1000000, True)
+    gs = _load(n, edges, kernel_timing=True)
+    ref = _oracle(n, edges)
+    for i in range(2):
+        before = gs.kernel_stats()["move_one_launch"]["ms"]
+        b = np.array([2 + i], np.uint32), np.array([40 + i], np.uint32), np.ones(1)
+        gs.apply_batch(*b)
+        ref.hit_leiden(*b)
+        _same(gs, ref)
+        ms = gs.kernel_stats()["move_one_launch"]["ms"] - before
+        assert ms < 1.5, ms
+    gs.close()
+
+
 # Hub rows side by side, in a batch above the one-launch limit: their sums run
 # beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
 # weights).  Same bits as the oracle's CSR and degrees.
