@@ -430,9 +430,15 @@ __device__ __forceinline__ void gang_label_sort(const Gang& G, GangSmem& S, u32 
 // position is the last of its 32, found by a 32-way search.  Segments of up to
 // 16 terms take a lane, longer ones the warp (`buf`: CHAIN_TILE doubles of it).
 // ANY_ORDER: sums that are exact in every order, the long ones lane by lane.
-template <bool ANY_ORDER = false, typename T, typename DN>
+// init(label): what a segment's sum starts from.
+struct FromZero {
+  template <typename T>
+  __device__ __forceinline__ double operator()(T) const { return 0.0; }
+};
+template <bool ANY_ORDER = false, typename T, typename DN, typename IN = FromZero>
 __device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T* lab,
-                                                  const double* x, double* buf, DN done) {
+                                                  const double* x, double* buf, DN done,
+                                                  IN init = IN{}) {
   const u32 lane = threadIdx.x & 31;
   for (u32 t0 = G.warp() * 32; t0 < n; t0 += G.warps() * 32) {
     const u32 t = t0 + lane;
@@ -466,7 +472,7 @@ __device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T*
     const u32 end = above ? t0 + __ffs(above) - 1 : end_last;
     const u32 len = head ? end - t : 0;
     if (len && len <= 16) {
-      double s = 0.0;
+      double s = init(c);
       u32 q = t;
       for (; q + 4 <= end; q += 4) {
         const double y0 = x[q], y1 = x[q + 1], y2 = x[q + 2], y3 = x[q + 3];
@@ -481,13 +487,13 @@ __device__ __forceinline__ void gang_segment_sums(const Gang& G, u32 n, const T*
     for (u32 bm = __ballot_sync(0xffffffffu, len > 16); bm; bm &= bm - 1) {
       const u32 l = __ffs(bm) - 1;
       const u32 e = __shfl_sync(0xffffffffu, end, l);
-      double s = 0.0;
+      double s = init(__shfl_sync(0xffffffffu, c, l));
       if (ANY_ORDER) {
 #pragma unroll 8
         for (u32 q = t0 + l + lane; q < e; q += 32) s += x[q];
         for (u32 o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       } else {
-        s = warp_long_sum(t0 + l, e, 0.0, x, buf);
+        s = warp_long_sum(t0 + l, e, s, x, buf);
       }
       if (lane == l) done(c, s);
     }

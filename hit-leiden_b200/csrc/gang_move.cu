@@ -86,7 +86,8 @@ struct GangMoveArgs {
   u8 *status, *nmask;
   u32* role;
   unsigned long long* res;
-  u64 *okey, *okey2, *otmp;  // d(C) updates: (community << 32 | 2 rank + enters)
+  u64 *okey, *okey2, *otmp;  // d(C) updates: (community << 32 | 2 rank + enters), sorted:
+  double* oterm;             // the communities and the signed degrees
   u32 *otv;
   u64* items;                // moved rows: (rank << 32 | slice)
   u32 items_cap;
@@ -563,21 +564,20 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     const u32 nops = R.nops;
     if (gt == 0) C.moves += nops / 2;
     if (!A.integral && nops) {
-      // d(C) -= k / += k in selected order, per community
+      // d(C) -= k / += k in selected order, per community: an ordered sum that
+      // starts from d(C) (a community that gains or loses thousands of vertices
+      // in a round is one long chain)
       gang_sort(
           G, S, nops, [&](u32 i) { return A.okey[i]; }, [](u32 i) { return i; }, A.otmp, A.otv,
-          [&](u32 r, u64 key, u32) { A.okey2[r] = key; });
-      for (u32 t = gt; t < nops; t += gts) {
-        const u32 c = (u32)(A.okey2[t] >> 32);
-        if (t && (u32)(A.okey2[t - 1] >> 32) == c) continue;
-        double x = A.d[c];
-        for (u32 j = t; j < nops && (u32)(A.okey2[j] >> 32) == c; ++j) {
-          const u32 op = (u32)A.okey2[j];
-          const double kv = A.k[A.sel_node[op >> 1]];
-          x = (op & 1) ? __dadd_rn(x, kv) : __dsub_rn(x, kv);
-        }
-        A.d[c] = x;
-      }
+          [&](u32 r, u64 key, u32) {
+            const u32 op = (u32)key;
+            const double kv = A.k[A.sel_node[op >> 1]];
+            A.okey2[r] = key >> 32;
+            A.oterm[r] = (op & 1) ? kv : -kv;
+          });
+      gang_segment_sums(
+          G, nops, A.okey2, A.oterm, M.w.sw[tid >> 5], [&](u64 c, double x) { A.d[c] = x; },
+          [&](u64 c) { return A.d[c]; });
     }
     // ---- the next frontier and K (throughput.rs:189-199), after all moves ----
     const u32 nitems = min(R.nitems, A.items_cap);
@@ -700,19 +700,20 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
     A.okey2 = S.keys2.p;
     A.otmp = S.rkeys.p;
     A.otv = S.idx.p;
+    S.fvals.ensure(E.mem, std::max<size_t>(n, 2 * (size_t)fr));
+    A.oterm = S.fvals.p;
     if (setup) {
       S.used.ensure(E.mem, n);
       S.rank.ensure(E.mem, n);
       S.order.ensure(E.mem, n);
       S.order2.ensure(E.mem, n);
       S.gm_hist.ensure(E.mem, (size_t)256 * GANG_WARPS * shape.blocks);
-      S.fvals.ensure(E.mem, n);
       A.lab = S.used.p;
       A.lab2 = S.rank.p;
       A.idx = S.order.p;
       A.idx2 = S.order2.p;
       A.hist = S.gm_hist.p;
-      A.kval = S.fvals.p;
+      A.kval = S.fvals.p;  // before any round
     }
   }
   if (L.g.nnz > GM_MAXDEG) {  // a row may be a hub

@@ -102,6 +102,30 @@ def test_degrees_of_giant_communities():
     gs.close()
 
 
+# Eight thousand vertices change community in one round, f64 weights: d(C) of
+# the two communities takes their degrees in selected order, by a warp each (2.8
+# ms of movement by a thread each, 0.9 so).
+def test_thousands_of_moves_into_one_community():
+    leaves = 8000
+    n, edges = _double_star(leaves, False)
+    gs, ref = _load(n, edges, kernel_timing=True), _oracle(n, edges)
+    at = np.arange(2, leaves + 2, dtype=np.uint32)
+    best = 1e9
+    for i in range(4):
+        for w in (5.25, -5.25):
+            b = np.ones(leaves, np.uint32), at, np.full(leaves, w)
+            before = gs.kernel_stats()["move_one_launch"]["ms"]
+            moved = gs.apply_batch(*b).moves
+            ms = gs.kernel_stats()["move_one_launch"]["ms"] - before
+            if w > 0.0:
+                assert moved > leaves
+                best = min(best, ms)
+            ref.hit_leiden(*b)
+            _same(gs, ref)
+    assert best < 1.8, best
+    gs.close()
+
+
 # Hub rows side by side, in a batch above the one-launch limit: their sums run
 # beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
 # weights).  Same bits as the oracle's CSR and degrees.
