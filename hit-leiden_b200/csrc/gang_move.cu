@@ -26,7 +26,15 @@ enum : u32 { GM_UNDECIDED = 0, GM_ACCEPTED = 1, GM_REJECTED = 2 };
 
 struct MoveRound {  // of one parity; the other one's is cleared meanwhile
   u32 nv, nh, ncand, nops, nitems, work, hwork, big, wv, wh;
+  u32 huge, whuge;  // a row of the frontier (to evaluate) outgrows the hub tables
 };
+
+// No hub table holds a row of this round: nothing further is taken up.
+__device__ __forceinline__ void gm_big(MoveRound& R) {
+  R.big = 1;
+  atomicMax(&R.work, 1u << 30);
+  atomicMax(&R.hwork, 1u << 30);
+}
 
 struct MoveCnt {  // zeroed by the host
   MoveRound r[2];
@@ -113,10 +121,12 @@ __device__ __forceinline__ void gm_activate(const GangMoveArgs& A, u32 b, u32 v)
   u32* word = &A.bits[b][v >> 5];
   if ((*word & m) || (atomicOr(word, m) & m)) return;
   MoveRound& R = A.cnt->r[b];
-  if (A.off[v + 1] - A.off[v] <= GM_MAXDEG) {
+  const u64 deg = A.off[v + 1] - A.off[v];
+  if (deg <= GM_MAXDEG) {
     const u32 at = atomicAdd(&R.nv, 1u);
     if (at < A.list_cap) A.verts[b][at] = v;
   } else {
+    if (deg > HUB_MAXDEG) R.huge = 1;
     const u32 at = atomicAdd(&R.nh, 1u);
     if (at < A.list_cap) A.hubs[b][at] = v;
   }
@@ -375,10 +385,14 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
     if (gt == 0) {
       MoveRound& N = C.r[b ^ 1];
       N.nv = N.nh = N.ncand = N.nops = N.nitems = N.work = N.hwork = N.big = N.wv = N.wh = 0;
+      N.huge = N.whuge = 0;
     }
     const u32 *verts = A.verts[b], *hubs = A.hubs[b];
     u32 ev = nv, eh = nh;  // vertices to evaluate
     unsigned long long pruned_round = 0;
+    // a row too long for the tables hands the round back before any evaluation,
+    // unless its bound rules it out
+    bool huge = R.huge != 0;
     if (A.prune.b && it > 0) {
       // rows of earlier rounds hold bounds: most need no evaluation
       for (u32 i = gt; i < nv + nh; i += gts) {
@@ -388,6 +402,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
             prune_rules_out(A.prune, shift, v, A.k[v], A.d[A.f[v]], A.tw, A.gamma)) {
           pruned_round += A.off[v + 1] - A.off[v];
         } else if (hub) {
+          if (A.off[v + 1] - A.off[v] > HUB_MAXDEG) R.whuge = 1;
           A.whubs[atomicAdd(&R.wh, 1u)] = v;
         } else {
           A.wverts[atomicAdd(&R.wv, 1u)] = v;
@@ -398,6 +413,11 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       eh = R.wh;
       verts = A.wverts;
       hubs = A.whubs;
+      huge = R.whuge != 0;
+    }
+    if (huge) {
+      status = MOVE_BIG_HUB;
+      break;
     }
     if (eh) {
       for (;;) {
@@ -409,13 +429,12 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
         const u32 v = hubs[i];
         const u64 o0 = A.off[v], o1 = A.off[v + 1];
         const u32 cur = A.f[v];
-        if (o1 - o0 > HUB_MAXDEG ||
-            !hub_sums<GANG_WARPS>(
+        if (!hub_sums<GANG_WARPS>(
                 M.h, o0, o1, A.col, A.w, A.integral,
                 [&](u32 nb) { return nb == v ? NONE32 : A.f[nb]; },
                 A.gslot + (size_t)G.rank * HUB_MAXDEG,
                 A.gw ? A.gw + (size_t)G.rank * HUB_MAXDEG : nullptr)) {
-          if (tid == 0) R.big = 1;
+          if (tid == 0) gm_big(R);
           continue;
         }
         const double kv = A.k[v], dcur = A.d[cur];

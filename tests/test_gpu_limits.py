@@ -126,6 +126,37 @@ def test_thousands_of_moves_into_one_community():
     gs.close()
 
 
+# Rows at and above the 16,384 entries the hub tables take: a longer one hands
+# the round back before it is evaluated, from a batch that touches it, from one
+# that makes its neighbours move, and where its bound rules it out.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("deg", [16384, 16385, 30000])
+def test_hub_longer_than_its_tables(deg, integral):
+    rng = np.random.default_rng(deg)
+    n = 40000
+    s, d, w = gh.random_graph(rng, n, 120000, integral)
+    hub = rng.choice(np.arange(1, n, dtype=np.uint32), deg, replace=False)
+    keep = s != 0
+    keep &= d != 0
+    s, d, w = s[keep], d[keep], w[keep]
+    s = np.concatenate([s, np.zeros(deg, np.uint32)])
+    d = np.concatenate([d, hub])
+    w = np.concatenate([w, np.ones(deg) if integral else rng.uniform(0.5, 2.0, deg)])
+    gs, ref = _load(n, (s, d, w)), _oracle(n, (s, d, w))
+    _same(gs, ref)
+    for i in range(3):
+        k = (10, 3000, 9000)[i]
+        u = rng.integers(0, n, k).astype(np.uint32)
+        v = rng.integers(0, n, k).astype(np.uint32)
+        if i == 0:
+            u[:5] = 0
+        b = u, v, np.full(k, 3.0) if integral else rng.uniform(2.0, 4.0, k)
+        gs.apply_batch(*b)
+        ref.hit_leiden(*b)
+        _same(gs, ref)
+    gs.close()
+
+
 # Hub rows side by side, in a batch above the one-launch limit: their sums run
 # beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
 # weights).  Same bits as the oracle's CSR and degrees.
