@@ -37,7 +37,9 @@ enum : u32 { DET_OK = 0, DET_POP_LIMIT = 1, DET_ID_SPACE = 2 };
 // Σw and the first CSR position of every key of row [o0, o1) into the dense
 // scratch (bw, bp), the distinct keys into klist (count in *nk).  `key(q)`
 // returns the entry's key or NONE32 to skip it.  Integral weights: the whole
-// block, atomics (every order gives the same sums).  Otherwise warp 0, in CSR
+// block, atomics of the keys of 32 entries each (every order gives the same
+// sums; most of a hub's neighbours may share one community, and an atomic an
+// entry took 20 us for a row of 1,800).  Otherwise warp 0, in CSR
 // order: a 32-entry tile at a time, entries of one key folded by its first
 // lane in lane order, tiles in order.
 template <typename K>
@@ -46,12 +48,27 @@ __device__ __forceinline__ void det_row_sums(u64 o0, u64 o1, const double* w, bo
                                              double* tile) {
   const u32 tid = threadIdx.x, lane = tid & 31;
   if (!ordered) {
-    for (u64 q = o0 + tid; q < o1; q += DET_THREADS) {
-      const u32 c = key(q);
-      if (c == NONE32) continue;
-      atomicAdd(&bw[c], w[q]);
-      const u32 old = atomicMin(&bp[c], (u32)(q - o0));
-      if (old == NONE32) klist[atomicAdd(nk, 1u)] = c;
+    for (u64 q0 = o0 + (tid - lane); q0 < o1; q0 += 4 * DET_THREADS) {
+      u32 c[4];
+      double x[4];
+#pragma unroll
+      for (u32 j = 0; j < 4; ++j) {
+        const u64 q = q0 + j * DET_THREADS + lane;
+        c[j] = q < o1 ? key(q) : NONE32;
+        x[j] = q < o1 ? w[q] : 0.0;
+      }
+#pragma unroll
+      for (u32 j = 0; j < 4; ++j) {
+        if (q0 + j * DET_THREADS >= o1) break;  // warp-uniform
+        const u64 q = q0 + j * DET_THREADS + lane;
+        const u32 grp = __match_any_sync(0xffffffffu, c[j]);
+        const bool lead = c[j] != NONE32 && !(grp & ((1u << lane) - 1u));
+        const double y = warp_group_sum(grp, lead, x[j]);
+        if (!lead) continue;
+        atomicAdd(&bw[c[j]], y);
+        const u32 old = atomicMin(&bp[c[j]], (u32)(q - o0));
+        if (old == NONE32) klist[atomicAdd(nk, 1u)] = c[j];
+      }
     }
     return;
   }
@@ -77,35 +94,44 @@ __device__ __forceinline__ void det_row_sums(u64 o0, u64 o1, const double* w, bo
   }
 }
 
-// Block argmax of (gain, first position, key) over positive gains: the
-// largest gain, ties to the smallest position.  Returns in thread 0.
+// Largest gain over the lanes (g of lanes without a candidate: 0), ties to the
+// smallest position; the winning lane, or 32 when no gain is positive.
+__device__ __forceinline__ u32 det_warp_best(double g, u32 p) {
+  const u64 key = g > 0.0 ? (u64)__double_as_longlong(g) : 0ull;  // positive: bits ascend
+  const u32 hi = (u32)(key >> 32), lo = (u32)key;
+  const u32 mh = __reduce_max_sync(0xffffffffu, hi);
+  if (!mh) return 32;
+  const u32 ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const bool best = hi == mh && lo == ml;
+  const u32 mp = __reduce_min_sync(0xffffffffu, best ? p : NONE32);
+  return __ffs(__ballot_sync(0xffffffffu, best && p == mp)) - 1;
+}
+
+// Block argmax of (gain, first position, key) over positive gains (p: NONE32
+// without one): the largest gain, ties to the smallest position.  Returns in the
+// first warp.
 __device__ __forceinline__ void det_argmax(double& g, u32& p, u32& k, double* r_g, u32* r_p,
                                            u32* r_k) {
-  const u32 tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-  for (int o = 16; o; o >>= 1) {
-    const double og = __shfl_xor_sync(0xffffffffu, g, o);
-    const u32 op = __shfl_xor_sync(0xffffffffu, p, o);
-    const u32 ok = __shfl_xor_sync(0xffffffffu, k, o);
-    if (op != NONE32 && (p == NONE32 || og > g || (og == g && op < p))) {
-      g = og;
-      p = op;
-      k = ok;
-    }
-  }
+  const u32 lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  auto warp_best = [&]() {
+    const u32 bl = det_warp_best(p != NONE32 ? g : 0.0, p);
+    g = __shfl_sync(0xffffffffu, g, bl & 31);
+    p = __shfl_sync(0xffffffffu, p, bl & 31);
+    k = __shfl_sync(0xffffffffu, k, bl & 31);
+    if (bl == 32) p = NONE32;
+  };
+  warp_best();
   if (lane == 0) {
     r_g[wib] = g;
     r_p[wib] = p;
     r_k[wib] = k;
   }
   __syncthreads();
-  if (tid == 0) {
-    for (u32 x = 1; x < DET_WARPS; ++x) {
-      if (r_p[x] != NONE32 && (p == NONE32 || r_g[x] > g || (r_g[x] == g && r_p[x] < p))) {
-        g = r_g[x];
-        p = r_p[x];
-        k = r_k[x];
-      }
-    }
+  if (wib == 0) {
+    g = lane < DET_WARPS ? r_g[lane] : 0.0;
+    p = lane < DET_WARPS ? r_p[lane] : NONE32;
+    k = lane < DET_WARPS ? r_k[lane] : NONE32;
+    warp_best();
   }
 }
 
@@ -144,7 +170,9 @@ struct DetMoveArgs {
 // the rest stay active and are evaluated again after the move.  The number taken
 // grows while nothing moves.  The active set is a three-level bit set in shared
 // memory, and so are the labels and the community degrees of small levels.
-// Rows above DET_WARP_ROW entries take the whole block, one at a time.
+// Rows above DET_WARP_ROW entries take the whole block, one at a time, and end
+// the list: where every other pop is such a row, evaluations beyond it would be
+// done again and again.
 constexpr u32 DET_AHEAD = 128;       // vertices evaluated together at most
 constexpr u32 DET_WARP_ROW = 128;
 constexpr u32 DET_TAB = 2 * DET_WARP_ROW;
@@ -152,7 +180,6 @@ constexpr u32 DET_F_LOCAL = 32768;   // nodes whose labels fit shared memory
 constexpr u32 DET_D_LOCAL = 10240;   // ... whose community degrees do, too
 constexpr size_t DET_SMEM_MAX = 216 * 1024;
 constexpr u32 DET_BITS_LOCAL = 1u << 20;  // nodes whose bit sets fit shared memory
-constexpr u32 DET_BIG = 0xFFFFFFFDu;      // result of a row left to the block
 
 struct DetWarp {
   double tv[DET_TAB];
@@ -197,19 +224,6 @@ __device__ __forceinline__ u32 det_lowest(const DetBits& B, u32 n2) {
   return NONE32;
 }
 
-// Largest gain over the lanes (g of lanes without a candidate: 0), ties to the
-// smallest position; the winning lane, or 32 when no gain is positive.
-__device__ __forceinline__ u32 det_warp_best(double g, u32 p) {
-  const u64 key = g > 0.0 ? (u64)__double_as_longlong(g) : 0ull;  // positive: bits ascend
-  const u32 hi = (u32)(key >> 32), lo = (u32)key;
-  const u32 mh = __reduce_max_sync(0xffffffffu, hi);
-  if (!mh) return 32;
-  const u32 ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  const bool best = hi == mh && lo == ml;
-  const u32 mp = __reduce_min_sync(0xffffffffu, best ? p : NONE32);
-  return __ffs(__ballot_sync(0xffffffffu, best && p == mp)) - 1;
-}
-
 // False when the computed gain of moving to (w_to, d_to) is certainly <= 0: the
 // division-free proxy Q = 2m·c·gain lies below zero by more than the rounding
 // of both (GainScreen in hl_internal.cuh).  Two divisions cost as much as the
@@ -231,7 +245,8 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
   extern __shared__ __align__(16) unsigned char det_raw[];
   DetSmem& M = *reinterpret_cast<DetSmem*>(det_raw);
   __shared__ u32 s_list[DET_AHEAD], s_to[DET_AHEAD], s_deg[DET_AHEAD];
-  __shared__ u32 s_nlist, s_first, s_nk, s_best, s_stop;
+  __shared__ u64 s_off[DET_AHEAD];
+  __shared__ u32 s_nlist, s_first, s_big, s_nk, s_best, s_stop;
   __shared__ double s_bestg;
   __shared__ double r_g[DET_WARPS];
   __shared__ u32 r_p[DET_WARPS], r_k[DET_WARPS];
@@ -276,6 +291,7 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
     }
   __syncthreads();
   u32 ahead = DET_WARPS;  // vertices taken together
+  unsigned long long trav = 0;
   while (true) {
     // ---- the next active vertices in order ----
     if (wib == 0) {
@@ -299,26 +315,28 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
       }
       if (lane == 0) {
         s_nlist = cnt;
-        s_first = NONE32;
+        s_first = s_big = NONE32;
         s_nk = 0;
       }
     }
     __syncthreads();
     const u32 nlist = s_nlist;
     if (nlist == 0) break;
-    // ---- their best moves on the current state ----
-    for (u32 i = wib; i < nlist; i += DET_WARPS) {
+    // ---- their rows; the first long one ends the list ----
+    if (tid < nlist) {
+      const u32 v = s_list[tid];
+      const u64 o0 = A.off[v], len = A.off[v + 1] - o0;
+      s_off[tid] = o0;
+      s_deg[tid] = (u32)len;
+      if (len > DET_WARP_ROW) atomicMin(&s_big, tid);
+    }
+    __syncthreads();
+    const u32 big = s_big, neval = min(nlist, big);
+    // ---- the best moves of those before it on the current state ----
+    for (u32 i = wib; i < neval; i += DET_WARPS) {
       const u32 v = s_list[i];
-      const u64 o0 = A.off[v];
-      const u32 deg = (u32)(A.off[v + 1] - o0);
-      if (deg > DET_WARP_ROW) {
-        if (lane == 0) {
-          s_deg[i] = 0;  // counted by the block
-          s_to[i] = DET_BIG;
-          atomicMin(&s_first, i);
-        }
-        continue;
-      }
+      const u64 o0 = s_off[i];
+      const u32 deg = s_deg[i];
       const u32 cur = f[v];
       const double kv = A.k[v];
       const double dcur = d_of(cur);
@@ -421,33 +439,35 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
       }
       if (may_empty && empty_gain(wcur, A.tw, A.gamma, kv, dcur) > bestg) to = DET_EMPTY;
       if (lane == 0) {
-        s_deg[i] = deg;
         s_to[i] = to;
         if (to != NONE32) atomicMin(&s_first, i);
       }
       __syncwarp();
     }
-    __syncthreads();
-    // ---- the pops: all up to the first that moves ----
-    const u32 first = s_first;
+    if (neval) __syncthreads();
+    // ---- the pops: all up to the first that moves, or the long row ----
+    const u32 first = min(s_first, big);
     const u32 popped = first == NONE32 ? nlist : first + 1;
     if (tid < popped) {
       B.clear(s_list[tid]);
-      atomicAdd(&s_trav, (unsigned long long)s_deg[tid]);
+      trav += s_deg[tid];
     }
     if (tid == 0) {
       s_pops += popped;
       if (s_pops > A.max_pops) s_stop = DET_POP_LIMIT;
     }
     __syncthreads();
-    ahead = first == NONE32 ? min(2 * ahead, DET_AHEAD) : DET_WARPS;
+    // a list that ends at a long row was too long by what it listed beyond it
+    ahead = first == NONE32 ? min(2 * ahead, DET_AHEAD)
+            : first == big  ? min(2 * popped, DET_WARPS)
+                            : DET_WARPS;
     if (s_stop != DET_OK) break;
     if (first == NONE32) continue;
     const u32 v = s_list[first];
     const u32 cur = f[v];
-    const u64 o0 = A.off[v], o1 = A.off[v + 1];
-    u32 best = s_to[first];
-    if (best != DET_BIG) {
+    const u64 o0 = s_off[first], o1 = o0 + s_deg[first];
+    u32 best = first != big ? s_to[first] : NONE32;
+    if (first != big) {
       // ---- the move (:1168-1187), by one warp ----
       if (wib == 0) {
         const double kv = A.k[v];
@@ -503,8 +523,10 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
     for (u32 i = tid; i < nk; i += DET_THREADS) {
       const u32 c = A.klist[i];
       if (c == cur) continue;
-      const double gn = move_gain(A.bw[c], wcur, A.tw, A.gamma, kv, dcur, d_of(c));
+      const double wc = A.bw[c], dc = d_of(c);
       const u32 pc = A.bp[c];
+      if (!det_may_gain(wc, dc, wcur, A.tw, A.gamma, kv, dcur)) continue;
+      const double gn = move_gain(wc, wcur, A.tw, A.gamma, kv, dcur, dc);
       if (gn > 0.0 && (p == NONE32 || gn > g || (gn == g && pc < p))) {
         g = gn;
         p = pc;
@@ -519,12 +541,13 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
         best = kk;
         bestg = g;
       }
-      const double eg = empty_gain(wcur, A.tw, A.gamma, kv, dcur);
-      if (eg > bestg) {
-        bestg = eg;
-        best = DET_EMPTY;
+      if (det_may_gain(0.0, 0.0, wcur, A.tw, A.gamma, kv, dcur)) {
+        const double eg = empty_gain(wcur, A.tw, A.gamma, kv, dcur);
+        if (eg > bestg) {
+          bestg = eg;
+          best = DET_EMPTY;
+        }
       }
-      s_trav += o1 - o0;
       if (bestg > 0.0) {
         if (best == DET_EMPTY) {
           if ((u64)s_empty >= A.dcap) s_stop = DET_ID_SPACE;
@@ -564,6 +587,8 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_move(DetMoveArgs A) {
     }
     __syncthreads();
   }
+  if (trav) atomicAdd(&s_trav, trav);
+  __syncthreads();
   if (tid == 0) {
     A.out[0] = s_pops;
     A.out[1] = s_moves;

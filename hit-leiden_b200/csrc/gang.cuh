@@ -106,13 +106,7 @@ __device__ __forceinline__ void warp_add_by_id(double* d, u32 c, double x, bool 
   const u32 lane = threadIdx.x & 31;
   const u32 grp = __match_any_sync(0xffffffffu, on ? c : NONE32);
   const bool lead = on && !(grp & ((1u << lane) - 1u));
-  for (u32 m = __ballot_sync(0xffffffffu, lead && (grp & (grp - 1))); m; m &= m - 1) {
-    const u32 l = __ffs(m) - 1;
-    const u32 of = __shfl_sync(0xffffffffu, grp, l);
-    double y = (of >> lane) & 1u ? x : 0.0;
-    for (u32 o = 16; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    if (lane == l) x = y;
-  }
+  x = warp_group_sum(grp, lead, x);
   if (lead) atomicAdd(&d[c], x);
 }
 

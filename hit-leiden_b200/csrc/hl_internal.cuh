@@ -515,6 +515,30 @@ __device__ __forceinline__ double warp_long_sum(u64 a, u64 b, double acc, const 
   }
 }
 
+// Sum of x over the lanes of each group (`grp`: the lane's group, `lead`: its
+// first lane), at the leaders; in any order, exact for integral x.
+__device__ __forceinline__ double warp_group_sum(u32 grp, bool lead, double x) {
+  const u32 lane = threadIdx.x & 31;
+  const bool large = __popc(grp) > 8;
+  double s = x;
+  // small groups side by side, a member a step
+  u32 rest = lead && !large ? grp & (grp - 1) : 0u;
+  while (__any_sync(0xffffffffu, rest != 0)) {
+    const double y = __shfl_sync(0xffffffffu, x, rest ? __ffs(rest) - 1 : lane);
+    if (rest) s += y;
+    rest &= rest - 1;
+  }
+  // the others (three at most) one after another
+  for (u32 m = __ballot_sync(0xffffffffu, lead && large); m; m &= m - 1) {
+    const u32 l = __ffs(m) - 1;
+    const u32 of = __shfl_sync(0xffffffffu, grp, l);
+    double y = (of >> lane) & 1u ? x : 0.0;
+    for (u32 o = 16; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (lane == l) s = y;
+  }
+  return s;
+}
+
 // Sum of xs[a..b) in any order, exact for integral terms, by a block of 256
 // threads (sh: 8 words); thread 0 holds it.
 __device__ __forceinline__ double block_sum_any(const double* xs, u64 a, u64 b, double* sh) {

@@ -157,6 +157,65 @@ def test_hub_longer_than_its_tables(deg, integral):
     gs.close()
 
 
+def _same_det(gs, ref):
+    assert np.array_equal(gs.community_mapping_per_level[0], ref.get_map(0, O.MAP_F))
+    assert np.array_equal(gs.current_subcommunity_mapping_per_level[0],
+                          ref.get_map(0, O.MAP_S_CUR))
+
+
+def _load_det(n, edges, gamma=1.0, **config):
+    gs = hl.PartitionState.load(
+        hl.GraphInput.from_arrays("det", n, *edges),
+        hl.RunConfig(mode=hl.RunMode.Deterministic, max_iterations=1, resolution=gamma, **config))
+    ref = O.State(n, levels=1, mode=O.MODE_DETERMINISTIC, gamma=gamma)
+    ref.push_empty_graph()
+    ref.hit_leiden(*edges)
+    return gs, ref
+
+
+# Deterministic mode where every other row is above the 128 entries a warp
+# takes: lists that end at a long row at any place, keys shared by many of a
+# row's entries and by none.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("gamma", [0.2, 1.0, 4.0])
+def test_deterministic_long_rows(integral, gamma):
+    rng = np.random.default_rng(17)
+    n = 900
+    s = (n * rng.random(60000) ** 3).astype(np.uint32)
+    d = (n * rng.random(60000) ** 1.5).astype(np.uint32)
+    s, d = s[s != d], d[s != d]
+    w = np.ones(len(s)) if integral else rng.uniform(0.5, 2.0, len(s))
+    gs, ref = _load_det(n, (s, d, w), gamma)
+    _same_det(gs, ref)
+    for k in (1, 30, 300):
+        u, v = rng.integers(0, n, k).astype(np.uint32), rng.integers(0, n, k).astype(np.uint32)
+        b = u, v, np.full(k, 40.0) if integral else rng.uniform(10.0, 60.0, k)
+        gs.apply_batch(*b)
+        ref.hit_leiden(*b)
+        _same_det(gs, ref)
+    gs.close()
+
+
+# The walk's time on a graph of hubs (R-MAT 2^17): 4.8 to 6.2 ms of movement a
+# pass while rows beyond a long one were evaluated in vain, 2.5 so.
+def test_deterministic_hub_rows_time():
+    scale = 17
+    n, s, d = W.rmat_torch(scale, 16, 3)
+    u, v, _ = W.rmat_batch_torch(scale, s, d, 80, 1.0, 5)
+    s, d, u, v = (x.cpu().numpy().astype(np.uint32) for x in (s, d, u, v))
+    gs = hl.PartitionState.load(
+        hl.GraphInput.from_arrays("det", n, s, d, np.ones(len(s))),
+        hl.RunConfig(mode=hl.RunMode.Deterministic, resolution=0.2, kernel_timing=True))
+    best = 1e9
+    for _ in range(5):
+        before = gs.kernel_stats()["stage_move"]["ms"]
+        gs.apply_batch(u, v, np.ones(len(u)))
+        gs.apply_batch(u, v, -np.ones(len(u)))
+        best = min(best, gs.kernel_stats()["stage_move"]["ms"] - before)
+    gs.close()
+    assert best < 3.8, best
+
+
 # Hub rows side by side, in a batch above the one-launch limit: their sums run
 # beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
 # weights).  Same bits as the oracle's CSR and degrees.
