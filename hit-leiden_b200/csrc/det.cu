@@ -715,87 +715,22 @@ struct DetRefArgs {
   unsigned long long* out;  // [0] merges
 };
 
-// w(S, C_parent) (hit_leiden.rs:1528-1541): S's members in node order (the
-// initial ones and those merged since, two ascending lists), each member's
-// row in CSR order, entries whose neighbour lies in C_parent.  With integral
-// weights the block sums in any order; otherwise warp 0 folds in that order.
-__device__ double det_wsp(const DetRefArgs& A, u32 S, u32 parent, double* r_g) {
-  const u32 tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-  const u32 ms = A.mstart[S];
-  const u32 mc = ms == NONE32 ? 0u : A.mcount[S];
-  const u32* f = A.f;
-  const u32* col = A.col;
-  const double* w = A.w;
-  if (!A.ordered) {
-    double acc = 0.0;
-    // initial members: a warp per member row
-    for (u32 i = wib; i < mc; i += DET_WARPS) {
-      const u32 m = A.members[ms + i];
-      for (u64 q = A.off[m] + lane; q < A.off[m + 1]; q += 32)
-        if (f[col[q]] == parent) acc += w[q];
-    }
-    // merged singletons
-    for (u32 m = A.xhead[S]; m != NONE32; m = A.xnext[m])
-      for (u64 q = A.off[m] + tid; q < A.off[m + 1]; q += DET_THREADS)
-        if (f[col[q]] == parent) acc += w[q];
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) r_g[wib] = acc;
-    __syncthreads();
-    double tot = 0.0;
-    if (tid == 0)
-      for (u32 x = 0; x < DET_WARPS; ++x) tot += r_g[x];
-    __syncthreads();
-    return tot;  // thread 0
-  }
-  double acc = 0.0;
-  if (tid < 32) {
-    u32 i = 0;
-    u32 x = A.xhead[S];
-    while (i < mc || x != NONE32) {
-      u32 m;
-      if (x == NONE32 || (i < mc && A.members[ms + i] < x)) {
-        m = A.members[ms + i];
-        ++i;
-      } else {
-        m = x;
-        x = A.xnext[x];
-      }
-      acc = warp_ordered_sum(A.off[m], A.off[m + 1], acc, [&](u64 t) { return w[t]; },
-                             [&](u64 t) { return f[col[t]] == parent; });
-    }
-  }
-  __syncthreads();
-  return acc;  // thread 0 (all of warp 0)
-}
-
-// w(S, C_parent) by one warp (det_wsp's sums and order).  With integral weights
-// (any order) a lane takes a member, rows above 32 entries the whole warp.
-__device__ __forceinline__ double det_wsp_warp(const DetRefArgs& A, u32 S, u32 parent) {
-  const u32 lane = threadIdx.x & 31;
+// w(S, C_parent) (hit_leiden.rs:1528-1541): S's members (the initial ones and
+// those merged since, two ascending lists), each member's row, entries whose
+// neighbour lies in C_parent.
+//
+// Integral weights, in any order: thread t's share of nt (whole warps).  A lane
+// takes a member, rows above 32 entries the whole warp.
+__device__ __forceinline__ double det_wsp_any(const DetRefArgs& A, u32 S, u32 parent, u32 t,
+                                              u32 nt) {
+  const u32 lane = t & 31;
   const u32 ms = A.mstart[S];
   const u32 mc = ms == NONE32 ? 0u : A.mcount[S];
   const u32* f = A.f;
   const u32* col = A.col;
   const double* w = A.w;
   double acc = 0.0;
-  u32 x = A.xhead[S];
-  if (A.ordered) {
-    u32 i = 0;
-    while (i < mc || x != NONE32) {
-      u32 m;
-      if (x == NONE32 || (i < mc && A.members[ms + i] < x)) {
-        m = A.members[ms + i];
-        ++i;
-      } else {
-        m = x;
-        x = A.xnext[x];
-      }
-      acc = warp_ordered_sum(A.off[m], A.off[m + 1], acc, [&](u64 t) { return w[t]; },
-                             [&](u64 t) { return f[col[t]] == parent; });
-    }
-    return acc;
-  }
-  for (u32 i0 = 0; i0 < mc; i0 += 32) {
+  for (u32 i0 = t - lane; i0 < mc; i0 += nt) {
     const u32 m = i0 + lane < mc ? A.members[ms + i0 + lane] : NONE32;
     const u64 a = m != NONE32 ? A.off[m] : 0, b = m != NONE32 ? A.off[m + 1] : 0;
     if (b - a <= 32)
@@ -808,10 +743,52 @@ __device__ __forceinline__ double det_wsp_warp(const DetRefArgs& A, u32 S, u32 p
         if (f[col[q]] == parent) acc += w[q];
     }
   }
-  for (; x != NONE32; x = A.xnext[x])
-    for (u64 q = A.off[x] + lane; q < A.off[x + 1]; q += 32)
+  for (u32 x = A.xhead[S]; x != NONE32; x = A.xnext[x])
+    for (u64 q = A.off[x] + t; q < A.off[x + 1]; q += nt)
       if (f[col[q]] == parent) acc += w[q];
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
+// Other weights, by one warp: members in node order, rows in CSR order.
+__device__ __forceinline__ double det_wsp_ordered(const DetRefArgs& A, u32 S, u32 parent) {
+  const u32 ms = A.mstart[S];
+  const u32 mc = ms == NONE32 ? 0u : A.mcount[S];
+  const u32* f = A.f;
+  const u32* col = A.col;
+  const double* w = A.w;
+  double acc = 0.0;
+  u32 i = 0;
+  u32 x = A.xhead[S];
+  while (i < mc || x != NONE32) {
+    u32 m;
+    if (x == NONE32 || (i < mc && A.members[ms + i] < x)) {
+      m = A.members[ms + i];
+      ++i;
+    } else {
+      m = x;
+      x = A.xnext[x];
+    }
+    acc = warp_ordered_sum(A.off[m], A.off[m + 1], acc, [&](u64 t) { return w[t]; },
+                           [&](u64 t) { return f[col[t]] == parent; });
+  }
+  return acc;
+}
+
+// The same by the block; thread 0 holds it.
+__device__ double det_wsp(const DetRefArgs& A, u32 S, u32 parent, double* r_g) {
+  const u32 tid = threadIdx.x;
+  double acc = 0.0;
+  if (!A.ordered) {
+    acc = det_wsp_any(A, S, parent, tid, DET_THREADS);
+    if ((tid & 31) == 0) r_g[tid >> 5] = acc;
+    __syncthreads();
+    if (tid == 0)
+      for (u32 x = 1; x < DET_WARPS; ++x) acc += r_g[x];
+  } else if (tid < 32) {
+    acc = det_wsp_ordered(A, S, parent);
+  }
+  __syncthreads();
   return acc;
 }
 
@@ -834,10 +811,17 @@ __device__ __forceinline__ void det_merge(const DetRefArgs& A, u32 v, u32 cs, u3
   else if (A.wvalid[best]) A.wsp[best] += wv;
 }
 
+// Entries of a sub-community from which the block sums w(S, C): a warp takes some
+// 1.5 us for 32 short rows or 32 entries of a long one, the block's barriers 2.
+constexpr double DET_WSP_BLOCK = 4096.0;
+
+enum : u32 { DET_STAYS = 0, DET_MERGED = 1, DET_BLOCK = 2 };
+
 // One singleton by one warp (rows of up to DET_WARP_ROW entries): per-key sums
 // in the warp's table, the candidates in gain order until the T-filter lets one
-// pass.  No block barriers: they were most of a step.
-__device__ __forceinline__ bool det_refine_warp(const DetRefArgs& A, DetWarp& T, u32 v, u32 cs) {
+// pass.  No block barriers: they were most of a step.  DET_BLOCK: the step is the
+// block's, a candidate is too large for one warp; nothing has changed then.
+__device__ __forceinline__ u32 det_refine_warp(const DetRefArgs& A, DetWarp& T, u32 v, u32 cs) {
   const u32 lane = threadIdx.x & 31;
   const u64 o0 = A.off[v];
   const u32 deg = (u32)(A.off[v + 1] - o0);
@@ -928,7 +912,7 @@ __device__ __forceinline__ bool det_refine_warp(const DetRefArgs& A, DetWarp& T,
       }
     }
     const u32 bl = det_warp_best(g, p);
-    if (bl == 32) return false;
+    if (bl == 32) return DET_STAYS;
     const u32 slot = __shfl_sync(0xffffffffu, at, bl);
     const u32 cand = T.tk[slot];
     const double ds = A.dS[cand];  // (:1514-1548)
@@ -938,7 +922,9 @@ __device__ __forceinline__ bool det_refine_warp(const DetRefArgs& A, DetWarp& T,
       if (A.wvalid[cand]) {
         x = A.wsp[cand];
       } else {
-        x = det_wsp_warp(A, cand, cc);
+        // (an integral d_S is at least the number of S's entries)
+        if (!A.ordered && ds > DET_WSP_BLOCK) return DET_BLOCK;
+        x = A.ordered ? det_wsp_ordered(A, cand, cc) : det_wsp_any(A, cand, cc, lane, 32);
         if (lane == 0) {
           A.wsp[cand] = x;
           A.wvalid[cand] = 1;
@@ -950,7 +936,7 @@ __device__ __forceinline__ bool det_refine_warp(const DetRefArgs& A, DetWarp& T,
     if (!skip) {
       if (lane == 0) det_merge(A, v, cs, cand, kv, wv);
       __syncwarp();
-      return true;
+      return DET_MERGED;
     }
     if (lane == 0) T.tk[slot] = NONE32;
     __syncwarp();
@@ -970,21 +956,23 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_refine(DetRefArgs A) {
   __shared__ DetWarp s_warp;
   __shared__ u32 s_i;
   for (u32 i = 0;; ++i) {
-    // the first warp walks until a row needs the block
+    // the first warp walks until a step needs the block
     if (tid < 32) {
       for (; i < A.nr; ++i) {
         const u32 v = A.rlist[i];
         const u32 cs = A.s[v];
         if (A.sizes[cs] != 1u) continue;  // singleton check (:1398-1400)
         if (A.off[v + 1] - A.off[v] > DET_WARP_ROW) break;
-        if (det_refine_warp(A, s_warp, v, cs)) ++merges;
+        const u32 r = det_refine_warp(A, s_warp, v, cs);
+        if (r == DET_BLOCK) break;
+        if (r == DET_MERGED) ++merges;
       }
       if (tid == 0) s_i = i;
     }
     __syncthreads();
     i = s_i;
     if (i >= A.nr) break;
-    // ---- a long row, by the whole block ----
+    // ---- a long row or a large candidate, by the whole block ----
     const u32 v = A.rlist[i];
     const u32 cs = A.s[v];
     const u32 cc = A.f[v];
@@ -1069,7 +1057,19 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_refine(DetRefArgs A) {
     }
     const u32 best = s_best;
     const double bestg = s_bestg;
-    // the row's same-community weight, for the merged vertex's T-filter share
+    // w(v, C), which w(best, C) grows by (integral weights: kept, not summed again)
+    double wv = -1.0;
+    if (!A.ordered && best != cs) {
+      double acc = 0.0;
+      for (u32 j = tid; j < nk; j += DET_THREADS) acc += A.bw[A.klist[j]];
+      for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if ((tid & 31) == 0) r_g[tid >> 5] = acc;
+      __syncthreads();
+      if (tid == 0) {
+        wv = 0.0;
+        for (u32 x = 0; x < DET_WARPS; ++x) wv += r_g[x];
+      }
+    }
     __syncthreads();
     for (u32 j = tid; j < nk; j += DET_THREADS) {
       const u32 c = A.klist[j];
@@ -1079,7 +1079,7 @@ __global__ void __launch_bounds__(DET_THREADS) k_det_refine(DetRefArgs A) {
     __syncthreads();
     if (best != cs && bestg > 0.0) {
       if (tid == 0) {
-        det_merge(A, v, cs, best, kv, -1.0);
+        det_merge(A, v, cs, best, kv, wv);
         ++merges;
       }
       __syncthreads();

@@ -196,6 +196,24 @@ def test_deterministic_long_rows(integral, gamma):
     gs.close()
 
 
+# A singleton with a short row beside sub-communities on both sides of the size
+# from which the block sums w(S, C); the sum is kept while members join.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("leaves", [500, 2047, 2048, 3000])
+def test_deterministic_merges_beside_large_subcommunities(leaves, integral):
+    n, edges = _double_star(leaves, integral)
+    gs, ref = _load_det(n, edges)
+    _same_det(gs, ref)
+    for i in range(3):
+        at = slice(i * 20, i * 20 + 1 + 9 * i)
+        cut = edges[0][at], edges[1][at], -edges[2][at]
+        for b in (cut, (cut[0], cut[1], -cut[2])):
+            gs.apply_batch(*b)
+            ref.hit_leiden(*b)
+            _same_det(gs, ref)
+    gs.close()
+
+
 # The walk's time on a graph of hubs (R-MAT 2^17): 4.8 to 6.2 ms of movement a
 # pass while rows beyond a long one were evaluated in vain, 2.5 so.
 def test_deterministic_hub_rows_time():
