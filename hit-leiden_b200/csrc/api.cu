@@ -353,6 +353,31 @@ static void level_emit(Engine& E, Level& L, u32 p) {
   E.level_fn(E.level_user, p, (uint64_t)nodes.size(), nodes.data(), ids.data());
 }
 
+// The one-launch stages take scratch for whatever a level may need before they
+// start (the refinement 61 bytes a vertex and sub-community id, the movement
+// bounds 24 a vertex, the aggregation up to 65,536 records).  A handle with a
+// budget uses them where a bound of all its memory fits the budget, so that no
+// budget refuses a batch that the multi-kernel stages alone could apply.  Per
+// level two CSR buffers (24 bytes an entry) and the node arrays; scratch of less
+// than 4,400 bytes a vertex, 400 an entry and 200 an update over all buffers
+// (those of n or 2n+2 elements, of the aggregation's records and of the hub
+// passes' keys); half of it again, because a buffer that grows takes half more
+// than it had; and the hub passes' global tables.
+void Engine::plan_scratch(u64 n, u64 entries, u64 updates, u64 nlevels) {
+  lean = false;
+  if (!mem.budget) return;
+  for (const Level& l : levels) {
+    n = std::max<u64>(n, std::max(l.g.n, l.s_bound));
+    entries = std::max(entries, l.g.nnz);
+  }
+  entries += 2 * updates;
+  nlevels = std::max<u64>(nlevels, levels.size());
+  const u64 level_bytes = nlevels * (24 * entries + 40 * n);
+  const u64 scratch = 4400 * n + 400 * entries + 200 * updates;
+  const u64 tables = std::min<u64>(4ull << 30, 32768 * n) + 2304 * n;
+  lean = (level_bytes + scratch) / 2 * 3 + tables + (64ull << 20) > mem.budget;
+}
+
 static void hit_leiden_batch(EngineBox& B, const DevEdges& delta) {
   Engine& E = *B.E;
   hl_batch_stats& st = E.st;
@@ -622,6 +647,7 @@ static void create_impl(const hl_config* cfg, uint32_t n, const uint32_t* src, c
   stats_begin(E);
   HL_CUDA(cudaEventRecord(E.ev0, E.stream));
   E.in_bootstrap = true;
+  E.plan_scratch(n, 2 * m, m, E.cfg.max_levels);
   bootstrap(*B, n, G);
   E.in_bootstrap = false;
   if (E.levels[0].tw >= 4503599627370496.0) E.integral = false;  // 2^52
@@ -651,6 +677,7 @@ static void apply_impl(hl_graph* g, const uint32_t* src, const uint32_t* dst, co
   // device_ms starts with the batch resident on the device: the host→device
   // copy of a host batch is not part of it.
   HL_CUDA(cudaEventRecord(E.ev0, E.stream));
+  E.plan_scratch(0, 0, k, 1);
   check_endpoints(E, D, E.levels[0].g.n);
   if (E.integral && !edges_integral(E, D)) E.integral = false;
   hit_leiden_batch(B, D);
@@ -835,6 +862,15 @@ static void get_partition_impl(const hl_graph* g, uint32_t* out) {
   // size of the largest, plus two
   u32 top = 0;
   for (const Level& l : E.levels) top = std::max(top, l.g.n);
+  E.plan_scratch(0, 0, 0, 1);
+  if (E.lean) {  // nothing stays
+    DBuf<u32> tmp;
+    tmp.ensure(E.mem, n);
+    canonicalize_device(E, L.f.p, n, tmp.p);
+    HL_CUDA(cudaMemcpyAsync(out, tmp.p, sizeof(u32) * n, cudaMemcpyDeviceToHost, E.stream));
+    E.sync();
+    return;
+  }
   E.sc.canon.ensure(E.mem, n);
   canonicalize_bounded(E, L.f.p, n, 2 * top + 2, E.sc.canon.p);
   HL_CUDA(cudaMemcpyAsync(out, E.sc.canon.p, sizeof(u32) * n, cudaMemcpyDeviceToHost, E.stream));

@@ -302,8 +302,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_aggregate(GangAggArgs 
 }
 
 bool gang_aggregate_fits(Engine& E, const Level& L, const DevEdges& delta) {
-  (void)E;
-  return L.g.n > 0 && delta.k <= AGG_MAX_REC;
+  return !E.lean && L.g.n > 0 && delta.k <= AGG_MAX_REC;
 }
 
 // Grows level H to `hn` nodes, projects the communities of L onto it and, with

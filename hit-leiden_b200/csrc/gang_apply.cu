@@ -41,7 +41,7 @@ struct GangApplyArgs {
   u64 *rkeys, *rkeys2; // row-operations (row << 32 | neighbour)
   u32 *rvals, *rvals2;
   u32* dpre;           // deletes before each sorted row-operation
-  u64* opos;           // position of each sorted row-operation in the old entries
+  u64* opos;           // position of each sorted row-operation in the old entries (= rkeys)
   u32* touched;        // bit per row: its weights changed
   u32* rows;           // those rows, listed
   u32* longrows;       // ... and those of LONG_SUM entries or more
@@ -258,8 +258,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_apply(GangApplyArgs A)
 constexpr u64 GANG_ROOM_MAX = 1ull << 22;  // entries
 
 bool gang_apply_fits(Engine& E, const Level& L, const DevEdges& b, bool drop_loops) {
-  (void)E;
-  return b.k > 0 && b.k <= GANG_BATCH_MAX && !drop_loops && L.g.n > 0;
+  return !E.lean && b.k > 0 && b.k <= GANG_BATCH_MAX && !drop_loops && L.g.n > 0;
 }
 
 void gang_apply(Engine& E, Level& L, const DevEdges& b) {
@@ -283,7 +282,6 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   S.rvals.ensure(E.mem, rmax);
   S.rvals2.ensure(E.mem, rmax);
   S.opdelpre.ensure(E.mem, rmax + 1);
-  S.opos.ensure(E.mem, rmax);
   S.ga_touched.ensure(E.mem, (n + 31) / 32);
   S.rowlist.ensure(E.mem, rmax);
   S.longrows.ensure(E.mem, std::min<u64>(rmax, Gr.nnz / LONG_SUM + 1));
@@ -316,7 +314,7 @@ void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   A.rvals = S.rvals.p;
   A.rvals2 = S.rvals2.p;
   A.dpre = S.opdelpre.p;
-  A.opos = S.opos.p;
+  A.opos = S.rkeys.p;  // the unsorted keys are done with
   A.touched = S.ga_touched.p;
   A.rows = S.rowlist.p;
   A.longrows = S.longrows.p;

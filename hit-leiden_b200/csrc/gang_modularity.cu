@@ -244,13 +244,22 @@ double modularity(Engine& E, Level& L, const u32* part) {
   if (!n || L.tw == 0.0) return 0.0;
   Scratch& S = E.sc;
   cudaStream_t st = E.stream;
-  const GangShape shape = gang_shape(E, 8ull * n + L.g.nnz);
-  S.used.ensure(E.mem, n);
-  S.rank.ensure(E.mem, n);
-  S.order.ensure(E.mem, n);
-  S.order2.ensure(E.mem, n);
+  GangShape shape = gang_shape(E, 8ull * n + L.g.nnz);
+  // a tight budget: no label sort where none is needed, digit counts (16 KB a
+  // block) of no more than 8 bytes a vertex, and nothing stays
+  E.plan_scratch(0, 0, 0, 1);
+  if (E.lean && shape.grid && n / 2048 < shape.blocks) shape = GangShape{8, false};
+  if (E.lean && !shape.grid && n / 2048 < shape.blocks) shape = GangShape{1, false};
+  const bool keep_kval = !E.lean || S.fvals.cap > 0;
+  if (E.lean) S.cnt.ensure(E.mem, 16);
+  if (!E.lean || !E.integral || reduce_max_u32(E, part, n, S.cnt.p + 12) >= n) {
+    S.used.ensure(E.mem, n);
+    S.rank.ensure(E.mem, n);
+    S.order.ensure(E.mem, n);
+    S.order2.ensure(E.mem, n);
+    S.gm_hist.ensure(E.mem, (size_t)256 * GANG_WARPS * shape.blocks);
+  }
   S.fvals.ensure(E.mem, n);
-  S.gm_hist.ensure(E.mem, (size_t)256 * GANG_WARPS * shape.blocks);
   S.gang_part.ensure(E.mem, GANG_MAX_BLOCKS);
   S.red.ensure(E.mem, 4 * GANG_MAX_BLOCKS);
   GangModArgs A{};
@@ -278,6 +287,8 @@ double modularity(Engine& E, Level& L, const u32* part) {
   E.sync();
   double q[2];
   std::memcpy(q, E.hs.p, sizeof(q));
+  if (E.lean) S.gm_hist.release();
+  if (!keep_kval) S.fvals.release();
   return (q[0] - q[1]) / L.tw;
 }
 

@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
 static std::atomic<bool> g_move_attr[64];
 
 bool gang_move_fits(Engine& E, const Level& L) {
-  return L.g.n > 0 &&
+  return !E.lean && L.g.n > 0 &&
          (E.cfg.mode == HL_MODE_DETERMINISTIC || !(E.cfg.flags & HL_FLAG_NO_SMALL_ROUNDS));
 }
 

@@ -578,7 +578,7 @@ static std::atomic<bool> g_ref_attr[64];
 // The bootstrap refines every vertex of every level from the identity: worth
 // one launch while one block per SM has few singletons a warp.
 bool gang_refine_fits(Engine& E, const Level& L) {
-  return L.g.n > 0 && L.g.n < (1u << 30) &&
+  return !E.lean && L.g.n > 0 && L.g.n < (1u << 30) &&
          (!E.in_bootstrap || L.g.n <= 16 * GANG_WARPS * GANG_MAX_BLOCKS);
 }
 

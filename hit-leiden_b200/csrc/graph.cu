@@ -636,9 +636,9 @@ void apply_delta(Engine& E, Level& L, const DevEdges& b, u32 new_n, bool keep_lo
       return cub::DeviceScan::ExclusiveSum(t, bytes, a, o, (int64_t)R + 1, st);
     });
   }
-  S.opos.ensure(E.mem, R);
+  u64* opos = S.rkeys.p;  // the unsorted keys are done with
   ++E.nlaunch, k_rowop_positions<<<grid_for(R), 256, 0, st>>>(S.rkeys2.p, S.rvals2.p, R,
-                                                               L.g.off.p, L.g.col.p, S.opos.p);
+                                                               L.g.off.p, L.g.col.p, opos);
   HL_LAUNCH_CHECK();
   S.newoff.ensure(E.mem, (size_t)n + 1);
   DevGraph& G = L.g;
@@ -648,7 +648,7 @@ void apply_delta(Engine& E, Level& L, const DevEdges& b, u32 new_n, bool keep_lo
   ncol.ensure_slack(E.mem, nnz_new ? nnz_new : 1);
   nw.ensure_slack(E.mem, nnz_new ? nnz_new : 1);
   cudaEvent_t kev = E.kt_begin();
-  const RowOps O{(u32)R, S.rkeys2.p, S.rvals2.p, S.opdelpre.p, S.opos.p};
+  const RowOps O{(u32)R, S.rkeys2.p, S.rvals2.p, S.opdelpre.p, opos};
   ++E.nlaunch, k_rebuild<<<grid_for(G.nnz / 8 + R + n), 256, 0, st>>>(
       O, n, G.nnz, G.off.p, G.col.p, G.w.p, S.neww.p, S.newoff.p, ncol.p, nw.p, nnz_new,
       S.cnt.p + 4);

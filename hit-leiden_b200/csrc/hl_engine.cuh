@@ -54,7 +54,6 @@ struct Scratch {
   DBuf<double> neww;
   DBuf<u32> nops_del, nops_ins, pos_del, pos_ins;
   DBuf<u32> opdel, opdelpre;  // apply_delta: delete flags of the sorted operations, their scan
-  DBuf<u64> opos;             // apply_delta: their positions in the old entries
   DBuf<u64> newoff;
   DBuf<u32> rowlist;
   // node flags (level size)
@@ -221,6 +220,11 @@ struct Engine {
   u32 prune_rounds = 0;  // multi-kernel evaluations of the running movement
   Prune prune;           // the running movement's bounds (b == nullptr: off)
   bool shared = false;   // other graphs are being updated on the GPU meanwhile
+  // The handle's budget may not hold what the one-launch stages and the movement
+  // bounds take: this call keeps to the multi-kernel stages, which size their
+  // scratch by what they find (plan_scratch).
+  bool lean = false;
+  void plan_scratch(u64 n, u64 entries, u64 updates, u64 nlevels);
   u64 sum_nv_batch = 0;  // frontier sizes of the multi-kernel evaluations, this call
   // degree-bin thresholds picked by the autotuner (0 = compile-time default)
   struct Tune {
@@ -318,6 +322,7 @@ struct RefineOut {
   u32 singles = 0;  // refined singletons (gang_refine)
 };
 RefineOut inc_refinement(Engine& E, Level& L, bool cc_same_community);
+u32 reduce_max_u32(Engine& E, const u32* x, u32 n, u32* out);
 
 // gang_refine.cu: the refinement in one launch; the status names the step the
 // multi-kernel path continues from

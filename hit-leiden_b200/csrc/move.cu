@@ -555,13 +555,24 @@ void select_decoupled_dev(Engine& E, u32 M) {
   E.kagg[KT_SELECT].bytes += (u64)M * 9 * iters;  // from/to/status/nmask per iteration
 }
 
+__global__ void k_bits_from_flags(const u8* flags, u32 n, u32* bits) {
+  const u32 words = (n + 31) >> 5;
+  for (u64 wi = blockIdx.x * (u64)blockDim.x + threadIdx.x; wi < words;
+       wi += (u64)gridDim.x * blockDim.x) {
+    u32 x = 0;
+    for (u32 j = 0; j < 32 && (wi << 5) + j < n; ++j)
+      if (flags[(wi << 5) + j]) x |= 1u << j;
+    bits[wi] = x;
+  }
+}
+
 // The bounds of one movement; off where they do not hold (γ < 0) or no row is
 // long enough for them.
 void prune_begin(Engine& E, const Level& L) {
   E.prune = Prune{};
   E.prune_rounds = 0;
   const u32 n = L.g.n;
-  if (!n || E.cfg.mode == HL_MODE_DETERMINISTIC || !(E.cfg.resolution >= 0.0) ||
+  if (!n || E.lean || E.cfg.mode == HL_MODE_DETERMINISTIC || !(E.cfg.resolution >= 0.0) ||
       !(L.tw > 0.0) || L.g.nnz <= PRUNE_MIN_DEG)
     return;
   Scratch& S = E.sc;
@@ -637,6 +648,16 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
     compact_labels_if_needed(E, L.f.p, n, n);
     ensure_comm_arrays(E, ncap);
     recompute_comm_degrees(E, L, L.f.p, (u32)ncap, S.d.p);
+    if (E.cfg.mode == HL_MODE_DETERMINISTIC) {
+      const size_t n0 = ((size_t)n + 31) / 32, n1 = (n0 + 31) / 32;
+      S.det_bits.ensure(E.mem, n0 + n1 + (n1 + 31) / 32);  // the walk's bit sets of large levels
+      ++E.nlaunch, k_bits_from_flags<<<grid_for(n0), 256, 0, st>>>(S.active.p, n, S.det_bits.p);
+      HL_LAUNCH_CHECK();
+      inc_movement_det(E, L, S.det_bits.p, S.d.p, ncap, mark_moved, &out.moves, &out.traversed);
+      out.iterations = 1;
+      E.kagg[KT_MOVE_EVAL].bytes += 16ull * out.traversed;
+      return out;
+    }
     if (E.prune.b) {
       HL_CUDA(cudaMemsetAsync(E.prune.valid, 0, sizeof(u32) * (((size_t)n + 31) / 32), st));
       HL_CUDA(cudaMemsetAsync(E.prune.drop, 0, sizeof(double) * ncap, st));

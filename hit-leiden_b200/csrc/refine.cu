@@ -399,7 +399,7 @@ __global__ void k_apply_merges(const u32* single, u32 ns, const u32* to, const d
   if (local) atomicAdd(count, local);
 }
 
-static u32 reduce_max_u32(Engine& E, const u32* x, u32 n, u32* out) {
+u32 reduce_max_u32(Engine& E, const u32* x, u32 n, u32* out) {
   cub_run(E, [&](void* t, size_t& b) {
     return cub::DeviceReduce::Max(t, b, x, out, (int64_t)n, E.stream);
   });

@@ -234,6 +234,111 @@ def test_deterministic_hub_rows_time():
     assert best < 3.8, best
 
 
+def _hubs(n, m, integral, hubs):
+    rng = np.random.default_rng(5)
+    s, d = rng.integers(0, n, m), rng.integers(0, n, m)
+    for h in range(hubs):
+        s = np.concatenate([s, np.full(n // 4, h)])
+        d = np.concatenate([d, rng.choice(n, n // 4, replace=False)])
+    s, d = s[s != d].astype(np.uint32), d[s != d].astype(np.uint32)
+    return s, d, rng.integers(1, 4, len(s)).astype(float) if integral else rng.uniform(0.5, 2.0,
+                                                                                       len(s))
+
+
+# Budgets that just hold a load, two batches, their partitions and modularities
+# by the multi-kernel stages: the one-launch stages and the bounds take more, and
+# a handle that cannot hold that does without them.  Results as without a budget.
+@pytest.mark.parametrize("n,m,integral,hubs,mode,levels,budget", [
+    (20000, 80000, True, 0, "Throughput", 10, 28131662),
+    (20000, 80000, False, 0, "Throughput", 10, 33116190),
+    (20000, 60000, True, 6, "Throughput", 10, 31103129),
+    (20000, 60000, False, 6, "Throughput", 10, 163400974),
+    (50000, 100000, False, 0, "Throughput", 1, 33567747),
+    (3000, 9000, True, 0, "Deterministic", 10, 3903253),
+    (3000, 9000, False, 0, "Deterministic", 10, 5542577)])
+def test_tight_budgets(n, m, integral, hubs, mode, levels, budget):
+    edges = _hubs(n, m, integral, hubs)
+    rng = np.random.default_rng(6)
+    batches = [_updates(rng, n, edges, k, integral) for k in (50, 2000)]
+    out = []
+    for b in (budget, 0):
+        gs = hl.PartitionState.load(
+            hl.GraphInput.from_arrays("budget", n, *edges),
+            hl.RunConfig(mode=hl.RunMode[mode], max_iterations=levels, hbm_budget=b))
+        out.append([])
+        for u, v, w in batches:
+            gs.apply_batch(u, v, w)
+            out[-1] += [gs.partition(), gs.modularity(), *gs.community_mapping_per_level,
+                        *gs.current_subcommunity_mapping_per_level]
+        gs.close()
+    assert len(out[0]) == len(out[1])
+    for a, b in zip(*out):
+        if isinstance(a, float):
+            assert abs(a - b) <= 1e-12 * max(1.0, abs(b))
+        else:
+            assert np.array_equal(a, b)
+
+
+# A generous budget keeps the one-launch stages.  Its CSR buffers have no room up
+# front, so the delta goes in two launches that share one counter block: the size
+# first, then the rest.  Weight changes only, then structure, several times over.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("mode", ["Throughput", "Deterministic"])
+def test_generous_budget(integral, mode):
+    n = 4000
+    edges = _hubs(n, 12000, integral, 2)
+    key = np.unique(np.minimum(edges[0], edges[1]).astype(np.int64) * n
+                    + np.maximum(edges[0], edges[1]))
+    edges = ((key // n).astype(np.uint32), (key % n).astype(np.uint32), edges[2][:len(key)])
+    cfg = hl.RunConfig(mode=hl.RunMode[mode], max_iterations=1, hbm_budget=8 << 30,
+                       kernel_timing=True)
+    gs = hl.PartitionState.load(hl.GraphInput.from_arrays("budget", n, *edges), cfg)
+    ref = O.State(n, levels=1,
+                  mode=O.MODE_THROUGHPUT if mode == "Throughput" else O.MODE_DETERMINISTIC)
+    ref.push_empty_graph()
+    ref.hit_leiden(*edges)
+    rng = np.random.default_rng(9)
+    e = rng.choice(len(edges[0]), 300, replace=False)
+    more = np.ones(300) if integral else rng.uniform(0.5, 1.0, 300)
+    weights = edges[0][e], edges[1][e], more  # existing edges only
+    for i in range(8):
+        b = weights if i in (0, 1, 4) else _updates(rng, n, edges, (1, 40, 600)[i % 3], integral)
+        before = gs.kernel_stats()["apply_one_launch"]["launches"]
+        gs.apply_batch(*b)
+        assert gs.kernel_stats()["apply_one_launch"]["launches"] > before
+        ref.hit_leiden(*b)
+        _same_det(gs, ref)
+        off, col, wt = gs.supergraph(0)
+        ro, rc, rw = ref.graph(0).csr()
+        assert np.array_equal(off, ro) and np.array_equal(col, rc) and gh.same_bits(wt, rw)
+    gs.close()
+
+
+# A level of more entries than the second buffer gets room for up front: the
+# same two launches, without a budget.
+def test_delta_of_a_large_level_in_two_launches():
+    rng = np.random.default_rng(2)
+    n, m = 400000, 2200000
+    s, d, w = gh.random_graph(rng, n, m, False)
+    g = O.Graph.from_edges(n, s, d, w).apply_delta([], [], [], keep_self_loops=True)
+    off, col, _ = g.csr()
+    assert len(col) > 1 << 22
+    for k in (1, 3000):
+        e = rng.integers(0, len(s), k)
+        u = np.concatenate([rng.integers(0, n, k).astype(np.uint32), s[e]])
+        v = np.concatenate([rng.integers(0, n, k).astype(np.uint32), d[e]])
+        x = np.concatenate([rng.uniform(0.5, 2.0, k), -w[e]])
+        ref = g.apply_delta(u, v, x, keep_self_loops=True)
+        got = gh.apply_delta(g, u, v, x, keep_loops=True)
+        for a, b in zip(got, ref.csr()):
+            assert gh.same_bits(a, b)
+    # and weight changes alone, which need no second buffer
+    ref = g.apply_delta(s[:500], d[:500], np.ones(500), keep_self_loops=True)
+    got = gh.apply_delta(g, s[:500], d[:500], np.ones(500), keep_loops=True)
+    for a, b in zip(got, ref.csr()):
+        assert gh.same_bits(a, b)
+
+
 # Hub rows side by side, in a batch above the one-launch limit: their sums run
 # beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
 # weights).  Same bits as the oracle's CSR and degrees.
