@@ -103,9 +103,11 @@ void Engine::side_begin() {
   HL_CUDA(cudaEventRecord(side_go, stream));
   HL_CUDA(cudaStreamWaitEvent(side, side_go, 0));
 }
-void Engine::side_end() {
-  cudaEventRecord(side_done, side);
-  cudaStreamWaitEvent(stream, side_done, 0);
+cudaError_t Engine::side_end() {
+  cudaError_t e = cudaEventRecord(side_done, side);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, side_done, 0);
+  if (e != cudaSuccess) cudaStreamSynchronize(side);  // the order by waiting
+  return e;
 }
 void Engine::sync() {
   if (ktiming) ++kagg[KT_HOST_SYNC].launches;

@@ -1904,11 +1904,12 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   struct Join {  // the engine's stream goes on after the other one, also on an exception
     Engine& E;
     bool forked = false;
-    void now() {
-      if (forked) E.side_end();
+    cudaError_t now() {
+      const cudaError_t e = forked ? E.side_end() : cudaSuccess;
       forked = false;
+      return e;
     }
-    ~Join() { now(); }
+    ~Join() { (void)now(); }
   } join{E};
   if (!fork) rest(st);
   cudaEvent_t e_h = E.kt_begin();
@@ -2004,7 +2005,7 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
     }
   }
   E.kt_end(KT_EVAL_HUGE, e_h);
-  join.now();
+  HL_CUDA(join.now());
   E.kt_end(kind == EVAL_MOVE ? KT_MOVE_EVAL : KT_REFINE_EVAL, ev);
 }
 

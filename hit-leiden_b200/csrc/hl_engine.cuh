@@ -195,7 +195,7 @@ struct Engine {
   cudaStream_t side = nullptr;
   cudaEvent_t side_go = nullptr, side_done = nullptr;
   void side_begin();
-  void side_end();
+  cudaError_t side_end();
   MemCtx mem;
   Scratch sc;
   std::vector<Level> levels;
