@@ -24,16 +24,16 @@ namespace hl {
 // Blocks of 64 words, portable across devices; at most PINNED_KEEP wait for
 // their next use, the rest are given back at once.
 constexpr size_t PINNED_KEEP = 64;
+// Never destroyed: a handle may be given back by a destructor or an exit handler
+// of the program that runs after this library's own.  The system takes the
+// blocks back with the process.
 struct PinnedPool {
   std::mutex mu;
   std::vector<u64*> free;
-  ~PinnedPool() {
-    for (u64* p : free) cudaFreeHost(p);
-  }
 };
 static PinnedPool& pinned_pool() {
-  static PinnedPool pool;
-  return pool;
+  static PinnedPool* pool = new PinnedPool;
+  return *pool;
 }
 u64* pinned_take() {
   PinnedPool& P = pinned_pool();

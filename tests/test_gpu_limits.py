@@ -479,3 +479,39 @@ def test_uncapped_rounds(max_rounds):
         ref.hit_leiden(*b)
         _same(gs, ref)
     gs.close()
+
+
+# A program's exit handler destroys handles after the library's own statics are
+# gone: the pool their staging blocks go back to must still be there (an abort
+# of the program on a second free otherwise).
+def test_handles_outlive_static_destruction(tmp_path):
+    import shutil
+    import subprocess
+    from pathlib import Path
+    root = Path(hl.__file__).resolve().parents[1]
+    gcc = shutil.which("gcc")
+    if gcc is None:
+        pytest.skip("no C compiler")
+    src = tmp_path / "late.c"
+    src.write_text("""
+#include <stdlib.h>
+#include "hl.h"
+static hl_graph* g[3];
+static void bye(void) { hl_destroy(g[1]); hl_destroy(g[2]); }
+int main(void) {
+  uint32_t u[3] = {0, 1, 2}, v[3] = {1, 2, 3};
+  hl_config c;
+  hl_config_default(&c);
+  if (atexit(bye)) return 3;
+  for (int i = 0; i < 3; ++i)
+    if (hl_create(&c, 4, u, v, 0, 3, &g[i]) != HL_OK) return 2;
+  hl_destroy(g[0]);
+  return 0;
+}
+""")
+    exe = tmp_path / "late"
+    lib = Path(hl.__file__).resolve().parent / "libhl.so"
+    subprocess.run([gcc, "-I", str(root / "include"), str(src), str(lib), "-o", str(exe),
+                    f"-Wl,-rpath,{lib.parent}"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stderr)
