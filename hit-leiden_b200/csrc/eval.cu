@@ -1723,8 +1723,10 @@ void run_eval(Engine& E, int kind, const u32* verts, u32 nv, const Level& L, con
   S.order2.ensure(E.mem, nv);
   S.used.ensure(E.mem, nv);
   S.rank.ensure(E.mem, nv);
-  S.cnt.ensure(E.mem, 16);
-  u32* cnt = S.cnt.p + 2;  // NBINS bin counters (cnt[2..8])
+  // the stages' own counters are cnt[0..15]: the bins' come after them
+  static_assert(NBINS <= 16, "cnt has 32 words");
+  S.cnt.ensure(E.mem, 32);
+  u32* cnt = S.cnt.p + 16;
   HL_CUDA(cudaMemsetAsync(cnt, 0, NBINS * sizeof(u32), st));
   // [0] deferred rows, [2..3] largest degree of the block bin, [4..5] work
   // counters of the block kernel's two passes
