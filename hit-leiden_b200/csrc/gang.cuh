@@ -100,14 +100,29 @@ __device__ __forceinline__ u32 block_scan(GangSmem& S, u32 x, u32& total) {
 }
 
 // d[c] += x for the lanes with `on` (the whole warp calls it), where sums are
-// exact in any order: the lanes of one id add up first.  One community may hold
-// most of a level, and 2M atomics on its word take 3 ms, a sixteenth of that so.
+// exact in any order.  One community may hold most of a level, and 2M atomics on
+// its word take 3 ms: the ids of the first two lanes left are looked for in the
+// others, and what eight lanes or more share adds up before its atomic.
 __device__ __forceinline__ void warp_add_by_id(double* d, u32 c, double x, bool on) {
   const u32 lane = threadIdx.x & 31;
-  const u32 grp = __match_any_sync(0xffffffffu, on ? c : NONE32);
-  const bool lead = on && !(grp & ((1u << lane) - 1u));
-  x = warp_group_sum(grp, lead, x);
-  if (lead) atomicAdd(&d[c], x);
+  u32 rest = __ballot_sync(0xffffffffu, on);
+#pragma unroll
+  for (u32 t = 0; t < 2; ++t) {
+    if (!rest) return;
+    const u32 l = __ffs(rest) - 1;
+    const u32 cl = __shfl_sync(0xffffffffu, c, l);
+    const u32 same = __ballot_sync(0xffffffffu, ((rest >> lane) & 1u) && c == cl);
+    const bool mine = (same >> lane) & 1u;
+    if (__popc(same) >= 8) {
+      double y = mine ? x : 0.0;
+      for (u32 o = 16; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+      if (lane == l) atomicAdd(&d[c], y);
+    } else if (mine) {
+      atomicAdd(&d[c], x);
+    }
+    rest &= ~same;
+  }
+  if ((rest >> lane) & 1u) atomicAdd(&d[c], x);
 }
 
 // Exclusive prefix sums of val(0..N-1), handed to out(i, prefix); returns the

@@ -311,7 +311,6 @@ bool gang_aggregate_fits(Engine& E, const Level& L, const DevEdges& delta) {
 bool gang_aggregate(Engine& E, Level& L, Level& H, const DevEdges& delta, bool aggregate,
                     DBuf<u32>& ou, DBuf<u32>& ov, DBuf<double>& ow, u64* count) {
   Scratch& S = E.sc;
-  cudaStream_t st = E.stream;
   const u32 n = L.g.n, h_old = H.g.n;
   const u32 hn = std::max(h_old, E.new_base + E.n_new);
   const GangShape shape = gang_shape(E, 2ull * n + L.g.nnz / 8 + 32ull * delta.k);

@@ -263,7 +263,6 @@ bool gang_apply_fits(Engine& E, const Level& L, const DevEdges& b, bool drop_loo
 
 void gang_apply(Engine& E, Level& L, const DevEdges& b) {
   Scratch& S = E.sc;
-  cudaStream_t st = E.stream;
   DevGraph& Gr = L.g;
   const u32 n = Gr.n;
   const u32 k = (u32)b.k;

@@ -243,7 +243,6 @@ double modularity(Engine& E, Level& L, const u32* part) {
   const u32 n = L.g.n;
   if (!n || L.tw == 0.0) return 0.0;
   Scratch& S = E.sc;
-  cudaStream_t st = E.stream;
   GangShape shape = gang_shape(E, 8ull * n + L.g.nnz);
   // a tight budget: no label sort where none is needed, digit counts (16 KB a
   // block) of no more than 8 bytes a vertex, and nothing stays

@@ -676,7 +676,6 @@ bool gang_move_fits(Engine& E, const Level& L) {
 u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_active,
               bool mark_moved, u32 frontier, u32& it, GangMoveStats& ms) {
   Scratch& S = E.sc;
-  cudaStream_t st = E.stream;
   const u32 n = L.g.n;
   const int dev = E.device;
   if (dev >= 0 && dev < 64 && !g_move_attr[dev]) {

@@ -24,7 +24,7 @@ constexpr u32 REF_MAX_REC = 65536;  // records sorted here
 
 struct RefCnt {  // zeroed by the host
   u32 smax, nitems, nsplit, nrefined, nsingle, nsitems, nbig, ncand;
-  u32 nmitems, nrec, nparent, nseg, namb, merges, not_identity, pad_;
+  u32 nmitems, nrec, namb, merges, not_identity, pad_;
 };
 
 struct RefOut {
@@ -59,7 +59,7 @@ struct GangRefArgs {
   u64 *skey, *skey2;             // split components (s << 32 | root)
   u32 *sidx, *sidx2;
   u32* origin;           // per new id: the sub-community it was split from
-  u32 *rlist, *single, *clist, *plist;
+  u32 *rlist, *single, *clist;
   u64 *rec, *rid, *rtmp;  // (id << 33 | is community << 32 | vertex)
   u32 *ridx, *rtidx;
   double* rval;
@@ -451,9 +451,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_refine(GangRefArgs A) 
     G.sync();
     for (u32 i = gt; i < ncand; i += gts) {
       const u32 c = A.f[A.minmem[A.clist[i]]];
-      if (!bit_first(A.parent, c)) continue;
-      A.plist[atomicAdd(&C.nparent, 1u)] = c;
-      A.dcomm[c] = 0.0;
+      if (bit_first(A.parent, c)) A.dcomm[c] = 0.0;
     }
     G.sync();
     // ---- w(S, C_parent) in any order, d of the parents ----
@@ -586,7 +584,6 @@ bool gang_refine_fits(Engine& E, const Level& L) {
 // from the step *status names (REF_*).
 u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   Scratch& S = E.sc;
-  cudaStream_t st = E.stream;
   const u32 n = L.g.n;
   const int dev = E.device;
   if (dev >= 0 && dev < 64 && !g_ref_attr[dev]) {
@@ -613,7 +610,6 @@ u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   S.act.ensure(E.mem, n);
   S.cand_idx.ensure(E.mem, n);
   S.cand_node.ensure(E.mem, scap);
-  S.sel_node.ensure(E.mem, n);
   const u64 nrec = E.integral ? 1 : std::min<u64>(2ull * n, REF_MAX_REC);
   S.rkeys.ensure(E.mem, nrec);
   S.rkeys2.ensure(E.mem, nrec);
@@ -665,7 +661,6 @@ u32 gang_refine(Engine& E, Level& L, bool cc_same_community, RefineOut& out) {
   A.rlist = S.act.p;
   A.single = S.cand_idx.p;
   A.clist = S.cand_node.p;
-  A.plist = S.sel_node.p;
   A.rec = S.rkeys.p;
   A.rid = S.rkeys2.p;
   A.rtmp = S.keys.p;

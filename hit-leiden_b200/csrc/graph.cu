@@ -5,8 +5,8 @@
 // batch's deltas in batch order (a stable sort keeps that order); keys whose
 // weight ends at <= 1e-12 disappear.  Instead of rebuilding a hash map of all
 // m edges, only the changed keys are resolved: weight updates are written in
-// place, and inserts/deletes become sorted row-operations that a warp-per-row
-// merge folds into a fresh CSR with rows still sorted by neighbour id.
+// place, and inserts/deletes become sorted row-operations by which every
+// surviving entry moves into a fresh CSR (csr_rebuild.cuh).
 #include "csr_rebuild.cuh"
 #include "hl_engine.cuh"
 
@@ -91,17 +91,6 @@ void graph_grow_nodes(Engine& E, Level& L, u32 n) {
   L.g.n = n;
   if (L.s_bound && L.s_bound < n) L.s_bound = n;
   HL_LAUNCH_CHECK();
-}
-
-__device__ __forceinline__ u64 lower_bound_u64(const u64* a, u64 lo, u64 hi, u64 x) {
-  while (lo < hi) {
-    u64 mid = (lo + hi) >> 1;
-    if (a[mid] < x)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
 }
 
 __global__ void k_check_endpoints(const u32* u, const u32* v, u64 k, u32 n, u32* bad) {

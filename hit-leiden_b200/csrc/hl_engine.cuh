@@ -50,7 +50,7 @@ struct Scratch {
   // delta application
   DBuf<u64> keys, keys2, rkeys, rkeys2;
   DBuf<u32> idx, idx2, segid, seg_start, rvals, rvals2;
-  DBuf<u8> op, ktouched, isdel, isins;
+  DBuf<u8> op, ktouched;
   DBuf<double> neww;
   DBuf<u32> nops_del, nops_ins, pos_del, pos_ins;
   DBuf<u32> opdel, opdelpre;  // apply_delta: delete flags of the sorted operations, their scan
@@ -60,7 +60,7 @@ struct Scratch {
   DBuf<u8> active, next, changed, affected, refined;
   DBuf<u32> act, cand_idx, cnt;
   DBuf<u32> cand_to, cand_node;
-  DBuf<double> cand_gain, cand_k;
+  DBuf<double> cand_gain;
   DBuf<u64> gkey, gkey2;
   DBuf<u32> sel_from, sel_to, sel_node, order, order2;
   DBuf<u8> status, nmask;
@@ -69,7 +69,7 @@ struct Scratch {
   DBuf<double> d;       // community degrees (2n)
   DBuf<u32> used, rank;
   // refinement
-  DBuf<u32> par, uroot, csize, ncomp, newid, minmem;
+  DBuf<u32> par, uroot, csize, newid, minmem;
   DBuf<u64> keep;
   DBuf<u8> affsc, cand_sc, blocked;
   DBuf<u32> sizes;
@@ -77,7 +77,6 @@ struct Scratch {
   DBuf<u64> wcnt;       // T-filter: terms of each any-order sum
   DBuf<u8> amb;         // T-filter: S whose decision needs the ordered sum
   DBuf<u32> longrows;   // T-filter: member rows summed by a whole block
-  DBuf<u32> upd_node, upd_to;
   // reductions
   DBuf<double> red, red2;
   DBuf<u64> red64;
