@@ -18,13 +18,14 @@ static u32 sm_count(int device) {
 // at once waits for all of their kernels: there clusters go on to a few million
 // entries (48 graphs of 1k-30k vertices on 16 host threads: 18.5 ms a batch
 // each with grids, 12 ms with clusters; one graph at a time: 97 and 104 ms).
-constexpr u64 GANG_BLOCK_WORK = 4096;
 constexpr u64 GANG_CLUSTER_WORK = 400000;
 constexpr u64 GANG_SHARED_WORK = 4000000;
 
+u64 gang_cluster_work(const Engine& E) { return E.shared ? GANG_SHARED_WORK : GANG_CLUSTER_WORK; }
+
 GangShape gang_shape(Engine& E, u64 work) {
   if (work <= GANG_BLOCK_WORK) return GangShape{1, false};
-  if (work <= (E.shared ? GANG_SHARED_WORK : GANG_CLUSTER_WORK)) return GangShape{8, false};
+  if (work <= gang_cluster_work(E)) return GangShape{8, false};
   const u32 sms = sm_count(E.device);
   return GangShape{sms < GANG_MAX_BLOCKS ? sms : GANG_MAX_BLOCKS, true};
 }

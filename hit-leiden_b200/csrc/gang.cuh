@@ -517,6 +517,8 @@ struct GangShape {
   bool grid;  // cooperative grid instead of a cluster
 };
 
+constexpr u64 GANG_BLOCK_WORK = 4096;           // entries up to which one block takes a stage
+u64 gang_cluster_work(const Engine& E);          // ... a cluster of 8
 // Shape for a stage that touches about `work` entries.
 GangShape gang_shape(Engine& E, u64 work);
 // Launch of a gang kernel with one argument struct.

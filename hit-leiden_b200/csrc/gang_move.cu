@@ -43,7 +43,7 @@ struct MoveCnt {  // zeroed by the host
 };
 
 struct MoveOutDev {
-  u32 status, it, round, pad_;
+  u32 status, it, round, frontier;
   u64 epoch;
   unsigned long long moves, cands, trav, nfront, pruned;
 };
@@ -82,7 +82,8 @@ struct GangMoveArgs {
   u32* bits[2];      // frontier bit sets
   u32* verts[2];     // frontier: rows of up to GM_MAXDEG entries
   u32* hubs[2];      // ... and longer ones
-  u32 list_cap;
+  u32 list_cap;      // entries of a list
+  u32 max_frontier;  // vertices up to which a round stays in this launch
   u32 *wverts, *whubs;  // those of them that need an evaluation
   Prune prune;
   u32* to;           // per vertex: its candidate's target
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       if (A.more && nv + nh) status = MOVE_BIG_FRONTIER;
       break;
     }
-    if (nv > A.list_cap || nh > A.list_cap || nv + nh > A.list_cap) {
+    if (nv > A.max_frontier || nh > A.max_frontier || nv + nh > A.max_frontier) {
       status = MOVE_BIG_FRONTIER;
       break;
     }
@@ -651,6 +652,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_move(GangMoveArgs A) {
       *A.prune.worst = 0;
     }
     A.out->status = status;
+    A.out->frontier = C.r[b].nv + C.r[b].nh;
     A.out->it = it;
     A.out->round = round;
     A.out->epoch = epoch;
@@ -781,6 +783,18 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   A.wverts = S.sm_list_a.p + 2 * (size_t)fr;
   A.whubs = S.sm_list_a.p + 3 * (size_t)fr;
   A.list_cap = fr;
+  // A launch whose blocks were chosen for a few vertices must not go on when the
+  // frontier has grown to what the whole GPU should evaluate (20k vertices with
+  // 320k entries, 40-2,000 updates that wake them all: 13-14.5 ms on 8 blocks,
+  // 3.0-3.8 with the hand-over, 8.3-10.3 by multi-kernel rounds).  A cluster may
+  // take twice the work it was chosen for; one block 32 times, because a
+  // hand-over costs 30 us (8 times: 2,000 updates of 3,000 vertices 4.0 -> 4.3 ms).
+  A.max_frontier = fr;
+  if (!shape.grid) {
+    const u64 work = shape.blocks > 1 ? 2 * gang_cluster_work(E) : 32 * GANG_BLOCK_WORK;
+    const u64 most = work > n ? (work - n) / (4 * avg) : 0;
+    A.max_frontier = (u32)std::min<u64>(fr, std::max<u64>(most, 64));
+  }
   A.prune = E.prune;
   A.to = S.cand_to.p;
   A.ckey = S.gkey.p;
@@ -815,6 +829,7 @@ u32 gang_move(Engine& E, Level& L, const DevEdges& delta, bool setup, bool all_a
   if (o.status == MOVE_LABELS) return o.status;
   if (setup) E.k_flags_set = false;
   it = o.it;
+  ms.frontier = o.frontier;
   ms.moves += o.moves;
   ms.cands += o.cands;
   ms.trav += o.trav + o.pruned;  // rows ruled out count as traversed

@@ -339,6 +339,7 @@ void stats_count_flags(Engine& E, const u8* flags, u32 n, u32 slot);
 enum : u32 { MOVE_DONE = 0, MOVE_BIG_FRONTIER = 1, MOVE_BIG_HUB = 2, MOVE_LABELS = 3 };
 struct GangMoveStats {
   u64 moves = 0, cands = 0, trav = 0;
+  u32 frontier = 0;  // of the round the last launch handed over
 };
 constexpr u32 GM_FRONTIER = 32768;  // frontier (and candidate) limit
 bool gang_move_fits(Engine& E, const Level& L);

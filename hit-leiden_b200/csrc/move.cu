@@ -603,6 +603,7 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   u32 it = 0;
   GangMoveStats gm;
   bool gang_on = gang_move_fits(E, L);
+  u32 last_na = NONE32;  // frontier of the last round (NONE32: not known)
   prune_begin(E, L);
   if (gang_on) {
     S.cnt.ensure(E.mem, 16);
@@ -629,6 +630,7 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
       return out;
     }
     if (why == MOVE_BIG_HUB) gang_on = false;
+    else last_na = gm.frontier;  // another launch, with more blocks, if its lists hold them
   } else {
     HL_CUDA(cudaMemsetAsync(S.active.p, all_active ? 1 : 0, n ? n : 1, st));
     HL_CUDA(cudaMemsetAsync(S.changed.p, 0, n ? n : 1, st));
@@ -688,13 +690,17 @@ MoveOut inc_movement(Engine& E, Level& L, const DevEdges& delta, bool all_active
   HL_CUDA(cudaMemsetAsync(S.acc_cnt.p, 0, sizeof(u32), st));  // accepted moves, all rounds
   // Small frontiers run whole rounds in one launch (gang_move.cu); the host
   // rounds take over while the frontier is large or a hub outgrows its tables.
-  u32 last_na = NONE32;
   while (it < max_rounds) {
     if (gang_on && last_na <= GM_FRONTIER) {
       const u32 why = gang_move(E, L, DevEdges{}, false, false, mark_moved, last_na, it, gm);
       if (why == MOVE_DONE) break;
-      if (why == MOVE_BIG_HUB) gang_on = false;
       if (it >= max_rounds) break;
+      if (why == MOVE_BIG_HUB) {
+        gang_on = false;
+      } else if (gm.frontier <= GM_FRONTIER) {
+        last_na = gm.frontier;
+        continue;
+      }
     }
     // Active list, ascending (iter_ones order).
     cub_run(E, [&](void* t, size_t& b) {

@@ -339,6 +339,24 @@ def test_delta_of_a_large_level_in_two_launches():
         assert gh.same_bits(a, b)
 
 
+# A few seeds wake the whole level: a launch whose blocks were chosen for the
+# seeds hands over to one with more of them, from one block and from a cluster.
+@pytest.mark.parametrize("integral", [True, False])
+@pytest.mark.parametrize("n,m", [(900, 3000), (1500, 60000), (20000, 160000)])
+def test_frontier_outgrows_its_launch(n, m, integral):
+    rng = np.random.default_rng(n)
+    s, d, w = gh.random_graph(rng, n, m, integral)
+    g = O.Graph.from_edges(n, s, d, w).apply_delta([], [], [], keep_self_loops=True)
+    f = np.arange(n, dtype=np.uint32)
+    sub = gh.random_partition(rng, n, n // 3)
+    delta = s[:2], d[:2], np.ones(2)
+    for rounds in (1, 4, 20):
+        ref = O.inc_movement(g, *delta, f.copy(), sub, 1.0, O.MODE_THROUGHPUT, max_rounds=rounds)
+        got = gh.inc_movement(g, *delta, f, sub, 1.0, max_rounds=rounds)
+        assert ref[3] == got[3] and all(np.array_equal(ref[i], got[i]) for i in range(3))
+    assert ref[1].sum() > n // 2  # most vertices have moved
+
+
 # Hub rows side by side, in a batch above the one-launch limit: their sums run
 # beside each other (one warp took 32 rows in turn: 4.5 ms here with f64
 # weights).  Same bits as the oracle's CSR and degrees.
