@@ -14,6 +14,8 @@ namespace hl {
 
 constexpr u32 AGG_SLICE = 512;       // entries of a row a warp emits
 constexpr u32 AGG_LANE = 16;         // sums up to this length: a lane each
+// Records sorted here: those of a largest batch (GANG_BATCH_MAX), two an update;
+// the sort's ranks grow with the square, and the radix sort takes over.
 constexpr u32 AGG_MAX_REC = 65536;
 
 struct AggCnt {  // zeroed by the host

@@ -101,8 +101,9 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_gang_modularity(GangModArgs
   };
   if (A.integral && C.maxlab < A.n) {
     // ---- Σ_C d(C)²/2m: integral degrees add up in any order, in shared memory
-    // while the labels fit it.  A sort and one ordered chain a community instead
-    // take 890 us on a partition of a few large communities, this form 320.
+    // while the labels fit it: no label sort and no ordered sum (300k vertices in
+    // 2 and 30 communities: 289 and 332 us in the multi-kernel form, 182 and 184
+    // so).
     const u32 nc = C.maxlab + 1;
     const bool local = nc <= GANG_WORDS;
     for (u32 c = gt; c < nc; c += gts) A.kval[c] = 0.0;

@@ -20,7 +20,7 @@ namespace hl {
 constexpr u32 REF_SLICE = 256;
 constexpr u32 REF_MAXDEG = 256;    // singleton rows evaluated here
 constexpr u32 REF_TAB = 2 * REF_MAXDEG;
-constexpr u32 REF_MAX_REC = 65536;  // records sorted here
+constexpr u32 REF_MAX_REC = 65536;  // records sorted here (as AGG_MAX_REC)
 
 struct RefCnt {  // zeroed by the host
   u32 smax, nitems, nsplit, nrefined, nsingle, nsitems, nbig, ncand;

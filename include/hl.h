@@ -71,7 +71,9 @@ typedef struct {
                         /* up to this cap (default 10, RunConfig.max_iterations)   */
   uint32_t max_rounds;  /* throughput movement round cap (hit_leiden.rs:1077); 20  */
   uint32_t flags;       /* HL_FLAG_*                                               */
-  uint64_t hbm_budget;  /* bytes this handle may allocate on the device; 0 = no cap */
+  uint64_t hbm_budget;  /* bytes this handle may allocate on the device; 0 = no cap.*/
+                        /* A budget that may not hold the one-launch stages'       */
+                        /* scratch keeps to the multi-kernel stages: same results  */
   int32_t device;       /* CUDA device ordinal                                     */
 } hl_config;
 
